@@ -41,12 +41,14 @@ extern "C" {
                                cluster where a cluster's shared memory holds the system with at
                                most 48 chunks of 32 slots per CTA and colour (one per warp where a
                                cluster of up to 16 CTAs allows), persistent up to about
-                               three 512-monomer tiles per SM (bond codes), else graph */
+                               three 512-monomer tiles per SM (bond codes), else graph, with
+                               persistent runs of 6 MCS or more where the slots fit the SMs */
 #define BFM_MODE_LAUNCH 1   /* check + perform launch per sub-step (the reference's structure) */
 #define BFM_MODE_GRAPH 2    /* the same launches captured into CUDA graphs */
 #define BFM_MODE_RESIDENT 3 /* one CTA per system, lattice in shared memory (box <= 64^3) */
 #define BFM_MODE_PERSISTENT 4 /* bond codes: one cooperative launch runs a whole chunk of sub-steps,
-                                 grid barriers between the phases (gather systems use GRAPH) */
+                                 each SM holding its share of the slots, grid barriers between the
+                                 phases (gather systems, and more than about 2 M monomers, use GRAPH) */
 #define BFM_MODE_CLUSTER 5    /* bond codes: one thread-block cluster (2-16 CTAs) holds the system's
                                  lattice and state in its shared memory for a whole chunk of
                                  sub-steps (systems too large for one CTA, up to about 200 KB x 16) */
@@ -125,12 +127,13 @@ int bfm_set_grid_block(bfm_handle h, int block);
  * reference counterpart (the reference's perform runs one thread per monomer of the colour). */
 int bfm_set_perform(bfm_handle h, int warps, int group);
 /* The path the next run takes (after bfm_initialize): the mode set by bfm_set_mode with
- * BFM_MODE_AUTO resolved, and a mode the system cannot use replaced by BFM_MODE_GRAPH. */
+ * BFM_MODE_AUTO resolved for a run of one MCS, and a mode the system cannot use replaced by
+ * BFM_MODE_GRAPH. */
 int bfm_get_path(bfm_handle h, int* mode);
 /* Fault injection for tests (no counterpart in the reference): the next BFM_MODE_PERSISTENT launch
- * of this handle runs as a cooperative grid (never as one cluster, whose barriers are in hardware)
- * and starts its grid-barrier arrival count where no barrier can complete, so every
- * CTA's wait runs out at its time limit (2 s) and the run reports the timeout (BFM_ERR_CUDA).
+ * of this handle starts its grid-barrier arrival count where no barrier can complete, so every
+ * CTA's wait runs out at its time limit (20 s, the first wait's) and the run reports the timeout
+ * (BFM_ERR_CUDA).
  * Nothing faults on the GPU and the device stays usable; this system's state is not. */
 int bfm_inject_barrier_stall(bfm_handle h);
 /* Device representation of the bonds, chosen before bfm_initialize: BFM_REPR_AUTO (bond codes —

@@ -535,13 +535,31 @@ __host__ __device__ __forceinline__ uint4 make_rec(uint32_t p, unsigned long lon
 // axes: da = D.front (+2 d) from the monomer's address, D.step (+d) from its target's; the low
 // six bits of its address select the masks (ptab: global memory through L1, or shared memory)
 // and the neighbouring bricks along u and v are one step of the brick index along those axes.
+// front_plane_words gives the words and the masks' table index (words of untouched bricks are valid
+// addresses too; touch says which count), front_plane the masks as well.
+__host__ __device__ __forceinline__ void front_plane_words(uint32_t (&w)[4], uint32_t& ti, uint32_t& touch,
+                                                           DirParams const& D, uint32_t base, uint32_t da, uint32_t dir)
+{
+    uint32_t const f = ((((base | ~D.ma) + da) & D.ma) | (((base | ~D.mu) + D.mu) & D.mu)) |
+                       (((base | ~D.mv) + D.mv) & D.mv);
+    ti = ((dir >> 1) * 64u + (f & 63u)) * 4u;
+    w[0] = f >> 6;
+    w[1] = addr_add(w[0], D.bv, 1u);
+    w[2] = addr_add(w[0], D.bu, 1u);
+    w[3] = addr_add(w[2], D.bv, 1u);
+    // the run of three cells along u (v) spills into the next brick when it starts at in-brick
+    // coordinate 2 or 3, i.e. when the high in-brick bit of that axis (one of bits 1, 3, 5) is set;
+    // loads predicated on this need not wait for the masks
+    uint32_t const tu = (f & D.mu & 0x2Au) != 0u, tv = (f & D.mv & 0x2Au) != 0u;
+    touch = 1u | (tv << 1) | (tu << 2) | ((tu & tv) << 3);
+}
+
 template <bool kSharedTables>
 __host__ __device__ __forceinline__ void front_plane(Plane& pl, unsigned long long const* ptab, DirParams const& D,
                                                      uint32_t base, uint32_t da, uint32_t dir)
 {
-    uint32_t const f = ((((base | ~D.ma) + da) & D.ma) | (((base | ~D.mu) + D.mu) & D.mu)) |
-                       (((base | ~D.mv) + D.mv) & D.mv);
-    uint32_t const ti = ((dir >> 1) * 64u + (f & 63u)) * 4u;
+    uint32_t ti;
+    front_plane_words(pl.w, ti, pl.touch, D, base, da, dir);
     ulonglong2 m01, m23;
 #ifdef __CUDA_ARCH__
     if (!kSharedTables) {
@@ -553,21 +571,10 @@ __host__ __device__ __forceinline__ void front_plane(Plane& pl, unsigned long lo
         m01 = *reinterpret_cast<ulonglong2 const*>(ptab + ti);
         m23 = *reinterpret_cast<ulonglong2 const*>(ptab + ti + 2);
     }
-    uint32_t const w00 = f >> 6;
-    uint32_t const w10 = addr_add(w00, D.bu, 1u);
-    pl.w[0] = w00;
     pl.m[0] = m01.x;
-    pl.w[1] = addr_add(w00, D.bv, 1u);
     pl.m[1] = m01.y;
-    pl.w[2] = w10;
     pl.m[2] = m23.x;
-    pl.w[3] = addr_add(w10, D.bv, 1u);
     pl.m[3] = m23.y;
-    // the run of three cells along u (v) spills into the next brick when it starts at in-brick
-    // coordinate 2 or 3, i.e. when the high in-brick bit of that axis (one of bits 1, 3, 5) is set;
-    // loads predicated on this need not wait for the masks
-    uint32_t const tu = (f & D.mu & 0x2Au) != 0u, tv = (f & D.mv & 0x2Au) != 0u;
-    pl.touch = 1u | (tv << 1) | (tu << 2) | ((tu & tv) << 3);
 }
 
 // Host: bit d of ok[idx] is set when the bond with table index idx (neighbour - monomer, every
@@ -616,6 +623,28 @@ __device__ __forceinline__ W code_shift(W code, uint32_t axis, int32_t delta)
         }
     }
     return out;
+}
+
+// A move along dir, on all fields of the code word at once (they lie 9 bits apart, so a carry out of
+// one field's 3-bit component falls into bits the component mask drops): the mover's code word after
+// the move (own components change by -d), and in `flip` the bits its neighbours' reverse fields
+// change in, neighbour k's in field k (the reverse component is the negation mod 8 of the own one).
+// Unused fields stay zero in both.
+template <typename W>
+__device__ __forceinline__ W code_move(W code, uint32_t dir, W& flip)
+{
+    uint32_t const n = uint32_t(code >> CodeWord<W>::kCountShift) & 7u;
+    constexpr W kOnes = CodeWord<W>::kSlots == 3 ? W(0x40201u) : W(0x40201ull | (0x40201ull << 27));
+    W const one = (kOnes << (3u * (dir >> 1))) & ((W(1) << (9u * n)) - W(1)), mask = (one << 3) - one;
+    W const x = code & mask, y = (x + ((dir & 1u) ? mask : one)) & mask;
+    flip = (((x ^ mask) + one) ^ ((y ^ mask) + one)) & mask;
+    return (code ^ x) | y;
+}
+// The bits that a neighbour's code word changes in: field q of flip, moved to its reverse slot.
+template <typename W>
+__device__ __forceinline__ W code_flip(W flip, uint32_t q, uint32_t reverse)
+{
+    return W((flip >> (9u * q)) & W(511u)) << (9u * reverse);
 }
 
 // True if every bond of the code word stays in the allowed set after a move along dir.

@@ -29,6 +29,9 @@ namespace {
 constexpr uint32_t kStepCap = 8192;       // step entries staged per host->device copy
 constexpr uint32_t kGraphMcs = 32;        // MCS per captured graph chunk
 constexpr uint32_t kSlotAlign = 32;
+// AUTO: runs of large systems shorter than this replay graphs (a persistent launch loads and writes
+// back every slot: on the 256^3 melt 4 MCS take 96 us as a graph and 109 persistent, 6 MCS 140 and 133)
+constexpr int32_t kSlabMcs = 6;
 
 bool pow2(uint32_t v) { return v && !(v & (v - 1)); }
 
@@ -545,6 +548,7 @@ void Updater::initialize()
     cuda_check(cudaStreamSynchronize(s), "initialize");
     buildObservables();
     planCluster();
+    slab_plan(grpSize_.data(), nC, maxc_, nwords, codeMode_, smCount_, slab_);
     subStep_ = 0;
     mcsDone_ = 0;
     lastColor_ = kNoColor;
@@ -1082,7 +1086,7 @@ float Updater::runTimed(int32_t nMcs)
     if (nMcs > 0 && (uint64_t)nMcs * grpSize_.size() <= 0xFFFFFFFFull) {
         cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
         ensureStaging();
-        if (effectiveMode() == kModeGraph) prepareGraphs((uint32_t)nMcs * (uint32_t)grpSize_.size());
+        if (effectiveMode(nMcs) == kModeGraph) prepareGraphs((uint32_t)nMcs * (uint32_t)grpSize_.size());
     }
     cudaEvent_t a, b;
     cuda_check(cudaEventCreate(&a), "cudaEventCreate");
@@ -1234,34 +1238,34 @@ void Updater::enqueueCluster(uint32_t nSteps)
 int Updater::path() const
 {
     requireInit("path");
-    return effectiveMode();
+    return effectiveMode(1);
 }
 
-int Updater::autoMode() const
+int Updater::autoMode(int32_t nMcs) const
 {
     // One system on a B200, per MCS: the resident kernel (one SM) while the largest colour group is
     // at most 2 x 1024 monomers (1.2K-3.3K-monomer chains 3.8-6.6 us, against 5.5-7.8 on a
     // cluster; 6.5K-8K: 11.4-13.2 against 8.3-8.8); then a cluster of CTAs holding the system in
     // distributed shared memory where each CTA walks at most 48 chunks of 32 slots per colour,
-    // one per warp where a cluster of up to 16 CTAs allows (planCluster; 8K-47K monomers: 8.3-14.7
-    // us against 12.8-16.0 persistent); then the
-    // persistent sweep while its tiles fit about three per SM (to 262K monomers: 16-19 us against
-    // 18-22 graph); beyond, the graph of separate launches (1M monomers: 30 us against 36).
+    // one per warp where a cluster of up to 16 CTAs allows (planCluster); then the persistent sweep
+    // (60K monomers 8.6 us against 15.2 for the graph of launches, 131K 9.6 against 13.4, 1M 14.9
+    // against 21.7), from three tiles per SM on only for runs of at least kSlabMcs MCS; else the
+    // graph.
     if (residentEligible() && maxGroup_ <= 2u * kResidentBlock) return kModeResident;
     if (clusterEligible() && clusterTier_ >= 3) return kModeCluster;
-    if (codeMode_ != kCodeNone) {
+    if (slab_.ctas != 0) {
         uint32_t const tiles = (maxGroup_ + kBcTileSpan - 1) / kBcTileSpan;
-        if (tiles <= 3u * smCount_) return kModePersistent;
+        if (tiles <= 3u * smCount_ || nMcs >= kSlabMcs) return kModePersistent;
     }
     return kModeGraph;
 }
 
-int Updater::effectiveMode() const
+int Updater::effectiveMode(int32_t nMcs) const
 {
     int m = mode_;
-    if (m == kModeAuto) m = autoMode();
+    if (m == kModeAuto) m = autoMode(nMcs);
     if (m == kModeResident && !residentEligible()) m = kModeGraph;
-    if (m == kModePersistent && codeMode_ == kCodeNone) m = kModeGraph;   // bond codes only
+    if (m == kModePersistent && slab_.ctas == 0) m = kModeGraph;   // bond codes, slots that fit
     if (m == kModeCluster && !clusterEligible()) m = kModeGraph;
     return m;
 }
@@ -1277,7 +1281,7 @@ void Updater::run(int32_t nMcs)
     ensureStaging();
     lastRunSnap_ = false;   // enqueueGraph sets both again
     lastRunLead_ = false;
-    int const m = effectiveMode();
+    int const m = effectiveMode(nMcs);
     if (m != kModeGraph) flushTickets();
     if (m == kModeResident) enqueueResident(nSteps);
     else if (m == kModeGraph) enqueueGraph(nSteps);
@@ -1287,21 +1291,6 @@ void Updater::run(int32_t nMcs)
     mcsDone_ += (uint64_t)nMcs;
     hostStale_ = true;
 }
-
-namespace {
-// CTAs per SM of the persistent kernel (launch_sweep_bc: 4, 5 or 6); 4, the default, is as fast
-// as the others up to a few hundred thousand monomers and faster above. The environment variable
-// BFM_SWEEP_SHAPE overrides it for tuning
-int sweep_shape()
-{
-    static int const shape = [] {
-        char const* e = std::getenv("BFM_SWEEP_SHAPE");
-        int const v = e ? std::atoi(e) : 0;
-        return (v >= 0 && v < kSweepShapes) ? v : 0;
-    }();
-    return shape;
-}
-}  // namespace
 
 void Updater::enqueuePersistent(uint32_t nSteps)
 {
@@ -1318,16 +1307,12 @@ void Updater::enqueuePersistent(uint32_t nSteps)
         // barrier's target is reached); the fault word stays set once a launch has failed
         cuda_check(cudaMemsetAsync(&dev_.gs->count, stallNext_ ? 0x80 : 0, sizeof(unsigned int), stream_),
                    "clear grid barrier");
-        // an injected stall tests the grid barrier in global memory, so that launch is cooperative
-        bool const allowCluster = !stallNext_;
         stallNext_ = false;
-        uint32_t grid = 0;
-        cuda_check(launch_sweep_bc(dev_.h, dev_.dSteps, chunk, maxGroup_, dev_.gs, codeMode_, sweep_shape(),
-                                   allowCluster, stream_, &grid),
-                   "persistent sweep");
+        cuda_check(launch_slab_bc(dev_.h, dev_.dSteps, chunk, slab_, dev_.gs, codeMode_, stream_), "persistent sweep");
         ++launches_;
         done += chunk;
     }
+    lastColor_ = kNoColor;   // the launch zeroed its last marks
     // the fault word comes back with the next synchronisation
     cuda_check(cudaMemcpyAsync(hGs_, dev_.gs, sizeof(GridSync), cudaMemcpyDeviceToHost, stream_), "grid status");
     d2hBytes_ += sizeof(GridSync);

@@ -270,6 +270,7 @@ private:
     uint32_t clusterPer_ = 0;                  // chunks of 32 slots per warp and colour
     size_t clusterSmem_ = 0;                   // dynamic shared memory per CTA
     uint32_t clusterTier_ = 0;                 // 3: AUTO takes the plan, 2: a Batch does, 1: forced only
+    SlabPlan slab_;                            // the persistent sweep's plan (ctas == 0: does not fit)
     uint32_t hStepCap_ = 0;
     struct GraphExec {
         uint32_t nSteps, parity0;               // chunk length, parity of its first sub-step
@@ -295,8 +296,8 @@ private:
     cudaGraphExec_t graphFor(uint32_t nSteps, uint32_t parity0, bool snap);
     void seedChain(cudaStream_t s);           // the device chain restarts at the host's position
     void producerOff(cudaStream_t s);         // the device producer stops writing entries
-    int effectiveMode() const;                // the path run() takes (mode_ with AUTO resolved)
-    int autoMode() const;                     // the path BFM_MODE_AUTO takes for this system
+    int effectiveMode(int32_t nMcs) const;    // the path run(nMcs) takes (mode_ with AUTO resolved)
+    int autoMode(int32_t nMcs) const;         // the path BFM_MODE_AUTO takes for this system
     void prepareGraphs(uint32_t nSteps);      // capture the graphs a graph-path run of nSteps replays
     // bond codes: unfolded positions (slot order) to image offsets in place (SysDev x, y, z)
     void toImageOffsets(std::vector<int32_t>& hx, std::vector<int32_t>& hy, std::vector<int32_t>& hz) const;

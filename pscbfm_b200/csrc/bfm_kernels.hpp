@@ -88,17 +88,30 @@ inline bool perform_shape_ok(int warps, int group)
 cudaError_t launch_perform_bc(SysDev const& hostDesc, SysDev const* dSys, TileRef const* dTiles, uint32_t nTiles,
                               StepEntry const* dSteps, uint32_t codeMode, cudaStream_t s, int shape = -1,
                               PerformArgs const& pa = PerformArgs{});
-// Persistent sweep (bond codes, one system): nSteps sub-steps of check, barrier, perform in one
-// launch of at most the co-resident CTA count: a grid of at most 16 CTAs as one thread-block
-// cluster (hardware barriers) where allowCluster and the device can run it, otherwise a
-// cooperative launch with grid barriers in global memory. gs->count must be zeroed before the
-// launch; after it, gs->fault != 0 means a grid-barrier wait ran out and the system's state is not
-// usable. shape selects the CTAs per SM the register budget must fit: 0 -> 4, 1 -> 5, 2 -> 6 (two
-// monomers per thread, one mover-list segment per tile).
-constexpr int kSweepShapes = 3;
-cudaError_t launch_sweep_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, uint32_t maxGroup,
-                            GridSync* gs, uint32_t codeMode, int shape, bool allowCluster, cudaStream_t s,
-                            uint32_t* gridOut);
+// Persistent sweep (bond codes, one system): nSteps sub-steps in one cooperative launch of
+// plan.ctas CTAs, each holding its share of the slots in shared memory (k_slab_bc). slab_plan
+// returns false where the system does not fit (more than kSlabColors colours, or too many slots per
+// CTA). gs->count must be zeroed before the launch; after it, gs->fault != 0 means a grid-barrier
+// wait ran out and the system's state is not usable.
+// threads per CTA (one CTA per SM); 64-bit codes keep up to six neighbours of a mover in registers
+constexpr uint32_t kSlabBlock32 = 640, kSlabBlock64 = 512;
+constexpr uint32_t kSlabColors = 8;          // bond codes: at most 6 bonds, so at most 7 colours
+constexpr uint32_t kSlabEntBits = 13;         // list entries: a slot's index in its colour's part, and 3 direction bits
+// bits of a local index in a 16-bit neighbour reference, below the reverse slot (0-2, or 0-5 with 64-bit codes)
+__host__ __device__ constexpr uint32_t slab_ref_bits(bool code64) { return code64 ? 13u : 14u; }
+constexpr uint32_t kSlabMinChunks = 8;       // chunks of 32 slots per CTA and colour, before more CTAs join
+constexpr size_t kSlabMaxSmem = 226 * 1024;
+struct SlabPlan {
+    uint32_t ctas = 0;         // 0: the system does not fit
+    uint32_t cap = 0, capG = 0;   // slots a CTA holds in all and of its largest colour group
+    uint32_t clearAll = 0;     // zero the previous temporary lattice whole
+    bool cache = false;        // the neighbour references and inner direction hashes fit in shared memory too
+    size_t smem = 0;
+};
+bool slab_plan(uint32_t const* grpSize, uint32_t nColors, uint32_t maxc, uint32_t nwords, uint32_t codeMode,
+               uint32_t sms, SlabPlan& plan);
+cudaError_t launch_slab_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
+                           GridSync* gs, uint32_t codeMode, cudaStream_t s);
 size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t codeMode);
 // Cluster-resident sweep (bond codes): one cluster of 2^logC CTAs of kResidentBlock threads per
 // system of dList[0..nClusters) (logC 1..4), state in the cluster's shared memory for nSteps

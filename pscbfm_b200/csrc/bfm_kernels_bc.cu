@@ -14,9 +14,8 @@
 // listed at t-1. Every independent load of a pass is issued before any dependent one; a single-system
 // launch takes the descriptor as a grid-constant parameter.
 //
-// Persistent (k_sweep_bc): the same bodies for a whole run of sub-steps in one launch: a grid of
-// at most 16 CTAs as one thread-block cluster with hardware barriers between the phases, a larger
-// one as a cooperative launch with time-bounded grid barriers.
+// Persistent (k_slab_bc): a whole run of sub-steps in one cooperative launch with time-bounded grid
+// barriers; the lattices in global memory, each CTA's share of the slots in its shared memory.
 //
 // Resident (k_resident_bc): one CTA owns a small system for a chunk of sub-steps; lattice, one
 // temporary lattice, pk and bond codes in shared memory; the check appends tentative movers to a
@@ -59,17 +58,6 @@ __device__ __forceinline__ bool bonds_ok(W code, uint32_t dir, uint8_t const* ok
     return (m >> dir) & 1u;
 }
 
-// Loads of state the sweep changes (packed coordinates, codes, flags, lattices): through the
-// read-only data path where one launch only reads them (kNc), plain loads in the persistent
-// kernel, where other CTAs wrote them earlier in the same launch (the read-only path is not
-// coherent with those writes).
-template <bool kNc, typename T>
-__device__ __forceinline__ T ldm(T const* p)
-{
-    if constexpr (kNc) return __ldg(p);
-    else return *p;
-}
-
 // Mover lists: the check of sub-step t appends each tentative mover of tile k (kBcTileSpan
 // in-colour indices) to segment k of list[parity] (entry: slot g in bits 0-26, direction in
 // 27-29), the lattice address of its target (the temporary-lattice cell it marked) to the same
@@ -85,7 +73,7 @@ constexpr int kPerfQ = 4;
 
 // ---------------------------------------------------------------------------------- check
 
-template <typename W, int MPT, bool kNc = true>
+template <typename W, int MPT>
 __device__ __forceinline__ void check_body(SysDev const& S, uint32_t const* dtab, StepEntry const& st, uint32_t start,
                                            uint32_t* segCount, uint2* stage)
 {
@@ -105,7 +93,7 @@ __device__ __forceinline__ void check_body(SysDev const& S, uint32_t const* dtab
 #pragma unroll
     for (int q = 0; q < MPT; ++q) {
         uint32_t const i = start + tid + (uint32_t)q * B;
-        RV const r = i < st.cnt ? ldm<kNc>(REC + st.off + i) : RV{};
+        RV const r = i < st.cnt ? __ldg(REC + st.off + i) : RV{};
         pk[q] = r.x;
         code[q] = rec_code_of(r);
     }
@@ -146,7 +134,7 @@ __device__ __forceinline__ void check_body(SysDev const& S, uint32_t const* dtab
         unsigned long long hit = 0ull;
 #pragma unroll
         for (int r = 0; r < 4; ++r)
-            if (live && ((pl.touch >> r) & 1u)) hit |= ldm<kNc>(S.lat + pl.w[r]) & pl.m[r];
+            if (live && ((pl.touch >> r) & 1u)) hit |= __ldg(S.lat + pl.w[r]) & pl.m[r];
         bool const go = live && hit == 0ull;
         uint32_t const bal = __ballot_sync(0xffffffffu, go);
         uint32_t base = 0;
@@ -178,7 +166,7 @@ __device__ __forceinline__ void image_step(SysDev const& S, uint32_t g, uint32_t
 // live[q]: re-test the front plane on the temporary lattice and apply the free moves. The plane
 // and the old position follow from the target's address, so the monomer's own address is not
 // loaded. Returns the moves applied.
-template <typename W, int N, bool kNc>
+template <typename W, int N>
 __device__ __forceinline__ uint32_t perform_movers(SysDev const& S, uint32_t const* dtab,
                                                    unsigned long long const* tcur, uint32_t const (&ent)[N],
                                                    uint32_t const (&to)[N], bool const (&live)[N])
@@ -210,7 +198,7 @@ __device__ __forceinline__ uint32_t perform_movers(SysDev const& S, uint32_t con
         hit[q] = 0ull;
 #pragma unroll
         for (int r = 0; r < 4; ++r)
-            if (live[q] && ((pl[q].touch >> r) & 1u)) hit[q] |= ldm<kNc>(tcur + pl[q].w[r]) & pl[q].m[r];
+            if (live[q] && ((pl[q].touch >> r) & 1u)) hit[q] |= __ldg(tcur + pl[q].w[r]) & pl[q].m[r];
     }
     uint32_t nAcc = 0;
 #pragma unroll
@@ -248,92 +236,6 @@ __device__ __forceinline__ uint32_t perform_movers(SysDev const& S, uint32_t con
     return nAcc;
 }
 
-// Entries e, e + B, ... (MPT of them, those below total) of the concatenated mover lists of nT
-// tiles (pre: the lists' starting offsets, lbase / tbase: the first tile's segment of the entries
-// and of the target addresses), through perform_movers. Returns the moves applied.
-template <typename W, int MPT, bool kNc>
-__device__ __forceinline__ uint32_t perform_chunk(SysDev const& S, uint32_t const* dtab,
-                                                  unsigned long long const* tcur, uint32_t const* lbase,
-                                                  uint32_t const* tbase, uint32_t const* pre, uint32_t nT,
-                                                  uint32_t total, uint32_t e)
-{
-    uint32_t const B = blockDim.x;
-    uint32_t ent[MPT], to[MPT];
-    bool live[MPT];
-#pragma unroll
-    for (int q = 0; q < MPT; ++q) {
-        uint32_t const eq = e + (uint32_t)q * B;
-        uint32_t j = 0;
-        while (j + 1 < nT && eq >= pre[j + 1]) ++j;
-        live[q] = eq < total;
-        uint32_t const li = j * kBcTileSpan + (eq - pre[j]);
-        ent[q] = live[q] ? ldm<kNc>(lbase + li) : 0u;
-        to[q] = live[q] ? ldm<kNc>(tbase + li) : 0u;
-    }
-    return perform_movers<W, MPT, kNc>(S, dtab, tcur, ent, to, live);
-}
-
-// The persistent sweep's perform. For tiles tile0 .. tile0+nT-1 (at most 16): zeroes the
-// temporary-lattice words the previous sub-step's movers marked, then walks this sub-step's
-// tentative movers as one dense range
-// (no thread waits on a monomer that did not move). pre is 2 (nT+1) words of shared memory: the
-// starting offsets of the current and of the previous lists. A tile's list counts only if the
-// tile lies inside that sub-step's colour group (older lengths may remain in count[]). Every thread
-// of the CTA calls this; st.color == kNoColor only scrubs.
-template <typename W, int MPT, bool kNc = true>
-__device__ __forceinline__ void perform_body(SysDev const& S, uint32_t const* dtab, StepEntry const& st,
-                                             uint32_t tile0, uint32_t nT, uint32_t* tally, uint32_t* pre)
-{
-    uint32_t const B = blockDim.x, tid = threadIdx.x;
-    unsigned long long const* const tcur = S.tmp + (size_t)st.parity * S.nwords;
-    unsigned long long* const tprev = S.tmp + (size_t)(st.parity ^ 1u) * S.nwords;
-    uint32_t const* const lbase = S.mlist + (size_t)st.parity * S.listStride + (size_t)tile0 * kBcTileSpan;
-    uint32_t const* const tbase = S.mword + (size_t)st.parity * S.listStride + (size_t)tile0 * kBcTileSpan;
-    uint32_t const* const wprev = S.mword + (size_t)(st.parity ^ 1u) * S.listStride + (size_t)tile0 * kBcTileSpan;
-    uint32_t const* const cnt = S.mcount + (size_t)st.parity * S.countStride + tile0;
-    uint32_t const* const cntPrev = S.mcount + (size_t)(st.parity ^ 1u) * S.countStride + tile0;
-    uint32_t* const preP = pre + nT + 1;
-    bool const active = st.color != kNoColor;
-    // the list lengths, this sub-step's in lanes 0..nT-1 and the previous sub-step's in lanes
-    // 16..16+nT-1, loaded by one warp before the barrier and scanned after it
-    uint32_t const j = tid & 15u;
-    uint32_t c = 0;
-    if (tid < 32 && j < nT) {
-        uint32_t const start = (tile0 + j) * kBcTileSpan;
-        if (tid < 16) c = (active && start < st.cnt) ? ldm<kNc>(cnt + j) : 0u;
-        else c = start < st.pcnt ? ldm<kNc>(cntPrev + j) : 0u;
-    }
-    __syncthreads();   // pre of an earlier call has been read; the caller's shared writes are visible
-    if (tid < 32) {
-#pragma unroll
-        for (uint32_t o = 1; o < 16; o <<= 1) {
-            uint32_t const v = __shfl_up_sync(0xffffffffu, c, o, 16);
-            if (j >= o) c += v;
-        }
-        uint32_t* const dst = tid < 16 ? pre : preP;
-        if (j < nT) dst[j + 1] = c;
-        if (j == 0) dst[0] = 0u;
-    }
-    __syncthreads();
-    // scrub of the previous sub-step: every set bit of tmp[parity^1] belongs to one of its
-    // tentative movers, so zeroing a whole marked word only clears bits that are due. The first
-    // words are loaded before the movers' chain starts and zeroed after it, so the two overlap.
-    uint32_t const totalP = preP[nT];
-    auto scrubWord = [&](uint32_t e) {
-        uint32_t j = 0;
-        while (j + 1 < nT && e >= preP[j + 1]) ++j;
-        return ldm<kNc>(wprev + j * kBcTileSpan + (e - preP[j])) >> 6;
-    };
-    uint32_t const w0 = tid < totalP ? scrubWord(tid) : 0u;
-    uint32_t const total = pre[nT];
-    uint32_t nAcc = 0;
-    for (uint32_t e0 = 0; e0 < total; e0 += B * MPT)
-        nAcc += perform_chunk<W, MPT, kNc>(S, dtab, tcur, lbase, tbase, pre, nT, total, e0 + tid);
-    if (tid < totalP) tprev[w0] = 0ull;
-    for (uint32_t e = tid + B; e < totalP; e += B) tprev[scrubWord(e)] = 0ull;
-    if (nAcc) atomicAdd(tally, nAcc);
-}
-
 // Grid-phase perform of one tile by a group of G warps (`sub` = this warp's index in the group):
 // the group walks list segment `tile` of this sub-step (parity p: its tentative movers) and of the
 // previous one (parity p ^ 1: it zeroes the temporary-lattice words those movers marked), warp
@@ -345,7 +247,7 @@ __device__ __forceinline__ void perform_body(SysDev const& S, uint32_t const* dt
 // take further passes. The warp's copy of the direction table (dtab) is written from d0, d1 (words
 // lane and lane + 32, loaded by the caller) once those loads are out, so the table's round trip
 // overlaps the lists'. Returns the moves this warp applied.
-template <typename W, bool kNc, int Q>
+template <typename W, int Q>
 __device__ __forceinline__ uint32_t perform_tile(SysDev const& S, uint32_t* dtab, uint32_t d0, uint32_t d1,
                                                  uint32_t p, uint32_t tile, bool doCur, bool doPrev, uint32_t sub,
                                                  uint32_t G, uint32_t& listLen)
@@ -357,8 +259,8 @@ __device__ __forceinline__ uint32_t perform_tile(SysDev const& S, uint32_t* dtab
     uint32_t const* const wp = S.mword + (size_t)(p ^ 1u) * S.listStride + seg;
     unsigned long long const* const tcur = S.tmp + (size_t)p * S.nwords;
     unsigned long long* const tprev = S.tmp + (size_t)(p ^ 1u) * S.nwords;
-    uint32_t const cnt = doCur ? ldm<kNc>(S.mcount + (size_t)p * S.countStride + tile) : 0u;
-    uint32_t const pcnt = doPrev ? ldm<kNc>(S.mcount + (size_t)(p ^ 1u) * S.countStride + tile) : 0u;
+    uint32_t const cnt = doCur ? __ldg(S.mcount + (size_t)p * S.countStride + tile) : 0u;
+    uint32_t const pcnt = doPrev ? __ldg(S.mcount + (size_t)(p ^ 1u) * S.countStride + tile) : 0u;
     listLen = cnt;
     uint32_t const first = sub * 32u + lane, stride = 32u * G;
     uint32_t ent[Q], to[Q], pw[Q];
@@ -366,16 +268,16 @@ __device__ __forceinline__ uint32_t perform_tile(SysDev const& S, uint32_t* dtab
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         uint32_t const e = first + stride * (uint32_t)q;   // < 32 G Q <= kBcTileSpan
-        ent[q] = doCur ? ldm<kNc>(lc + e) : 0u;
-        to[q] = doCur ? ldm<kNc>(wc + e) : 0u;
-        pw[q] = doPrev ? ldm<kNc>(wp + e) : 0u;
+        ent[q] = doCur ? __ldg(lc + e) : 0u;
+        to[q] = doCur ? __ldg(wc + e) : 0u;
+        pw[q] = doPrev ? __ldg(wp + e) : 0u;
     }
     dtab[lane] = d0;
     if (lane + 32u < kDirTab) dtab[lane + 32u] = d1;
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < Q; ++q) live[q] = first + stride * (uint32_t)q < cnt;
-    uint32_t nAcc = perform_movers<W, Q, kNc>(S, dtab, tcur, ent, to, live);
+    uint32_t nAcc = perform_movers<W, Q>(S, dtab, tcur, ent, to, live);
 #pragma unroll
     for (int q = 0; q < Q; ++q)
         if (first + stride * (uint32_t)q < pcnt) tprev[pw[q] >> 6] = 0ull;
@@ -385,16 +287,16 @@ __device__ __forceinline__ uint32_t perform_tile(SysDev const& S, uint32_t* dtab
         for (int q = 0; q < Q; ++q) {
             uint32_t const e = b + first + stride * (uint32_t)q;
             live[q] = e < cnt;
-            ent[q] = live[q] ? ldm<kNc>(lc + e) : 0u;
-            to[q] = live[q] ? ldm<kNc>(wc + e) : 0u;
+            ent[q] = live[q] ? __ldg(lc + e) : 0u;
+            to[q] = live[q] ? __ldg(wc + e) : 0u;
         }
-        nAcc += perform_movers<W, Q, kNc>(S, dtab, tcur, ent, to, live);
+        nAcc += perform_movers<W, Q>(S, dtab, tcur, ent, to, live);
     }
     for (uint32_t b = pass; b < pcnt; b += pass) {
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             uint32_t const e = b + first + stride * (uint32_t)q;
-            if (e < pcnt) tprev[ldm<kNc>(wp + e) >> 6] = 0ull;
+            if (e < pcnt) tprev[__ldg(wp + e) >> 6] = 0ull;
         }
     }
     return nAcc;
@@ -520,7 +422,7 @@ __global__ void __launch_bounds__(32 * PW) k_perform_bc(const __grid_constant__ 
         uint32_t listLen = 0;
         uint32_t const nAcc = __reduce_add_sync(
             0xffffffffu,
-            perform_tile<W, true, Q>(S, dtabs[wid], d0, d1, p, tile, cur, prev, sub, (uint32_t)G, listLen));
+            perform_tile<W, Q>(S, dtabs[wid], d0, d1, p, tile, cur, prev, sub, (uint32_t)G, listLen));
         uint32_t const stripe = (blockIdx.x * PW + wid) % kStatSlots;
         // the tile's list length (its tentative moves) is counted once, by the group's first warp
         if (lane == 0 && sub == 0 && listLen)
@@ -532,7 +434,9 @@ __global__ void __launch_bounds__(32 * PW) k_perform_bc(const __grid_constant__ 
 
 // ---------------------------------------------------------------------------------- persistent
 
-constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;   // a wait longer than 2 s is a fault
+// A wait longer than 2 s is a fault; a launch's first wait may take 20 s, since it ends only once every
+// CTA has found a free SM (another stream's kernel may hold some for a while).
+constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull, kFirstBarrierTimeoutNs = 20000000000ull;
 
 __device__ __forceinline__ unsigned int ld_acquire_gpu(unsigned int const* p)
 {
@@ -553,112 +457,485 @@ __device__ __forceinline__ void red_release_gpu_add(unsigned int* p, unsigned in
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// All CTAs of the cooperative grid meet; every write before the barrier is visible to every
-// thread after it. After the CTA barrier, thread 0 adds the CTA's arrival to a count that only
-// grows (a release add, which orders the whole CTA's earlier writes before it) and waits with
-// acquire loads until the count reaches this barrier's target, gridDim.x above the previous one.
-// Nothing is reset between barriers, and the signed difference keeps the comparison right
-// across a wrap of the count. The wait is bounded by time and by a poll count; on every thread
-// of the CTA it returns false if it ran out or another CTA's did (GridSync::fault): the kernel
-// then leaves, and the host reports the fault.
-__device__ __forceinline__ bool grid_barrier(GridSync* gs, unsigned int& target, unsigned int* okSm)
+// One thread of each CTA, after a CTA barrier that ordered the CTA's earlier writes before it: adds
+// the CTA's arrival to a count that only grows (a release add) and waits with acquire loads until
+// the count reaches this barrier's target, nCtas above the previous one. Nothing is reset between
+// barriers, and the signed difference keeps the comparison right across a wrap of the count. The
+// wait is bounded by time and by a poll count; false if it ran out or another CTA's did
+// (GridSync::fault): the kernel then leaves, and the host reports the fault.
+__device__ __forceinline__ bool grid_meet(GridSync* gs, unsigned int& target, unsigned int nCtas)
 {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int ok = 1u;
-        target += gridDim.x;
-        red_release_gpu_add(&gs->count, 1u);
-        if (int(ld_acquire_gpu(&gs->count) - target) < 0) {
-            unsigned long long const t0 = global_ns();
-            unsigned int polls = 0u;
-            while (int(ld_acquire_gpu(&gs->count) - target) < 0) {
-                // a time limit, and a poll count as a second bound that does not trust the timer
-                if ((++polls & 255u) == 0u) {
-                    if (ld_acquire_gpu(&gs->fault) != 0u) {
-                        ok = 0u;
-                        break;
-                    }
-                    if (global_ns() - t0 > kBarrierTimeoutNs || polls > (1u << 24)) {
-                        if (atomicExch(&gs->fault, 1u) == 0u) gs->where = target / gridDim.x;
-                        ok = 0u;
-                        break;
-                    }
+    target += nCtas;
+    red_release_gpu_add(&gs->count, 1u);
+    if (int(ld_acquire_gpu(&gs->count) - target) < 0) {
+        bool const first = target == nCtas;
+        unsigned long long const t0 = global_ns(), limit = first ? kFirstBarrierTimeoutNs : kBarrierTimeoutNs;
+        unsigned int polls = 0u;
+        while (int(ld_acquire_gpu(&gs->count) - target) < 0) {
+            // a time limit, and a poll count as a second bound that does not trust the timer
+            if ((++polls & 255u) == 0u) {
+                if (ld_acquire_gpu(&gs->fault) != 0u) return false;
+                if (global_ns() - t0 > limit || polls > (first ? 1u << 27 : 1u << 24)) {
+                    if (atomicExch(&gs->fault, 1u) == 0u) gs->where = target / nCtas;
+                    return false;
                 }
-                __nanosleep(20);
             }
+            __nanosleep(20);
         }
-        *okSm = ok;
     }
-    __syncthreads();
-    return *okSm != 0u;
+    return true;
 }
 
-// The whole grid as one thread-block cluster: the hardware cluster barrier, with release and
-// acquire semantics at cluster scope, orders every thread's earlier global writes before any
-// thread's later reads. Every CTA of the sweep reaches the same sequence of barriers.
-__device__ __forceinline__ void cluster_barrier()
+// Slab-resident layout (k_slab_bc): CTA r of C holds, of every colour group of n slots in
+// chunks of 32, chunks [r nch / C, (r + 1) nch / C), nch = ceil(n / 32): contiguous slots, in the
+// group's order, so the neighbours of a chain numbered along its bonds mostly lie in the same CTA.
+struct SlabPart {
+    uint32_t first[kSlabColors], count[kSlabColors], base[kSlabColors];   // first slot, slots, local index
+};
+
+// A code word's top bit in shared memory (above the fields and the count): some neighbour of the slot
+// lies in another CTA, so its code word lives in global memory, where that CTA can change it.
+template <typename W>
+__device__ __forceinline__ constexpr W slab_shared_flag()
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return W(1) << (8 * sizeof(W) - 1);
 }
 
-// One system, a whole run of sub-steps in one cooperative launch: per sub-step the check phase
-// over every tile, a grid barrier, the perform phase and (between sub-steps) another barrier. CTA b
-// takes tiles b, b + gridDim.x, ... of kGridBlock * MPT in-colour indices. Same bodies as
-// k_check_bc / k_perform_bc, with plain loads of the state other CTAs change during the launch;
-// the step entries are prefetched one sub-step ahead and the move counters flushed once.
-template <typename W, int MPT, int kMinBlocks, bool kCluster, int B = (int)kGridBlock>
-__global__ void __launch_bounds__(B, kMinBlocks)
-    k_sweep_bc(const __grid_constant__ SysDev S, StepEntry const* __restrict__ steps, uint32_t nSteps,
-               uint32_t nTiles, GridSync* gs)
+// Local index of slot g in this CTA, or kNoMark if another CTA holds it.
+__device__ __forceinline__ uint32_t slab_local(SlabPart const& P, uint32_t nColors, uint32_t g)
 {
-    static_assert(B * MPT == (int)kBcTileSpan, "a tile is one list segment");
-    __shared__ __align__(16) uint32_t dtab[kDirTab];
-    __shared__ uint32_t tallyT, tallyA, okSm, segCount, pre[4];
-    __shared__ uint2 stage[kBcTileSpan];   // the warps' candidates (check_body)
+    for (uint32_t c = 0; c < nColors; ++c) {
+        uint32_t const d = g - P.first[c];
+        if (d < P.count[c]) return P.base[c] + d;
+    }
+    return kNoMark;
+}
+
+// Adds v to a counter in shared memory and returns its old value, as one instruction: written with
+// atomicAdd, the compiler gathers the adds of a warp first, 20 instructions for the one lane that adds.
+__device__ __forceinline__ uint32_t shared_add(uint32_t* p, uint32_t v)
+{
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v)
+                 : "memory");
+    return old;
+}
+__device__ __forceinline__ void shared_xor(uint32_t* p, uint32_t v) { atomicXor(p, v); }
+// (a 64-bit exclusive or as two on the halves: shared memory has no native 64-bit one)
+__device__ __forceinline__ void shared_xor(unsigned long long* p, unsigned long long v)
+{
+    unsigned int* const h = reinterpret_cast<unsigned int*>(p);
+    if ((unsigned int)v) atomicXor(h, (unsigned int)v);
+    if ((unsigned int)(v >> 32)) atomicXor(h + 1, (unsigned int)(v >> 32));
+}
+
+// The words a front plane touches and their masks, prepared ahead of the reads (a word that is not
+// touched has an empty mask; reads of it are left out).
+struct PlaneRef {
+    uint32_t w[4];
+    unsigned long long m[4];
+};
+__device__ __forceinline__ void plane_ref(PlaneRef& r, unsigned long long const* ptab, DirParams const& D,
+                                          uint32_t base, uint32_t da, uint32_t dir)
+{
+    uint32_t ti, touch;
+    front_plane_words(r.w, ti, touch, D, base, da, dir);
+    ulonglong2 const m01 = *reinterpret_cast<ulonglong2 const*>(ptab + ti);
+    ulonglong2 const m23 = *reinterpret_cast<ulonglong2 const*>(ptab + ti + 2);
+    r.m[0] = m01.x;
+    r.m[1] = m01.y;
+    r.m[2] = m23.x;
+    r.m[3] = m23.y;
+}
+// An 8-byte load where `on`, else 0, as one predicated instruction: the loads of a plane go out back
+// to back. Coherent with other CTAs' writes after a grid barrier (its acquire drops the L1's lines),
+// cached in the L1 within a phase.
+__device__ __forceinline__ unsigned long long load_if(unsigned long long const* p, bool on)
+{
+    unsigned long long v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.u64 %0, 0;\n\t@q ld.global.u64 %0, [%1];\n\t}"
+                 : "=l"(v)
+                 : "l"(p), "r"((uint32_t)on)
+                 : "memory");
+    return v;
+}
+// The set cells of the plane in lattice L (0 where not live).
+__device__ __forceinline__ unsigned long long plane_hits(PlaneRef const& r, bool live, unsigned long long const* L)
+{
+    unsigned long long v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = load_if(L + r.w[k], live && r.m[k] != 0ull);
+    return (v[0] & r.m[0]) | (v[1] & r.m[1]) | (v[2] & r.m[2]) | (v[3] & r.m[3]);
+}
+
+// One system, a whole run of sub-steps in one cooperative launch, one CTA per SM. Lattice and
+// temporary lattices stay in global memory (the L2); each CTA keeps the lattice addresses and code
+// words of its slots (SlabPart) in shared memory. Per sub-step two grid barriers: after the check
+// (every mark is set) and after the perform (the lattice is settled). The last warp waits at the
+// barriers; the others meanwhile do all of the next phase that depends on this CTA's own slots only:
+// bond tests, candidates and their planes before the check's lattice reads; the list of movers,
+// their codes, neighbour references and planes, the clearing of the previous marks and the
+// directions of the next sub-step before the perform's temporary-lattice reads. What is left between
+// two barriers is one round of L2 reads and the writes that follow from it.
+//   kCache: the slots' inner direction hashes and neighbour references in shared memory too.
+//   clearAll: the previous temporary lattice is zeroed whole, each CTA its share, instead of by the
+//   targets listed in it (a dense system marks most of its words).
+// Bound: on the 256^3 melt (N = 1,048,576) by the scattered L2 accesses (about 0.8 loads and 0.57
+// atomics per clock and SM) and instruction issue (27 K warp instructions per SM and sub-step); below
+// 200K monomers by the barriers (1.3-1.8 us each with the writes before them) and one L2 round trip
+// after each. Per MCS: melt 14.9 us (graph of launches 21.7), 131K monomers 9.6 (13.4; 15 with the
+// cooperative sweep that kept every record in global memory), 60K 8.6 (15.2).
+// 640 threads: 20 warps of 96 registers hold two prepared candidates per thread (the melt has 1.9
+// per thread) and its movers fit one pass; 1024 threads of 64 registers spilled and took 18 us.
+template <typename W, int B, bool kCache>
+__global__ void __launch_bounds__(B, 1)
+    k_slab_bc(const __grid_constant__ SysDev S, StepEntry const* __restrict__ steps, uint32_t nSteps, uint32_t cap,
+              uint32_t capG, uint32_t clearAll, GridSync* gs)
+{
+    constexpr uint32_t kSlots = CodeWord<W>::kSlots;
+    constexpr W kShared = slab_shared_flag<W>();
+    constexpr uint32_t nWork = B / 32 - 1, kThreads = nWork * 32;   // the last warp waits at the barriers
+    constexpr uint32_t kGroup = 3;   // slots of a thread worked on together, so that their latencies overlap
+    constexpr uint32_t kDirs = 9;    // directions (3 bits each) a thread keeps at a time
+    constexpr int kPre = 2;          // candidates of a thread prepared ahead of the barrier
+    constexpr uint32_t kEntMask = (1u << kSlabEntBits) - 1u;   // list entries: index in the part | dir << kSlabEntBits
+    constexpr uint32_t kRefBits = slab_ref_bits(sizeof(W) == 8), kRefMask = (1u << kRefBits) - 1u, kAway = 0xFFFFu;
+    constexpr uint32_t kFarBit = 1u << 31;
+    __shared__ SlabPart P;
+    __shared__ uint32_t nCand, nMov, tallyA;
+    extern __shared__ unsigned long long smem[];
+    uint32_t const tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    bool const waiter = warp == nWork;
+    uint32_t const C = gridDim.x, rank = blockIdx.x;
+    unsigned long long* const ptab = smem;                                   // 768 plane masks
+    uint32_t* const dtab = reinterpret_cast<uint32_t*>(smem + 768);          // kDirTab words
+    W* const code = reinterpret_cast<W*>(smem + 768 + kDirTab / 2);          // cap slots
+    uint32_t* const pk = reinterpret_cast<uint32_t*>(code + cap);            // cap slots
+    uint16_t* const cand = reinterpret_cast<uint16_t*>(pk + cap);            // capG candidates
+    uint16_t* const list = cand + capG;                                      // capG movers
+    uint32_t* const tgt = reinterpret_cast<uint32_t*>(list + capG);          // !clearAll: capG marked addresses
+    uint8_t* const mok = reinterpret_cast<uint8_t*>(tgt + (clearAll ? 0u : capG));   // 512 move-table bytes
+    uint32_t* const inner = reinterpret_cast<uint32_t*>(mok + 512);          // kCache: cap hashes
+    uint16_t* const refs = reinterpret_cast<uint16_t*>(inner + cap);         // kCache: maxc x cap references
     if (ld_acquire_gpu(&gs->fault) != 0u) return;   // an earlier launch failed: the state is not usable
-    if (threadIdx.x < kDirTab) dtab[threadIdx.x] = S.dirTab[threadIdx.x];
-    if (threadIdx.x == 0) {
-        tallyT = 0u;
+    uint32_t const nColors = S.nColors, np = S.npad;
+    if (tid == 0) {
+        uint32_t b = 0;
+        for (uint32_t c = 0; c < nColors; ++c) {
+            uint32_t const nch = (S.grp[2 * c + 1] + 31u) >> 5;
+            uint32_t const lo = rank * nch / C, hi = (rank + 1u) * nch / C;
+            P.first[c] = S.grp[2 * c] + 32u * lo;
+            P.count[c] = 32u * (hi - lo);
+            P.base[c] = b;
+            b += 32u * (hi - lo);
+        }
+        nCand = 0u;
+        nMov = 0u;
         tallyA = 0u;
     }
+    for (uint32_t w = tid; w < 768; w += B) ptab[w] = S.planeTab[w];
+    if (tid < kDirTab) dtab[tid] = S.dirTab[tid];
+    for (uint32_t w = tid; w < 512; w += B) mok[w] = S.moveOk[w];
     __syncthreads();
-    constexpr uint32_t span = kBcTileSpan;
-    unsigned int target = 0u;   // this CTA's count target of the next barrier
+    using RV = typename SlotRec<W>::V;
+    for (uint32_t c = 0; c < nColors; ++c)
+        for (uint32_t d = tid; d < P.count[c]; d += B) {
+            uint32_t const g = P.first[c] + d, l = P.base[c] + d;
+            RV const r = reinterpret_cast<RV const*>(S.rec)[g];
+            W cw = rec_code_of(r);
+            uint32_t const n = uint32_t(cw >> CodeWord<W>::kCountShift) & 7u;
+            for (uint32_t q = 0; q < n; ++q) {
+                uint32_t const ref = S.nbrr[(size_t)q * np + g], at = slab_local(P, nColors, ref & kSlotMask);
+                if (at == kNoMark) cw |= kShared;
+                if (kCache) refs[q * cap + l] = at == kNoMark ? kAway : at | ((ref >> kSlotShift) << kRefBits);
+            }
+            code[l] = cw;
+            pk[l] = r.x;
+            if (kCache) inner[l] = move_hash(g - S.grp[2 * c]);
+        }
+    __syncthreads();
+    if (kCache) {
+        // a neighbour held here whose code word other CTAs change too lives in global memory as well
+        for (uint32_t c = 0; c < nColors; ++c)
+            for (uint32_t d = tid; d < P.count[c]; d += B) {
+                uint32_t const l = P.base[c] + d, n = uint32_t(code[l] >> CodeWord<W>::kCountShift) & 7u;
+                for (uint32_t q = 0; q < n; ++q) {
+                    uint32_t const r = refs[q * cap + l];
+                    if (r != kAway && (code[r & kRefMask] & kShared) != W(0)) refs[q * cap + l] = kAway;
+                }
+            }
+        __syncthreads();
+    }
+    // neighbour q of slot g (local index l): the local index of its slot | its reverse slot << kSlotShift,
+    // or the slot itself with kFarBit where its code word lives in global memory
+    auto neighbour = [&](uint32_t q, uint32_t g, uint32_t l) {
+        if (kCache) {
+            uint32_t const r = refs[q * cap + l];
+            if (r != kAway) return (r & kRefMask) | ((r >> kRefBits) << kSlotShift);
+            return __ldg(S.nbrr + (size_t)q * np + g) | kFarBit;
+        }
+        uint32_t const ref = __ldg(S.nbrr + (size_t)q * np + g), at = slab_local(P, nColors, ref & kSlotMask);
+        if (at == kNoMark || (code[at] & kShared) != W(0)) return ref | kFarBit;
+        return at | ((ref >> kSlotShift) << kSlotShift);
+    };
+    // directions of this thread's slots tid + k kThreads of the part, k from k0, of a sub-step
+    auto directions = [&](StepEntry const& e, uint32_t k0) {
+        uint32_t const n = P.count[e.color], i0 = P.first[e.color] - e.off;
+        uint32_t const* const h = inner + P.base[e.color];
+        uint32_t d = 0;
+        for (uint32_t k = 0, i = tid + k0 * kThreads; k < kDirs && i < n; k += kGroup) {
+#pragma unroll
+            for (uint32_t q = 0; q < kGroup; ++q, i += kThreads) {
+                uint32_t const in = kCache ? h[i < n ? i : tid] : move_hash(i0 + i);
+                d |= (move_hash(in ^ e.seed) % 6u) << (3u * (k + q));
+            }
+        }
+        return d;
+    };
+    // a warp's append: the place of each lane with `on` in a list whose length is *count
+    uint32_t const lanesBelow = (1u << lane) - 1u;
+    auto append = [&](bool on, uint32_t* count) {
+        uint32_t const bal = __ballot_sync(0xffffffffu, on);
+        uint32_t at = 0;
+        if (lane == 0) at = shared_add(count, (uint32_t)__popc(bal));
+        return __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanesBelow);
+    };
+    unsigned int target = 0u;   // (the waiter's) count target of the next barrier
+    bool const walled = S.walls != 0u;
+    uint32_t const cw0 = (uint32_t)((uint64_t)S.nwords * rank / C), cw1 = (uint32_t)((uint64_t)S.nwords * (rank + 1u) / C);
+    uint32_t prevMov = 0u, nAcc = 0u, nTent = 0u, par = 0u, dirs = 0u;
     unsigned long long att = 0ull;
     StepEntry next = steps[0];
+    if (!waiter) dirs = directions(next, 0);
     for (uint32_t t = 0; t < nSteps; ++t) {
         StepEntry const st = next;
         if (t + 1 < nSteps) next = steps[t + 1];
-        bool const active = st.color != kNoColor;
-        for (uint32_t k = blockIdx.x; k < nTiles; k += gridDim.x) {
-            uint32_t const start = k * span;
-            if (!active || start >= st.cnt) break;
-            if (threadIdx.x == 0) segCount = 0u;   // published by check_body's first barrier
-            check_body<W, MPT, false>(S, dtab, st, start, &segCount, stage);
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                S.mcount[(size_t)st.parity * S.countStride + k] = segCount;
-                tallyT += segCount;
+        par = st.parity;
+        att += st.cnt;
+        uint32_t const first = P.first[st.color], base = P.base[st.color];
+        unsigned long long* const tcur = S.tmp + (size_t)par * S.nwords;
+        bool bad = false;   // (the waiter's) barrier wait ran out
+        // check, part 1 (own slots only): walls and bonds -> candidates, and their planes
+        uint32_t nc = 0, ent[kPre], to[kPre], far = 0u, go = 0u;   // far, go: bit q, candidate q
+        PlaneRef pr[kPre];
+        auto candidate = [&](bool live, uint32_t e, uint32_t& en, uint32_t& target1, PlaneRef& r) {
+            en = live ? cand[e] : 0u;
+            uint32_t const l = base + (en & kEntMask), p = pk[l], dir = en >> kSlabEntBits;
+            DirParams const D = dir_params(dtab, dir);
+            plane_ref(r, ptab, D, p, D.front, dir);
+            target1 = addr_add(p, D.ma, D.step);
+            return (code[l] & kShared) != W(0);
+        };
+        // the bond test of a candidate whose code word lives in global memory
+        auto far_ok = [&](uint32_t en) {
+            return bonds_ok<W, true>(__ldcg(rec_code<W>(S.rec, first + (en & kEntMask))), en >> kSlabEntBits, mok);
+        };
+        if (waiter) {
+            if (lane == 0) {
+                nMov = 0u;
+                bad = t > 0 && !grid_meet(gs, target, C);
+            }
+            __syncwarp();
+        } else {
+            // slots held here, and those before the group's end (the last chunk may be padded)
+            uint32_t const n = P.count[st.color], left = min(n, st.cnt - (first - st.off));
+            uint32_t const t0 = warp * 32u;   // (n is a multiple of 32: a warp's slots end together)
+            for (uint32_t k = 0; t0 + k * kThreads < n; k += kGroup) {
+                if (k != 0 && k % kDirs == 0) dirs = directions(st, k);
+                W cw[kGroup];
+                uint32_t bal[kGroup], dir[kGroup], total = 0;
+#pragma unroll
+                for (uint32_t q = 0; q < kGroup; ++q) {
+                    uint32_t const i = tid + (k + q) * kThreads;
+                    cw[q] = i < n ? code[base + i] : W(0);
+                    dir[q] = dirs & 7u;
+                    dirs >>= 3;
+                }
+#pragma unroll
+                for (uint32_t q = 0; q < kGroup; ++q) {
+                    uint32_t const i = tid + (k + q) * kThreads;
+                    bool ok = bonds_ok<W, true>(cw[q], dir[q], mok) || (cw[q] & kShared) != W(0);
+                    ok = ok && i < left;
+                    if (walled && ok) {
+                        uint2 const mw = make_uint2(dtab[dir[q] * 4u], dtab[kDirHalf + dir[q] * 4u + 3u]);   // Ma, wall
+                        ok = (pk[base + i] & mw.x) != mw.y;
+                    }
+                    bal[q] = __ballot_sync(0xffffffffu, ok);
+                    total += __popc(bal[q]);
+                }
+                uint32_t at = 0;
+                if (lane == 0) at = shared_add(&nCand, total);
+                at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+                for (uint32_t q = 0; q < kGroup; ++q) {
+                    if ((bal[q] >> lane) & 1u)
+                        cand[at + __popc(bal[q] & lanesBelow)] =
+                            (uint16_t)((tid + (k + q) * kThreads) | (dir[q] << kSlabEntBits));
+                    at += __popc(bal[q]);
+                }
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");   // the working warps
+            nc = nCand;
+#pragma unroll
+            for (int q = 0; q < kPre; ++q) {
+                // (a thread without a candidate takes entry 0's slot, and its answer is not used)
+                bool const live = q * kThreads + tid < nc;
+                if (q * kThreads + t0 < nc && candidate(live, q * kThreads + tid, ent[q], to[q], pr[q]) && live)
+                    far |= 1u << q;
             }
         }
-        if (active) att += st.cnt;
-        if constexpr (kCluster) cluster_barrier();
-        else if (!grid_barrier(gs, target, &okSm)) return;
-        uint32_t const reach = max(active ? st.cnt : 0u, st.pcnt);   // movers now, marks of t-1
-        for (uint32_t k = blockIdx.x; k < nTiles; k += gridDim.x) {
-            if (k * span >= reach) break;
-            perform_body<W, MPT, false>(S, dtab, st, k, 1u, &tallyA, pre);
+        if (__syncthreads_or(bad)) return;
+        // check, part 2: the front planes; free candidates mark their target
+        if (!waiter) {
+            uint32_t const w0 = warp * 32u;   // (the tests on it are the same for the whole warp)
+            unsigned long long hit[kPre];
+#pragma unroll
+            for (int q = 0; q < kPre; ++q)
+                if (q * kThreads + w0 < nc) hit[q] = plane_hits(pr[q], q * kThreads + tid < nc, S.lat);
+#pragma unroll
+            for (int q = 0; q < kPre; ++q)
+                if (q * kThreads + tid < nc && hit[q] == 0ull && (!((far >> q) & 1u) || far_ok(ent[q]))) {
+                    atomicOr(tcur + (to[q] >> 6), 1ull << (to[q] & 63u));
+                    go |= 1u << q;
+                }
+            for (uint32_t e0 = kPre * kThreads + w0; e0 < nc; e0 += kThreads) {
+                uint32_t en = 0, target1 = 0;
+                PlaneRef r;
+                bool ok = e0 + lane < nc;
+                bool const f = candidate(ok, e0 + lane, en, target1, r);
+                ok = ok && plane_hits(r, ok, S.lat) == 0ull && (!f || far_ok(en));
+                if (ok) atomicOr(tcur + (target1 >> 6), 1ull << (target1 & 63u));
+                uint32_t const at = append(ok, &nMov);
+                if (ok) list[at] = (uint16_t)en;
+            }
         }
-        if (t + 1 < nSteps) {
-            if constexpr (kCluster) cluster_barrier();
-            else if (!grid_barrier(gs, target, &okSm)) return;
+        __syncthreads();
+        // perform, part 1: the movers, and what they need besides the temporary lattice
+        uint32_t nm = 0, mL = 0, mTo = 0, mW0 = 0, mW1 = 0, nb[kSlots];
+        W moved = W(0), flip[kSlots];
+        unsigned long long mB0 = 0ull, mB1 = 0ull;
+        PlaneRef mr{};
+        bool mFar = false;
+        int32_t wraps = -1;   // the periodic axis the move wraps, + 4 going up
+        auto fetch = [&](uint32_t e) {
+            uint32_t const en = list[e], dir = en >> kSlabEntBits, g = first + (en & kEntMask);
+            mL = base + (en & kEntMask);
+            DirParams const D = dir_params(dtab, dir);
+            uint32_t const from = pk[mL];
+            mTo = addr_add(from, D.ma, D.step);
+            plane_ref(mr, ptab, D, mTo, D.step, dir);
+            W own = code[mL];
+            mFar = (own & kShared) != W(0);
+            if (mFar) own = __ldcg(rec_code<W>(S.rec, g));
+            W f;
+            moved = code_move(own, dir, f);
+            uint32_t const n = uint32_t(own >> CodeWord<W>::kCountShift) & 7u;
+#pragma unroll
+            for (uint32_t q = 0; q < kSlots; ++q) {
+                flip[q] = W(0);
+                if (q < n) {
+                    nb[q] = neighbour(q, g, mL);
+                    flip[q] = code_flip(f, q, (nb[q] >> kSlotShift) & 7u);
+                }
+            }
+            mW0 = from >> 6;
+            mW1 = mTo >> 6;
+            mB0 = 1ull << (from & 63u);
+            mB1 = 1ull << (mTo & 63u);
+            if (mW0 == mW1) {
+                mB0 |= mB1;
+                mB1 = 0ull;
+            }
+            wraps = (((dir & 1u) ? mTo : from) & D.ma) == 0u ? int32_t((dir >> 1) | ((dir & 1u) << 2)) : -1;
+        };
+        if (waiter) {
+            if (lane == 0) {
+                nCand = 0u;
+                bad = !grid_meet(gs, target, C);
+            }
+            __syncwarp();
+        } else {
+            if (warp * 32u < nc) {
+                static_assert(kPre == 2, "the candidates of a warp go to the list together");
+                uint32_t const b0 = __ballot_sync(0xffffffffu, go & 1u), b1 = __ballot_sync(0xffffffffu, go & 2u);
+                uint32_t at = 0;
+                if (lane == 0) at = shared_add(&nMov, (uint32_t)(__popc(b0) + __popc(b1)));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (go & 1u) list[at + __popc(b0 & lanesBelow)] = (uint16_t)ent[0];
+                if (go & 2u) list[at + __popc(b0) + __popc(b1 & lanesBelow)] = (uint16_t)ent[1];
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+            nm = nMov;
+            if (tid < nm) fetch(tid);
+            unsigned long long* const tprev = S.tmp + (size_t)(par ^ 1u) * S.nwords;
+            if (clearAll) {
+                for (uint32_t w = cw0 + tid; w < cw1; w += kThreads) tprev[w] = 0ull;
+            } else {
+                for (uint32_t e = tid; e < prevMov || e < nm; e += kThreads) {
+                    if (e < prevMov) tprev[tgt[e] >> 6] = 0ull;
+                    if (e < nm) {
+                        uint32_t const en = list[e];
+                        DirParams const D = dir_params(dtab, en >> kSlabEntBits);
+                        tgt[e] = addr_add(pk[base + (en & kEntMask)], D.ma, D.step);
+                    }
+                }
+            }
+            if (t + 1 < nSteps) dirs = directions(next, 0);
         }
+        if (__syncthreads_or(bad)) return;
+        // perform, part 2: front planes on the temporary lattice; the free movers move
+        if (!waiter) {
+            for (uint32_t e = tid; e < nm; e += kThreads) {
+                if (e != tid) fetch(e);
+                if (plane_hits(mr, true, tcur) != 0ull) continue;
+                ++nAcc;
+                atomicXor(S.lat + mW0, mB0);
+                if (mB1 != 0ull) atomicXor(S.lat + mW1, mB1);
+                pk[mL] = mTo;
+                if (mFar) *rec_code<W>(S.rec, first + (mL - base)) = moved;
+                else code[mL] = moved;
+#pragma unroll
+                for (uint32_t q = 0; q < kSlots; ++q) {
+                    if (flip[q] == W(0)) continue;
+                    if (nb[q] & kFarBit) atomicXor(rec_code<W>(S.rec, nb[q] & kSlotMask), flip[q]);
+                    else shared_xor(code + (nb[q] & kSlotMask), flip[q]);
+                }
+                if (wraps >= 0) {   // about one move in a lattice side: the image offset changes
+                    int32_t const a = wraps & 3, side = int32_t(S.mask[a] + 1u);
+                    atomicAdd((a == 0 ? S.x : (a == 1 ? S.y : S.z)) + first + (mL - base), (wraps & 4) ? side : -side);
+                }
+            }
+        }
+        nTent += nm;
+        prevMov = nm;
+        __syncthreads();   // this CTA's slots are settled for the next check's first part
     }
+    // every perform has read the last marks: zero them, and write the slots back
+    bool bad = false;
+    if (waiter && lane == 0) bad = !grid_meet(gs, target, C);
+    __syncwarp();
+    if (__syncthreads_or(bad)) return;
+    unsigned long long* const tlast = S.tmp + (size_t)par * S.nwords;
+    if (clearAll) {
+        for (uint32_t w = cw0 + tid; w < cw1; w += B) tlast[w] = 0ull;
+    } else if (!waiter) {
+        for (uint32_t e = tid; e < prevMov; e += kThreads) tlast[tgt[e] >> 6] = 0ull;
+    }
+    for (uint32_t c = 0; c < nColors; ++c)
+        for (uint32_t d = tid; d < P.count[c]; d += B) {
+            uint32_t const g = P.first[c] + d, l = P.base[c] + d;
+            if ((code[l] & kShared) != W(0)) *rec_pk<W>(S.rec, g) = pk[l];   // its code word is in place
+            else reinterpret_cast<RV*>(S.rec)[g] = make_rec(pk[l], code[l]);
+        }
+    uint32_t const asum = __reduce_add_sync(0xffffffffu, nAcc);
+    if (lane == 0 && asum) atomicAdd(&tallyA, asum);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        tally_flush(tallyT, S.stats, 1);
+    if (tid == 0) {
+        tally_flush(nTent, S.stats, 1);
         tally_flush(tallyA, S.stats, 2);
-        if (blockIdx.x == 0 && att) atomicAdd(S.stats, att);
+        if (rank == 0 && att) atomicAdd(S.stats, att);
     }
 }
 
@@ -1187,89 +1464,70 @@ cudaError_t launch_perform_bc(SysDev const& hostDesc, SysDev const* dSys, TileRe
     return cudaErrorInvalidValue;
 }
 
+bool slab_plan(uint32_t const* grpSize, uint32_t nColors, uint32_t maxc, uint32_t nwords, uint32_t codeMode,
+               uint32_t sms, SlabPlan& plan)
+{
+    plan = SlabPlan{};
+    if (codeMode == kCodeNone || nColors == 0 || nColors > kSlabColors) return false;
+    uint32_t maxCh = 1;
+    for (uint32_t c = 0; c < nColors; ++c) maxCh = std::max(maxCh, (grpSize[c] + 31u) >> 5);
+    uint32_t const C = std::min(sms, (maxCh + kSlabMinChunks - 1u) / kSlabMinChunks);
+    uint32_t cap = 0, capG = 0, n = 0;
+    for (uint32_t c = 0; c < nColors; ++c) {
+        uint32_t const own = 32u * ((((grpSize[c] + 31u) >> 5) + C - 1u) / C);
+        cap += own;
+        n += grpSize[c];
+        capG = std::max(capG, own);
+    }
+    size_t const w = codeMode == kCode64 ? 8 : 4;
+    if (capG > 1u << kSlabEntBits) return false;
+    // dense systems clear the temporary lattice whole (nwords x 8 B against two scattered accesses per mark)
+    uint32_t const clearAll = nwords <= 2u * n ? 1u : 0u;
+    size_t const smem = 768 * 8 + kDirTab * 4 + (size_t)cap * (w + 4) + (size_t)capG * (clearAll ? 4 : 8) + 512;
+    if (smem > kSlabMaxSmem) return false;
+    size_t const cache = (size_t)cap * 4 + (size_t)maxc * cap * 2;
+    bool const fits = smem + cache <= kSlabMaxSmem && cap < (1u << slab_ref_bits(codeMode == kCode64));
+    plan = SlabPlan{C, cap, capG, clearAll, fits, fits ? smem + cache : smem};
+    return true;
+}
+
 namespace {
 
-// A sweep grid of at most this many CTAs runs as one cluster (a non-portable size above 8)
-constexpr uint32_t kMaxSweepCluster = 16;
-
-template <typename W, int MPT, int kMinBlocks, int B = (int)kGridBlock>
-cudaError_t launch_sweep_bc_k(SysDev const& S, StepEntry const* dSteps, uint32_t nSteps, uint32_t maxGroup,
-                              GridSync* gs, bool allowCluster, cudaStream_t s, uint32_t* gridOut)
+template <typename W, int B, bool kCache>
+cudaError_t launch_slab_bc_w(SysDev const& S, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
+                             GridSync* gs, cudaStream_t s)
 {
-    // co-resident CTAs per SM and SM count, once per device and instantiation; which cluster sizes
-    // can run, once per device, instantiation and size
-    static thread_local int occ[64] = {}, nsm[64] = {};
-    static thread_local signed char clusterOk[64][kMaxSweepCluster + 1] = {};
+    static thread_local size_t attrSet[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (!occ[dev & 63]) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[dev & 63], k_sweep_bc<W, MPT, kMinBlocks, false, B>,
-                                                          B, 0);
+    size_t& have = attrSet[dev & 63];
+    if (plan.smem > have) {
+        e = cudaFuncSetAttribute(k_slab_bc<W, B, kCache>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
         if (e != cudaSuccess) return e;
-        e = cudaDeviceGetAttribute(&nsm[dev & 63], cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-        if (occ[dev & 63] < 1) return cudaErrorInvalidConfiguration;
+        have = plan.smem;
     }
-    uint32_t nTiles = (maxGroup + kBcTileSpan - 1) / kBcTileSpan;
-    if (nTiles == 0) nTiles = 1;
-    uint32_t const grid = std::min<uint32_t>(nTiles, (uint32_t)(occ[dev & 63] * nsm[dev & 63]));
-    if (gridOut) *gridOut = grid;
-    void* args[] = {const_cast<SysDev*>(&S), &dSteps, &nSteps, &nTiles, &gs};
-    if (allowCluster && grid <= kMaxSweepCluster) {
-        // the whole grid as one cluster, its barriers in hardware, where the device can run it
-        auto kernel = k_sweep_bc<W, MPT, kMinBlocks, true, B>;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = grid;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(B);
-        cfg.stream = s;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        signed char& ok = clusterOk[dev & 63][grid];
-        if (ok == 0) {
-            ok = -1;
-            if (grid <= 8 || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                                 cudaSuccess) {
-                int clusters = 0;
-                if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters >= 1) ok = 1;
-            }
-            cudaGetLastError();   // a size the device refuses is not an error of this call
-        }
-        if (ok == 1) return cudaLaunchKernelExC(&cfg, reinterpret_cast<void const*>(kernel), args);
-    }
-    return cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(k_sweep_bc<W, MPT, kMinBlocks, false, B>),
-                                       dim3(grid), dim3(B), args, 0, s);
-}
-
-template <typename W>
-cudaError_t launch_sweep_bc_w(SysDev const& S, StepEntry const* dSteps, uint32_t nSteps, uint32_t maxGroup,
-                              GridSync* gs, bool allowCluster, int shape, cudaStream_t s, uint32_t* gridOut)
-{
-    switch (shape) {
-    case 0: return launch_sweep_bc_k<W, kCheckMpt, 4>(S, dSteps, nSteps, maxGroup, gs, allowCluster, s, gridOut);
-    case 1: return launch_sweep_bc_k<W, kCheckMpt, 5>(S, dSteps, nSteps, maxGroup, gs, allowCluster, s, gridOut);
-    case 2: return launch_sweep_bc_k<W, kCheckMpt, 6>(S, dSteps, nSteps, maxGroup, gs, allowCluster, s, gridOut);
-    default: return cudaErrorInvalidValue;
-    }
+    uint32_t cap = plan.cap, capG = plan.capG, clearAll = plan.clearAll;
+    void* args[] = {const_cast<SysDev*>(&S), &dSteps, &nSteps, &cap, &capG, &clearAll, &gs};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(k_slab_bc<W, B, kCache>), dim3(plan.ctas), dim3(B),
+                                       args, plan.smem, s);
 }
 
 }  // namespace
 
-cudaError_t launch_sweep_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, uint32_t maxGroup,
-                            GridSync* gs, uint32_t codeMode, int shape, bool allowCluster, cudaStream_t s,
-                            uint32_t* gridOut)
+cudaError_t launch_slab_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
+                           GridSync* gs, uint32_t codeMode, cudaStream_t s)
 {
     if (nSteps == 0) return cudaSuccess;
+    if (plan.ctas == 0) return cudaErrorInvalidValue;
+    using U = unsigned long long;
+    constexpr int B32 = (int)kSlabBlock32, B64 = (int)kSlabBlock64;
     if (codeMode == kCode32)
-        return launch_sweep_bc_w<uint32_t>(hostDesc, dSteps, nSteps, maxGroup, gs, allowCluster, shape, s, gridOut);
+        return plan.cache ? launch_slab_bc_w<uint32_t, B32, true>(hostDesc, dSteps, nSteps, plan, gs, s)
+                         : launch_slab_bc_w<uint32_t, B32, false>(hostDesc, dSteps, nSteps, plan, gs, s);
     if (codeMode == kCode64)
-        return launch_sweep_bc_w<unsigned long long>(hostDesc, dSteps, nSteps, maxGroup, gs, allowCluster, shape, s,
-                                                     gridOut);
+        return plan.cache ? launch_slab_bc_w<U, B64, true>(hostDesc, dSteps, nSteps, plan, gs, s)
+                         : launch_slab_bc_w<U, B64, false>(hostDesc, dSteps, nSteps, plan, gs, s);
     return cudaErrorInvalidValue;
 }
 
