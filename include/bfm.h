@@ -37,10 +37,9 @@ extern "C" {
 #define BFM_ERR_BUSY 7             /* server: result not ready yet */
 
 /* engine paths (bfm_set_mode) */
-#define BFM_MODE_AUTO 0     /* resident for small systems (largest colour group <= 2048 and fits one CTA),
-                               cluster where a cluster's shared memory holds the system with at
-                               most 48 chunks of 32 slots per CTA and colour (one per warp where a
-                               cluster of up to 16 CTAs allows), persistent up to about
+#define BFM_MODE_AUTO 0     /* resident for small systems (largest colour group <= 1024 and fits one CTA),
+                               cluster where a cluster of up to 16 CTAs holds the system with few slots
+                               per CTA (to about 26 K monomers in a 64^3 box), persistent up to about
                                three 512-monomer tiles per SM (bond codes), else graph, with
                                persistent runs of 6 MCS or more where the slots fit the SMs */
 #define BFM_MODE_LAUNCH 1   /* check + perform launch per sub-step (the reference's structure) */

@@ -129,18 +129,19 @@ void Batch::rebuild()
     uint32_t clusterCtas = 0;
     for (uint32_t m = 0; m < M; ++m) {
         Updater* u = members_[m];
-        uint32_t const C = 1u << u->clusterLogC();
+        Updater::ClusterPlan const& cp = u->batchCluster();
+        uint32_t const C = 1u << cp.logC;
         if (residentOn_ && u->residentEligible()) {
             ResidentGroup& g = resGroup(u->codeMode());
             g.members.push_back(m);
             g.smem = std::max(g.smem, u->residentSmem());
             while (g.perThread * kResidentBlock < u->maxGroup()) g.perThread *= 2;
             wholeRun_[m] = 1;
-        } else if (clusterOn_ && u->clusterEligible() && u->clusterForBatch() && clusterCtas + C <= smCount_ / 2u) {
-            ClusterGroup& g = clusterGroup(u->codeMode(), u->clusterLogC());
+        } else if (clusterOn_ && cp.logC != 0 && clusterCtas + C <= smCount_ / 2u) {
+            ClusterGroup& g = clusterGroup(u->codeMode(), cp.logC);
             g.members.push_back(m);
-            g.smem = std::max(g.smem, u->clusterSmem());
-            g.perThread = std::max(g.perThread, u->clusterPer());
+            g.smem = std::max(g.smem, cp.smem);
+            g.perThread = std::max(g.perThread, cp.perWarp);
             clusterCtas += C;
             wholeRun_[m] = 1;
         } else {
@@ -172,7 +173,7 @@ void Batch::rebuild()
         for (uint32_t m : g.members) {
             Updater const* u = members_[m];
             smem = std::max(smem, cluster_bc_smem_bytes(u->desc().nwords, u->desc().npad, g.logC, g.perThread,
-                                                        g.codeMode));
+                                                        u->desc().maxc, g.codeMode));
         }
         g.smem = smem;
         if (!cluster_bc_runnable(g.logC, g.perThread, g.smem, g.codeMode))
@@ -447,7 +448,7 @@ std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
     bool anyResident = false, anyCluster[2] = {false, false};
     for (Updater* u : members_) {
         anyResident = anyResident || u->residentEligible();
-        bool const cl = u->clusterEligible() && u->clusterForBatch();
+        bool const cl = u->batchCluster().logC != 0;
         anyCluster[0] = anyCluster[0] || cl;
         anyCluster[1] = anyCluster[1] || (cl && !u->residentEligible());
     }

@@ -847,7 +847,7 @@ size_t Updater::residentSmem() const
 {
     uint32_t const ntab = dev_.h.nb[0] + dev_.h.nb[1] + dev_.h.nb[2];
     return codeMode_ == kCodeNone ? resident_smem_bytes(dev_.h.nwords, ntab)
-                                  : resident_bc_smem_bytes(dev_.h.nwords, npad_, maxGroup_, codeMode_);
+                                  : resident_bc_smem_bytes(dev_.h.nwords, npad_, maxGroup_, maxc_, codeMode_);
 }
 
 bool Updater::residentEligible() const
@@ -1179,40 +1179,37 @@ void Updater::enqueueResident(uint32_t nSteps)
 
 void Updater::planCluster()
 {
-    // Tiers, each the smallest cluster (2..16 CTAs) the device can run whose CTAs walk at most so
-    // many chunks of 32 slots per colour: 32 (one per warp) and then 48 (1.5 per warp), the plans
-    // BFM_MODE_AUTO takes; 64 (2 per warp), the plan a Batch takes; 256 (8 per warp),
-    // BFM_MODE_CLUSTER only. Each chunk a warp walks waits on remote shared memory, so the
-    // kernel's time per sub-step grows with the chunks per warp more than with the cluster size.
-    // Alone on a B200 (chains in 64^3 and 128^3 boxes, 11K-60K monomers, two barriers per
-    // sub-step): one chunk per warp 8.9-11.3 us per MCS, up to 48 chunks per CTA 11.6-14.7, both
-    // ahead of the persistent sweep (12.8-16.0); at 51-59 about even with it (15.3-16.9 against
-    // 15.8) while still ahead of the graph of launches (17.9-18.1), the path a Batch runs such a
-    // system on otherwise; at 8 chunks per warp 25-32.
-    constexpr uint32_t kLimits[4] = {32u, 48u, 64u, 256u};
-    constexpr uint32_t kTier[4] = {3u, 3u, 2u, 1u};
-    clusterLogC_ = 0;
-    clusterPer_ = 0;
-    clusterSmem_ = 0;
-    clusterTier_ = 0;
+    // Alone: the largest cluster the device can run (remote accesses, the barriers and each warp's chain
+    // of dependent reads bound the kernel, so more CTAs with fewer slots are faster: 64^3 chains, N = 8192,
+    // us per MCS on 2, 4, 8, 16 CTAs: 11.4, 9.1, 6.6, 5.7; the 11K network on 8 and 16: 8.8, 6.8). AUTO
+    // takes it (clusterAuto_) while a CTA's chunks of 32 slots per colour and its share of the lattice
+    // stay small; beyond, the persistent sweep, which reads the lattice from the L2, is at least as fast
+    // (us per MCS, cluster against persistent: N = 8K in 64^3 5.7 and 8.3, 16K 7.0 and 8.2, 26K 8.5 and
+    // 8.2; in 128^3, 11K (network) 6.8 and 10.7, 26K 10.5 and 8.5, 45K 15.6 and 8.5).
+    // In a Batch: the smallest cluster whose CTAs walk at most two chunks per warp and colour, the better
+    // use of the SMs when several systems share them.
+    cluster_ = batchCluster_ = ClusterPlan{};
+    clusterAuto_ = false;
     if (codeMode_ == kCodeNone) return;
     uint32_t const chunks = (maxGroup_ + 31u) / 32u;
-    for (uint32_t tier = 0; tier < 4; ++tier)
-        for (uint32_t logC = 1; logC <= 4; ++logC) {
-            uint32_t const C = 1u << logC;
-            if (dev_.h.nwords < C) continue;
-            uint32_t const perCta = (chunks + C - 1u) / C, perWarp = (perCta + 31u) / 32u;
-            if (perCta > kLimits[tier]) continue;
-            uint32_t per = 1;
-            while (per < perWarp) per *= 2;
-            size_t const smem = cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, per, codeMode_);
-            if (smem > kResidentMaxSmem || !cluster_bc_runnable(logC, per, smem, codeMode_)) continue;
-            clusterLogC_ = logC;
-            clusterPer_ = per;
-            clusterSmem_ = smem;
-            clusterTier_ = kTier[tier];
-            return;
-        }
+    auto plan = [&](uint32_t logC, uint32_t limit, ClusterPlan& out) {
+        uint32_t const C = 1u << logC, perCta = (chunks + C - 1u) / C, perWarp = (perCta + 31u) / 32u;
+        if (dev_.h.nwords < C || perCta > limit) return false;
+        uint32_t per = 1;
+        while (per < perWarp) per *= 2;
+        size_t const smem = cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, per, maxc_, codeMode_);
+        if (smem > kResidentMaxSmem || !cluster_bc_runnable(logC, per, smem, codeMode_)) return false;
+        out = ClusterPlan{logC, per, smem};
+        return true;
+    };
+    for (uint32_t logC = 4; logC >= 1; --logC)
+        if (plan(logC, 256u, cluster_)) break;
+    if (cluster_.logC) {
+        uint32_t const C = 1u << cluster_.logC;
+        clusterAuto_ = (chunks + C - 1u) / C * 128u + dev_.h.nwords / C <= 4352u;
+    }
+    for (uint32_t logC = 1; logC <= 4; ++logC)
+        if (plan(logC, 64u, batchCluster_)) break;
 }
 
 void Updater::enqueueCluster(uint32_t nSteps)
@@ -1226,8 +1223,8 @@ void Updater::enqueueCluster(uint32_t nSteps)
                    "steps H2D");
         h2dBytes_ += sizeof(StepEntry) * chunk;
         cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
-        cuda_check(launch_cluster_bc(dev_.dDesc, dev_.dList, 1, clusterLogC_, clusterPer_, dev_.dSteps, 1, chunk,
-                                     clusterSmem_, codeMode_, stream_),
+        cuda_check(launch_cluster_bc(dev_.dDesc, dev_.dList, 1, cluster_.logC, cluster_.perWarp, dev_.dSteps, 1, chunk,
+                                     cluster_.smem, codeMode_, stream_),
                    "cluster");
         ++launches_;
         done += chunk;
@@ -1243,16 +1240,14 @@ int Updater::path() const
 
 int Updater::autoMode(int32_t nMcs) const
 {
-    // One system on a B200, per MCS: the resident kernel (one SM) while the largest colour group is
-    // at most 2 x 1024 monomers (1.2K-3.3K-monomer chains 3.8-6.6 us, against 5.5-7.8 on a
-    // cluster; 6.5K-8K: 11.4-13.2 against 8.3-8.8); then a cluster of CTAs holding the system in
-    // distributed shared memory where each CTA walks at most 48 chunks of 32 slots per colour,
-    // one per warp where a cluster of up to 16 CTAs allows (planCluster); then the persistent sweep
-    // (60K monomers 8.6 us against 15.2 for the graph of launches, 131K 9.6 against 13.4, 1M 14.9
-    // against 21.7), from three tiles per SM on only for runs of at least kSlabMcs MCS; else the
-    // graph.
-    if (residentEligible() && maxGroup_ <= 2u * kResidentBlock) return kModeResident;
-    if (clusterEligible() && clusterTier_ >= 3) return kModeCluster;
+    // One system on a B200, us per MCS: the resident kernel (one SM) while the largest colour group is
+    // at most 1024 monomers (1.2K-monomer chains 3.5 against 4.6 on a cluster of 16 CTAs, 2K 4.3 against
+    // 4.6, 3.3K 5.3-5.6 against 4.8, 8K 10.6 against 5.7); then a cluster of CTAs holding the system in distributed shared
+    // memory (planCluster); then the persistent sweep (60K monomers 8.6 against 15.2 for the graph of
+    // launches, 131K 9.6 against 13.4, 1M 14.9 against 21.7), from three tiles per SM on only for runs of
+    // at least kSlabMcs MCS; else the graph.
+    if (residentEligible() && maxGroup_ <= kResidentBlock) return kModeResident;
+    if (clusterAuto_) return kModeCluster;
     if (slab_.ctas != 0) {
         uint32_t const tiles = (maxGroup_ + kBcTileSpan - 1) / kBcTileSpan;
         if (tiles <= 3u * smCount_ || nMcs >= kSlabMcs) return kModePersistent;

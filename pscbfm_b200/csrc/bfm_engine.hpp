@@ -128,14 +128,14 @@ public:
     size_t deviceBytes() const { return dev_.bytes; }
     uint32_t maxGroup() const { return maxGroup_; }
     bool residentEligible() const;
-    bool clusterEligible() const { return clusterLogC_ != 0; }
-    // the cluster-resident kernel's plan: log2 CTAs per cluster, chunks per warp, shared memory,
-    // and whether BFM_MODE_AUTO (clusterFast) or a Batch (clusterForBatch) takes it (planCluster)
-    uint32_t clusterLogC() const { return clusterLogC_; }
-    uint32_t clusterPer() const { return clusterPer_; }
-    size_t clusterSmem() const { return clusterSmem_; }
-    bool clusterFast() const { return clusterTier_ >= 3; }
-    bool clusterForBatch() const { return clusterTier_ >= 2; }
+    bool clusterEligible() const { return cluster_.logC != 0; }
+    // the cluster-resident kernel's plan: log2 CTAs per cluster (0: does not fit), chunks of 32 slots
+    // per warp and colour, dynamic shared memory per CTA (planCluster)
+    struct ClusterPlan {
+        uint32_t logC = 0, perWarp = 0;
+        size_t smem = 0;
+    };
+    ClusterPlan const& batchCluster() const { return batchCluster_; }   // inside a Batch
     int gpu() const { return gpu_; }
     void validate();                         // host-side EV and bond-set check (checkSystem)
 
@@ -266,10 +266,8 @@ private:
     bool gsPending_ = false;                   // hGs_ is being refreshed by the stream
     bool stallNext_ = false;                   // injectBarrierStall
     uint32_t smCount_ = 148;                   // SMs of the device (setGpu)
-    uint32_t clusterLogC_ = 0;                 // cluster of 2^logC CTAs holds the system (0: does not fit)
-    uint32_t clusterPer_ = 0;                  // chunks of 32 slots per warp and colour
-    size_t clusterSmem_ = 0;                   // dynamic shared memory per CTA
-    uint32_t clusterTier_ = 0;                 // 3: AUTO takes the plan, 2: a Batch does, 1: forced only
+    ClusterPlan cluster_, batchCluster_;       // alone, and inside a Batch
+    bool clusterAuto_ = false;                 // AUTO takes the cluster-resident kernel
     SlabPlan slab_;                            // the persistent sweep's plan (ctas == 0: does not fit)
     uint32_t hStepCap_ = 0;
     struct GraphExec {
@@ -366,7 +364,7 @@ public:
         residentOn_ = on;
     }
     // members too large for one CTA whose cluster plan beats the grid-phase kernels
-    // (Updater::clusterForBatch: at most two chunks of 32 slots per warp and colour) run in the
+    // (Updater::batchCluster: at most two chunks of 32 slots per warp and colour) run in the
     // cluster-resident kernel, while the batch's clusters take at most half of the SMs (the rest
     // stay with the grid-phase kernels)
     void setClusterEnabled(bool on)

@@ -406,17 +406,9 @@ template <int K>
 static cudaError_t launch_resident_k(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, StepEntry const* dSteps,
                                      uint32_t nSys, uint32_t nSteps, size_t smem, cudaStream_t s)
 {
-    // the attribute is per function and per device context; raise it to what this launch needs
-    static thread_local size_t attrSet[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    static thread_local bool done[64] = {};
+    cudaError_t const e = allow_smem(k_resident<K>, done);
     if (e != cudaSuccess) return e;
-    size_t& have = attrSet[dev & 63];
-    if (smem > have) {
-        e = cudaFuncSetAttribute(k_resident<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        have = smem;
-    }
     k_resident<K><<<nCta, kResidentBlock, smem, s>>>(dSys, dList, dSteps, nSys, nSteps);
     return cudaGetLastError();
 }

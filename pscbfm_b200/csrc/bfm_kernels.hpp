@@ -16,6 +16,19 @@ constexpr uint32_t kResidentBlock = 1024;     // threads per CTA of the resident
 // dynamic shared memory of the resident kernel: the 227 KB opt-in limit minus room for its
 // static shared memory (the copied system descriptor)
 constexpr size_t kResidentMaxSmem = 226 * 1024;
+// Raises a kernel's dynamic shared memory limit to kResidentMaxSmem, once per device and thread (done: that
+// kernel's own flags). Always to the same value: the limit belongs to the function, not to the
+// launch, so a thread that set what its own launch needs would lower it under another thread's.
+template <typename F>
+cudaError_t allow_smem(F* kernel, bool (&done)[64])
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || done[dev & 63]) return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentMaxSmem);
+    done[dev & 63] = e == cudaSuccess;
+    return e;
+}
 constexpr int32_t kPadCoord = INT32_MIN;      // x of an unused (padding) slot
 
 // One CTA of a grid-phase launch: system index and first in-colour index it covers.
@@ -100,7 +113,7 @@ constexpr uint32_t kSlabEntBits = 13;         // list entries: a slot's index in
 // bits of a local index in a 16-bit neighbour reference, below the reverse slot (0-2, or 0-5 with 64-bit codes)
 __host__ __device__ constexpr uint32_t slab_ref_bits(bool code64) { return code64 ? 13u : 14u; }
 constexpr uint32_t kSlabMinChunks = 8;       // chunks of 32 slots per CTA and colour, before more CTAs join
-constexpr size_t kSlabMaxSmem = 226 * 1024;
+constexpr size_t kSlabMaxSmem = kResidentMaxSmem;
 struct SlabPlan {
     uint32_t ctas = 0;         // 0: the system does not fit
     uint32_t cap = 0, capG = 0;   // slots a CTA holds in all and of its largest colour group
@@ -112,13 +125,15 @@ bool slab_plan(uint32_t const* grpSize, uint32_t nColors, uint32_t maxc, uint32_
                uint32_t sms, SlabPlan& plan);
 cudaError_t launch_slab_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
                            GridSync* gs, uint32_t codeMode, cudaStream_t s);
-size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t codeMode);
+// Dynamic shared memory of the bond-code resident kernel, with the neighbour references where they fit too.
+size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t maxc, uint32_t codeMode);
 // Cluster-resident sweep (bond codes): one cluster of 2^logC CTAs of kResidentBlock threads per
 // system of dList[0..nClusters) (logC 1..4), state in the cluster's shared memory for nSteps
 // sub-steps whose entries are dSteps[t * stride + system]; perThread (1, 2, 4, 8) chunks of 32
 // slots per warp and colour. cluster_bc_runnable: whether the device can run that configuration
 // (kernel attributes set, cudaOccupancyMaxActiveClusters >= 1).
-size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t perThread, uint32_t codeMode);
+size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t perThread, uint32_t maxc,
+                             uint32_t codeMode);
 bool cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode);
 cudaError_t launch_cluster_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
                               uint32_t perThread, StepEntry const* dSteps, uint32_t stride, uint32_t nSteps,

@@ -17,9 +17,9 @@
 // Persistent (k_slab_bc): a whole run of sub-steps in one cooperative launch with time-bounded grid
 // barriers; the lattices in global memory, each CTA's share of the slots in its shared memory.
 //
-// Resident (k_resident_bc): one CTA owns a small system for a chunk of sub-steps; lattice, one
-// temporary lattice, pk and bond codes in shared memory; the check appends tentative movers to a
-// shared list (warp ballot + one atomic per warp), so the perform runs with full warps.
+// Resident (k_resident_bc): one CTA owns a small system for a chunk of sub-steps; lattice, temporary
+// lattices, addresses, bond codes and neighbour references in shared memory; tentative movers go to
+// a shared list (warp ballot + one atomic per warp), so the perform runs with full warps.
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -58,6 +58,44 @@ __device__ __forceinline__ bool bonds_ok(W code, uint32_t dir, uint8_t const* ok
     return (m >> dir) & 1u;
 }
 
+// Adds v to a counter in shared memory and returns its old value, as one instruction: written with
+// atomicAdd, the compiler gathers the adds of a warp first, 20 instructions for the one lane that adds.
+__device__ __forceinline__ uint32_t shared_add(uint32_t* p, uint32_t v)
+{
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v)
+                 : "memory");
+    return old;
+}
+__device__ __forceinline__ void shared_xor(uint32_t* p, uint32_t v) { atomicXor(p, v); }
+// (a 64-bit exclusive or as two on the halves: shared memory has no native 64-bit one)
+__device__ __forceinline__ void shared_xor(unsigned long long* p, unsigned long long v)
+{
+    unsigned int* const h = reinterpret_cast<unsigned int*>(p);
+    if ((unsigned int)v) atomicXor(h, (unsigned int)v);
+    if ((unsigned int)(v >> 32)) atomicXor(h + 1, (unsigned int)(v >> 32));
+}
+
+// The words a front plane touches and their masks, prepared ahead of the reads (a word that is not
+// touched has an empty mask; reads of it are left out).
+struct PlaneRef {
+    uint32_t w[4];
+    unsigned long long m[4];
+};
+__device__ __forceinline__ void plane_ref(PlaneRef& r, unsigned long long const* ptab, DirParams const& D,
+                                          uint32_t base, uint32_t da, uint32_t dir)
+{
+    uint32_t ti, touch;
+    front_plane_words(r.w, ti, touch, D, base, da, dir);
+    ulonglong2 const m01 = *reinterpret_cast<ulonglong2 const*>(ptab + ti);
+    ulonglong2 const m23 = *reinterpret_cast<ulonglong2 const*>(ptab + ti + 2);
+    r.m[0] = m01.x;
+    r.m[1] = m01.y;
+    r.m[2] = m23.x;
+    r.m[3] = m23.y;
+}
 // Mover lists: the check of sub-step t appends each tentative mover of tile k (kBcTileSpan
 // in-colour indices) to segment k of list[parity] (entry: slot g in bits 0-26, direction in
 // 27-29), the lattice address of its target (the temporary-lattice cell it marked) to the same
@@ -511,44 +549,6 @@ __device__ __forceinline__ uint32_t slab_local(SlabPart const& P, uint32_t nColo
     return kNoMark;
 }
 
-// Adds v to a counter in shared memory and returns its old value, as one instruction: written with
-// atomicAdd, the compiler gathers the adds of a warp first, 20 instructions for the one lane that adds.
-__device__ __forceinline__ uint32_t shared_add(uint32_t* p, uint32_t v)
-{
-    uint32_t old;
-    asm volatile("atom.shared.add.u32 %0, [%1], %2;"
-                 : "=r"(old)
-                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v)
-                 : "memory");
-    return old;
-}
-__device__ __forceinline__ void shared_xor(uint32_t* p, uint32_t v) { atomicXor(p, v); }
-// (a 64-bit exclusive or as two on the halves: shared memory has no native 64-bit one)
-__device__ __forceinline__ void shared_xor(unsigned long long* p, unsigned long long v)
-{
-    unsigned int* const h = reinterpret_cast<unsigned int*>(p);
-    if ((unsigned int)v) atomicXor(h, (unsigned int)v);
-    if ((unsigned int)(v >> 32)) atomicXor(h + 1, (unsigned int)(v >> 32));
-}
-
-// The words a front plane touches and their masks, prepared ahead of the reads (a word that is not
-// touched has an empty mask; reads of it are left out).
-struct PlaneRef {
-    uint32_t w[4];
-    unsigned long long m[4];
-};
-__device__ __forceinline__ void plane_ref(PlaneRef& r, unsigned long long const* ptab, DirParams const& D,
-                                          uint32_t base, uint32_t da, uint32_t dir)
-{
-    uint32_t ti, touch;
-    front_plane_words(r.w, ti, touch, D, base, da, dir);
-    ulonglong2 const m01 = *reinterpret_cast<ulonglong2 const*>(ptab + ti);
-    ulonglong2 const m23 = *reinterpret_cast<ulonglong2 const*>(ptab + ti + 2);
-    r.m[0] = m01.x;
-    r.m[1] = m01.y;
-    r.m[2] = m23.x;
-    r.m[3] = m23.y;
-}
 // An 8-byte load where `on`, else 0, as one predicated instruction: the loads of a plane go out back
 // to back. Coherent with other CTAs' writes after a grid barrier (its acquire drops the L1's lines),
 // cached in the L1 within a phase.
@@ -941,191 +941,370 @@ __global__ void __launch_bounds__(B, 1)
 
 // ---------------------------------------------------------------------------------- resident
 
+// Half bricks: the kernels that keep the lattices in shared memory read them as 32-bit words of
+// 4 x 4 x 2 cells (word a >> 5 of lattice address a; the z axis's in-word coordinate has one bit). A
+// front plane still touches at most 2 x 2 of them, with half the bytes of the lattice and of the
+// masks to read: shared-memory wavefronts (bank conflicts of random words) bound those kernels, and a
+// plane on 64-bit words took 52 of a warp's 80 per check, on half bricks 25. Marks and flips
+// are 32-bit atomics (shared memory has no native 64-bit ones).
+constexpr uint32_t kHalfPlanes = 3 * 32;   // table entries of four masks: axis, in-word position
+
+// Entry e of the mask table: for the axis e >> 5 and the first cell's position e & 31 in its word, the
+// plane's cells in the word itself and its neighbours along v, u, and both (front_plane_words' order).
+__device__ __forceinline__ uint4 half_plane_masks(uint32_t e)
+{
+    uint32_t const a = e >> 5, u = a == 0 ? 1u : 0u, v = a == 2 ? 1u : 2u;
+    uint32_t m[4] = {0u, 0u, 0u, 0u};
+    for (uint32_t k = 0; k < 9; ++k) {
+        uint32_t const c[3] = {e & 3u, (e >> 2) & 3u, (e >> 4) & 1u}, size[3] = {4u, 4u, 2u};
+        uint32_t w = 0, bit = 0;
+        for (uint32_t ax = 0; ax < 3; ++ax) {
+            uint32_t const at = c[ax] + (ax == u ? k % 3u : 0u) + (ax == v ? k / 3u : 0u);
+            if (at >= size[ax]) w |= ax == u ? 2u : 1u;
+            bit |= (at % size[ax]) << (2u * ax);
+        }
+        for (uint32_t j = 0; j < 4; ++j)
+            if (w == j) m[j] |= 1u << bit;
+    }
+    return make_uint4(m[0], m[1], m[2], m[3]);
+}
+
+// The tables of the kernels with half bricks, by the CTA's threads: masks, and the direction table
+// with the u and v masks of a half-brick index in place of those of a brick index.
+__device__ __forceinline__ void half_tables(SysDev const& S, uint4* masks, uint32_t* dtab)
+{
+    for (uint32_t e = threadIdx.x; e < kHalfPlanes; e += blockDim.x) masks[e] = half_plane_masks(e);
+    if (threadIdx.x < kDirTab) {
+        uint32_t const w = threadIdx.x, d = w % 24u / 4u, k = w % 4u;
+        bool const uv = w >= kDirHalf && (k == 1u || k == 2u);
+        dtab[w] = uv ? S.dirTab[d * 4u + k + 1u] >> 5 : S.dirTab[w];
+    }
+}
+
+// The set cells of the front plane of a move along dir in lattice L of half bricks (front_plane's
+// arguments): all four words are read, each is a word of the lattice.
+struct HalfPlane {
+    uint32_t w[4];
+    uint4 m;
+};
+__device__ __forceinline__ void half_plane(HalfPlane& r, uint4 const* masks, DirParams const& D, uint32_t base,
+                                           uint32_t da, uint32_t dir)
+{
+    uint32_t const f = ((((base | ~D.ma) + da) & D.ma) | (((base | ~D.mu) + D.mu) & D.mu)) |
+                       (((base | ~D.mv) + D.mv) & D.mv);
+    r.w[0] = f >> 5;
+    r.w[1] = addr_add(r.w[0], D.bv, 1u);
+    r.w[2] = addr_add(r.w[0], D.bu, 1u);
+    r.w[3] = addr_add(r.w[2], D.bv, 1u);
+    r.m = masks[(dir >> 1) * 32u + (f & 31u)];
+}
+__device__ __forceinline__ uint32_t half_hits(HalfPlane const& r, uint32_t const* L)
+{
+    return (L[r.w[0]] & r.m.x) | (L[r.w[1]] & r.m.y) | (L[r.w[2]] & r.m.z) | (L[r.w[3]] & r.m.w);
+}
+
+// Shared memory of k_resident_bc (resident_bc_smem_bytes); nb: neighbour references kept here (0: they
+// stay in global memory).
+constexpr uint32_t kStepBlock = 16;   // step entries staged in shared memory at a time (static shared memory stays below 1 KB)
+__host__ __device__ __forceinline__ size_t resident_layout(uint32_t nwords, uint32_t npad, uint32_t maxGroup,
+                                                           uint32_t codeBytes, uint32_t nb)
+{
+    return kHalfPlanes * 16 + kDirTab * 4 + (size_t)nwords * 3 * 8 + (size_t)npad * (codeBytes + 4) + 512 +
+           (size_t)((maxGroup + 1u) & ~1u) * 4 + (size_t)nb * npad * 2;
+}
+
 // The whole system in one CTA's shared memory for nSteps sub-steps: lattice, one temporary
-// lattice per sub-step parity (the previous one cleared while the next check runs), packed
-// coordinates, bond codes and the mover list; one CTA per system of sysList, entries of sub-step t
-// at steps[t * nSys + system]. Two CTA barriers per sub-step (after the check, after the perform).
-template <typename W, int K>
+// lattice per sub-step parity (the previous one cleared while the next check runs), lattice
+// addresses, bond codes, neighbour references (where they fit: 2 bytes each) and lists; one CTA per
+// system of sysList, entries of sub-step t at steps[t * nSys + system].
+// The bond test and the front plane are evaluated side by side, without branches, so that their
+// chains of dependent reads overlap; the directions of sub-step t + 1 are drawn during the perform
+// of t, whose movers take the threads from the last one down, where a small system has no slots.
+// Two forms of the check:
+//   kDirect: each slot's bonds and plane by its own thread, two CTA barriers per sub-step (groups of at
+//   most 1024 slots, and those too large for 16-bit list entries);
+//   else the slots that pass the wall and bond tests (a third of a melt's) are listed first, so the
+//   planes run on full warps: three barriers, and less work from 2 slots per thread on.
+// Bound by shared-memory wavefronts (bank conflicts), the integer pipe and the chain of dependent reads
+// of each phase. us per MCS: 1.2K-monomer chains 3.9 -> 3.5, 2K 5.0 -> 4.3, 3.3K 6.3 -> 5.3, 8K 13.0 -> 10.6.
+template <typename W, bool kDirect>
 __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const* __restrict__ sysv,
                                                                     uint32_t const* __restrict__ sysList,
                                                                     StepEntry const* __restrict__ steps,
                                                                     uint32_t nSys, uint32_t nSteps)
 {
+    constexpr uint32_t kSlots = CodeWord<W>::kSlots, B = kResidentBlock, kDirs = 10;
+    constexpr uint32_t kRefBits = slab_ref_bits(sizeof(W) == 8), kRefMask = (1u << kRefBits) - 1u;
     __shared__ SysDev S;
-    __shared__ uint32_t listCount[2];   // per sub-step parity
+    __shared__ __align__(16) StepEntry stepSm[kStepBlock];
+    __shared__ uint32_t nMov[2], nCand, maxGroup;   // nMov: per sub-step parity
     extern __shared__ unsigned long long smem[];
     uint32_t const sysId = sysList[blockIdx.x];
     copy_desc(S, sysv + sysId);
     __syncthreads();
-    uint32_t const nw = S.nwords, np = S.npad;
-    uint32_t const B = blockDim.x, tid = threadIdx.x, lane = tid & 31u;
-    unsigned long long* const ptab = smem;                  // 768 plane masks
-    uint32_t* const dtab = reinterpret_cast<uint32_t*>(smem + 768);   // kDirTab words (16-byte aligned)
-    unsigned long long* const lat = smem + 768 + kDirTab / 2;
-    unsigned long long* const tmp = lat + nw;               // 2 x nw words (per sub-step parity)
-    W* const code = reinterpret_cast<W*>(tmp + 2u * nw);
+    uint32_t const nw = S.nwords, np = S.npad, maxc = S.maxc;
+    uint32_t const tid = threadIdx.x, lane = tid & 31u;
+    if (tid == 0) {
+        uint32_t m = 0;
+        for (uint32_t c = 0; c < S.nColors; ++c) m = max(m, S.grp[2 * c + 1]);
+        maxGroup = m;
+        nMov[0] = nMov[1] = nCand = 0u;
+    }
+    __syncthreads();
+    uint4* const masks = reinterpret_cast<uint4*>(smem);    // kHalfPlanes entries
+    uint32_t* const dtab = reinterpret_cast<uint32_t*>(masks + kHalfPlanes);   // kDirTab words (16-byte aligned)
+    uint32_t* const lat = dtab + kDirTab;                   // 2 nw half bricks
+    uint32_t* const tmp = lat + 2u * nw;                    // twice 2 nw half bricks (per sub-step parity)
+    W* const code = reinterpret_cast<W*>(tmp + 4u * nw);
     uint32_t* const pk = reinterpret_cast<uint32_t*>(code + np);
     uint8_t* const mok = reinterpret_cast<uint8_t*>(pk + np);   // 512 move-table bytes
+    uint32_t const mg = (maxGroup + 1u) & ~1u;
+    // kDirect: movers, slot | dir << 28; else candidates and movers, index in the group | dir << 13
     uint32_t* const list = reinterpret_cast<uint32_t*>(mok + 512);
-    for (uint32_t w = tid; w < 768; w += B) ptab[w] = S.planeTab[w];
-    if (tid < kDirTab) dtab[tid] = S.dirTab[tid];
+    uint16_t* const cand = reinterpret_cast<uint16_t*>(list);
+    uint16_t* const movers = cand + mg;
+    uint16_t* const refs = movers + mg;                     // maxc x np references, where they fit
+    uint32_t dynBytes;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynBytes));
+    bool const cached = np < (1u << kRefBits) && resident_layout(nw, np, maxGroup, sizeof(W), maxc) <= dynBytes;
+    half_tables(S, masks, dtab);
     for (uint32_t w = tid; w < 512; w += B) mok[w] = S.moveOk[w];
-    for (uint32_t w = tid; w < nw; w += B) {
-        lat[w] = S.lat[w];
-        tmp[w] = 0ull;
-        tmp[nw + w] = 0ull;
+    for (uint32_t w = tid; w < 2u * nw; w += B) {
+        lat[w] = reinterpret_cast<uint32_t const*>(S.lat)[w];
+        tmp[w] = 0u;
+        tmp[2u * nw + w] = 0u;
     }
     for (uint32_t g = tid; g < np; g += B) {
         code[g] = *rec_code<W>(S.rec, g);
         pk[g] = *rec_pk<W>(S.rec, g);
     }
-    if (tid < 2) listCount[tid] = 0;
-    uint32_t nTent = 0, nAcc = 0;
+    if (cached)
+        for (uint32_t g = tid; g < maxc * np; g += B) {   // reference q of slot g at q np + g, as in nbrr
+            uint32_t const r = S.nbrr[g];
+            refs[g] = (uint16_t)((r & kSlotMask) | ((r >> kSlotShift) << kRefBits));
+        }
+    uint32_t nAcc = 0, nTent = 0;
     unsigned long long nAtt = 0;
-    StepEntry next = nSteps ? steps[sysId] : StepEntry{};
-    __syncthreads();
+    bool const walled = S.walls != 0u;
 
-    uint32_t par = 0;
+    uint32_t const lanesBelow = (1u << lane) - 1u;
+    auto append = [&](bool on, uint32_t* count) {
+        uint32_t const bal = __ballot_sync(0xffffffffu, on);
+        uint32_t at = 0;
+        if (lane == 0) at = shared_add(count, (uint32_t)__popc(bal));
+        return __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanesBelow);
+    };
+    // directions of in-colour indices tid + k B, k from k0, 3 bits each
+    auto directions = [&](StepEntry const& e, uint32_t k0) {
+        uint32_t d = 0;
+        for (uint32_t k = 0, i = tid + k0 * B; k < kDirs && i < e.cnt; ++k, i += B) d |= move_dir(i, e.seed) << (3u * k);
+        return d;
+    };
+    // the check of slot l: the move's target, and whether the front plane is free and, if asked, the
+    // wall and bond tests pass, in one straight line of code
+    auto check = [&](uint32_t l, uint32_t dir, bool tests, uint32_t& to) {
+        uint32_t const p = pk[l];
+        DirParams const D = dir_params(dtab, dir);
+        bool const ok = !tests || (bonds_ok<W, true>(code[l], dir, mok) & ((p & D.ma) != D.wall));
+        HalfPlane pl;
+        half_plane(pl, masks, D, p, D.front, dir);
+        to = addr_add(p, D.ma, D.step);
+        return ok & (half_hits(pl, lat) == 0u);
+    };
+    uint32_t par = 0, dirs = 0;
+    bool drawn = false;   // dirs belong to the next active sub-step
     for (uint32_t t = 0; t < nSteps; ++t) {
-        StepEntry const st = next;
-        if (t + 1 < nSteps) next = steps[(size_t)(t + 1) * nSys + sysId];   // prefetch
+        if (t % kStepBlock == 0) {   // (the last barrier of the sub-step before ended the reads of the old ones)
+            uint32_t const n = min(kStepBlock, nSteps - t);
+            for (uint32_t k = tid; k < 2u * n; k += B)
+                reinterpret_cast<uint4*>(stepSm)[k] =
+                    reinterpret_cast<uint4 const*>(steps + (size_t)(t + k / 2u) * nSys + sysId)[k & 1u];
+            __syncthreads();   // (the first also publishes the state loaded above)
+            drawn = false;
+        }
+        uint32_t const ts = t % kStepBlock;
+        StepEntry const st = stepSm[ts];
         if (st.color == kNoColor) continue;
+        if (!drawn) dirs = directions(st, 0);
         nAtt += st.cnt;
-        unsigned long long* const tmpCur = tmp + par * nw;
-        // the previous sub-step's marks and list count: read by no thread after the barrier that
-        // ended that sub-step, written by none before the barrier that ends this one
-        for (uint32_t w = tid; w < nw; w += B) tmp[(par ^ 1u) * nw + w] = 0ull;
-        if (tid == 0) listCount[par ^ 1u] = 0;
-        // check: tentative movers -> tmp bit + shared list (one atomic per warp)
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            uint32_t const i = tid + (uint32_t)k * B;
-            bool go = false;
-            uint32_t entry = 0;
-            if (i < st.cnt) {
-                uint32_t const g = st.off + i;
-                uint32_t const dir = move_dir(i, st.seed);
-                uint32_t const p = pk[g];
-                DirParams const D = dir_params(dtab, dir);
-                if ((p & D.ma) != D.wall && bonds_ok<W, true>(code[g], dir, mok)) {
-                    Plane pl;
-                    front_plane<true>(pl, ptab, D, p, D.front, dir);
-                    unsigned long long hit = 0ull;
-#pragma unroll
-                    for (int r = 0; r < 4; ++r)
-                        if (pl.m[r]) hit |= lat[pl.w[r]] & pl.m[r];   // masks from shared memory
-                    if (hit == 0ull) {
-                        uint32_t const to = addr_add(p, D.ma, D.step);
-                        atomicOr(tmpCur + (to >> 6), 1ull << (to & 63u));
-                        go = true;
-                        entry = g | (dir << kSlotShift);
-                    }
-                }
+        uint32_t* const marks = tmp + par * 2u * nw;
+        uint32_t const cnt = st.cnt, off = st.off;
+        if (kDirect) {
+            for (uint32_t k = 0, i0 = tid & ~31u; i0 < cnt; ++k, i0 += B) {   // warp-uniform
+                if (k != 0 && k % kDirs == 0) dirs = directions(st, k);
+                uint32_t const i = i0 + lane, dir = dirs & 7u, l = off + min(i, cnt - 1u);
+                dirs >>= 3;
+                uint32_t to;
+                bool const go = check(l, dir, true, to) & (i < cnt);
+                if (go) atomicOr(marks + (to >> 5), 1u << (to & 31u));
+                uint32_t const at = append(go, &nMov[par]);
+                if (go) list[at] = l | (dir << kSlotShift);
             }
-            uint32_t const bal = __ballot_sync(0xffffffffu, go);
-            if (bal) {
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(&listCount[par], (uint32_t)__popc(bal));
-                base = __shfl_sync(0xffffffffu, base, 0);
-                if (go) list[base + __popc(bal & ((1u << lane) - 1u))] = entry;
-                nTent += lane == 0 ? (uint32_t)__popc(bal) : 0u;
+        } else {
+            for (uint32_t k = 0, i0 = tid & ~31u; i0 < cnt; ++k, i0 += B) {
+                if (k != 0 && k % kDirs == 0) dirs = directions(st, k);
+                uint32_t const i = i0 + lane, dir = dirs & 7u, l = off + min(i, cnt - 1u);
+                dirs >>= 3;
+                bool ok = bonds_ok<W, true>(code[l], dir, mok) & (i < cnt);
+                if (walled) {
+                    uint2 const mw = make_uint2(dtab[dir * 4u], dtab[kDirHalf + dir * 4u + 3u]);   // Ma, wall
+                    ok = ok & ((pk[l] & mw.x) != mw.y);
+                }
+                uint32_t const at = append(ok, &nCand);
+                if (ok) cand[at] = (uint16_t)(i | (dir << kSlabEntBits));
+            }
+        }
+        // the previous sub-step's marks and mover count: read by no thread after the barrier that
+        // ended that sub-step, written by none before the barrier that ends this check
+        for (uint32_t w = B - 1u - tid; w < nw; w += B)
+            reinterpret_cast<unsigned long long*>(tmp + (par ^ 1u) * 2u * nw)[w] = 0ull;
+        if (tid == 0) nMov[par ^ 1u] = 0u;
+        if (!kDirect) {
+            __syncthreads();
+            uint32_t const nc = nCand;
+            for (uint32_t e0 = tid & ~31u; e0 < nc; e0 += B) {
+                bool const live = e0 + lane < nc;
+                uint32_t const en = live ? cand[e0 + lane] : 0u;
+                uint32_t to;
+                bool const go = check(off + (en & ((1u << kSlabEntBits) - 1u)), en >> kSlabEntBits, false, to) & live;
+                if (go) atomicOr(marks + (to >> 5), 1u << (to & 31u));
+                uint32_t const at = append(go, &nMov[par]);
+                if (go) movers[at] = (uint16_t)en;
             }
         }
         __syncthreads();
-        // perform over the compact list
-        uint32_t const nList = listCount[par];
-        for (uint32_t e = tid; e < nList; e += B) {
-            uint32_t const g = list[e] & kSlotMask, dir = list[e] >> kSlotShift;
-            uint32_t const p = pk[g];
-            // the neighbour references live in global memory: ask for them before the test, so
-            // their latency overlaps it
-            uint32_t nb[CodeWord<W>::kSlots];
-#pragma unroll
-            for (uint32_t q = 0; q < CodeWord<W>::kSlots; ++q)
-                nb[q] = q < S.maxc ? __ldg(S.nbrr + (size_t)q * np + g) : 0u;
-            Plane pl;
-            DirParams const D = dir_params(dtab, dir);
-            front_plane<true>(pl, ptab, D, p, D.front, dir);
-            unsigned long long hit = 0ull;
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-                if (pl.m[r]) hit |= tmpCur[pl.w[r]] & pl.m[r];
-            if (hit != 0ull) continue;
-            uint32_t const a = dir >> 1;
-            int32_t const s = (dir & 1u) ? 1 : -1;
-            uint32_t const p1 = addr_add(p, D.ma, D.step);
-            uint32_t const w0 = p >> 6, w1 = p1 >> 6;
-            if (w0 == w1) {
-                atomicXor(lat + w0, (1ull << (p & 63u)) | (1ull << (p1 & 63u)));
+        // perform over the movers
+        uint32_t const n = nMov[par];
+        if (!kDirect && tid == 0) nCand = 0u;
+        for (uint32_t e = B - 1u - tid; e < n; e += B) {
+            uint32_t l, dir;
+            if (kDirect) {
+                l = list[e] & kSlotMask;
+                dir = list[e] >> kSlotShift;
             } else {
-                atomicXor(lat + w0, 1ull << (p & 63u));
-                atomicXor(lat + w1, 1ull << (p1 & 63u));
+                l = off + (movers[e] & ((1u << kSlabEntBits) - 1u));
+                dir = movers[e] >> kSlabEntBits;
             }
-            pk[g] = p1;
-            image_step(S, g, a, s, p, p1, D.ma);
-            W const own = code[g];
-            code[g] = code_shift(own, a, -s);
-            uint32_t const n = uint32_t(own >> CodeWord<W>::kCountShift) & 7u;
+            uint32_t const p = pk[l];
+            W const own = code[l];
+            uint32_t const nn = uint32_t(own >> CodeWord<W>::kCountShift) & 7u;
+            uint32_t nb[kSlots];
 #pragma unroll
-            for (uint32_t q = 0; q < CodeWord<W>::kSlots; ++q) {
-                if (q < n) {
-                    uint32_t const ent = nb[q];
-                    uint32_t const c = (0u - (uint32_t(own >> (9u * q + 3u * a)) & 7u)) & 7u;
-                    uint32_t const nc = uint32_t(int32_t(c) + s) & 7u;
-                    atomicXor(code + (ent & kSlotMask), W(c ^ nc) << (9u * (ent >> kSlotShift) + 3u * a));
+            for (uint32_t q = 0; q < kSlots; ++q) {
+                nb[q] = 0u;
+                if (q < maxc) {
+                    if (cached) {
+                        uint32_t const r = refs[q * np + l];
+                        nb[q] = (r & kRefMask) | ((r >> kRefBits) << kSlotShift);
+                    } else if (q < nn) {
+                        nb[q] = __ldg(S.nbrr + (size_t)q * np + l);
+                    }
                 }
             }
+            DirParams const D = dir_params(dtab, dir);
+            uint32_t const to = addr_add(p, D.ma, D.step);
+            HalfPlane pl;
+            half_plane(pl, masks, D, to, D.step, dir);
+            W flip;
+            W const moved = code_move(own, dir, flip);
+            if (half_hits(pl, marks) != 0u) continue;
+            atomicXor(lat + (p >> 5), 1u << (p & 31u));
+            atomicXor(lat + (to >> 5), 1u << (to & 31u));
+            pk[l] = to;
+            code[l] = moved;
+#pragma unroll
+            for (uint32_t q = 0; q < kSlots; ++q) {
+                W const f = code_flip(flip, q, nb[q] >> kSlotShift);
+                if (f != W(0)) shared_xor(code + (nb[q] & kSlotMask), f);   // (f is 0 past the last bond)
+            }
+            image_step(S, l, dir >> 1, (dir & 1u) ? 1 : -1, p, to, D.ma);
             ++nAcc;
         }
+        nTent += n;
+        drawn = t + 1 < nSteps && ts + 1u < kStepBlock && stepSm[ts + 1u].color != kNoColor;
+        if (drawn) dirs = directions(stepSm[ts + 1u], 0);
         __syncthreads();   // every perform is done: the lattice is settled for the next check
         par ^= 1u;
     }
-    for (uint32_t w = tid; w < nw; w += B) S.lat[w] = lat[w];
+    __syncthreads();   // (a run that ended with idle sub-steps)
+    for (uint32_t w = tid; w < 2u * nw; w += B) reinterpret_cast<uint32_t*>(S.lat)[w] = lat[w];
     for (uint32_t g = tid; g < np; g += B) {
         *rec_code<W>(S.rec, g) = code[g];
         *rec_pk<W>(S.rec, g) = pk[g];
     }
-    uint32_t const tsum = __reduce_add_sync(0xffffffffu, nTent);
     uint32_t const asum = __reduce_add_sync(0xffffffffu, nAcc);
-    if (lane == 0) {
-        tally_flush(tsum, S.stats, 1);
-        tally_flush(asum, S.stats, 2);
+    if (lane == 0) tally_flush(asum, S.stats, 2);
+    if (tid == 0) {
+        tally_flush(nTent, S.stats, 1);
+        if (nAtt) atomicAdd(S.stats + (blockIdx.x % kStatSlots), nAtt);
     }
-    if (tid == 0 && nAtt) atomicAdd(S.stats + (blockIdx.x % kStatSlots), nAtt);
 }
 
 // ---------------------------------------------------------------------------------- cluster-resident
 
-// A 64-bit OR / XOR into distributed shared memory as 32-bit atomics on the two halves (the bits
-// are independent, so the result is the same). Measured on B200: 64-bit bitwise atomics on
-// another CTA's shared memory (through map_shared_rank, or atom.shared::cluster.*.b64) lose updates
-// when several CTAs hit the same word, while 32-bit ones do not.
-__device__ __forceinline__ void dsmem_or64(unsigned long long* p, unsigned long long v)
+// Distributed shared memory: the address of p (this CTA's shared memory) in the CTA of the given
+// rank, a read, and atomics without result where `on`. All are 32 bits wide: 64-bit bitwise atomics on
+// another CTA's shared memory (through map_shared_rank, or atom.shared::cluster.*.b64) were measured
+// on a B200 to lose updates when several CTAs hit the same word, 32-bit ones are exact.
+__device__ __forceinline__ uint32_t cluster_map(uint32_t sharedAddr, uint32_t rank)
 {
-    unsigned int* const h = reinterpret_cast<unsigned int*>(p);
-    if ((unsigned int)v) atomicOr(h, (unsigned int)v);
-    if ((unsigned int)(v >> 32)) atomicOr(h + 1, (unsigned int)(v >> 32));
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(sharedAddr), "r"(rank));
+    return a;
 }
-__device__ __forceinline__ void dsmem_xor64(unsigned long long* p, unsigned long long v)
+__device__ __forceinline__ uint32_t cluster_load(uint32_t a, bool on)
 {
-    unsigned int* const h = reinterpret_cast<unsigned int*>(p);
-    if ((unsigned int)v) atomicXor(h, (unsigned int)v);
-    if ((unsigned int)(v >> 32)) atomicXor(h + 1, (unsigned int)(v >> 32));
+    uint32_t v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.u32 %0, 0;\n\t@q ld.shared::cluster.u32 %0, [%1];\n\t}"
+                 : "=r"(v) : "r"(a), "r"((uint32_t)on) : "memory");
+    return v;
 }
-__device__ __forceinline__ void dsmem_xor(unsigned int* p, unsigned int v) { atomicXor(p, v); }
-__device__ __forceinline__ void dsmem_xor(unsigned long long* p, unsigned long long v) { dsmem_xor64(p, v); }
+__device__ __forceinline__ void cluster_or(uint32_t a, uint32_t v, bool on)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;\n\t}"
+                 :: "r"(a), "r"(v), "r"((uint32_t)on) : "memory");
+}
+__device__ __forceinline__ void cluster_xor(uint32_t a, uint32_t v, bool on)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.relaxed.cluster.shared::cluster.xor.b32 [%0], %1;\n\t}"
+                 :: "r"(a), "r"(v), "r"((uint32_t)on) : "memory");
+}
+__device__ __forceinline__ void cluster_xor(uint32_t a, unsigned long long v, bool on)
+{
+    cluster_xor(a, (uint32_t)v, on && (uint32_t)v != 0u);
+    cluster_xor(a + 4u, (uint32_t)(v >> 32), on && (v >> 32) != 0ull);
+}
+// The two halves of a cluster barrier: after the first every earlier access of the thread is on its
+// way, after the second those of all threads of the cluster are in place.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Shared memory of k_cluster_bc per CTA (cluster_bc_smem_bytes); nb: neighbour references kept here (0:
+// they stay in global memory).
+__host__ __device__ __forceinline__ size_t cluster_layout(uint32_t nwords, uint32_t npad, uint32_t logC,
+                                                          uint32_t groupSlots, uint32_t codeBytes, uint32_t nb)
+{
+    size_t const cap = cluster_slots_per_cta(npad, logC);
+    return kHalfPlanes * 16 + kDirTab * 4 + (size_t)(nwords >> logC) * 3 * 8 + cap * (codeBytes + 4) + 512 +
+           (size_t)groupSlots * 4 + cap * nb * 4;
+}
 
 // One thread-block cluster of 2^logC CTAs (1024 threads each) owns a system whose lattice,
-// temporary lattice, addresses and codes fit their shared memory together, for a whole run of
-// sub-steps (layout: cluster_word_rank, cluster_slot_rank). Each CTA checks the slots it holds,
-// lists its own tentative movers and performs them; lattice and temporary words and neighbours'
-// codes held by another CTA are reached through distributed shared memory. Two cluster barriers
-// per sub-step (after the check, after the perform) take the place of the resident kernel's CTA
-// barriers; the temporary lattice has one copy per sub-step parity, each CTA clearing its words of
-// the previous one while it checks. Every CTA of a cluster runs the same system and so reaches
-// the same barriers. A CTA leaves only after the last barrier, when no other CTA
-// accesses its shared memory any more. Grid: one cluster per system of sysList; the entries of
-// sub-step t are steps[t * stride + system].
+// temporary lattices, addresses and codes fit their shared memory together, for a whole run of
+// sub-steps (half bricks dealt out as cluster_word_rank says, slots as cluster_slot_rank). Each CTA
+// checks the slots it holds, lists its own tentative movers and performs them; words and
+// neighbours' codes held by another CTA are reached through distributed shared memory, the
+// neighbours' at addresses mapped once. Two cluster barriers per sub-step (after the check, after the
+// perform); the temporary lattice has one copy per sub-step parity. Between the two halves of the
+// first barrier a CTA clears its words of the previous copy and draws the directions of the next
+// sub-step, which nobody waits for. Every CTA of a cluster runs the same system and so reaches the
+// same barriers. A CTA leaves only after the last barrier, when no other CTA accesses its shared
+// memory any more. Grid: one cluster per system of sysList; the entries of sub-step t are
+// steps[t * stride + system]. K: chunks of 32 slots per warp and colour, at most.
+// Bound by remote accesses (0.33 remote atomics per clock and SM), two barriers of 0.3 us and the
+// chain of dependent reads of each phase; a lattice word is read only where the bond test passed and the
+// plane touches it. us per MCS, 16 CTAs: 8K chains 5.7 (8.6 on the four CTAs of one chunk per warp),
+// the 11K network 6.8 (8.3 on eight), 16K chains 7.0 (8.4).
 template <typename W, int K>
 __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* __restrict__ sysv,
                                                                    uint32_t const* __restrict__ sysList,
@@ -1133,155 +1312,174 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
                                                                    uint32_t stride, uint32_t nSteps)
 {
     namespace cg = cooperative_groups;
+    constexpr uint32_t kSlots = CodeWord<W>::kSlots, B = kResidentBlock;
+    static_assert(K <= 10, "a thread's directions share one word, three bits each");
     cg::cluster_group cluster = cg::this_cluster();
     uint32_t const C = cluster.num_blocks(), rank = cluster.block_rank();
     uint32_t logC = 0;
     while ((1u << logC) < C) ++logC;   // a power of two (launch_cluster_bc)
     __shared__ SysDev S;
-    __shared__ uint32_t listCount[2];   // per sub-step parity
+    __shared__ __align__(16) StepEntry stepSm[kStepBlock];
+    __shared__ uint32_t nMov[2];   // per sub-step parity
     extern __shared__ unsigned long long smem[];
     uint32_t const sysId = sysList[blockIdx.x >> logC];
     copy_desc(S, sysv + sysId);
     __syncthreads();
-    uint32_t const np = S.npad, nwC = S.nwords >> logC, cap = cluster_slots_per_cta(np, logC);
-    uint32_t const B = blockDim.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    unsigned long long* const ptab = smem;                                   // 768 plane masks
-    uint32_t* const dtab = reinterpret_cast<uint32_t*>(smem + 768);          // kDirTab words
-    unsigned long long* const lat = smem + 768 + kDirTab / 2;                // nwC words
-    unsigned long long* const tmp = lat + nwC;                               // 2 x nwC words
-    W* const code = reinterpret_cast<W*>(tmp + 2u * nwC);                    // cap slots
+    uint32_t const np = S.npad, nwC = S.nwords >> logC, cap = cluster_slots_per_cta(np, logC), maxc = S.maxc;
+    uint32_t const tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    uint4* const masks = reinterpret_cast<uint4*>(smem);                     // kHalfPlanes entries
+    uint32_t* const dtab = reinterpret_cast<uint32_t*>(masks + kHalfPlanes); // kDirTab words
+    uint32_t* const lat = dtab + kDirTab;                                    // 2 nwC half bricks
+    uint32_t* const tmp = lat + 2u * nwC;                                    // twice 2 nwC half bricks
+    W* const code = reinterpret_cast<W*>(tmp + 4u * nwC);                    // cap slots
     uint32_t* const pk = reinterpret_cast<uint32_t*>(code + cap);            // cap slots
     uint8_t* const mok = reinterpret_cast<uint8_t*>(pk + cap);               // 512 move-table bytes
-    uint32_t* const list = reinterpret_cast<uint32_t*>(mok + 512);           // K x 1024 entries
-    for (uint32_t w = tid; w < 768; w += B) ptab[w] = S.planeTab[w];
-    if (tid < kDirTab) dtab[tid] = S.dirTab[tid];
+    uint32_t* const list = reinterpret_cast<uint32_t*>(mok + 512);           // K x 1024 movers: local slot | dir << 28
+    uint32_t* const refs = list + K * B;                                     // maxc x cap references, where they fit
+    uint32_t dynBytes;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynBytes));
+    bool const cached = cluster_layout(S.nwords, np, logC, K * B, sizeof(W), maxc) <= dynBytes;
+    uint32_t const latAddr = (uint32_t)__cvta_generic_to_shared(lat), tmpAddr = (uint32_t)__cvta_generic_to_shared(tmp),
+                   codeAddr = (uint32_t)__cvta_generic_to_shared(code);
+    // neighbour reference (slot | reverse slot << 28): the mapped address of its code word, with the
+    // reverse slot (0-2, or 0-5 with 64-bit codes) in the low bits the word's alignment leaves free
+    auto mapped = [&](uint32_t ref) {
+        uint32_t const g = ref & kSlotMask;
+        return cluster_map(codeAddr + cluster_slot_local(g, logC) * (uint32_t)sizeof(W), cluster_slot_rank(g, logC)) |
+               (ref >> kSlotShift);
+    };
+    half_tables(S, masks, dtab);
     for (uint32_t w = tid; w < 512; w += B) mok[w] = S.moveOk[w];
-    for (uint32_t l = tid; l < nwC; l += B) {
-        lat[l] = S.lat[(l << logC) | rank];
-        tmp[l] = 0ull;
-        tmp[nwC + l] = 0ull;
+    for (uint32_t l = tid; l < 2u * nwC; l += B) {
+        lat[l] = reinterpret_cast<uint32_t const*>(S.lat)[(l << logC) | rank];
+        tmp[l] = 0u;
+        tmp[2u * nwC + l] = 0u;
     }
     for (uint32_t l = tid; l < cap; l += B) {
         uint32_t const g = cluster_slot_of(l, rank, logC);
         bool const in = g < np;
         code[l] = in ? *rec_code<W>(S.rec, g) : W(0);
         pk[l] = in ? *rec_pk<W>(S.rec, g) : 0u;
+        if (cached)
+            for (uint32_t q = 0; q < maxc; ++q) refs[q * cap + l] = in ? mapped(S.nbrr[(size_t)q * np + g]) : 0u;
     }
-    if (tid < 2) listCount[tid] = 0;
+    if (tid < 2) nMov[tid] = 0u;
     cluster.sync();   // every CTA's part of the state is in place before any remote access
 
-    auto latAt = [&](uint32_t w) { return cluster.map_shared_rank(lat + (w >> logC), w & (C - 1u)); };
-    // the temporary lattice and the list count alternate with the parity of the sub-steps run, so
-    // each CTA clears the previous sub-step's words while it checks: two cluster barriers per
-    // sub-step (after the check, after the perform)
-    auto tmpAt = [&](uint32_t par, uint32_t w) {
-        return cluster.map_shared_rank(tmp + par * nwC + (w >> logC), w & (C - 1u));
+    auto wordAt = [&](uint32_t base, uint32_t w) {
+        return cluster_map(base + 4u * cluster_word_local(w, logC), cluster_word_rank(w, logC));
     };
-    auto codeAt = [&](uint32_t g) {
-        return cluster.map_shared_rank(code + cluster_slot_local(g, logC), cluster_slot_rank(g, logC));
+    auto hits = [&](HalfPlane const& r, uint32_t base, bool on) {
+        uint32_t const v0 = cluster_load(wordAt(base, r.w[0]), on), v1 = cluster_load(wordAt(base, r.w[1]), on && r.m.y),
+                       v2 = cluster_load(wordAt(base, r.w[2]), on && r.m.z), v3 = cluster_load(wordAt(base, r.w[3]), on && r.m.w);
+        return (v0 & r.m.x) | (v1 & r.m.y) | (v2 & r.m.z) | (v3 & r.m.w);
     };
-
-    uint32_t nTent = 0, nAcc = 0;
+    // this warp's chunks of a colour group (which starts at a chunk): the k-th starts at slot
+    // chunk(e) * 32 + k * 1024 C
+    auto chunk = [&](StepEntry const& e) {
+        uint32_t const c0 = e.off >> 5;
+        return c0 + ((rank - c0) & (C - 1u)) + warp * C;
+    };
+    auto directions = [&](StepEntry const& e) {
+        uint32_t const c = chunk(e), i0 = c * 32u + lane - e.off;
+        uint32_t d = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < (uint32_t)K; ++k) {
+            uint32_t const i = i0 + k * B * C;
+            if (i - lane >= e.cnt) break;   // the same for the whole warp
+            d |= move_dir(i, e.seed) << (3u * k);
+        }
+        return d;
+    };
+    uint32_t const lanesBelow = (1u << lane) - 1u;
+    uint32_t nTent = 0, nAcc = 0, par = 0, dirs = 0;
+    bool drawn = false;   // dirs belong to the next active sub-step
     unsigned long long nAtt = 0;
-    StepEntry next = nSteps ? steps[sysId] : StepEntry{};
-    uint32_t par = 0;
     for (uint32_t t = 0; t < nSteps; ++t) {
-        StepEntry const st = next;
-        if (t + 1 < nSteps) next = steps[(size_t)(t + 1) * stride + sysId];   // prefetch
+        if (t % kStepBlock == 0) {   // (the last barrier of the sub-step before ended the reads of the old ones)
+            uint32_t const n = min(kStepBlock, nSteps - t);
+            for (uint32_t k = tid; k < 2u * n; k += B)
+                reinterpret_cast<uint4*>(stepSm)[k] =
+                    reinterpret_cast<uint4 const*>(steps + (size_t)(t + k / 2u) * stride + sysId)[k & 1u];
+            __syncthreads();
+            drawn = false;
+        }
+        uint32_t const ts = t % kStepBlock;
+        StepEntry const st = stepSm[ts];
         if (st.color == kNoColor) continue;
+        if (!drawn) dirs = directions(st);
         if (rank == 0) nAtt += st.cnt;
-        // the previous sub-step's marks and list count: no CTA reads them after the barrier that
-        // ended that sub-step, and none writes them before the barrier that ends this one
-        for (uint32_t l = tid; l < nwC; l += B) tmp[(par ^ 1u) * nwC + l] = 0ull;
-        if (tid == 0) listCount[par ^ 1u] = 0;
-        // check: this CTA's chunks of 32 slots of the colour group (the group starts at a chunk)
-        uint32_t const end = st.off + st.cnt, c0 = st.off >> 5, cEnd = (end + 31u) >> 5;
-        uint32_t const cFirst = c0 + ((rank - c0) & (C - 1u));
+        uint32_t const marks = tmpAddr + par * 8u * nwC;
+        // check: this warp's chunks of the colour group
+        uint32_t const end = st.off + st.cnt, c0 = chunk(st);
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            uint32_t const c = cFirst + (warp + (uint32_t)k * 32u) * C;
-            uint32_t const g = c * 32u + lane;
-            bool go = false;
-            uint32_t entry = 0;
-            if (c < cEnd && g < end) {
-                uint32_t const l = cluster_slot_local(g, logC);
-                uint32_t const dir = move_dir(g - st.off, st.seed);
-                uint32_t const p = pk[l];
-                DirParams const D = dir_params(dtab, dir);
-                if ((p & D.ma) != D.wall && bonds_ok<W, true>(code[l], dir, mok)) {
-                    Plane pl;
-                    front_plane<true>(pl, ptab, D, p, D.front, dir);
-                    unsigned long long hit = 0ull;
-#pragma unroll
-                    for (int r = 0; r < 4; ++r)
-                        if (pl.m[r]) hit |= *latAt(pl.w[r]) & pl.m[r];
-                    if (hit == 0ull) {
-                        uint32_t const to = addr_add(p, D.ma, D.step);
-                        dsmem_or64(tmpAt(par, to >> 6), 1ull << (to & 63u));
-                        go = true;
-                        entry = l | (dir << kSlotShift);
-                    }
-                }
-            }
-            uint32_t const bal = __ballot_sync(0xffffffffu, go);
-            if (bal) {
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(&listCount[par], (uint32_t)__popc(bal));
-                base = __shfl_sync(0xffffffffu, base, 0);
-                if (go) list[base + __popc(bal & ((1u << lane) - 1u))] = entry;
-                nTent += lane == 0 ? (uint32_t)__popc(bal) : 0u;
-            }
-        }
-        cluster.sync();   // every CTA's marks are in place
-        // perform over this CTA's list
-        uint32_t const nList = listCount[par];
-        for (uint32_t e = tid; e < nList; e += B) {
-            uint32_t const l = list[e] & kSlotMask, dir = list[e] >> kSlotShift;
-            uint32_t const g = cluster_slot_of(l, rank, logC);
-            uint32_t const p = pk[l];
-            uint32_t nb[CodeWord<W>::kSlots];
-#pragma unroll
-            for (uint32_t q = 0; q < CodeWord<W>::kSlots; ++q)
-                nb[q] = q < S.maxc ? __ldg(S.nbrr + (size_t)q * np + g) : 0u;
-            Plane pl;
+        for (uint32_t k = 0; k < (uint32_t)K; ++k) {
+            uint32_t const g = (c0 + k * 32u * C) * 32u + lane;
+            if (g - lane >= end) break;   // the same for the whole warp
+            uint32_t const l = cluster_slot_local(g, logC), dir = (dirs >> (3u * k)) & 7u, p = pk[l];
             DirParams const D = dir_params(dtab, dir);
-            front_plane<true>(pl, ptab, D, p, D.front, dir);
-            unsigned long long hit = 0ull;
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-                if (pl.m[r]) hit |= *tmpAt(par, pl.w[r]) & pl.m[r];
-            if (hit != 0ull) continue;
-            uint32_t const a = dir >> 1;
-            int32_t const s = (dir & 1u) ? 1 : -1;
-            uint32_t const p1 = addr_add(p, D.ma, D.step);
-            uint32_t const w0 = p >> 6, w1 = p1 >> 6;
-            if (w0 == w1) {
-                dsmem_xor64(latAt(w0), (1ull << (p & 63u)) | (1ull << (p1 & 63u)));
-            } else {
-                dsmem_xor64(latAt(w0), 1ull << (p & 63u));
-                dsmem_xor64(latAt(w1), 1ull << (p1 & 63u));
-            }
-            pk[l] = p1;
-            image_step(S, g, a, s, p, p1, D.ma);
-            W const own = code[l];
-            code[l] = code_shift(own, a, -s);
-            uint32_t const n = uint32_t(own >> CodeWord<W>::kCountShift) & 7u;
-#pragma unroll
-            for (uint32_t q = 0; q < CodeWord<W>::kSlots; ++q) {
-                if (q < n) {
-                    uint32_t const ent = nb[q];
-                    uint32_t const cr = (0u - (uint32_t(own >> (9u * q + 3u * a)) & 7u)) & 7u;
-                    uint32_t const nc = uint32_t(int32_t(cr) + s) & 7u;
-                    dsmem_xor(codeAt(ent & kSlotMask), W(cr ^ nc) << (9u * (ent >> kSlotShift) + 3u * a));
-                }
-            }
-            ++nAcc;
+            bool const ok = bonds_ok<W, true>(code[l], dir, mok) & ((p & D.ma) != D.wall) & (g < end);
+            HalfPlane pl;
+            half_plane(pl, masks, D, p, D.front, dir);
+            uint32_t const to = addr_add(p, D.ma, D.step);
+            bool const go = ok & (hits(pl, latAddr, ok) == 0u);
+            cluster_or(wordAt(marks, to >> 5), 1u << (to & 31u), go);
+            uint32_t const bal = __ballot_sync(0xffffffffu, go);
+            uint32_t at = 0;
+            if (lane == 0) at = shared_add(&nMov[par], (uint32_t)__popc(bal));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanesBelow);
+            if (go) list[at] = l | (dir << kSlotShift);
         }
-        cluster.sync();   // every perform is done: the lattice is settled for the next check
+        cluster_arrive();   // this CTA's marks are on their way
+        // the previous sub-step's marks and mover count: no CTA reads them after the barrier that
+        // ended that sub-step, and none writes them before the barrier that ends this one
+        for (uint32_t w = B - 1u - tid; w < nwC; w += B)
+            reinterpret_cast<unsigned long long*>(tmp + (par ^ 1u) * 2u * nwC)[w] = 0ull;
+        if (tid == 0) nMov[par ^ 1u] = 0u;
+        drawn = t + 1 < nSteps && ts + 1u < kStepBlock && stepSm[ts + 1u].color != kNoColor;
+        if (drawn) dirs = directions(stepSm[ts + 1u]);
+        cluster_wait();   // every CTA's marks are in place
+        // perform over this CTA's movers, from the last thread down
+        uint32_t const n = nMov[par];
+        for (uint32_t e = B - 1u - tid; e < n; e += B) {
+            uint32_t const l = list[e] & kSlotMask, dir = list[e] >> kSlotShift, p = pk[l];
+            W const own = code[l];
+            uint32_t const nn = uint32_t(own >> CodeWord<W>::kCountShift) & 7u;
+            uint32_t nb[kSlots];
+#pragma unroll
+            for (uint32_t q = 0; q < kSlots; ++q) {
+                nb[q] = 0u;
+                if (q < nn)
+                    nb[q] = cached ? refs[q * cap + l]
+                                   : mapped(__ldg(S.nbrr + (size_t)q * np + cluster_slot_of(l, rank, logC)));
+            }
+            DirParams const D = dir_params(dtab, dir);
+            uint32_t const to = addr_add(p, D.ma, D.step);
+            HalfPlane pl;
+            half_plane(pl, masks, D, to, D.step, dir);
+            W flip;
+            W const moved = code_move(own, dir, flip);
+            bool const free = hits(pl, marks, true) == 0u;
+            cluster_xor(wordAt(latAddr, p >> 5), 1u << (p & 31u), free);
+            cluster_xor(wordAt(latAddr, to >> 5), 1u << (to & 31u), free);
+#pragma unroll
+            for (uint32_t q = 0; q < kSlots; ++q)
+                cluster_xor(nb[q] & ~(uint32_t)(sizeof(W) - 1), code_flip(flip, q, nb[q] & (uint32_t)(sizeof(W) - 1)),
+                            free && q < nn);
+            if (free) {
+                pk[l] = to;
+                code[l] = moved;
+                image_step(S, cluster_slot_of(l, rank, logC), dir >> 1, (dir & 1u) ? 1 : -1, p, to, D.ma);
+                ++nAcc;
+            }
+        }
+        nTent += n;
+        cluster_arrive();
+        cluster_wait();   // every perform is done: the lattice is settled for the next check
         par ^= 1u;
     }
     // after the last cluster barrier no CTA reaches into another's shared memory
-    for (uint32_t l = tid; l < nwC; l += B) S.lat[(l << logC) | rank] = lat[l];
+    for (uint32_t l = tid; l < 2u * nwC; l += B) reinterpret_cast<uint32_t*>(S.lat)[(l << logC) | rank] = lat[l];
     for (uint32_t l = tid; l < cap; l += B) {
         uint32_t const g = cluster_slot_of(l, rank, logC);
         if (g < np) {
@@ -1289,13 +1487,12 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
             *rec_pk<W>(S.rec, g) = pk[l];
         }
     }
-    uint32_t const tsum = __reduce_add_sync(0xffffffffu, nTent);
     uint32_t const asum = __reduce_add_sync(0xffffffffu, nAcc);
-    if (lane == 0) {
-        tally_flush(tsum, S.stats, 1);
-        tally_flush(asum, S.stats, 2);
+    if (lane == 0) tally_flush(asum, S.stats, 2);
+    if (tid == 0) {
+        tally_flush(nTent, S.stats, 1);
+        if (nAtt) atomicAdd(S.stats + (blockIdx.x % kStatSlots), nAtt);
     }
-    if (tid == 0 && nAtt) atomicAdd(S.stats + (blockIdx.x % kStatSlots), nAtt);
 }
 
 // ---------------------------------------------------------------------------------- launchers
@@ -1497,16 +1694,9 @@ template <typename W, int B, bool kCache>
 cudaError_t launch_slab_bc_w(SysDev const& S, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
                              GridSync* gs, cudaStream_t s)
 {
-    static thread_local size_t attrSet[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    static thread_local bool done[64] = {};
+    cudaError_t const e = allow_smem(k_slab_bc<W, B, kCache>, done);
     if (e != cudaSuccess) return e;
-    size_t& have = attrSet[dev & 63];
-    if (plan.smem > have) {
-        e = cudaFuncSetAttribute(k_slab_bc<W, B, kCache>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
-        if (e != cudaSuccess) return e;
-        have = plan.smem;
-    }
     uint32_t cap = plan.cap, capG = plan.capG, clearAll = plan.clearAll;
     void* args[] = {const_cast<SysDev*>(&S), &dSteps, &nSteps, &cap, &capG, &clearAll, &gs};
     return cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(k_slab_bc<W, B, kCache>), dim3(plan.ctas), dim3(B),
@@ -1531,29 +1721,23 @@ cudaError_t launch_slab_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint
     return cudaErrorInvalidValue;
 }
 
-size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t codeMode)
+size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t maxc, uint32_t codeMode)
 {
-    size_t const w = codeMode == kCode64 ? 8 : 4;
-    return 768 * 8 + kDirTab * 4 + (size_t)nwords * 3 * 8 + (size_t)npad * (w + 4) + 512 + (size_t)maxGroup * 4;
+    uint32_t const w = codeMode == kCode64 ? 8 : 4;
+    size_t const all = resident_layout(nwords, npad, maxGroup, w, maxc);
+    return all <= kResidentMaxSmem ? all : resident_layout(nwords, npad, maxGroup, w, 0);
 }
 
 namespace {
 
-template <typename W, int K>
+template <typename W, bool kDirect>
 cudaError_t launch_resident_bc_k(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, StepEntry const* dSteps,
                                  uint32_t nSys, uint32_t nSteps, size_t smem, cudaStream_t s)
 {
-    static thread_local size_t attrSet[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    static thread_local bool done[64] = {};
+    cudaError_t const e = allow_smem(k_resident_bc<W, kDirect>, done);
     if (e != cudaSuccess) return e;
-    size_t& have = attrSet[dev & 63];
-    if (smem > have) {
-        e = cudaFuncSetAttribute(k_resident_bc<W, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        have = smem;
-    }
-    k_resident_bc<W, K><<<nCta, kResidentBlock, smem, s>>>(dSys, dList, dSteps, nSys, nSteps);
+    k_resident_bc<W, kDirect><<<nCta, kResidentBlock, smem, s>>>(dSys, dList, dSteps, nSys, nSteps);
     return cudaGetLastError();
 }
 
@@ -1561,14 +1745,12 @@ template <typename W>
 cudaError_t launch_resident_bc_w(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, uint32_t perThread,
                                  StepEntry const* dSteps, uint32_t nSys, uint32_t nSteps, size_t smem, cudaStream_t s)
 {
-    switch (perThread) {
-    case 1: return launch_resident_bc_k<W, 1>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s);
-    case 2: return launch_resident_bc_k<W, 2>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s);
-    case 4: return launch_resident_bc_k<W, 4>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s);
-    case 8: return launch_resident_bc_k<W, 8>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s);
-    case 16: return launch_resident_bc_k<W, 16>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s);
-    default: return cudaErrorInvalidValue;
-    }
+    // lists of 16-bit entries index up to 1 << kSlabEntBits slots of a group
+    constexpr uint32_t kListed = (1u << kSlabEntBits) / kResidentBlock;
+    if (perThread < 1 || perThread > 16) return cudaErrorInvalidValue;
+    return perThread == 1 || perThread > kListed
+               ? launch_resident_bc_k<W, true>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s)
+               : launch_resident_bc_k<W, false>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s);
 }
 
 }  // namespace
@@ -1586,12 +1768,12 @@ cudaError_t launch_resident_bc(SysDev const* dSys, uint32_t const* dList, uint32
     return cudaErrorInvalidValue;
 }
 
-size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t perThread, uint32_t codeMode)
+size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t perThread, uint32_t maxc,
+                             uint32_t codeMode)
 {
-    size_t const w = codeMode == kCode64 ? 8 : 4;
-    size_t const cap = cluster_slots_per_cta(npad, logC);
-    return 768 * 8 + kDirTab * 4 + (size_t)(nwords >> logC) * 3 * 8 + cap * (w + 4) + 512 +
-           (size_t)perThread * kResidentBlock * 4;
+    uint32_t const w = codeMode == kCode64 ? 8 : 4;
+    size_t const all = cluster_layout(nwords, npad, logC, perThread * kResidentBlock, w, maxc);
+    return all <= kResidentMaxSmem ? all : cluster_layout(nwords, npad, logC, perThread * kResidentBlock, w, 0);
 }
 
 namespace {
@@ -1602,7 +1784,8 @@ cudaError_t cluster_bc_config(uint32_t logC, size_t smem, cudaLaunchConfig_t& cf
 {
     auto kernel = k_cluster_bc<W, K>;
     uint32_t const C = 1u << logC;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static thread_local bool done[64] = {};
+    cudaError_t e = allow_smem(kernel, done);
     if (e != cudaSuccess) return e;
     if (C > 8) {
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

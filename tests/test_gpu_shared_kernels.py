@@ -1,0 +1,74 @@
+"""The kernels that hold a system in shared memory (one CTA, or a cluster of CTAs) against the oracle
+where their layouts can go wrong: lattices of one and two words, every remainder of the slots per
+warp, both forms of the resident check and the group size between them, groups too large for 16-bit
+list entries, neighbour references that do not fit, walls, three colours, 64-bit codes, and calls that
+end inside and on the edges of a block of step entries. Integers: every comparison is exact."""
+import numpy as np
+import pytest
+
+import pscbfm_b200 as P
+from oracle import oracle as O
+from pscbfm_b200 import systems as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _free(n, side):
+    """n unbonded monomers on a 2-spaced grid: one colour group of n."""
+    k = np.arange(n)
+    h = side // 2
+    xyz = 2 * np.stack([k % h, (k // h) % h, k // (h * h)], axis=1)
+    return S.from_bonds((side,) * 3, xyz, np.zeros((0, 2)), seed=29)
+
+
+SYSTEMS = {
+    "one_word_lattice": lambda: S.from_bonds((4, 4, 4), [[0, 0, 0], [2, 2, 2]], [], seed=2),
+    "two_word_lattice": lambda: S.from_bonds((8, 4, 4), [[0, 0, 0], [2, 0, 0], [4, 0, 0]], [(0, 1), (1, 2)], seed=3),
+    "group_1024": lambda: S.serpentine_chains(32, 32, 0.5, seed=5),
+    "group_1056": lambda: S.serpentine_chains(32, 33, 0.52, seed=6),
+    "ragged_3_per_thread": lambda: S.serpentine_chains((64, 32, 32), 31, 0.63, seed=7),
+    "free_8200_direct": lambda: _free(8200, 64),
+    "refs_do_not_fit": lambda: S.serpentine_chains(64, 64, 0.3, seed=8),
+    "walls": lambda: S.walled(S.serpentine_chains((30, 64, 50), 17, 0.4, seed=9), walls=7),
+    "three_colours": lambda: S.rings_and_free(32),
+    "codes_64bit": lambda: S.square_network(64),
+}
+
+
+@pytest.mark.parametrize("mode", ["resident", "cluster"])
+@pytest.mark.parametrize("name", list(SYSTEMS))
+def test_shared_memory_kernels_vs_oracle(name, mode):
+    s = SYSTEMS[name]()
+    m = {"resident": P.MODE_RESIDENT, "cluster": P.MODE_CLUSTER}[mode]
+    u = P.UpdaterGPUScBFM_AB_Type(0)
+    u.load_system(s, mode=m)
+    if mode == "resident" or name not in ("one_word_lattice",):
+        assert u.path() == m
+    nc = u.n_colors()[0]
+    done = 0
+    # sub-steps per call: below, on and across the blocks of 16 step entries
+    for mcs in (1, 16 // nc, 16 // nc + 1, 33):
+        u.runSimulationOnGPU(mcs)
+        done += mcs
+    want, ost = O.run(s, done)
+    st = u.stats()
+    assert np.array_equal(u.get_coords(), want)
+    assert (st["attempted"], st["tentative"], st["accepted"]) == ost
+    u.validate()
+    u.close()
+
+
+def test_idle_members_beside_longer_ones():
+    """A batch whose members stop at different sub-steps: the shared-memory kernels skip the idle entries
+    that follow a member's last sub-step, inside and across blocks of step entries."""
+    systems = [S.serpentine_chains(32, 16, 0.3, seed=40), S.small_chains(), S.crosslinked_network(),
+               S.rings_and_free(32), S.serpentine_chains(64, 64, 0.6, seed=41)]
+    members = [P.UpdaterGPUScBFM_AB_Type(0).load_system(s) for s in systems]
+    b = P.Batch(members)
+    plan = [[1, 9, 40, 5, 17], [8, 0, 3, 33, 0], [16, 16, 1, 0, 7]]
+    for mcs in plan:
+        b.run_each(mcs)
+    for s, m, t in zip(systems, members, np.sum(plan, axis=0)):
+        assert np.array_equal(m.get_coords(), O.run(s, int(t))[0]), s.name
+        m.validate()
+    b.close()
