@@ -130,8 +130,8 @@ int bfm_set_perform(bfm_handle h, int warps, int group);
  * BFM_MODE_GRAPH. */
 int bfm_get_path(bfm_handle h, int* mode);
 /* Fault injection for tests (no counterpart in the reference): the next BFM_MODE_PERSISTENT launch
- * of this handle starts its grid-barrier arrival count where no barrier can complete, so every
- * CTA's wait runs out at its time limit (20 s, the first wait's) and the run reports the timeout
+ * of this handle (or the next run of a batch that holds it on CTAs of its own) starts its grid-barrier arrival count where no barrier can complete, so every
+ * CTA's wait runs out at its time limit (20 s) and the run reports the timeout
  * (BFM_ERR_CUDA).
  * Nothing faults on the GPU and the device stays usable; this system's state is not. */
 int bfm_inject_barrier_stall(bfm_handle h);
@@ -238,10 +238,10 @@ int bfm_batch_launch_count(bfm_batch_handle b, uint64_t* out);
 int bfm_batch_synchronize(bfm_batch_handle b);
 /* 0: every system on the grid path; 1 (default): small systems on the resident kernel. */
 int bfm_batch_set_resident(bfm_batch_handle b, int on);
-/* 1 (default): systems too large for one CTA that a cluster of CTAs holds with at most two chunks
- * of 32 monomers per warp and colour (bond codes; there the cluster-resident kernel of
- * BFM_MODE_CLUSTER beats the grid-phase kernels) run in that kernel while the batch's clusters take
- * at most half of the SMs; 0: they share the grid-phase kernels. */
+/* 1 (default): bond-code systems too large for one CTA run on CTAs of their own for the whole run, as
+ * many as hold them in shared memory and share the SMs evenly (to about 500 K monomers; beside a larger
+ * or a gather system, which needs the grid-phase kernels, they take at most half of the SMs); 0: they
+ * share the grid-phase kernels. Results do not change. */
 int bfm_batch_set_cluster(bfm_batch_handle b, int on);
 /* Member i advances mcs[i] MCS (0 = it idles); one launch sequence for all, like bfm_batch_run. */
 int bfm_batch_run_each(bfm_batch_handle b, const int32_t* mcs);

@@ -2,11 +2,9 @@
 //
 // Systems whose lattices (and, in the bond-code representation, packed coordinates and bond
 // codes) fit one CTA's shared memory run in the resident kernel, one CTA per system, one launch
-// per run. Systems of the bond-code representation that a cluster of 2-16 CTAs holds in its
-// distributed shared memory with at most two chunks of 32 slots per warp and colour (where that
-// kernel beats the grid-phase kernels) run in the cluster-resident kernel, one cluster per system and one
-// launch per run and cluster size, while the batch's clusters take at most half of the SMs. The
-// other systems share the grid-phase kernels: one check and one perform launch per
+// per run. Larger systems of the bond-code representation run in the slab sweep, each on CTAs of its
+// own, several systems in one cooperative launch per run (planSlabs). What fits neither shares
+// the grid-phase kernels: one check and one perform launch per
 // sub-step and representation cover the active colour group of every such system at once, and
 // chunks of those launches are captured into a CUDA graph once and replayed. Each system draws its
 // own sub-steps from its own stream exactly as it would alone, so its trajectory is unchanged by
@@ -14,10 +12,11 @@
 //
 // A run stages the step entries of all its sub-steps with one host-to-device copy; the resident
 // and the grid-phase launches then proceed on two streams without meeting until the run ends, and
-// the host returns as soon as the work is queued. Each cluster group runs on a stream of its own. Member streams are ordered before the run and
+// the host returns as soon as the work is queued. The slab sweeps run on a stream of their own. Member streams are ordered before the run and
 // after it with events, never with host waits.
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <stdexcept>
 
@@ -41,7 +40,7 @@ Batch::Batch(int gpu, Updater* const* members, uint32_t n) : gpu_(gpu)
         cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, gpu_) == cudaSuccess && sms > 0)
-        smCount_ = (uint32_t)sms;
+        smCount_ = slabSms_ = (uint32_t)sms;
 }
 
 Batch::~Batch()
@@ -49,7 +48,7 @@ Batch::~Batch()
     cudaSetDevice(gpu_);
     if (stream_) cudaStreamSynchronize(stream_);
     if (stream2_) cudaStreamSynchronize(stream2_);
-    for (cudaStream_t q : side_) cudaStreamSynchronize(q);
+    if (side_) cudaStreamSynchronize(side_);
     if (graph_) cudaGraphExecDestroy(graph_);
     if (arena_) cudaFreeAsync(arena_, stream_);
     if (dStepsAll_) cudaFreeAsync(dStepsAll_, stream_);
@@ -57,8 +56,8 @@ Batch::~Batch()
     cudaFreeHost(hSteps_);
     for (cudaEvent_t e : {join_, fork_, stepsFree_, done_, ready_})
         if (e) cudaEventDestroy(e);
-    for (cudaEvent_t e : sideJoin_) cudaEventDestroy(e);
-    for (cudaStream_t q : side_) cudaStreamDestroy(q);
+    if (sideJoin_) cudaEventDestroy(sideJoin_);
+    if (side_) cudaStreamDestroy(side_);
     if (stream_) cudaStreamDestroy(stream_);
     if (stream2_) cudaStreamDestroy(stream2_);
 }
@@ -73,7 +72,8 @@ uint32_t Batch::residentCount() const
 uint32_t Batch::clusterCount() const
 {
     uint32_t n = 0;
-    for (auto const& g : cluster_) n += (uint32_t)g.members.size();
+    for (auto const& w : slab_)
+        for (SlabRef const& r : w.refs) n += r.rank == 0 ? 1u : 0u;
     return n;
 }
 
@@ -102,11 +102,10 @@ void Batch::rebuild()
     // the previous launches may still read the arena
     cuda_check(cudaStreamSynchronize(stream_), "batch");
     cuda_check(cudaStreamSynchronize(stream2_), "batch");
-    for (cudaStream_t q : side_) cuda_check(cudaStreamSynchronize(q), "batch");
+    if (side_) cuda_check(cudaStreamSynchronize(side_), "batch");
     uint32_t const M = (uint32_t)members_.size();
     grid_.clear();
     resident_.clear();
-    cluster_.clear();
     wholeRun_.assign(M, 0);
     auto gridGroup = [&](uint32_t mode) -> GridGroup& {
         for (auto& g : grid_)
@@ -120,29 +119,33 @@ void Batch::rebuild()
         resident_.push_back(ResidentGroup{mode, {}, nullptr, 1, 0});
         return resident_.back();
     };
-    auto clusterGroup = [&](uint32_t mode, uint32_t logC) -> ClusterGroup& {
-        for (auto& g : cluster_)
-            if (g.codeMode == mode && g.logC == logC) return g;
-        cluster_.push_back(ClusterGroup{mode, logC, {}, nullptr, 1, 0, cluster_.size()});
-        return cluster_.back();
-    };
-    uint32_t clusterCtas = 0;
+    std::vector<char> slabbed;
+    slab_ = planSlabs(slabbed, residentsAfter_);
+    if (!slab_.empty() && !side_) {
+        cuda_check(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
+        cuda_check(cudaEventCreateWithFlags(&sideJoin_, cudaEventDisableTiming), "cudaEventCreate");
+    }
+    bool faulted = false;   // a report belongs to the member it was made for: kept by it, not reused
+    for (uint32_t m = 0; m < reportCap_; ++m) faulted = faulted || reports_.get()[m].fault != 0u;
+    if (!slab_.empty() && (M > reportCap_ || faulted)) {
+        void* p = nullptr;
+        void* d = nullptr;
+        cuda_check(cudaHostAlloc(&p, sizeof(GridFault) * M, cudaHostAllocMapped), "cudaHostAlloc(reports)");
+        std::memset(p, 0, sizeof(GridFault) * M);
+        reports_ = std::shared_ptr<GridFault>(static_cast<GridFault*>(p), [](GridFault* q) { cudaFreeHost(q); });
+        cuda_check(cudaHostGetDevicePointer(&d, p, 0), "reports device address");
+        dReports_ = static_cast<GridFault*>(d);
+        reportCap_ = M;
+    }
     for (uint32_t m = 0; m < M; ++m) {
         Updater* u = members_[m];
-        Updater::ClusterPlan const& cp = u->batchCluster();
-        uint32_t const C = 1u << cp.logC;
         if (residentOn_ && u->residentEligible()) {
             ResidentGroup& g = resGroup(u->codeMode());
             g.members.push_back(m);
             g.smem = std::max(g.smem, u->residentSmem());
             while (g.perThread * kResidentBlock < u->maxGroup()) g.perThread *= 2;
             wholeRun_[m] = 1;
-        } else if (clusterOn_ && cp.logC != 0 && clusterCtas + C <= smCount_ / 2u) {
-            ClusterGroup& g = clusterGroup(u->codeMode(), cp.logC);
-            g.members.push_back(m);
-            g.smem = std::max(g.smem, cp.smem);
-            g.perThread = std::max(g.perThread, cp.perWarp);
-            clusterCtas += C;
+        } else if (slabbed[m]) {
             wholeRun_[m] = 1;
         } else {
             GridGroup& g = gridGroup(u->codeMode());
@@ -157,28 +160,7 @@ void Batch::rebuild()
     size_t total = up256(sizeof(SysDev) * M) + up256(sizeof(StepEntry) * stepCap_ * M);
     for (auto const& g : grid_) total += up256(sizeof(TileRef) * g.tiles.size()) + up256(sizeof(TileRef) * g.ptiles.size());
     for (auto const& g : resident_) total += up256(sizeof(uint32_t) * g.members.size());
-    for (auto const& g : cluster_) total += up256(sizeof(uint32_t) * g.members.size());
-    while (side_.size() < cluster_.size()) {
-        cudaStream_t q = nullptr;
-        cudaEvent_t e = nullptr;
-        cuda_check(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreate");
-        side_.push_back(q);
-        cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-        sideJoin_.push_back(e);
-    }
-    for (auto& g : cluster_) {
-        // one launch runs every cluster of the group at one size; a member planned with fewer
-        // chunks per warp runs as well with more (the kernel walks only its own chunks)
-        size_t smem = 0;
-        for (uint32_t m : g.members) {
-            Updater const* u = members_[m];
-            smem = std::max(smem, cluster_bc_smem_bytes(u->desc().nwords, u->desc().npad, g.logC, g.perThread,
-                                                        u->desc().maxc, g.codeMode));
-        }
-        g.smem = smem;
-        if (!cluster_bc_runnable(g.logC, g.perThread, g.smem, g.codeMode))
-            throw std::runtime_error("[Batch] a cluster group's configuration does not run on this device");
-    }
+    for (auto const& w : slab_) total += up256(sizeof(SlabRef) * w.refs.size());
     if (total > arenaBytes_) {   // grows only: membership changes reuse the arena
         if (arena_) cuda_check(cudaFreeAsync(arena_, stream_), "cudaFreeAsync(batch)");
         arena_ = nullptr;
@@ -214,12 +196,12 @@ void Batch::rebuild()
                                    cudaMemcpyHostToDevice, stream_),
                    "upload resident list");
     }
-    for (auto& g : cluster_) {
-        g.dList = reinterpret_cast<uint32_t*>(p);
-        p += up256(sizeof(uint32_t) * g.members.size());
-        cuda_check(cudaMemcpyAsync(g.dList, g.members.data(), sizeof(uint32_t) * g.members.size(),
-                                   cudaMemcpyHostToDevice, stream_),
-                   "upload cluster list");
+    for (auto& w : slab_) {
+        w.dRefs = reinterpret_cast<SlabRef*>(p);
+        p += up256(sizeof(SlabRef) * w.refs.size());
+        cuda_check(cudaMemcpyAsync(w.dRefs, w.refs.data(), sizeof(SlabRef) * w.refs.size(), cudaMemcpyHostToDevice,
+                                   stream_),
+                   "upload slab CTAs");
     }
     // the host vectors above die with this call: finish their copies now
     cuda_check(cudaStreamSynchronize(stream_), "batch uploads");
@@ -228,6 +210,98 @@ void Batch::rebuild()
         graph_ = nullptr;
     }
     built_ = true;
+}
+
+bool Batch::slabFits(Updater const& u) const
+{
+    SlabPlan plan;
+    return u.slabPlan(smCount_ / 2u, plan) && plan.cache;
+}
+
+std::vector<Batch::SlabWave> Batch::planSlabs(std::vector<char>& taken, bool& residentsAfter) const
+{
+    // The members in the slab sweep (taken) and their CTAs, in cooperative launches of at most `budget` CTAs
+    // that run one after the other. Each CTA takes an SM, so the fewest CTAs that hold a member do the most
+    // work per SM (moves per us and SM at 0.9K, 1.9K, 3.7K and 7.5K slots per CTA and colour: 208, 331, 419
+    // and 458); members are packed that way, longest first. The SMs a wave leaves idle then go, one by one,
+    // to its member with the most slots per CTA, which runs longest. A member the grid-phase kernels
+    // have to take anyway (it does not fit, or gathers) keeps half of the SMs.
+    uint32_t const M = (uint32_t)members_.size();
+    taken.assign(M, 0);
+    residentsAfter = false;
+    std::vector<SlabWave> waves;
+    if (!clusterOn_) return waves;
+    uint32_t residents = 0;
+    bool gridAnyway = false;
+    struct Item {
+        uint32_t m;
+        SlabPlan plan;
+    };
+    std::vector<Item> items;
+    for (uint32_t m = 0; m < M; ++m) {
+        Updater const& u = *members_[m];
+        if (residentOn_ && u.residentEligible()) {
+            ++residents;
+            continue;
+        }
+        if (!slabFits(u)) {
+            gridAnyway = true;
+            continue;
+        }
+        Item it{m, {}};
+        for (uint32_t C = 1; !(u.slabPlan(C, it.plan) && it.plan.cache); ++C) {}   // ends: slabFits
+        items.push_back(it);
+    }
+    // A cooperative launch waits until all its CTAs have found an SM, so it must never queue behind the
+    // batch's own resident kernels, which keep theirs for the whole run: a few residents get SMs of
+    // their own, many run after the slab sweeps.
+    residentsAfter = residents > slabSms_ / 4u;
+    uint32_t const budget =
+        std::max(1u, gridAnyway ? slabSms_ / 2u : slabSms_ - (residentsAfter ? 0u : residents));
+    std::stable_sort(items.begin(), items.end(), [&](Item const& a, Item const& b) {
+        return members_[a.m]->nMonomers() > members_[b.m]->nMonomers();
+    });
+    std::vector<std::vector<Item>> packed;
+    std::vector<uint32_t> used;
+    for (Item const& it : items) {
+        uint32_t const mode = members_[it.m]->codeMode();
+        size_t w = 0;
+        while (w < packed.size() &&
+               (used[w] + it.plan.ctas > budget || members_[packed[w][0].m]->codeMode() != mode))
+            ++w;
+        if (w == packed.size()) {
+            packed.emplace_back();
+            used.push_back(0);
+        }
+        packed[w].push_back(it);
+        used[w] += it.plan.ctas;
+    }
+    for (size_t w = 0; w < packed.size(); ++w) {
+        for (;;) {
+            Item* pick = nullptr;
+            for (Item& it : packed[w])
+                if (it.plan.perCta > kSlabGrowSlots && (!pick || it.plan.perCta > pick->plan.perCta)) pick = &it;
+            SlabPlan next;
+            if (!pick || used[w] >= budget || !members_[pick->m]->slabPlan(pick->plan.ctas + 1u, next) || !next.cache)
+                break;
+            pick->plan = next;
+            ++used[w];
+        }
+        SlabWave wave{members_[packed[w][0].m]->codeMode(), {}, 0, nullptr};
+        for (Item const& it : packed[w]) {
+            for (uint32_t r = 0; r < it.plan.ctas; ++r) wave.refs.push_back(SlabRef{it.m, r, it.plan.ctas, 0u});
+            wave.smem = std::max(wave.smem, it.plan.smem);
+            taken[it.m] = 1;
+        }
+        waves.push_back(std::move(wave));
+    }
+    return waves;
+}
+
+void Batch::setSlabSms(uint32_t sms)
+{
+    if (sms != slabSms_) built_ = false;
+    slabSms_ = sms;
 }
 
 cudaError_t Batch::launchGrid(StepEntry const* e)
@@ -357,20 +431,23 @@ void Batch::run(int32_t const* mcs)
         cuda_check(cudaMemcpyAsync(dStepsAll_, hSteps_, sizeof(StepEntry) * entries, cudaMemcpyHostToDevice, stream_),
                    "batch steps H2D");
         cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
-        if (!resident_.empty() || !cluster_.empty()) cuda_check(cudaEventRecord(fork_, stream_), "event");
-        for (auto const& g : cluster_) {
-            // one launch per cluster size for the whole run, each on a stream of its own
-            cudaStream_t const q = side_[g.side];
-            cuda_check(cudaStreamWaitEvent(q, fork_, 0), "wait");
-            cuda_check(launch_cluster_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.logC, g.perThread, dStepsAll_,
-                                         M, (uint32_t)T, g.smem, g.codeMode, q),
-                       "batch cluster");
-            cuda_check(cudaEventRecord(sideJoin_[g.side], q), "event");
-            ++launches_;
+        if (!resident_.empty() || !slab_.empty()) cuda_check(cudaEventRecord(fork_, stream_), "event");
+        if (!slab_.empty()) {
+            cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
+            for (auto const& w : slab_) {
+                for (SlabRef const& r : w.refs)
+                    if (r.rank == 0) members_[r.sys]->applyStall(side_);
+                cuda_check(launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, dStepsAll_, M,
+                                             (uint32_t)T, dReports_, w.codeMode, side_),
+                           "batch slab");
+                ++launches_;
+            }
+            cuda_check(cudaEventRecord(sideJoin_, side_), "event");
         }
         if (!resident_.empty()) {
             // one launch per group for the whole run, on the second stream
             cuda_check(cudaStreamWaitEvent(stream2_, fork_, 0), "wait");
+            if (!slab_.empty() && residentsAfter_) cuda_check(cudaStreamWaitEvent(stream2_, sideJoin_, 0), "wait");
             for (auto const& g : resident_) {
                 cuda_check(g.codeMode == kCodeNone
                                ? launch_resident(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, dStepsAll_,
@@ -402,11 +479,12 @@ void Batch::run(int32_t const* mcs)
             cuda_check(cudaEventRecord(join_, stream2_), "event");
             cuda_check(cudaStreamWaitEvent(stream_, join_, 0), "wait");
         }
-        for (auto const& g : cluster_) cuda_check(cudaStreamWaitEvent(stream_, sideJoin_[g.side], 0), "wait");
+        if (!slab_.empty()) cuda_check(cudaStreamWaitEvent(stream_, sideJoin_, 0), "wait");
     }
     cuda_check(cudaEventRecord(done_, stream_), "event");
     for (uint32_t m = 0; m < M; ++m) {
-        members_[m]->noteExternalRun(need[m], (uint64_t)mcs[m], !wholeRun_[m], members_[m]->lastColor());
+        members_[m]->noteExternalRun(need[m], (uint64_t)mcs[m], !wholeRun_[m], members_[m]->lastColor(),
+                                     slab_.empty() ? nullptr : std::shared_ptr<GridFault>(reports_, reports_.get() + m));
         members_[m]->streamWait(done_);
     }
 }
@@ -443,18 +521,18 @@ std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
     if (mcsPerTrial <= 0) throw std::invalid_argument("[Batch::autotune] trials need at least one MCS");
     cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
     if (!built_) rebuild();
-    // cluster on and off differ only where a member that does not run resident could run in a
-    // cluster
+    // cluster on and off differ only where a member that does not run resident fits the slab sweep
     bool anyResident = false, anyCluster[2] = {false, false};
     for (Updater* u : members_) {
         anyResident = anyResident || u->residentEligible();
-        bool const cl = u->batchCluster().logC != 0;
+        bool const cl = slabFits(*u);
         anyCluster[0] = anyCluster[0] || cl;
         anyCluster[1] = anyCluster[1] || (cl && !u->residentEligible());
     }
     // Three stages, each configuration timed over the same kind of MCS: first the paths (resident
     // kernel on / off x cluster kernel on / off, where either can matter) with the grid kernels'
-    // defaults; then, for the best paths and if some member runs on the grid-phase kernels, the
+    // defaults; then, for the best paths under which some member runs on the grid-phase kernels (with the
+    // slab sweeps off where they take every member), the
     // check's register budget (kGridShapes) x its CTA size (128, 256, 512 threads), as the
     // reference sweeps its block size (CRITICAL.cu:445-487); last, for the best of those, the
     // perform's warps per CTA x warps per tile.
@@ -482,20 +560,27 @@ std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
             first = false;
         }
     }
-    setResidentEnabled(best.resident);
-    setClusterEnabled(best.cluster);
-    rebuild();
+    bool clusterOn = best.cluster;
+    for (;;) {
+        setResidentEnabled(best.resident);
+        setClusterEnabled(clusterOn);
+        rebuild();
+        if (!grid_.empty() || !clusterOn) break;
+        clusterOn = false;
+    }
     if (!grid_.empty()) {
+        Trial grid{};
         for (int block : {128, 256, 512})
             for (int sh = 0; sh < kGridShapes; ++sh) {
-                Trial const t = time_it(best.resident, best.cluster, sh, block, 0, 0);
-                if (t.msPerMcs < best.msPerMcs) best = t;
+                Trial const t = time_it(best.resident, clusterOn, sh, block, 0, 0);
+                if (grid.msPerMcs == 0.f || t.msPerMcs < grid.msPerMcs) grid = t;
             }
-        Trial const base = best;
+        Trial const base = grid;
         for (auto pw : kPerformShapeTrials) {
             Trial const t = time_it(base.resident, base.cluster, base.shape, base.block, pw[0], pw[1]);
-            if (t.msPerMcs < best.msPerMcs) best = t;
+            if (t.msPerMcs < grid.msPerMcs) grid = t;
         }
+        if (grid.msPerMcs < best.msPerMcs) best = grid;
     }
     setResidentEnabled(best.resident);
     setClusterEnabled(best.cluster);
@@ -525,6 +610,7 @@ float Batch::runTimed(int32_t nMcs)
     cuda_check(cudaEventElapsedTime(&ms, a, b), "elapsed");
     cudaEventDestroy(a);
     cudaEventDestroy(b);
+    checkReports();
     return ms;
 }
 
@@ -532,6 +618,17 @@ void Batch::synchronize()
 {
     cuda_check(cudaStreamSynchronize(stream_), "batch");
     cuda_check(cudaStreamSynchronize(stream2_), "batch");
+    checkReports();
+}
+
+void Batch::checkReports()
+{
+    std::atomic_thread_fence(std::memory_order_acquire);
+    for (auto const& w : slab_)
+        for (SlabRef const& r : w.refs)
+            if (static_cast<GridFault const volatile*>(reports_.get())[r.sys].fault)
+                throw CudaError("[Batch::run] a grid barrier of a member's slab sweep timed out; the state of member " +
+                                std::to_string(r.sys) + " is not usable");
 }
 
 }  // namespace bfm

@@ -95,6 +95,7 @@ struct SysDev {
     uint32_t walls;                  // bit a: axis a is not periodic (corners stay in [0, L-2])
     uint32_t npad, nwords, maxc, nColors;
     struct StepGen* gen;             // device-side producer of the counter stream's sub-step entries
+    struct GridSync* gs;             // barrier of the slab sweep
     uint32_t mask[3];                // lattice side - 1 (a power of two; the box side but along a
                                      // walled axis whose side is not one)
     uint32_t lim[3];                 // box side - 1: on a walled axis a moved corner stays below it
@@ -104,13 +105,22 @@ struct SysDev {
     uint32_t forbid[16];             // bit i set <=> bond index i is forbidden
 };
 
-// Grid-wide barrier of the persistent sweep kernel: a count of arrivals that only grows during a
-// launch (the host zeroes it before every launch); barrier k of a launch completes when the count
-// reaches k x the grid size.
+// Barrier of the CTAs of one system's slab sweep: a count of arrivals that only grows; barrier k of a
+// launch completes when the count reaches base + k x the CTAs, and the launch's last CTA 0 leaves the
+// count it ended at in base.
 struct GridSync {
-    unsigned int count;   // arrivals so far in this launch
-    unsigned int fault;   // set when a wait ran out; every CTA then leaves and the host reports it
-    unsigned int where;   // the barrier (1, 2, ... within the launch) at which the first wait ran out
+    unsigned int count;   // arrivals so far
+    unsigned int base;    // the count at the start of the next launch
+    unsigned int fault;   // set when a wait ran out; every CTA then leaves and the host reports the fault
+    unsigned int pad;
+};
+// The report of a wait that ran out, in mapped host memory.
+struct GridFault {
+    unsigned int fault, where;   // where: the barrier (1, 2, ... within the launch)
+};
+// One CTA of a launch of several systems' slab sweeps.
+struct SlabRef {
+    uint32_t sys, rank, ctas, pad;
 };
 
 // Bond codes: field k (9 bits at 9k) of a monomer's code word is the bond index of

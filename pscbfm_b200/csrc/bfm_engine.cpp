@@ -470,7 +470,7 @@ void Updater::initialize()
     dev_.dSteps = reinterpret_cast<StepEntry*>(base + L.steps) + 1;
     dev_.stepCap = kStepCap;
     dev_.dList = reinterpret_cast<uint32_t*>(base + L.list);
-    dev_.gs = reinterpret_cast<GridSync*>(base + L.gs);
+    h.gs = reinterpret_cast<GridSync*>(base + L.gs);
     dev_.slotOf = reinterpret_cast<uint32_t*>(base + L.slotOf);
     dev_.xyzOut = reinterpret_cast<int32_t*>(base + L.xyzOut);
     dev_.snap = reinterpret_cast<unsigned long long*>(base + L.snap);
@@ -534,7 +534,7 @@ void Updater::initialize()
     cuda_check(cudaMemsetAsync(h.stats, 0, kStatBytes, s), "memset stats");
     cuda_check(cudaMemcpyAsync(dev_.dDesc, &h, sizeof(SysDev), cudaMemcpyHostToDevice, s), "upload descriptor");
     cuda_check(cudaMemsetAsync(dev_.dList, 0, 4, s), "memset list");
-    cuda_check(cudaMemsetAsync(dev_.gs, 0, sizeof(GridSync), s), "memset grid barrier");
+    cuda_check(cudaMemsetAsync(h.gs, 0, sizeof(GridSync), s), "memset grid barrier");
     cuda_check(cudaMemsetAsync(h.gen, 0, sizeof(StepGen), s), "memset step producer");   // off
     cuda_check(cudaMemsetAsync(dev_.snap, 0, 8ull * (4 * kSnapRing + 1), s), "memset snapshots");
     if (segs) {
@@ -548,7 +548,7 @@ void Updater::initialize()
     cuda_check(cudaStreamSynchronize(s), "initialize");
     buildObservables();
     planCluster();
-    slab_plan(grpSize_.data(), nC, maxc_, nwords, codeMode_, smCount_, slab_);
+    slab_plan(grpSize_.data(), nC, maxc_, nwords, codeMode_, slab_ctas(maxGroup_, smCount_), slab_);
     subStep_ = 0;
     mcsDone_ = 0;
     lastColor_ = kNoColor;
@@ -894,9 +894,9 @@ void Updater::ensureStaging()
     // pinned staging of the step entries, allocated on the first run of this system's own paths
     // (systems advanced only by a Batch never need it)
     if (hSteps_) return;
-    // one extra entry holds the copy of the persistent kernel's barrier state, and after it the
+    // one extra entry holds the persistent kernel's report of a failed barrier, and after it the
     // copy of the move counters
-    static_assert(sizeof(GridSync) <= sizeof(StepEntry), "GridSync fits one staging entry");
+    static_assert(sizeof(GridFault) <= sizeof(StepEntry), "GridFault fits one staging entry");
     // (entry kStepCap), then the producer's state and the first entry of a chain (kStepCap + 1,
     // kStepCap + 2, copied together to the producer's slot and the first entry slot)
     void* p = nullptr;
@@ -904,14 +904,16 @@ void Updater::ensureStaging()
                "cudaHostAlloc(steps)");
     hSteps_ = static_cast<StepEntry*>(p);
     hStepCap_ = kStepCap;
-    hGs_ = reinterpret_cast<GridSync*>(hSteps_ + kStepCap);
-    std::memset(hGs_, 0, sizeof(GridSync));
+    hGs_ = reinterpret_cast<GridFault*>(hSteps_ + kStepCap);
+    std::memset(hGs_, 0, sizeof(GridFault));
     hGen_ = reinterpret_cast<StepGen*>(hSteps_ + kStepCap + 1);
     hStats_ = reinterpret_cast<unsigned long long*>(hSteps_ + kStepCap + 3);
     if (!genFree_) cuda_check(cudaEventCreateWithFlags(&genFree_, cudaEventDisableTiming), "cudaEventCreate");
     void* d = nullptr;
     cuda_check(cudaHostGetDevicePointer(&d, hStats_, 0), "stats staging device address");
     dStats_ = static_cast<unsigned long long*>(d);
+    cuda_check(cudaHostGetDevicePointer(&d, hGs_, 0), "barrier report device address");
+    dGs_ = static_cast<GridFault*>(d);
 }
 
 void Updater::scrubPending(cudaStream_t s)
@@ -935,9 +937,11 @@ void Updater::scrubPending(cudaStream_t s)
     lastColor_ = kNoColor;
 }
 
-void Updater::noteExternalRun(uint64_t subSteps, uint64_t mcs, bool pendingMarks, uint32_t lastColor)
+void Updater::noteExternalRun(uint64_t subSteps, uint64_t mcs, bool pendingMarks, uint32_t lastColor,
+                              std::shared_ptr<GridFault> report)
 {
     (void)subSteps;
+    if (report) batchReport_ = std::move(report);
     lastRunSnap_ = false;
     lastRunLead_ = false;   // the batch flushed this system's waiting tickets before it ran
     mcsDone_ += mcs;
@@ -1186,30 +1190,21 @@ void Updater::planCluster()
     // stay small; beyond, the persistent sweep, which reads the lattice from the L2, is at least as fast
     // (us per MCS, cluster against persistent: N = 8K in 64^3 5.7 and 8.3, 16K 7.0 and 8.2, 26K 8.5 and
     // 8.2; in 128^3, 11K (network) 6.8 and 10.7, 26K 10.5 and 8.5, 45K 15.6 and 8.5).
-    // In a Batch: the smallest cluster whose CTAs walk at most two chunks per warp and colour, the better
-    // use of the SMs when several systems share them.
-    cluster_ = batchCluster_ = ClusterPlan{};
+    cluster_ = ClusterPlan{};
     clusterAuto_ = false;
     if (codeMode_ == kCodeNone) return;
     uint32_t const chunks = (maxGroup_ + 31u) / 32u;
-    auto plan = [&](uint32_t logC, uint32_t limit, ClusterPlan& out) {
+    for (uint32_t logC = 4; logC >= 1; --logC) {
         uint32_t const C = 1u << logC, perCta = (chunks + C - 1u) / C, perWarp = (perCta + 31u) / 32u;
-        if (dev_.h.nwords < C || perCta > limit) return false;
+        if (dev_.h.nwords < C || perCta > 256u) continue;
         uint32_t per = 1;
         while (per < perWarp) per *= 2;
         size_t const smem = cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, per, maxc_, codeMode_);
-        if (smem > kResidentMaxSmem || !cluster_bc_runnable(logC, per, smem, codeMode_)) return false;
-        out = ClusterPlan{logC, per, smem};
-        return true;
-    };
-    for (uint32_t logC = 4; logC >= 1; --logC)
-        if (plan(logC, 256u, cluster_)) break;
-    if (cluster_.logC) {
-        uint32_t const C = 1u << cluster_.logC;
-        clusterAuto_ = (chunks + C - 1u) / C * 128u + dev_.h.nwords / C <= 4352u;
+        if (smem > kResidentMaxSmem || !cluster_bc_runnable(logC, per, smem, codeMode_)) continue;
+        cluster_ = ClusterPlan{logC, per, smem};
+        clusterAuto_ = perCta * 128u + dev_.h.nwords / C <= 4352u;
+        return;
     }
-    for (uint32_t logC = 1; logC <= 4; ++logC)
-        if (plan(logC, 64u, batchCluster_)) break;
 }
 
 void Updater::enqueueCluster(uint32_t nSteps)
@@ -1287,6 +1282,13 @@ void Updater::run(int32_t nMcs)
     hostStale_ = true;
 }
 
+void Updater::applyStall(cudaStream_t s)
+{
+    // an arrival count from where no barrier's target is reached
+    if (stallNext_) cuda_check(cudaMemsetAsync(&dev_.h.gs->count, 0x80, sizeof(unsigned int), s), "stall grid barrier");
+    stallNext_ = false;
+}
+
 void Updater::enqueuePersistent(uint32_t nSteps)
 {
     scrubPending(stream_);   // marks of a previous grid-phase run, left for the next check
@@ -1298,20 +1300,13 @@ void Updater::enqueuePersistent(uint32_t nSteps)
                    "steps H2D");
         h2dBytes_ += sizeof(StepEntry) * chunk;
         cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
-        // the arrival count restarts at 0 (an injected stall starts it at 0x80808080, from where no
-        // barrier's target is reached); the fault word stays set once a launch has failed
-        cuda_check(cudaMemsetAsync(&dev_.gs->count, stallNext_ ? 0x80 : 0, sizeof(unsigned int), stream_),
-                   "clear grid barrier");
-        stallNext_ = false;
-        cuda_check(launch_slab_bc(dev_.h, dev_.dSteps, chunk, slab_, dev_.gs, codeMode_, stream_), "persistent sweep");
+        applyStall(stream_);
+        cuda_check(launch_slab_bc(dev_.h, dev_.dSteps, chunk, slab_, dGs_, codeMode_, stream_), "persistent sweep");
         ++launches_;
         done += chunk;
     }
     lastColor_ = kNoColor;   // the launch zeroed its last marks
-    // the fault word comes back with the next synchronisation
-    cuda_check(cudaMemcpyAsync(hGs_, dev_.gs, sizeof(GridSync), cudaMemcpyDeviceToHost, stream_), "grid status");
-    d2hBytes_ += sizeof(GridSync);
-    gsPending_ = true;
+    gsPending_ = true;   // the next synchronisation looks at the report
 }
 
 void Updater::runSimulationOnGPU(int32_t nMcs)
@@ -1328,14 +1323,23 @@ void Updater::streamWait(cudaEvent_t e)
 void Updater::synchronize()
 {
     if (stream_) cuda_check(cudaStreamSynchronize(stream_), "sweep");
+    auto failed = [](GridFault const volatile* f) {
+        if (!f || !f->fault) return;
+        std::ostringstream m;
+        m << "[runSimulationOnGPU] a grid barrier of the persistent sweep timed out (barrier " << f->where
+          << "); the system's state is not usable";
+        throw CudaError(m.str());
+    };
     if (gsPending_) {
         gsPending_ = false;
-        if (hGs_->fault) {
-            std::ostringstream m;
-            m << "[runSimulationOnGPU] a grid barrier of the persistent sweep timed out (barrier " << hGs_->where
-              << "); the system's state is not usable";
-            throw CudaError(m.str());
-        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        failed(hGs_);
+    }
+    if (batchReport_) {
+        std::shared_ptr<GridFault> const r = std::move(batchReport_);
+        batchReport_ = nullptr;
+        std::atomic_thread_fence(std::memory_order_acquire);
+        failed(r.get());
     }
 }
 
@@ -1672,6 +1676,7 @@ void Updater::freeDevice()
         cudaFreeHost(hSteps_);
         hSteps_ = nullptr;
         hGs_ = nullptr;
+        dGs_ = nullptr;
         hGen_ = nullptr;
         hStats_ = nullptr;
         dStats_ = nullptr;

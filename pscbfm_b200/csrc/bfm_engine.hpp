@@ -129,13 +129,11 @@ public:
     uint32_t maxGroup() const { return maxGroup_; }
     bool residentEligible() const;
     bool clusterEligible() const { return cluster_.logC != 0; }
-    // the cluster-resident kernel's plan: log2 CTAs per cluster (0: does not fit), chunks of 32 slots
-    // per warp and colour, dynamic shared memory per CTA (planCluster)
-    struct ClusterPlan {
-        uint32_t logC = 0, perWarp = 0;
-        size_t smem = 0;
-    };
-    ClusterPlan const& batchCluster() const { return batchCluster_; }   // inside a Batch
+    // whether ctas CTAs hold the system in the slab sweep (bond codes), and how
+    bool slabPlan(uint32_t ctas, SlabPlan& plan) const
+    {
+        return slab_plan(grpSize_.data(), (uint32_t)grpSize_.size(), maxc_, dev_.h.nwords, codeMode_, ctas, plan);
+    }
     int gpu() const { return gpu_; }
     void validate();                         // host-side EV and bond-set check (checkSystem)
 
@@ -145,7 +143,9 @@ public:
     uint32_t const* sortedSlot() const { return oldToNew_.data(); }
     StepEntry nextStep();                    // consumes the draws of one sub-step
     void scrubPending(cudaStream_t s);       // clears the temporary marks of the last sub-step
-    void noteExternalRun(uint64_t subSteps, uint64_t mcs, bool pendingMarks, uint32_t lastColor);
+    // report: where a launch of the run may report a failed barrier (looked at by the next synchronise)
+    void noteExternalRun(uint64_t subSteps, uint64_t mcs, bool pendingMarks, uint32_t lastColor,
+                         std::shared_ptr<GridFault> report = nullptr);
     uint32_t lastColor() const { return lastColor_; }
     void streamWait(cudaEvent_t e);          // orders this system's later work after e
     void flushTickets();                     // tickets waiting for a snapshot: from the counters, now
@@ -162,6 +162,7 @@ public:
     float runTimed(int32_t nMcs);            // run + CUDA-event time on the handle's stream (ms)
     // the next persistent launch starts its barrier count where no barrier completes (tests)
     void injectBarrierStall() { stallNext_ = true; }
+    void applyStall(cudaStream_t s);           // ahead of a launch on s: starts its count there if injected
     int path() const;                        // the path the next run takes (BFM_MODE_*)
     void timeKernels(int32_t nMcs, double out[4]);   // check ms, perform ms, launches of each
     uint64_t launches() const { return launches_; }  // kernels launched by this handle so far
@@ -180,7 +181,6 @@ private:
         StepEntry* dSteps = nullptr;
         uint32_t stepCap = 0;
         uint32_t* dList = nullptr;     // resident kernel system list (one entry: 0)
-        GridSync* gs = nullptr;        // grid barrier of the persistent kernel
         uint32_t* slotOf = nullptr;    // [n] sorted slot of each monomer (caller's order)
         int32_t* xyzOut = nullptr;     // [3 n] positions in the caller's order, for read-back
         unsigned long long* snap = nullptr;      // [kSnapRing][4] counter snapshots of graph replays
@@ -238,7 +238,9 @@ private:
     uint64_t chainSub_ = 0, chainSeed_ = 0;
     uint32_t chainPrev_ = kNoColor;
     uint32_t genOn_ = 0;                       // the device producer's `on`, as last written
-    GridSync* hGs_ = nullptr;                  // pinned copy of the persistent kernel's barrier state
+    GridFault* hGs_ = nullptr;                 // mapped report of the persistent kernel's barrier
+    GridFault* dGs_ = nullptr;                 // the same, as the device addresses it
+    std::shared_ptr<GridFault> batchReport_;   // the report of a Batch run not yet synchronised
     unsigned long long* hStats_ = nullptr;     // pinned copy of the move counters (stats)
     unsigned long long* hStatRing_ = nullptr;  // kStatRing mapped pinned slots (statsEnqueue)
     unsigned long long* dStatRing_ = nullptr;  // the same, as the device addresses them
@@ -263,10 +265,15 @@ private:
     bool leadSnapshots() const { return codeMode_ != kCodeNone; }
     cudaStream_t pubStream_ = nullptr;
     cudaEvent_t pubEv_ = nullptr;
-    bool gsPending_ = false;                   // hGs_ is being refreshed by the stream
+    bool gsPending_ = false;                   // a persistent launch may have reported to hGs_
     bool stallNext_ = false;                   // injectBarrierStall
     uint32_t smCount_ = 148;                   // SMs of the device (setGpu)
-    ClusterPlan cluster_, batchCluster_;       // alone, and inside a Batch
+    // the cluster-resident kernel's plan: log2 CTAs per cluster (0: does not fit), chunks of 32 slots
+    // per warp and colour, dynamic shared memory per CTA (planCluster)
+    struct ClusterPlan {
+        uint32_t logC = 0, perWarp = 0;
+        size_t smem = 0;
+    } cluster_;
     bool clusterAuto_ = false;                 // AUTO takes the cluster-resident kernel
     SlabPlan slab_;                            // the persistent sweep's plan (ctas == 0: does not fit)
     uint32_t hStepCap_ = 0;
@@ -318,7 +325,7 @@ public:
 };
 
 // A set of initialised updaters on one GPU advanced together: systems that fit one CTA run in the
-// resident kernel and systems that fit a cluster of CTAs in the cluster-resident kernel (one
+// resident kernel and larger bond-code systems in the slab sweep on several CTAs each (one
 // launch per run and group), the others share one grid-phase launch per phase and sub-step,
 // captured into a CUDA graph. Every system keeps its own draw stream, so its
 // trajectory is identical to running it alone.
@@ -363,15 +370,15 @@ public:
         if (on != residentOn_) built_ = false;
         residentOn_ = on;
     }
-    // members too large for one CTA whose cluster plan beats the grid-phase kernels
-    // (Updater::batchCluster: at most two chunks of 32 slots per warp and colour) run in the
-    // cluster-resident kernel, while the batch's clusters take at most half of the SMs (the rest
-    // stay with the grid-phase kernels)
+    // bond-code members too large for one CTA run in the slab sweep on several CTAs each (planSlabs)
     void setClusterEnabled(bool on)
     {
         if (on != clusterOn_) built_ = false;
         clusterOn_ = on;
     }
+    // SMs the slab sweeps may fill (default: all; a server's lanes share them)
+    void setSlabSms(uint32_t sms);
+    uint32_t smCount() const { return smCount_; }
     cudaStream_t stream() const { return stream_; }
     uint32_t residentCount() const;
     uint32_t clusterCount() const;
@@ -394,17 +401,18 @@ private:
         uint32_t perThread = 1;
         size_t smem = 0;
     };
-    // members of one representation with the same cluster size, one launch per run on a stream
-    // of their own (side_[side])
-    struct ClusterGroup {
+    // members of one representation in the slab sweep, one cooperative launch per run and wave, in order on
+    // one stream (side_[side])
+    struct SlabWave {
         uint32_t codeMode;
-        uint32_t logC;
-        std::vector<uint32_t> members;
-        uint32_t* dList = nullptr;
-        uint32_t perThread = 1;
+        std::vector<SlabRef> refs;      // the launch's CTAs
         size_t smem = 0;
-        size_t side = 0;
+        SlabRef* dRefs = nullptr;
     };
+    static constexpr uint32_t kSlabGrowSlots = 512;   // slots per CTA and colour, at least, where more CTAs join
+    bool slabFits(Updater const& u) const;
+    std::vector<SlabWave> planSlabs(std::vector<char>& taken, bool& residentsAfter) const;
+    void checkReports();                       // throws if a slab sweep of the last run failed
     void rebuild();
     void validateMembers(Updater* const* members, uint32_t n) const;
     cudaError_t launchGrid(StepEntry const* e);   // one sub-step of every grid group, entries [members]
@@ -413,13 +421,17 @@ private:
     void prepare(int32_t const* mcs);            // both, for a run of mcs[i] MCS per member
     int gpu_;
     std::vector<Updater*> members_;
-    std::vector<char> wholeRun_;               // member runs in a resident or cluster kernel
+    std::vector<char> wholeRun_;               // member runs in a resident kernel or a slab sweep
     std::vector<GridGroup> grid_;
     std::vector<ResidentGroup> resident_;
-    std::vector<ClusterGroup> cluster_;
-    std::vector<cudaStream_t> side_;           // streams of the cluster groups (grown, never shrunk)
-    std::vector<cudaEvent_t> sideJoin_;
-    uint32_t smCount_ = 148;
+    std::vector<SlabWave> slab_;
+    std::shared_ptr<GridFault> reports_;       // mapped host memory, one per member
+    GridFault* dReports_ = nullptr;
+    uint32_t reportCap_ = 0;
+    bool residentsAfter_ = false;              // the resident kernels run after the slab sweeps
+    cudaStream_t side_ = nullptr;              // the slab sweeps' stream
+    cudaEvent_t sideJoin_ = nullptr;
+    uint32_t smCount_ = 148, slabSms_ = 148;
     bool residentOn_ = true;
     bool clusterOn_ = true;
     bool built_ = false;

@@ -101,13 +101,14 @@ inline bool perform_shape_ok(int warps, int group)
 cudaError_t launch_perform_bc(SysDev const& hostDesc, SysDev const* dSys, TileRef const* dTiles, uint32_t nTiles,
                               StepEntry const* dSteps, uint32_t codeMode, cudaStream_t s, int shape = -1,
                               PerformArgs const& pa = PerformArgs{});
-// Persistent sweep (bond codes, one system): nSteps sub-steps in one cooperative launch of
-// plan.ctas CTAs, each holding its share of the slots in shared memory (k_slab_bc). slab_plan
-// returns false where the system does not fit (more than kSlabColors colours, or too many slots per
-// CTA). gs->count must be zeroed before the launch; after it, gs->fault != 0 means a grid-barrier
-// wait ran out and the system's state is not usable.
+// Slab sweeps (bond codes): nSteps sub-steps of a system by plan.ctas CTAs of a cooperative launch, each
+// holding its share of the slots in shared memory (slab_sweep): one system (k_slab_bc), or several in one
+// launch (k_slab_batch_bc). slab_plan returns false where the system does not fit ctas CTAs (more than
+// kSlabColors colours, or too many slots per CTA). report (mapped host memory): its fault word is set
+// when a grid-barrier wait ran out; the system's state is then not usable.
 // threads per CTA (one CTA per SM); 64-bit codes keep up to six neighbours of a mover in registers
-constexpr uint32_t kSlabBlock32 = 640, kSlabBlock64 = 512;
+constexpr uint32_t kSlabBlock32 = 640, kSlabBlock64 = 512, kSlabBlockSmall = 256;
+constexpr uint32_t kSlabSmallSlots = 1024;   // slots per CTA and colour, at most, of the small CTAs
 constexpr uint32_t kSlabColors = 8;          // bond codes: at most 6 bonds, so at most 7 colours
 constexpr uint32_t kSlabEntBits = 13;         // list entries: a slot's index in its colour's part, and 3 direction bits
 // bits of a local index in a 16-bit neighbour reference, below the reverse slot (0-2, or 0-5 with 64-bit codes)
@@ -116,15 +117,23 @@ constexpr uint32_t kSlabMinChunks = 8;       // chunks of 32 slots per CTA and c
 constexpr size_t kSlabMaxSmem = kResidentMaxSmem;
 struct SlabPlan {
     uint32_t ctas = 0;         // 0: the system does not fit
-    uint32_t cap = 0, capG = 0;   // slots a CTA holds in all and of its largest colour group
-    uint32_t clearAll = 0;     // zero the previous temporary lattice whole
+    uint32_t cap = 0, perCta = 0;   // slots a CTA holds in all, and of the largest colour group
+    uint32_t threads = 0;      // threads per CTA
+    bool clearAll = false;     // the temporary lattice is zeroed whole
     bool cache = false;        // the neighbour references and inner direction hashes fit in shared memory too
-    size_t smem = 0;
+    size_t smem = 0;           // dynamic shared memory per CTA
 };
 bool slab_plan(uint32_t const* grpSize, uint32_t nColors, uint32_t maxc, uint32_t nwords, uint32_t codeMode,
-               uint32_t sms, SlabPlan& plan);
+               uint32_t ctas, SlabPlan& plan);
+// CTAs of a cooperative launch for a system whose largest colour group is maxGroup
+uint32_t slab_ctas(uint32_t maxGroup, uint32_t sms);
 cudaError_t launch_slab_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
-                           GridSync* gs, uint32_t codeMode, cudaStream_t s);
+                           GridFault* report, uint32_t codeMode, cudaStream_t s);
+// Plans with the cache only; dRefs: the launch's CTAs; the entries of sub-step t are
+// dSteps[t * stride + system], the reports report[system].
+cudaError_t launch_slab_batch(SysDev const* dSys, SlabRef const* dRefs, uint32_t ctas, size_t smem,
+                              StepEntry const* dSteps, uint32_t stride, uint32_t nSteps, GridFault* report,
+                              uint32_t codeMode, cudaStream_t s);
 // Dynamic shared memory of the bond-code resident kernel, with the neighbour references where they fit too.
 size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t maxc, uint32_t codeMode);
 // Cluster-resident sweep (bond codes): one cluster of 2^logC CTAs of kResidentBlock threads per

@@ -89,8 +89,10 @@ __device__ __forceinline__ void plane_ref(PlaneRef& r, unsigned long long const*
 {
     uint32_t ti, touch;
     front_plane_words(r.w, ti, touch, D, base, da, dir);
-    ulonglong2 const m01 = *reinterpret_cast<ulonglong2 const*>(ptab + ti);
-    ulonglong2 const m23 = *reinterpret_cast<ulonglong2 const*>(ptab + ti + 2);
+    // entry ti / 4, its first two masks in the table's first half and the others in the second: 16-byte
+    // entries spread over all banks (21 wavefronts per warp, 28 with the 32-byte entries of planeTab)
+    ulonglong2 const m01 = *reinterpret_cast<ulonglong2 const*>(ptab + ti / 2u);
+    ulonglong2 const m23 = *reinterpret_cast<ulonglong2 const*>(ptab + 384u + ti / 2u);
     r.m[0] = m01.x;
     r.m[1] = m01.y;
     r.m[2] = m23.x;
@@ -472,9 +474,9 @@ __global__ void __launch_bounds__(32 * PW) k_perform_bc(const __grid_constant__ 
 
 // ---------------------------------------------------------------------------------- persistent
 
-// A wait longer than 2 s is a fault; a launch's first wait may take 20 s, since it ends only once every
-// CTA has found a free SM (another stream's kernel may hold some for a while).
-constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull, kFirstBarrierTimeoutNs = 20000000000ull;
+// A wait longer than this is a fault: a launch's first wait ends only once every CTA has found a free SM,
+// and another stream's kernel may hold some for a while.
+constexpr unsigned long long kBarrierTimeoutNs = 20000000000ull;
 
 __device__ __forceinline__ unsigned int ld_acquire_gpu(unsigned int const* p)
 {
@@ -497,24 +499,23 @@ __device__ __forceinline__ void red_release_gpu_add(unsigned int* p, unsigned in
 
 // One thread of each CTA, after a CTA barrier that ordered the CTA's earlier writes before it: adds
 // the CTA's arrival to a count that only grows (a release add) and waits with acquire loads until
-// the count reaches this barrier's target, nCtas above the previous one. Nothing is reset between
-// barriers, and the signed difference keeps the comparison right across a wrap of the count. The
-// wait is bounded by time and by a poll count; false if it ran out or another CTA's did
-// (GridSync::fault): the kernel then leaves, and the host reports the fault.
+// the count reaches this barrier's target, nCtas above the previous one (the first one's is
+// base + nCtas). Nothing is reset between barriers, and the signed difference keeps the comparison right
+// across a wrap of the count. The wait is bounded by time and by a poll count; false if it ran out or
+// another CTA's did (GridSync::fault): the kernel then leaves, and the host reports the fault.
 __device__ __forceinline__ bool grid_meet(GridSync* gs, unsigned int& target, unsigned int nCtas)
 {
     target += nCtas;
     red_release_gpu_add(&gs->count, 1u);
     if (int(ld_acquire_gpu(&gs->count) - target) < 0) {
-        bool const first = target == nCtas;
-        unsigned long long const t0 = global_ns(), limit = first ? kFirstBarrierTimeoutNs : kBarrierTimeoutNs;
+        unsigned long long const t0 = global_ns();
         unsigned int polls = 0u;
         while (int(ld_acquire_gpu(&gs->count) - target) < 0) {
             // a time limit, and a poll count as a second bound that does not trust the timer
             if ((++polls & 255u) == 0u) {
                 if (ld_acquire_gpu(&gs->fault) != 0u) return false;
-                if (global_ns() - t0 > limit || polls > (first ? 1u << 27 : 1u << 24)) {
-                    if (atomicExch(&gs->fault, 1u) == 0u) gs->where = target / nCtas;
+                if (global_ns() - t0 > kBarrierTimeoutNs || polls > (1u << 27)) {
+                    gs->fault = 1u;
                     return false;
                 }
             }
@@ -524,7 +525,12 @@ __device__ __forceinline__ bool grid_meet(GridSync* gs, unsigned int& target, un
     return true;
 }
 
-// Slab-resident layout (k_slab_bc): CTA r of C holds, of every colour group of n slots in
+// The two halves of a cluster barrier: after the first every earlier access of the thread is on its
+// way, after the second those of all threads of the cluster are in place.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Slab layout (slab_sweep): CTA r of C holds, of every colour group of n slots in
 // chunks of 32, chunks [r nch / C, (r + 1) nch / C), nch = ceil(n / 32): contiguous slots, in the
 // group's order, so the neighbours of a chain numbered along its bonds mostly lie in the same CTA.
 struct SlabPart {
@@ -570,29 +576,58 @@ __device__ __forceinline__ unsigned long long plane_hits(PlaneRef const& r, bool
     return (v[0] & r.m[0]) | (v[1] & r.m[1]) | (v[2] & r.m[2]) | (v[3] & r.m[3]);
 }
 
-// One system, a whole run of sub-steps in one cooperative launch, one CTA per SM. Lattice and
-// temporary lattices stay in global memory (the L2); each CTA keeps the lattice addresses and code
-// words of its slots (SlabPart) in shared memory. Per sub-step two grid barriers: after the check
-// (every mark is set) and after the perform (the lattice is settled). The last warp waits at the
-// barriers; the others meanwhile do all of the next phase that depends on this CTA's own slots only:
-// bond tests, candidates and their planes before the check's lattice reads; the list of movers,
-// their codes, neighbour references and planes, the clearing of the previous marks and the
-// directions of the next sub-step before the perform's temporary-lattice reads. What is left between
-// two barriers is one round of L2 reads and the writes that follow from it.
+// Shared memory of a CTA of the slab sweeps: cap slots in all, capG of the largest colour group.
+__host__ __device__ __forceinline__ size_t slab_layout(uint32_t cap, uint32_t capG, bool clearAll, bool cache,
+                                                       uint32_t maxc, uint32_t codeBytes)
+{
+    return 768 * 8 + kDirTab * 4 + (size_t)cap * (codeBytes + 4) + (size_t)capG * (clearAll ? 4 : 8) + 512 +
+           (cache ? (size_t)cap * 4 + (size_t)maxc * cap * 2 : 0);
+}
+// Slots a CTA of C holds at most of all colour groups and of the largest one, and the system's slots.
+template <typename F>
+__host__ __device__ __forceinline__ void slab_caps(F size, uint32_t nColors, uint32_t C, uint32_t& cap, uint32_t& capG,
+                                                   uint32_t& n)
+{
+    cap = capG = n = 0;
+    for (uint32_t c = 0; c < nColors; ++c) {
+        uint32_t const own = 32u * ((((size(c) + 31u) >> 5) + C - 1u) / C);
+        cap += own;
+        capG = capG > own ? capG : own;
+        n += size(c);
+    }
+}
+// Dense systems clear the temporary lattice whole: nwords x 8 B written in order, against one scattered
+// write per mark.
+__host__ __device__ __forceinline__ bool slab_clear_all(uint32_t nwords, uint32_t nSlots) { return nwords <= 2u * nSlots; }
+
+// The sweep of one system by C CTAs (this one's rank among them), a whole run of sub-steps in one launch.
+// Lattice and temporary lattices stay in global memory (the L2); each CTA keeps the lattice addresses and
+// code words of its slots (SlabPart) in shared memory. Per sub-step two barriers of the CTAs: after the
+// check (every mark is set) and after the perform (the lattice is settled). The last warp sees the CTA's
+// writes through and waits; the others meanwhile do all of the next phase that depends on this CTA's own
+// slots only: bond tests, candidates and their planes before the check's lattice reads; the list of
+// movers, their codes, neighbour references and planes, the clearing of the previous marks and the
+// directions of the next sub-step before the perform's temporary-lattice reads. What is left between two
+// barriers is one round of L2 reads and the writes that follow from it.
 //   kCache: the slots' inner direction hashes and neighbour references in shared memory too.
-//   clearAll: the previous temporary lattice is zeroed whole, each CTA its share, instead of by the
-//   targets listed in it (a dense system marks most of its words).
-// Bound: on the 256^3 melt (N = 1,048,576) by the scattered L2 accesses (about 0.8 loads and 0.57
-// atomics per clock and SM) and instruction issue (27 K warp instructions per SM and sub-step); below
-// 200K monomers by the barriers (1.3-1.8 us each with the writes before them) and one L2 round trip
-// after each. Per MCS: melt 14.9 us (graph of launches 21.7), 131K monomers 9.6 (13.4; 15 with the
-// cooperative sweep that kept every record in global memory), 60K 8.6 (15.2).
+// The CTAs are part of a cooperative launch and meet at a count in global memory (S.gs). A thread-block
+// cluster and its barrier in hardware were no faster (131K monomers on 16 CTAs 9.7 us per sub-step
+// against 8.9: every warp's wait drops the SM's L1 lines), and its CTAs have to fit one GPC.
+// kIdle: entries may be idle (kNoColor). cap, capG: slots of a CTA in all and of the largest colour group, at most (slab_caps); entries of
+// sub-step t at steps[t * stride].
+// Bound: on the 256^3 melt (N = 1,048,576, 148 CTAs) by the scattered L2 accesses (about 0.8 loads and
+// 0.57 atomics per clock and SM), the integer pipe and instruction issue (24 K warp instructions per SM
+// and sub-step); below 200K monomers by the barriers (1.3-1.8 us each with the writes before them) and
+// one L2 round trip after each. Per MCS: melt 14.9 us (graph of launches 21.7), 131K monomers 9.6 (13.4;
+// 15 with the cooperative sweep that kept every record in global memory), 60K 8.6 (15.2).
 // 640 threads: 20 warps of 96 registers hold two prepared candidates per thread (the melt has 1.9
-// per thread) and its movers fit one pass; 1024 threads of 64 registers spilled and took 18 us.
-template <typename W, int B, bool kCache>
-__global__ void __launch_bounds__(B, 1)
-    k_slab_bc(const __grid_constant__ SysDev S, StepEntry const* __restrict__ steps, uint32_t nSteps, uint32_t cap,
-              uint32_t capG, uint32_t clearAll, GridSync* gs)
+// per thread) and its movers fit one pass; 512 threads took 17.6 us per MCS there, 768 16.3, 1024 18.
+// CTAs with at most kSlabSmallSlots slots per colour have 256: fewer warps meet faster at the CTA's own
+// barriers (131K monomers 9.0 against 9.6 us per MCS, 210K 9.3 against 9.9, 60K 7.9 against 8.5).
+template <typename W, int B, bool kCache, bool kIdle>
+__device__ __forceinline__ void slab_sweep(SysDev const& S, StepEntry const* __restrict__ steps, uint32_t stride,
+                                           uint32_t nSteps, uint32_t C, uint32_t rank, uint32_t cap, uint32_t capG,
+                                           bool clearAll, GridFault* report)
 {
     constexpr uint32_t kSlots = CodeWord<W>::kSlots;
     constexpr W kShared = slab_shared_flag<W>();
@@ -608,17 +643,7 @@ __global__ void __launch_bounds__(B, 1)
     extern __shared__ unsigned long long smem[];
     uint32_t const tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     bool const waiter = warp == nWork;
-    uint32_t const C = gridDim.x, rank = blockIdx.x;
-    unsigned long long* const ptab = smem;                                   // 768 plane masks
-    uint32_t* const dtab = reinterpret_cast<uint32_t*>(smem + 768);          // kDirTab words
-    W* const code = reinterpret_cast<W*>(smem + 768 + kDirTab / 2);          // cap slots
-    uint32_t* const pk = reinterpret_cast<uint32_t*>(code + cap);            // cap slots
-    uint16_t* const cand = reinterpret_cast<uint16_t*>(pk + cap);            // capG candidates
-    uint16_t* const list = cand + capG;                                      // capG movers
-    uint32_t* const tgt = reinterpret_cast<uint32_t*>(list + capG);          // !clearAll: capG marked addresses
-    uint8_t* const mok = reinterpret_cast<uint8_t*>(tgt + (clearAll ? 0u : capG));   // 512 move-table bytes
-    uint32_t* const inner = reinterpret_cast<uint32_t*>(mok + 512);          // kCache: cap hashes
-    uint16_t* const refs = reinterpret_cast<uint16_t*>(inner + cap);         // kCache: maxc x cap references
+    GridSync* const gs = S.gs;
     if (ld_acquire_gpu(&gs->fault) != 0u) return;   // an earlier launch failed: the state is not usable
     uint32_t const nColors = S.nColors, np = S.npad;
     if (tid == 0) {
@@ -631,11 +656,19 @@ __global__ void __launch_bounds__(B, 1)
             P.base[c] = b;
             b += 32u * (hi - lo);
         }
-        nCand = 0u;
-        nMov = 0u;
-        tallyA = 0u;
+        nCand = nMov = tallyA = 0u;
     }
-    for (uint32_t w = tid; w < 768; w += B) ptab[w] = S.planeTab[w];
+    unsigned long long* const ptab = smem;                                   // 768 plane masks
+    uint32_t* const dtab = reinterpret_cast<uint32_t*>(smem + 768);          // kDirTab words
+    W* const code = reinterpret_cast<W*>(smem + 768 + kDirTab / 2);          // cap slots
+    uint32_t* const pk = reinterpret_cast<uint32_t*>(code + cap);            // cap slots
+    uint16_t* const cand = reinterpret_cast<uint16_t*>(pk + cap);            // capG candidates
+    uint16_t* const list = cand + capG;                                      // capG movers
+    uint32_t* const tgt = reinterpret_cast<uint32_t*>(list + capG);          // !clearAll: capG marked addresses
+    uint8_t* const mok = reinterpret_cast<uint8_t*>(tgt + (clearAll ? 0u : capG));   // 512 move-table bytes
+    uint32_t* const inner = reinterpret_cast<uint32_t*>(mok + 512);          // kCache: cap hashes
+    uint16_t* const refs = reinterpret_cast<uint16_t*>(inner + cap);         // kCache: maxc x cap references
+    for (uint32_t w = tid; w < 768; w += B) ptab[(w & 2u ? 384u : 0u) + (w >> 2) * 2u + (w & 1u)] = S.planeTab[w];
     if (tid < kDirTab) dtab[tid] = S.dirTab[tid];
     for (uint32_t w = tid; w < 512; w += B) mok[w] = S.moveOk[w];
     __syncthreads();
@@ -702,21 +735,34 @@ __global__ void __launch_bounds__(B, 1)
         if (lane == 0) at = shared_add(count, (uint32_t)__popc(bal));
         return __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanesBelow);
     };
-    unsigned int target = 0u;   // (the waiter's) count target of the next barrier
+    // a barrier of the CTAs in two halves, between which the workers prepare; a CTA barrier comes before
+    // the first. The waiter alone carries the CTA's writes over (it orders them after the CTA barrier)
+    unsigned int target = gs->base;   // (the waiter's) count target of the next barrier
+    auto meet_begin = [&]() {   // false on the waiter if a wait ran out
+        bool met = true;
+        if (waiter && lane == 0) met = grid_meet(gs, target, C);
+        __syncwarp();
+        return met;
+    };
+    auto meet_end = [&](bool met) {   // whether every CTA came
+        if (__syncthreads_or(!met) == 0) return true;
+        if (waiter && lane == 0) *report = GridFault{1u, (target - gs->base) / C};
+        return false;
+    };
     bool const walled = S.walls != 0u;
     uint32_t const cw0 = (uint32_t)((uint64_t)S.nwords * rank / C), cw1 = (uint32_t)((uint64_t)S.nwords * (rank + 1u) / C);
     uint32_t prevMov = 0u, nAcc = 0u, nTent = 0u, par = 0u, dirs = 0u;
+    bool began = false, drawn = false;   // a sub-step has run; dirs belong to the next one
     unsigned long long att = 0ull;
     StepEntry next = steps[0];
-    if (!waiter) dirs = directions(next, 0);
     for (uint32_t t = 0; t < nSteps; ++t) {
         StepEntry const st = next;
-        if (t + 1 < nSteps) next = steps[t + 1];
+        if (t + 1 < nSteps) next = steps[(size_t)(t + 1) * stride];
+        if (kIdle && st.color == kNoColor) continue;
         par = st.parity;
         att += st.cnt;
         uint32_t const first = P.first[st.color], base = P.base[st.color];
         unsigned long long* const tcur = S.tmp + (size_t)par * S.nwords;
-        bool bad = false;   // (the waiter's) barrier wait ran out
         // check, part 1 (own slots only): walls and bonds -> candidates, and their planes
         uint32_t nc = 0, ent[kPre], to[kPre], far = 0u, go = 0u;   // far, go: bit q, candidate q
         PlaneRef pr[kPre];
@@ -732,13 +778,10 @@ __global__ void __launch_bounds__(B, 1)
         auto far_ok = [&](uint32_t en) {
             return bonds_ok<W, true>(__ldcg(rec_code<W>(S.rec, first + (en & kEntMask))), en >> kSlabEntBits, mok);
         };
-        if (waiter) {
-            if (lane == 0) {
-                nMov = 0u;
-                bad = t > 0 && !grid_meet(gs, target, C);
-            }
-            __syncwarp();
-        } else {
+        if (waiter && lane == 0) nMov = 0u;
+        bool met = began ? meet_begin() : true;
+        if (!waiter) {
+            if (!drawn) dirs = directions(st, 0);
             // slots held here, and those before the group's end (the last chunk may be padded)
             uint32_t const n = P.count[st.color], left = min(n, st.cnt - (first - st.off));
             uint32_t const t0 = warp * 32u;   // (n is a multiple of 32: a warp's slots end together)
@@ -786,7 +829,12 @@ __global__ void __launch_bounds__(B, 1)
                     far |= 1u << q;
             }
         }
-        if (__syncthreads_or(bad)) return;
+        if (began) {
+            if (!meet_end(met)) return;
+        } else {
+            __syncthreads();
+        }
+        began = true;
         // check, part 2: the front planes; free candidates mark their target
         if (!waiter) {
             uint32_t const w0 = warp * 32u;   // (the tests on it are the same for the whole warp)
@@ -850,13 +898,10 @@ __global__ void __launch_bounds__(B, 1)
             }
             wraps = (((dir & 1u) ? mTo : from) & D.ma) == 0u ? int32_t((dir >> 1) | ((dir & 1u) << 2)) : -1;
         };
-        if (waiter) {
-            if (lane == 0) {
-                nCand = 0u;
-                bad = !grid_meet(gs, target, C);
-            }
-            __syncwarp();
-        } else {
+        if (waiter && lane == 0) nCand = 0u;
+        met = meet_begin();
+        drawn = t + 1 < nSteps && (!kIdle || next.color != kNoColor);
+        if (!waiter) {
             if (warp * 32u < nc) {
                 static_assert(kPre == 2, "the candidates of a warp go to the list together");
                 uint32_t const b0 = __ballot_sync(0xffffffffu, go & 1u), b1 = __ballot_sync(0xffffffffu, go & 2u);
@@ -882,9 +927,9 @@ __global__ void __launch_bounds__(B, 1)
                     }
                 }
             }
-            if (t + 1 < nSteps) dirs = directions(next, 0);
+            if (drawn) dirs = directions(next, 0);
         }
-        if (__syncthreads_or(bad)) return;
+        if (!meet_end(met)) return;
         // perform, part 2: front planes on the temporary lattice; the free movers move
         if (!waiter) {
             for (uint32_t e = tid; e < nm; e += kThreads) {
@@ -913,10 +958,8 @@ __global__ void __launch_bounds__(B, 1)
         __syncthreads();   // this CTA's slots are settled for the next check's first part
     }
     // every perform has read the last marks: zero them, and write the slots back
-    bool bad = false;
-    if (waiter && lane == 0) bad = !grid_meet(gs, target, C);
-    __syncwarp();
-    if (__syncthreads_or(bad)) return;
+    if (began && !meet_end(meet_begin())) return;
+    if (began && rank == 0 && waiter && lane == 0) gs->base = target;   // (every CTA has read it)
     unsigned long long* const tlast = S.tmp + (size_t)par * S.nwords;
     if (clearAll) {
         for (uint32_t w = cw0 + tid; w < cw1; w += B) tlast[w] = 0ull;
@@ -937,6 +980,34 @@ __global__ void __launch_bounds__(B, 1)
         tally_flush(tallyA, S.stats, 2);
         if (rank == 0 && att) atomicAdd(S.stats, att);
     }
+}
+
+template <typename W, int B, bool kCache>
+__global__ void __launch_bounds__(B, 1)
+    k_slab_bc(const __grid_constant__ SysDev S, StepEntry const* __restrict__ steps, uint32_t nSteps, uint32_t cap,
+              uint32_t capG, uint32_t clearAll, GridFault* report)
+{
+    slab_sweep<W, B, kCache, false>(S, steps, 1u, nSteps, gridDim.x, blockIdx.x, cap, capG, clearAll != 0u, report);
+}
+
+// Many systems in one cooperative launch: CTA b runs share refs[b].rank of system refs[b].sys with the
+// other CTAs of that system, and waits for no others; the entries of sub-step t are
+// steps[t * stride + system], the reports report[system].
+template <typename W, int B>
+__global__ void __launch_bounds__(B, 1)
+    k_slab_batch_bc(SysDev const* __restrict__ sysv, SlabRef const* __restrict__ refs,
+                    StepEntry const* __restrict__ steps, uint32_t stride, uint32_t nSteps, GridFault* report)
+{
+    __shared__ SysDev S;
+    __shared__ uint32_t caps[3];
+    SlabRef const r = refs[blockIdx.x];
+    copy_desc(S, sysv + r.sys);
+    __syncthreads();
+    if (threadIdx.x == 0)
+        slab_caps([&](uint32_t c) { return S.grp[2 * c + 1]; }, S.nColors, r.ctas, caps[0], caps[1], caps[2]);
+    __syncthreads();
+    slab_sweep<W, B, true, true>(S, steps + r.sys, stride, nSteps, r.ctas, r.rank, caps[0], caps[1],
+                                 slab_clear_all(S.nwords, caps[2]), report + r.sys);
 }
 
 // ---------------------------------------------------------------------------------- resident
@@ -1274,11 +1345,6 @@ __device__ __forceinline__ void cluster_xor(uint32_t a, unsigned long long v, bo
     cluster_xor(a, (uint32_t)v, on && (uint32_t)v != 0u);
     cluster_xor(a + 4u, (uint32_t)(v >> 32), on && (v >> 32) != 0ull);
 }
-// The two halves of a cluster barrier: after the first every earlier access of the thread is on its
-// way, after the second those of all threads of the cluster are in place.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 // Shared memory of k_cluster_bc per CTA (cluster_bc_smem_bytes); nb: neighbour references kept here (0:
 // they stay in global memory).
 __host__ __device__ __forceinline__ size_t cluster_layout(uint32_t nwords, uint32_t npad, uint32_t logC,
@@ -1662,62 +1728,101 @@ cudaError_t launch_perform_bc(SysDev const& hostDesc, SysDev const* dSys, TileRe
 }
 
 bool slab_plan(uint32_t const* grpSize, uint32_t nColors, uint32_t maxc, uint32_t nwords, uint32_t codeMode,
-               uint32_t sms, SlabPlan& plan)
+               uint32_t ctas, SlabPlan& plan)
 {
     plan = SlabPlan{};
-    if (codeMode == kCodeNone || nColors == 0 || nColors > kSlabColors) return false;
-    uint32_t maxCh = 1;
-    for (uint32_t c = 0; c < nColors; ++c) maxCh = std::max(maxCh, (grpSize[c] + 31u) >> 5);
-    uint32_t const C = std::min(sms, (maxCh + kSlabMinChunks - 1u) / kSlabMinChunks);
-    uint32_t cap = 0, capG = 0, n = 0;
-    for (uint32_t c = 0; c < nColors; ++c) {
-        uint32_t const own = 32u * ((((grpSize[c] + 31u) >> 5) + C - 1u) / C);
-        cap += own;
-        n += grpSize[c];
-        capG = std::max(capG, own);
-    }
-    size_t const w = codeMode == kCode64 ? 8 : 4;
+    if (codeMode == kCodeNone || nColors == 0 || nColors > kSlabColors || ctas == 0) return false;
+    uint32_t cap, capG, n;
+    slab_caps([&](uint32_t c) { return grpSize[c]; }, nColors, ctas, cap, capG, n);
     if (capG > 1u << kSlabEntBits) return false;
-    // dense systems clear the temporary lattice whole (nwords x 8 B against two scattered accesses per mark)
-    uint32_t const clearAll = nwords <= 2u * n ? 1u : 0u;
-    size_t const smem = 768 * 8 + kDirTab * 4 + (size_t)cap * (w + 4) + (size_t)capG * (clearAll ? 4 : 8) + 512;
-    if (smem > kSlabMaxSmem) return false;
-    size_t const cache = (size_t)cap * 4 + (size_t)maxc * cap * 2;
-    bool const fits = smem + cache <= kSlabMaxSmem && cap < (1u << slab_ref_bits(codeMode == kCode64));
-    plan = SlabPlan{C, cap, capG, clearAll, fits, fits ? smem + cache : smem};
+    uint32_t const w = codeMode == kCode64 ? 8 : 4;
+    bool const clearAll = slab_clear_all(nwords, n);
+    size_t const least = slab_layout(cap, capG, clearAll, false, maxc, w), all = slab_layout(cap, capG, clearAll, true, maxc, w);
+    if (least > kSlabMaxSmem) return false;
+    bool const cache = all <= kSlabMaxSmem && cap < (1u << slab_ref_bits(w == 8));
+    uint32_t const threads = cache && capG <= kSlabSmallSlots ? kSlabBlockSmall : (w == 8 ? kSlabBlock64 : kSlabBlock32);
+    plan = SlabPlan{ctas, cap, capG, threads, clearAll, cache, cache ? all : least};
     return true;
+}
+
+uint32_t slab_ctas(uint32_t maxGroup, uint32_t sms)
+{
+    return std::min(sms, std::max(1u, (((maxGroup + 31u) >> 5) + kSlabMinChunks - 1u) / kSlabMinChunks));
 }
 
 namespace {
 
 template <typename W, int B, bool kCache>
 cudaError_t launch_slab_bc_w(SysDev const& S, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
-                             GridSync* gs, cudaStream_t s)
+                             GridFault* report, cudaStream_t s)
 {
     static thread_local bool done[64] = {};
     cudaError_t const e = allow_smem(k_slab_bc<W, B, kCache>, done);
     if (e != cudaSuccess) return e;
-    uint32_t cap = plan.cap, capG = plan.capG, clearAll = plan.clearAll;
-    void* args[] = {const_cast<SysDev*>(&S), &dSteps, &nSteps, &cap, &capG, &clearAll, &gs};
+    uint32_t cap = plan.cap, perCta = plan.perCta, clearAll = plan.clearAll ? 1u : 0u;
+    void* args[] = {const_cast<SysDev*>(&S), &dSteps, &nSteps, &cap, &perCta, &clearAll, &report};
     return cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(k_slab_bc<W, B, kCache>), dim3(plan.ctas), dim3(B),
                                        args, plan.smem, s);
+}
+
+// Calls f.operator()<W, B, kCache>() for a code mode and a plan.
+template <typename W, int B, typename F>
+auto slab_dispatch_w(SlabPlan const& plan, F f)
+{
+    if (plan.threads == kSlabBlockSmall) return f.template operator()<W, (int)kSlabBlockSmall, true>();
+    return plan.cache ? f.template operator()<W, B, true>() : f.template operator()<W, B, false>();
+}
+template <typename F>
+auto slab_dispatch(uint32_t codeMode, SlabPlan const& plan, F f)
+{
+    return codeMode == kCode64 ? slab_dispatch_w<unsigned long long, (int)kSlabBlock64>(plan, f)
+                               : slab_dispatch_w<uint32_t, (int)kSlabBlock32>(plan, f);
+}
+
+struct SlabLaunch {
+    SysDev const& S;
+    StepEntry const* dSteps;
+    uint32_t nSteps;
+    SlabPlan const& plan;
+    GridFault* report;
+    cudaStream_t s;
+    template <typename W, int B, bool kCache>
+    cudaError_t operator()() const { return launch_slab_bc_w<W, B, kCache>(S, dSteps, nSteps, plan, report, s); }
+};
+
+template <typename W, int B>
+cudaError_t launch_slab_batch_w(SysDev const* dSys, SlabRef const* dRefs, uint32_t ctas, size_t smem,
+                                StepEntry const* dSteps, uint32_t stride, uint32_t nSteps, GridFault* report,
+                                cudaStream_t s)
+{
+    static thread_local bool done[64] = {};
+    cudaError_t const e = allow_smem(k_slab_batch_bc<W, B>, done);
+    if (e != cudaSuccess) return e;
+    void* args[] = {&dSys, &dRefs, &dSteps, &stride, &nSteps, &report};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(k_slab_batch_bc<W, B>), dim3(ctas), dim3(B), args,
+                                       smem, s);
 }
 
 }  // namespace
 
 cudaError_t launch_slab_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
-                           GridSync* gs, uint32_t codeMode, cudaStream_t s)
+                           GridFault* report, uint32_t codeMode, cudaStream_t s)
 {
     if (nSteps == 0) return cudaSuccess;
-    if (plan.ctas == 0) return cudaErrorInvalidValue;
-    using U = unsigned long long;
-    constexpr int B32 = (int)kSlabBlock32, B64 = (int)kSlabBlock64;
+    if (plan.ctas == 0 || codeMode == kCodeNone) return cudaErrorInvalidValue;
+    return slab_dispatch(codeMode, plan, SlabLaunch{hostDesc, dSteps, nSteps, plan, report, s});
+}
+
+cudaError_t launch_slab_batch(SysDev const* dSys, SlabRef const* dRefs, uint32_t ctas, size_t smem,
+                              StepEntry const* dSteps, uint32_t stride, uint32_t nSteps, GridFault* report,
+                              uint32_t codeMode, cudaStream_t s)
+{
+    if (ctas == 0 || nSteps == 0) return cudaSuccess;
     if (codeMode == kCode32)
-        return plan.cache ? launch_slab_bc_w<uint32_t, B32, true>(hostDesc, dSteps, nSteps, plan, gs, s)
-                         : launch_slab_bc_w<uint32_t, B32, false>(hostDesc, dSteps, nSteps, plan, gs, s);
+        return launch_slab_batch_w<uint32_t, (int)kSlabBlock32>(dSys, dRefs, ctas, smem, dSteps, stride, nSteps, report, s);
     if (codeMode == kCode64)
-        return plan.cache ? launch_slab_bc_w<U, B64, true>(hostDesc, dSteps, nSteps, plan, gs, s)
-                         : launch_slab_bc_w<U, B64, false>(hostDesc, dSteps, nSteps, plan, gs, s);
+        return launch_slab_batch_w<unsigned long long, (int)kSlabBlock64>(dSys, dRefs, ctas, smem, dSteps, stride, nSteps,
+                                                                          report, s);
     return cudaErrorInvalidValue;
 }
 
@@ -1778,34 +1883,47 @@ size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint
 
 namespace {
 
-template <typename W, int K>
-cudaError_t cluster_bc_config(uint32_t logC, size_t smem, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr,
-                              uint32_t nClusters, cudaStream_t s, bool& runnable)
+// The launch of nClusters clusters of 2^logC CTAs.
+cudaLaunchConfig_t cluster_bc_config(uint32_t logC, size_t smem, cudaLaunchAttribute* attr, uint32_t nClusters,
+                                     cudaStream_t s)
 {
-    auto kernel = k_cluster_bc<W, K>;
-    uint32_t const C = 1u << logC;
-    static thread_local bool done[64] = {};
-    cudaError_t e = allow_smem(kernel, done);
-    if (e != cudaSuccess) return e;
-    if (C > 8) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return e;
-    }
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.x = 1u << logC;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg = {};
-    cfg.gridDim = dim3(nClusters * C);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nClusters << logC);
     cfg.blockDim = dim3(kResidentBlock);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
-    runnable = e == cudaSuccess && clusters >= 1;
-    return e;
+    return cfg;
+}
+
+// Whether the device runs clusters of 2^logC CTAs with all the shared memory a CTA may take: asked once
+// per device, thread, kernel and size (the question takes the driver most of a millisecond).
+template <typename W, int K>
+bool cluster_bc_check(uint32_t logC)
+{
+    static thread_local signed char known[64][5] = {};
+    static thread_local bool done[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    signed char& k = known[dev & 63][logC];
+    if (k == 0) {
+        auto kernel = k_cluster_bc<W, K>;
+        cudaLaunchAttribute attr[1];
+        cudaLaunchConfig_t const cfg = cluster_bc_config(logC, kResidentMaxSmem, attr, 1, nullptr);
+        int clusters = 0;
+        cudaError_t e = allow_smem(kernel, done);
+        if (e == cudaSuccess && logC > 3)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
+        if (e != cudaSuccess) cudaGetLastError();   // a configuration the device refuses is an answer, not an error
+        k = e == cudaSuccess && clusters >= 1 ? 1 : -1;
+    }
+    return k > 0;
 }
 
 template <typename W, int K>
@@ -1813,12 +1931,9 @@ cudaError_t launch_cluster_bc_k(SysDev const* dSys, uint32_t const* dList, uint3
                                 StepEntry const* dSteps, uint32_t stride, uint32_t nSteps, size_t smem,
                                 cudaStream_t s)
 {
-    cudaLaunchConfig_t cfg;
+    if (!cluster_bc_check<W, K>(logC)) return cudaErrorInvalidConfiguration;
     cudaLaunchAttribute attr[1];
-    bool runnable = false;
-    cudaError_t e = cluster_bc_config<W, K>(logC, smem, cfg, attr, nClusters, s, runnable);
-    if (e != cudaSuccess) return e;
-    if (!runnable) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t const cfg = cluster_bc_config(logC, smem, attr, nClusters, s);
     return cudaLaunchKernelEx(&cfg, k_cluster_bc<W, K>, dSys, dList, dSteps, stride, nSteps);
 }
 
@@ -1837,21 +1952,15 @@ cudaError_t launch_cluster_bc_w(SysDev const* dSys, uint32_t const* dList, uint3
 }
 
 template <typename W>
-bool cluster_bc_runnable_w(uint32_t logC, uint32_t perThread, size_t smem)
+bool cluster_bc_runnable_w(uint32_t logC, uint32_t perThread)
 {
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[1];
-    bool runnable = false;
-    cudaError_t e = cudaErrorInvalidValue;
     switch (perThread) {
-    case 1: e = cluster_bc_config<W, 1>(logC, smem, cfg, attr, 1, nullptr, runnable); break;
-    case 2: e = cluster_bc_config<W, 2>(logC, smem, cfg, attr, 1, nullptr, runnable); break;
-    case 4: e = cluster_bc_config<W, 4>(logC, smem, cfg, attr, 1, nullptr, runnable); break;
-    case 8: e = cluster_bc_config<W, 8>(logC, smem, cfg, attr, 1, nullptr, runnable); break;
-    default: break;
+    case 1: return cluster_bc_check<W, 1>(logC);
+    case 2: return cluster_bc_check<W, 2>(logC);
+    case 4: return cluster_bc_check<W, 4>(logC);
+    case 8: return cluster_bc_check<W, 8>(logC);
+    default: return false;
     }
-    if (e != cudaSuccess) cudaGetLastError();   // a configuration the device refuses is an answer, not an error
-    return e == cudaSuccess && runnable;
 }
 
 }  // namespace
@@ -1859,8 +1968,8 @@ bool cluster_bc_runnable_w(uint32_t logC, uint32_t perThread, size_t smem)
 bool cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode)
 {
     if (logC < 1 || logC > 4 || smem > kResidentMaxSmem) return false;
-    if (codeMode == kCode32) return cluster_bc_runnable_w<uint32_t>(logC, perThread, smem);
-    if (codeMode == kCode64) return cluster_bc_runnable_w<unsigned long long>(logC, perThread, smem);
+    if (codeMode == kCode32) return cluster_bc_runnable_w<uint32_t>(logC, perThread);
+    if (codeMode == kCode64) return cluster_bc_runnable_w<unsigned long long>(logC, perThread);
     return false;
 }
 

@@ -367,7 +367,10 @@ void Server::workerMain()
                 std::vector<Updater*> members;
                 for (auto const& j : L.jobs) members.push_back(j->u.get());
                 if (L.batch) L.batch->setMembers(members.data(), (uint32_t)members.size());
-                else L.batch.reset(new Batch(gpu_, members.data(), (uint32_t)members.size()));
+                else {
+                    L.batch.reset(new Batch(gpu_, members.data(), (uint32_t)members.size()));
+                    L.batch->setSlabSms(L.batch->smCount() / kGridLanes);   // the grid lanes share the SMs
+                }
                 L.changed = false;
             }
             if (!L.done) cuda_check(cudaEventCreateWithFlags(&L.done, cudaEventDisableTiming), "cudaEventCreate");

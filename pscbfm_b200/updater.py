@@ -438,8 +438,8 @@ class Batch:
                 "mcs_spent": n.value * (1 + mcs_per_trial), "trials": t}
 
     def set_cluster(self, on: bool):
-        """Members too large for one CTA that a cluster of CTAs holds run in the cluster-resident
-        kernel (default on); off: they share the grid-phase kernels. Results do not change."""
+        """Bond-code members too large for one CTA run on CTAs of their own (default on); off: they share the
+        grid-phase kernels. Results do not change."""
         self._call("bfm_batch_set_cluster", 1 if on else 0)
 
     def run_each(self, mcs):

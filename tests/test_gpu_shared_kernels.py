@@ -72,3 +72,43 @@ def test_idle_members_beside_longer_ones():
         assert np.array_equal(m.get_coords(), O.run(s, int(t))[0]), s.name
         m.validate()
     b.close()
+
+
+def test_batch_slab_sweeps_in_waves_vs_oracle():
+    """More members than one cooperative launch holds (each of at least eight CTAs), beside resident members
+    and a 64-bit network: the launches run one after the other, and every trajectory is its own."""
+    big = S.serpentine_chains(128, 64, 0.45)
+    systems = [big] * 20 + [S.crosslinked_network(), S.serpentine_chains(128, 37, 0.1), S.serpentine_chains(32, 16, 0.3)]
+    members = [P.UpdaterGPUScBFM_AB_Type(0).load_system(s, seed=60 + i) for i, s in enumerate(systems)]
+    b = P.Batch(members)
+    n0 = b.launch_count()
+    b.run(2)
+    assert b.launch_count() - n0 <= 5   # two or three waves, the 64-bit wave, the resident launch
+    for i in (0, 7, 19, 20, 21, 22):
+        want, ost = O.run(systems[i], 2, seed=60 + i)
+        st = members[i].stats()
+        assert np.array_equal(members[i].get_coords(), want), i
+        assert (st["attempted"], st["tentative"], st["accepted"]) == ost
+        members[i].validate()
+    # alone, then in a batch again, then as two launches per sub-step
+    u = members[21]
+    u.set_mode(P.MODE_PERSISTENT)
+    u.runSimulationOnGPU(3)
+    b.run(1)
+    u.set_mode(P.MODE_GRAPH)
+    u.runSimulationOnGPU(2)
+    assert np.array_equal(u.get_coords(), O.run(systems[21], 8, seed=81)[0])
+    b.close()
+
+
+def test_batch_barrier_timeout_is_reported():
+    """A member whose barrier cannot complete (injected on the host) ends at the wait's time limit and the
+    batch's run reports it; the device stays usable for other members."""
+    s = S.serpentine_chains(128, 32, 0.1, seed=3)
+    members = [P.UpdaterGPUScBFM_AB_Type(0).load_system(s, seed=q) for q in (1, 2)]
+    b = P.Batch(members)
+    members[0].inject_barrier_stall()
+    with pytest.raises(P.BfmCudaError, match="timed out"):
+        b.run(2)
+    assert np.array_equal(members[1].get_coords(), O.run(s, 2, seed=2)[0])
+    b.close()
