@@ -432,13 +432,14 @@ void Batch::run(int32_t const* mcs)
                    "batch steps H2D");
         cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
         if (!resident_.empty() || !slab_.empty()) cuda_check(cudaEventRecord(fork_, stream_), "event");
+        StepSource const src{dStepsAll_, M, 0u, 0ull, 0ull};
         if (!slab_.empty()) {
             cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
             for (auto const& w : slab_) {
                 for (SlabRef const& r : w.refs)
                     if (r.rank == 0) members_[r.sys]->applyStall(side_);
-                cuda_check(launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, dStepsAll_, M,
-                                             (uint32_t)T, dReports_, w.codeMode, side_),
+                cuda_check(launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, src, (uint32_t)T,
+                                             dReports_, w.codeMode, side_),
                            "batch slab");
                 ++launches_;
             }
@@ -452,8 +453,8 @@ void Batch::run(int32_t const* mcs)
                 cuda_check(g.codeMode == kCodeNone
                                ? launch_resident(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, dStepsAll_,
                                                  M, (uint32_t)T, g.smem, stream2_)
-                               : launch_resident_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread,
-                                                    dStepsAll_, M, (uint32_t)T, g.smem, g.codeMode, stream2_),
+                               : launch_resident_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, src,
+                                                    (uint32_t)T, g.smem, g.codeMode, stream2_),
                            "batch resident");
                 ++launches_;
             }

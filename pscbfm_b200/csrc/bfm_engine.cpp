@@ -1156,6 +1156,24 @@ void Updater::timeKernels(int32_t nMcs, double out[4])
     out[3] = (double)n;
 }
 
+StepSource Updater::stepSource(uint32_t nSteps)
+{
+    // the entries of the next nSteps sub-steps for a kernel that runs them all: the counter stream's are
+    // made on the device, a callback's go up in one copy
+    if (drawKind_ == kDrawCounter) {
+        StepSource const src{nullptr, 0u, 1u, drawSeed_, subStep_};
+        subStep_ += nSteps;
+        return src;
+    }
+    cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
+    fillSteps(nSteps, hSteps_, false);
+    cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * nSteps, cudaMemcpyHostToDevice, stream_),
+               "steps H2D");
+    h2dBytes_ += sizeof(StepEntry) * nSteps;
+    cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
+    return StepSource{dev_.dSteps, 1u, 0u, 0ull, 0ull};
+}
+
 void Updater::enqueueResident(uint32_t nSteps)
 {
     scrubPending(stream_);
@@ -1164,17 +1182,19 @@ void Updater::enqueueResident(uint32_t nSteps)
     while (per * kResidentBlock < maxGroup_) per *= 2;
     for (uint32_t done = 0; done < nSteps;) {
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
-        cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
-        fillSteps(chunk, hSteps_, true);
-        cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * chunk, cudaMemcpyHostToDevice, stream_),
-                   "steps H2D");
-        h2dBytes_ += sizeof(StepEntry) * chunk;
-        cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
-        cuda_check(codeMode_ == kCodeNone
-                       ? launch_resident(dev_.dDesc, dev_.dList, 1, per, dev_.dSteps, 1, chunk, smem, stream_)
-                       : launch_resident_bc(dev_.dDesc, dev_.dList, 1, per, dev_.dSteps, 1, chunk, smem, codeMode_,
-                                            stream_),
-                   "resident");
+        if (codeMode_ == kCodeNone) {
+            cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
+            fillSteps(chunk, hSteps_, true);
+            cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * chunk, cudaMemcpyHostToDevice, stream_),
+                       "steps H2D");
+            h2dBytes_ += sizeof(StepEntry) * chunk;
+            cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
+            cuda_check(launch_resident(dev_.dDesc, dev_.dList, 1, per, dev_.dSteps, 1, chunk, smem, stream_), "resident");
+        } else {
+            cuda_check(launch_resident_bc(dev_.dDesc, dev_.dList, 1, per, stepSource(chunk), chunk, smem, codeMode_,
+                                          stream_),
+                       "resident");
+        }
         ++launches_;
         done += chunk;
     }
@@ -1212,13 +1232,7 @@ void Updater::enqueueCluster(uint32_t nSteps)
     scrubPending(stream_);
     for (uint32_t done = 0; done < nSteps;) {
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
-        cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
-        fillSteps(chunk, hSteps_, true);
-        cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * chunk, cudaMemcpyHostToDevice, stream_),
-                   "steps H2D");
-        h2dBytes_ += sizeof(StepEntry) * chunk;
-        cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
-        cuda_check(launch_cluster_bc(dev_.dDesc, dev_.dList, 1, cluster_.logC, cluster_.perWarp, dev_.dSteps, 1, chunk,
+        cuda_check(launch_cluster_bc(dev_.dDesc, dev_.dList, 1, cluster_.logC, cluster_.perWarp, stepSource(chunk), chunk,
                                      cluster_.smem, codeMode_, stream_),
                    "cluster");
         ++launches_;
@@ -1294,14 +1308,8 @@ void Updater::enqueuePersistent(uint32_t nSteps)
     scrubPending(stream_);   // marks of a previous grid-phase run, left for the next check
     for (uint32_t done = 0; done < nSteps;) {
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
-        cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
-        fillSteps(chunk, hSteps_, false);
-        cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * chunk, cudaMemcpyHostToDevice, stream_),
-                   "steps H2D");
-        h2dBytes_ += sizeof(StepEntry) * chunk;
-        cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
         applyStall(stream_);
-        cuda_check(launch_slab_bc(dev_.h, dev_.dSteps, chunk, slab_, dGs_, codeMode_, stream_), "persistent sweep");
+        cuda_check(launch_slab_bc(dev_.h, stepSource(chunk), chunk, slab_, dGs_, codeMode_, stream_), "persistent sweep");
         ++launches_;
         done += chunk;
     }

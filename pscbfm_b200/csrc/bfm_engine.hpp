@@ -196,6 +196,7 @@ private:
     void enqueueCluster(uint32_t nSteps);
     void planCluster();   // the cluster size and chunks per warp of the cluster-resident kernel
     void enqueuePersistent(uint32_t nSteps);
+    StepSource stepSource(uint32_t nSteps);   // the next nSteps entries, for one launch that runs them
     void fillSteps(uint32_t nSteps, StepEntry* hostBuf, bool residentParity);
     void freeDevice();
     void ensureStaging();

@@ -127,29 +127,26 @@ bool slab_plan(uint32_t const* grpSize, uint32_t nColors, uint32_t maxc, uint32_
                uint32_t ctas, SlabPlan& plan);
 // CTAs of a cooperative launch for a system whose largest colour group is maxGroup
 uint32_t slab_ctas(uint32_t maxGroup, uint32_t sms);
-cudaError_t launch_slab_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
+cudaError_t launch_slab_bc(SysDev const& hostDesc, StepSource const& src, uint32_t nSteps, SlabPlan const& plan,
                            GridFault* report, uint32_t codeMode, cudaStream_t s);
-// Plans with the cache only; dRefs: the launch's CTAs; the entries of sub-step t are
-// dSteps[t * stride + system], the reports report[system].
+// Plans with the cache only; dRefs: the launch's CTAs; the reports are report[system].
 cudaError_t launch_slab_batch(SysDev const* dSys, SlabRef const* dRefs, uint32_t ctas, size_t smem,
-                              StepEntry const* dSteps, uint32_t stride, uint32_t nSteps, GridFault* report,
-                              uint32_t codeMode, cudaStream_t s);
+                              StepSource const& src, uint32_t nSteps, GridFault* report, uint32_t codeMode,
+                              cudaStream_t s);
 // Dynamic shared memory of the bond-code resident kernel, with the neighbour references where they fit too.
 size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t maxc, uint32_t codeMode);
 // Cluster-resident sweep (bond codes): one cluster of 2^logC CTAs of kResidentBlock threads per
 // system of dList[0..nClusters) (logC 1..4), state in the cluster's shared memory for nSteps
-// sub-steps whose entries are dSteps[t * stride + system]; perThread (1, 2, 4, 8) chunks of 32
-// slots per warp and colour. cluster_bc_runnable: whether the device can run that configuration
-// (kernel attributes set, cudaOccupancyMaxActiveClusters >= 1).
+// sub-steps; perThread (1, 2, 4, 8) chunks of 32 slots per warp and colour. cluster_bc_runnable: whether
+// the device can run that configuration.
 size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t perThread, uint32_t maxc,
                              uint32_t codeMode);
 bool cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode);
 cudaError_t launch_cluster_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
-                              uint32_t perThread, StepEntry const* dSteps, uint32_t stride, uint32_t nSteps,
-                              size_t smem, uint32_t codeMode, cudaStream_t s);
+                              uint32_t perThread, StepSource const& src, uint32_t nSteps, size_t smem,
+                              uint32_t codeMode, cudaStream_t s);
 cudaError_t launch_resident_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, uint32_t perThread,
-                               StepEntry const* dSteps, uint32_t nSys, uint32_t nSteps, size_t smem, uint32_t codeMode,
-                               cudaStream_t s);
+                               StepSource const& src, uint32_t nSteps, size_t smem, uint32_t codeMode, cudaStream_t s);
 
 // Observables (bfm_observables.cu). Molecule of every slot (kNoColor for padding), first and last
 // slot of every molecule, and the reference positions for the mean squared displacement.

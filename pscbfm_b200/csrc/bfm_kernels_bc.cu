@@ -58,6 +58,8 @@ __device__ __forceinline__ bool bonds_ok(W code, uint32_t dir, uint8_t const* ok
     return (m >> dir) & 1u;
 }
 
+constexpr uint32_t kStepBlock = 8;   // step entries staged in shared memory at a time (static shared memory stays below 1 KB)
+
 // Adds v to a counter in shared memory and returns its old value, as one instruction: written with
 // atomicAdd, the compiler gathers the adds of a warp first, 20 instructions for the one lane that adds.
 __device__ __forceinline__ uint32_t shared_add(uint32_t* p, uint32_t v)
@@ -613,8 +615,8 @@ __host__ __device__ __forceinline__ bool slab_clear_all(uint32_t nwords, uint32_
 // The CTAs are part of a cooperative launch and meet at a count in global memory (S.gs). A thread-block
 // cluster and its barrier in hardware were no faster (131K monomers on 16 CTAs 9.7 us per sub-step
 // against 8.9: every warp's wait drops the SM's L1 lines), and its CTAs have to fit one GPC.
-// kIdle: entries may be idle (kNoColor). cap, capG: slots of a CTA in all and of the largest colour group, at most (slab_caps); entries of
-// sub-step t at steps[t * stride].
+// kIdle: entries may be idle (kNoColor). cap, capG: slots of a CTA in all and of the largest colour group,
+// at most (slab_caps). The waiter fetches the step entries a block ahead, during a perform.
 // Bound: on the 256^3 melt (N = 1,048,576, 148 CTAs) by the scattered L2 accesses (about 0.8 loads and
 // 0.57 atomics per clock and SM), the integer pipe and instruction issue (24 K warp instructions per SM
 // and sub-step); below 200K monomers by the barriers (1.3-1.8 us each with the writes before them) and
@@ -625,9 +627,9 @@ __host__ __device__ __forceinline__ bool slab_clear_all(uint32_t nwords, uint32_
 // CTAs with at most kSlabSmallSlots slots per colour have 256: fewer warps meet faster at the CTA's own
 // barriers (131K monomers 9.0 against 9.6 us per MCS, 210K 9.3 against 9.9, 60K 7.9 against 8.5).
 template <typename W, int B, bool kCache, bool kIdle>
-__device__ __forceinline__ void slab_sweep(SysDev const& S, StepEntry const* __restrict__ steps, uint32_t stride,
-                                           uint32_t nSteps, uint32_t C, uint32_t rank, uint32_t cap, uint32_t capG,
-                                           bool clearAll, GridFault* report)
+__device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& src, uint32_t sysId, uint32_t nSteps,
+                                           uint32_t C, uint32_t rank, uint32_t cap, uint32_t capG, bool clearAll,
+                                           GridFault* report)
 {
     constexpr uint32_t kSlots = CodeWord<W>::kSlots;
     constexpr W kShared = slab_shared_flag<W>();
@@ -639,6 +641,7 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepEntry const* __r
     constexpr uint32_t kRefBits = slab_ref_bits(sizeof(W) == 8), kRefMask = (1u << kRefBits) - 1u, kAway = 0xFFFFu;
     constexpr uint32_t kFarBit = 1u << 31;
     __shared__ SlabPart P;
+    __shared__ __align__(16) StepEntry stepSm[2][kStepBlock];   // the block of entries in use, and the next
     __shared__ uint32_t nCand, nMov, tallyA;
     extern __shared__ unsigned long long smem[];
     uint32_t const tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -754,11 +757,28 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepEntry const* __r
     uint32_t prevMov = 0u, nAcc = 0u, nTent = 0u, par = 0u, dirs = 0u;
     bool began = false, drawn = false;   // a sub-step has run; dirs belong to the next one
     unsigned long long att = 0ull;
-    StepEntry next = steps[0];
+    auto fetch_steps = [&](uint32_t block) {   // the waiter's lanes
+        uint32_t const t = block * kStepBlock + lane;
+        if (lane < kStepBlock && t < nSteps) stepSm[block & 1u][lane] = step_entry(src, sysId, t, S.grp, nColors);
+    };
+    if (waiter) {
+        fetch_steps(0);
+        fetch_steps(1);
+    }
+    __syncthreads();
     for (uint32_t t = 0; t < nSteps; ++t) {
-        StepEntry const st = next;
-        if (t + 1 < nSteps) next = steps[(size_t)(t + 1) * stride];
-        if (kIdle && st.color == kNoColor) continue;
+        StepEntry const st = stepSm[t / kStepBlock & 1u][t % kStepBlock];
+        StepEntry const& next = stepSm[(t + 1u) / kStepBlock & 1u][(t + 1u) % kStepBlock];
+        // the block before the one in use has been read by all: the next one takes its place
+        bool const refill = t != 0 && t % kStepBlock == 0;
+        if (kIdle && st.color == kNoColor) {
+            if (refill) {   // (the same on every thread)
+                __syncthreads();
+                if (waiter) fetch_steps(t / kStepBlock + 1u);
+                __syncthreads();
+            }
+            continue;
+        }
         par = st.parity;
         att += st.cnt;
         uint32_t const first = P.first[st.color], base = P.base[st.color];
@@ -953,6 +973,7 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepEntry const* __r
                 }
             }
         }
+        if (waiter && refill) fetch_steps(t / kStepBlock + 1u);
         nTent += nm;
         prevMov = nm;
         __syncthreads();   // this CTA's slots are settled for the next check's first part
@@ -984,19 +1005,18 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepEntry const* __r
 
 template <typename W, int B, bool kCache>
 __global__ void __launch_bounds__(B, 1)
-    k_slab_bc(const __grid_constant__ SysDev S, StepEntry const* __restrict__ steps, uint32_t nSteps, uint32_t cap,
+    k_slab_bc(const __grid_constant__ SysDev S, const __grid_constant__ StepSource src, uint32_t nSteps, uint32_t cap,
               uint32_t capG, uint32_t clearAll, GridFault* report)
 {
-    slab_sweep<W, B, kCache, false>(S, steps, 1u, nSteps, gridDim.x, blockIdx.x, cap, capG, clearAll != 0u, report);
+    slab_sweep<W, B, kCache, false>(S, src, 0u, nSteps, gridDim.x, blockIdx.x, cap, capG, clearAll != 0u, report);
 }
 
 // Many systems in one cooperative launch: CTA b runs share refs[b].rank of system refs[b].sys with the
-// other CTAs of that system, and waits for no others; the entries of sub-step t are
-// steps[t * stride + system], the reports report[system].
+// other CTAs of that system, and waits for no others; the reports are report[system].
 template <typename W, int B>
 __global__ void __launch_bounds__(B, 1)
     k_slab_batch_bc(SysDev const* __restrict__ sysv, SlabRef const* __restrict__ refs,
-                    StepEntry const* __restrict__ steps, uint32_t stride, uint32_t nSteps, GridFault* report)
+                    const __grid_constant__ StepSource src, uint32_t nSteps, GridFault* report)
 {
     __shared__ SysDev S;
     __shared__ uint32_t caps[3];
@@ -1006,7 +1026,7 @@ __global__ void __launch_bounds__(B, 1)
     if (threadIdx.x == 0)
         slab_caps([&](uint32_t c) { return S.grp[2 * c + 1]; }, S.nColors, r.ctas, caps[0], caps[1], caps[2]);
     __syncthreads();
-    slab_sweep<W, B, true, true>(S, steps + r.sys, stride, nSteps, r.ctas, r.rank, caps[0], caps[1],
+    slab_sweep<W, B, true, true>(S, src, r.sys, nSteps, r.ctas, r.rank, caps[0], caps[1],
                                  slab_clear_all(S.nwords, caps[2]), report + r.sys);
 }
 
@@ -1076,7 +1096,6 @@ __device__ __forceinline__ uint32_t half_hits(HalfPlane const& r, uint32_t const
 
 // Shared memory of k_resident_bc (resident_bc_smem_bytes); nb: neighbour references kept here (0: they
 // stay in global memory).
-constexpr uint32_t kStepBlock = 16;   // step entries staged in shared memory at a time (static shared memory stays below 1 KB)
 __host__ __device__ __forceinline__ size_t resident_layout(uint32_t nwords, uint32_t npad, uint32_t maxGroup,
                                                            uint32_t codeBytes, uint32_t nb)
 {
@@ -1087,7 +1106,7 @@ __host__ __device__ __forceinline__ size_t resident_layout(uint32_t nwords, uint
 // The whole system in one CTA's shared memory for nSteps sub-steps: lattice, one temporary
 // lattice per sub-step parity (the previous one cleared while the next check runs), lattice
 // addresses, bond codes, neighbour references (where they fit: 2 bytes each) and lists; one CTA per
-// system of sysList, entries of sub-step t at steps[t * nSys + system].
+// system of sysList.
 // The bond test and the front plane are evaluated side by side, without branches, so that their
 // chains of dependent reads overlap; the directions of sub-step t + 1 are drawn during the perform
 // of t, whose movers take the threads from the last one down, where a small system has no slots.
@@ -1101,8 +1120,7 @@ __host__ __device__ __forceinline__ size_t resident_layout(uint32_t nwords, uint
 template <typename W, bool kDirect>
 __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const* __restrict__ sysv,
                                                                     uint32_t const* __restrict__ sysList,
-                                                                    StepEntry const* __restrict__ steps,
-                                                                    uint32_t nSys, uint32_t nSteps)
+                                                                    StepSource const src, uint32_t nSteps)
 {
     constexpr uint32_t kSlots = CodeWord<W>::kSlots, B = kResidentBlock, kDirs = 10;
     constexpr uint32_t kRefBits = slab_ref_bits(sizeof(W) == 8), kRefMask = (1u << kRefBits) - 1u;
@@ -1187,9 +1205,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const*
     for (uint32_t t = 0; t < nSteps; ++t) {
         if (t % kStepBlock == 0) {   // (the last barrier of the sub-step before ended the reads of the old ones)
             uint32_t const n = min(kStepBlock, nSteps - t);
-            for (uint32_t k = tid; k < 2u * n; k += B)
-                reinterpret_cast<uint4*>(stepSm)[k] =
-                    reinterpret_cast<uint4 const*>(steps + (size_t)(t + k / 2u) * nSys + sysId)[k & 1u];
+            if (tid < n) stepSm[tid] = step_entry(src, sysId, t + tid, S.grp, S.nColors);
             __syncthreads();   // (the first also publishes the state loaded above)
             drawn = false;
         }
@@ -1365,8 +1381,7 @@ __host__ __device__ __forceinline__ size_t cluster_layout(uint32_t nwords, uint3
 // first barrier a CTA clears its words of the previous copy and draws the directions of the next
 // sub-step, which nobody waits for. Every CTA of a cluster runs the same system and so reaches the
 // same barriers. A CTA leaves only after the last barrier, when no other CTA accesses its shared
-// memory any more. Grid: one cluster per system of sysList; the entries of sub-step t are
-// steps[t * stride + system]. K: chunks of 32 slots per warp and colour, at most.
+// memory any more. Grid: one cluster per system of sysList. K: chunks of 32 slots per warp and colour, at most.
 // Bound by remote accesses (0.33 remote atomics per clock and SM), two barriers of 0.3 us and the
 // chain of dependent reads of each phase; a lattice word is read only where the bond test passed and the
 // plane touches it. us per MCS, 16 CTAs: 8K chains 5.7 (8.6 on the four CTAs of one chunk per warp),
@@ -1374,8 +1389,7 @@ __host__ __device__ __forceinline__ size_t cluster_layout(uint32_t nwords, uint3
 template <typename W, int K>
 __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* __restrict__ sysv,
                                                                    uint32_t const* __restrict__ sysList,
-                                                                   StepEntry const* __restrict__ steps,
-                                                                   uint32_t stride, uint32_t nSteps)
+                                                                   StepSource const src, uint32_t nSteps)
 {
     namespace cg = cooperative_groups;
     constexpr uint32_t kSlots = CodeWord<W>::kSlots, B = kResidentBlock;
@@ -1464,9 +1478,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
     for (uint32_t t = 0; t < nSteps; ++t) {
         if (t % kStepBlock == 0) {   // (the last barrier of the sub-step before ended the reads of the old ones)
             uint32_t const n = min(kStepBlock, nSteps - t);
-            for (uint32_t k = tid; k < 2u * n; k += B)
-                reinterpret_cast<uint4*>(stepSm)[k] =
-                    reinterpret_cast<uint4 const*>(steps + (size_t)(t + k / 2u) * stride + sysId)[k & 1u];
+            if (tid < n) stepSm[tid] = step_entry(src, sysId, t + tid, S.grp, S.nColors);
             __syncthreads();
             drawn = false;
         }
@@ -1753,14 +1765,14 @@ uint32_t slab_ctas(uint32_t maxGroup, uint32_t sms)
 namespace {
 
 template <typename W, int B, bool kCache>
-cudaError_t launch_slab_bc_w(SysDev const& S, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
+cudaError_t launch_slab_bc_w(SysDev const& S, StepSource src, uint32_t nSteps, SlabPlan const& plan,
                              GridFault* report, cudaStream_t s)
 {
     static thread_local bool done[64] = {};
     cudaError_t const e = allow_smem(k_slab_bc<W, B, kCache>, done);
     if (e != cudaSuccess) return e;
     uint32_t cap = plan.cap, perCta = plan.perCta, clearAll = plan.clearAll ? 1u : 0u;
-    void* args[] = {const_cast<SysDev*>(&S), &dSteps, &nSteps, &cap, &perCta, &clearAll, &report};
+    void* args[] = {const_cast<SysDev*>(&S), &src, &nSteps, &cap, &perCta, &clearAll, &report};
     return cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(k_slab_bc<W, B, kCache>), dim3(plan.ctas), dim3(B),
                                        args, plan.smem, s);
 }
@@ -1781,48 +1793,46 @@ auto slab_dispatch(uint32_t codeMode, SlabPlan const& plan, F f)
 
 struct SlabLaunch {
     SysDev const& S;
-    StepEntry const* dSteps;
+    StepSource const& src;
     uint32_t nSteps;
     SlabPlan const& plan;
     GridFault* report;
     cudaStream_t s;
     template <typename W, int B, bool kCache>
-    cudaError_t operator()() const { return launch_slab_bc_w<W, B, kCache>(S, dSteps, nSteps, plan, report, s); }
+    cudaError_t operator()() const { return launch_slab_bc_w<W, B, kCache>(S, src, nSteps, plan, report, s); }
 };
 
 template <typename W, int B>
-cudaError_t launch_slab_batch_w(SysDev const* dSys, SlabRef const* dRefs, uint32_t ctas, size_t smem,
-                                StepEntry const* dSteps, uint32_t stride, uint32_t nSteps, GridFault* report,
-                                cudaStream_t s)
+cudaError_t launch_slab_batch_w(SysDev const* dSys, SlabRef const* dRefs, uint32_t ctas, size_t smem, StepSource src,
+                                uint32_t nSteps, GridFault* report, cudaStream_t s)
 {
     static thread_local bool done[64] = {};
     cudaError_t const e = allow_smem(k_slab_batch_bc<W, B>, done);
     if (e != cudaSuccess) return e;
-    void* args[] = {&dSys, &dRefs, &dSteps, &stride, &nSteps, &report};
+    void* args[] = {&dSys, &dRefs, &src, &nSteps, &report};
     return cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(k_slab_batch_bc<W, B>), dim3(ctas), dim3(B), args,
                                        smem, s);
 }
 
 }  // namespace
 
-cudaError_t launch_slab_bc(SysDev const& hostDesc, StepEntry const* dSteps, uint32_t nSteps, SlabPlan const& plan,
+cudaError_t launch_slab_bc(SysDev const& hostDesc, StepSource const& src, uint32_t nSteps, SlabPlan const& plan,
                            GridFault* report, uint32_t codeMode, cudaStream_t s)
 {
     if (nSteps == 0) return cudaSuccess;
     if (plan.ctas == 0 || codeMode == kCodeNone) return cudaErrorInvalidValue;
-    return slab_dispatch(codeMode, plan, SlabLaunch{hostDesc, dSteps, nSteps, plan, report, s});
+    return slab_dispatch(codeMode, plan, SlabLaunch{hostDesc, src, nSteps, plan, report, s});
 }
 
 cudaError_t launch_slab_batch(SysDev const* dSys, SlabRef const* dRefs, uint32_t ctas, size_t smem,
-                              StepEntry const* dSteps, uint32_t stride, uint32_t nSteps, GridFault* report,
-                              uint32_t codeMode, cudaStream_t s)
+                              StepSource const& src, uint32_t nSteps, GridFault* report, uint32_t codeMode,
+                              cudaStream_t s)
 {
     if (ctas == 0 || nSteps == 0) return cudaSuccess;
     if (codeMode == kCode32)
-        return launch_slab_batch_w<uint32_t, (int)kSlabBlock32>(dSys, dRefs, ctas, smem, dSteps, stride, nSteps, report, s);
+        return launch_slab_batch_w<uint32_t, (int)kSlabBlock32>(dSys, dRefs, ctas, smem, src, nSteps, report, s);
     if (codeMode == kCode64)
-        return launch_slab_batch_w<unsigned long long, (int)kSlabBlock64>(dSys, dRefs, ctas, smem, dSteps, stride, nSteps,
-                                                                          report, s);
+        return launch_slab_batch_w<unsigned long long, (int)kSlabBlock64>(dSys, dRefs, ctas, smem, src, nSteps, report, s);
     return cudaErrorInvalidValue;
 }
 
@@ -1836,40 +1846,40 @@ size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup,
 namespace {
 
 template <typename W, bool kDirect>
-cudaError_t launch_resident_bc_k(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, StepEntry const* dSteps,
-                                 uint32_t nSys, uint32_t nSteps, size_t smem, cudaStream_t s)
+cudaError_t launch_resident_bc_k(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, StepSource const& src,
+                                 uint32_t nSteps, size_t smem, cudaStream_t s)
 {
     static thread_local bool done[64] = {};
     cudaError_t const e = allow_smem(k_resident_bc<W, kDirect>, done);
     if (e != cudaSuccess) return e;
-    k_resident_bc<W, kDirect><<<nCta, kResidentBlock, smem, s>>>(dSys, dList, dSteps, nSys, nSteps);
+    k_resident_bc<W, kDirect><<<nCta, kResidentBlock, smem, s>>>(dSys, dList, src, nSteps);
     return cudaGetLastError();
 }
 
 template <typename W>
 cudaError_t launch_resident_bc_w(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, uint32_t perThread,
-                                 StepEntry const* dSteps, uint32_t nSys, uint32_t nSteps, size_t smem, cudaStream_t s)
+                                 StepSource const& src, uint32_t nSteps, size_t smem, cudaStream_t s)
 {
     // lists of 16-bit entries index up to 1 << kSlabEntBits slots of a group
     constexpr uint32_t kListed = (1u << kSlabEntBits) / kResidentBlock;
     if (perThread < 1 || perThread > 16) return cudaErrorInvalidValue;
     return perThread == 1 || perThread > kListed
-               ? launch_resident_bc_k<W, true>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s)
-               : launch_resident_bc_k<W, false>(dSys, dList, nCta, dSteps, nSys, nSteps, smem, s);
+               ? launch_resident_bc_k<W, true>(dSys, dList, nCta, src, nSteps, smem, s)
+               : launch_resident_bc_k<W, false>(dSys, dList, nCta, src, nSteps, smem, s);
 }
 
 }  // namespace
 
 cudaError_t launch_resident_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, uint32_t perThread,
-                               StepEntry const* dSteps, uint32_t nSys, uint32_t nSteps, size_t smem, uint32_t codeMode,
+                               StepSource const& src, uint32_t nSteps, size_t smem, uint32_t codeMode,
                                cudaStream_t s)
 {
     if (nCta == 0 || nSteps == 0) return cudaSuccess;
     if (smem > kResidentMaxSmem) return cudaErrorInvalidValue;
     if (codeMode == kCode32)
-        return launch_resident_bc_w<uint32_t>(dSys, dList, nCta, perThread, dSteps, nSys, nSteps, smem, s);
+        return launch_resident_bc_w<uint32_t>(dSys, dList, nCta, perThread, src, nSteps, smem, s);
     if (codeMode == kCode64)
-        return launch_resident_bc_w<unsigned long long>(dSys, dList, nCta, perThread, dSteps, nSys, nSteps, smem, s);
+        return launch_resident_bc_w<unsigned long long>(dSys, dList, nCta, perThread, src, nSteps, smem, s);
     return cudaErrorInvalidValue;
 }
 
@@ -1928,25 +1938,25 @@ bool cluster_bc_check(uint32_t logC)
 
 template <typename W, int K>
 cudaError_t launch_cluster_bc_k(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
-                                StepEntry const* dSteps, uint32_t stride, uint32_t nSteps, size_t smem,
+                                StepSource const& src, uint32_t nSteps, size_t smem,
                                 cudaStream_t s)
 {
     if (!cluster_bc_check<W, K>(logC)) return cudaErrorInvalidConfiguration;
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t const cfg = cluster_bc_config(logC, smem, attr, nClusters, s);
-    return cudaLaunchKernelEx(&cfg, k_cluster_bc<W, K>, dSys, dList, dSteps, stride, nSteps);
+    return cudaLaunchKernelEx(&cfg, k_cluster_bc<W, K>, dSys, dList, src, nSteps);
 }
 
 template <typename W>
 cudaError_t launch_cluster_bc_w(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
-                                uint32_t perThread, StepEntry const* dSteps, uint32_t stride, uint32_t nSteps,
+                                uint32_t perThread, StepSource const& src, uint32_t nSteps,
                                 size_t smem, cudaStream_t s)
 {
     switch (perThread) {
-    case 1: return launch_cluster_bc_k<W, 1>(dSys, dList, nClusters, logC, dSteps, stride, nSteps, smem, s);
-    case 2: return launch_cluster_bc_k<W, 2>(dSys, dList, nClusters, logC, dSteps, stride, nSteps, smem, s);
-    case 4: return launch_cluster_bc_k<W, 4>(dSys, dList, nClusters, logC, dSteps, stride, nSteps, smem, s);
-    case 8: return launch_cluster_bc_k<W, 8>(dSys, dList, nClusters, logC, dSteps, stride, nSteps, smem, s);
+    case 1: return launch_cluster_bc_k<W, 1>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
+    case 2: return launch_cluster_bc_k<W, 2>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
+    case 4: return launch_cluster_bc_k<W, 4>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
+    case 8: return launch_cluster_bc_k<W, 8>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -1974,15 +1984,15 @@ bool cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_
 }
 
 cudaError_t launch_cluster_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
-                              uint32_t perThread, StepEntry const* dSteps, uint32_t stride, uint32_t nSteps,
+                              uint32_t perThread, StepSource const& src, uint32_t nSteps,
                               size_t smem, uint32_t codeMode, cudaStream_t s)
 {
     if (nClusters == 0 || nSteps == 0) return cudaSuccess;
     if (logC < 1 || logC > 4 || smem > kResidentMaxSmem) return cudaErrorInvalidValue;
     if (codeMode == kCode32)
-        return launch_cluster_bc_w<uint32_t>(dSys, dList, nClusters, logC, perThread, dSteps, stride, nSteps, smem, s);
+        return launch_cluster_bc_w<uint32_t>(dSys, dList, nClusters, logC, perThread, src, nSteps, smem, s);
     if (codeMode == kCode64)
-        return launch_cluster_bc_w<unsigned long long>(dSys, dList, nClusters, logC, perThread, dSteps, stride, nSteps,
+        return launch_cluster_bc_w<unsigned long long>(dSys, dList, nClusters, logC, perThread, src, nSteps,
                                                        smem, s);
     return cudaErrorInvalidValue;
 }

@@ -46,7 +46,7 @@ def test_shared_memory_kernels_vs_oracle(name, mode):
         assert u.path() == m
     nc = u.n_colors()[0]
     done = 0
-    # sub-steps per call: below, on and across the blocks of 16 step entries
+    # sub-steps per call: below, on and across the blocks of 8 step entries
     for mcs in (1, 16 // nc, 16 // nc + 1, 33):
         u.runSimulationOnGPU(mcs)
         done += mcs
@@ -56,6 +56,48 @@ def test_shared_memory_kernels_vs_oracle(name, mode):
     assert (st["attempted"], st["tentative"], st["accepted"]) == ost
     u.validate()
     u.close()
+
+
+@pytest.mark.parametrize("mode", ["resident", "cluster", "persistent"])
+def test_entries_made_on_the_device_vs_the_callbacks(mode):
+    """Kernels that run many sub-steps make the counter stream's entries themselves; a callback's come
+    from the host. Both forms of the same stream, and runs that change between them, give the same system,
+    also past 2^32 sub-steps."""
+    s = S.serpentine_chains(32, 16, 0.4, seed=12)
+    m = {"resident": P.MODE_RESIDENT, "cluster": P.MODE_CLUSTER, "persistent": P.MODE_PERSISTENT}[mode]
+    for first in (0, 2**32 - 5):
+        at = [0]
+
+        def draw():
+            v = P.updater.counter_draw(s.seed, at[0])
+            at[0] += 1
+            return v
+
+        a, b, c = (P.UpdaterGPUScBFM_AB_Type(0) for _ in range(3))
+        for u in (a, b, c):
+            u.load_system(s, mode=m)
+            u.set_substep(first)
+        c.set_mode(P.MODE_GRAPH)
+        nc = a.n_colors()[0]
+        done = first
+        for k, mcs in enumerate((1, 4, 7, 20)):
+            a.runSimulationOnGPU(mcs)
+            c.runSimulationOnGPU(mcs)
+            if k % 2 == 0:
+                b.runSimulationOnGPU(mcs)
+            else:
+                at[0] = 2 * done
+                b.set_draw_callback(draw)
+                b.runSimulationOnGPU(mcs)
+                b.set_seed(s.seed)
+                b.set_substep(done + mcs * nc)
+            done += mcs * nc
+            assert a.path() == m
+            assert np.array_equal(a.get_coords(), b.get_coords()), (mode, first, k)
+            assert np.array_equal(a.get_coords(), c.get_coords()), (mode, first, k)
+        for u in (a, b, c):
+            u.validate()
+            u.close()
 
 
 def test_idle_members_beside_longer_ones():
