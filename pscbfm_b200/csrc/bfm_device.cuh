@@ -112,7 +112,7 @@ struct GridSync {
     unsigned int count;   // arrivals so far
     unsigned int base;    // the count at the start of the next launch
     unsigned int fault;   // set when a wait ran out; every CTA then leaves and the host reports the fault
-    unsigned int pad;
+    unsigned int leaving; // CTAs of a kernel with a DoneSignal that have finished
 };
 // The report of a wait that ran out, in mapped host memory.
 struct GridFault {
@@ -166,6 +166,31 @@ __host__ __device__ __forceinline__ uint64_t sm64_mix(uint64_t z)
 __host__ __device__ __forceinline__ uint32_t counter_draw(uint64_t seed, uint64_t k)
 {
     return (uint32_t)(sm64_mix(sm64_mix(seed) + (k + 1) * 0x9E3779B97F4A7C15ull) >> 32);
+}
+
+// The end of a kernel, told to a host that waits for it: the last CTA writes seq to a word of mapped host
+// memory (flag == nullptr: nobody waits). On a B200 the host sees that write earlier than the completion
+// of the kernel on its stream: launch to return 10.8 to 13.1 us against 14.8 for a kernel that writes 24
+// bytes, and 16.5 against 18.8 us for the positions of 1.6K monomers.
+struct DoneSignal {
+    unsigned int* flag;
+    unsigned int seq;
+};
+// At the end of the kernel, by every thread of every CTA; the writes of all CTAs, to host memory too, are
+// visible to who has seen the flag. leaving: a zero, left a zero. (A system fence in every CTA on top of
+// the release of the flag took 4 us more.)
+__device__ __forceinline__ void signal_done(DoneSignal const& d, unsigned int* leaving)
+{
+    if (d.flag == nullptr) return;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (gridDim.x > 1u) {
+        unsigned int before;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(leaving) : "memory");
+        if (before != gridDim.x - 1u) return;
+        *leaving = 0u;
+    }
+    asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(d.flag), "r"(d.seq) : "memory");
 }
 
 // Where a kernel that runs many sub-steps takes their entries from: the host's array (entry of sub-step t

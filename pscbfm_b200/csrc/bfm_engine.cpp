@@ -7,10 +7,13 @@
 
 #include "bfm_engine.hpp"
 
+#include <cuda.h>
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <sstream>
 #include <string>
 
@@ -26,6 +29,13 @@ void cuda_check(cudaError_t e, char const* what)
 
 namespace {
 
+// Positions of up to this many bytes go straight from the gathering kernel into a caller's page-locked
+// buffer: no copy to queue, and its end seen by a word in host memory. us per call, with the copy and
+// so: 1.6K monomers 22.4 and 15.9, 8K 24.1 and 16.5, 52K 33.9 and 26.7, 131K 51.3 and 44.7 (48.8 where
+// the buffer is aligned to 4 bytes only); 1M 254 and 259 (301), where the link is the bound.
+constexpr size_t kDirectReadBytes = 2u << 20;
+constexpr size_t kFlagBytes = 64;   // apart of each other: two hosts' threads poll two lines
+constexpr int kFlagWaitUs = 200;   // the longest watch of the word a kernel writes, before the wait on its stream
 constexpr uint32_t kStepCap = 8192;       // step entries staged per host->device copy
 constexpr uint32_t kGraphMcs = 32;        // MCS per captured graph chunk
 constexpr uint32_t kSlotAlign = 32;
@@ -1331,6 +1341,11 @@ void Updater::streamWait(cudaEvent_t e)
 void Updater::synchronize()
 {
     if (stream_) cuda_check(cudaStreamSynchronize(stream_), "sweep");
+    checkReports();
+}
+
+void Updater::checkReports()
+{
     auto failed = [](GridFault const volatile* f) {
         if (!f || !f->fault) return;
         std::ostringstream m;
@@ -1353,13 +1368,114 @@ void Updater::synchronize()
 
 // ============================================================================ read back
 
+namespace {
+
+// The words kernels signal their end in (DoneSignal), one per updater that waits for kernels: 64 to a
+// page of mapped host memory, which lives while one of them is in use.
+struct DonePage {
+    char* base;
+    uint64_t used;
+};
+std::mutex doneLock;
+std::vector<DonePage> donePages;
+
+// Whether kernels of the current device can write all of [p, p + bytes): page-locked host memory of one
+// allocation or registration, mapped at its own address, not registered as read-only.
+bool device_writable_host(void const* p, size_t bytes)
+{
+    using Query = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static Query const query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Query>(f);
+    }();
+    if (!query) return false;
+    unsigned int type = 0, access = 0, mapped = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                  CU_POINTER_ATTRIBUTE_MAPPED,           CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void* into[] = {&type, &dev, &start, &size, &mapped, &access};
+    CUdeviceptr const at = reinterpret_cast<CUdeviceptr>(p);
+    if (query(6, what, into, at) != CUDA_SUCCESS) return false;
+    return type == CU_MEMORYTYPE_HOST && dev == at && (mapped & 0xffu) != 0u &&
+           access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE && start != 0 && at >= start && at - start <= size &&
+           size - (at - start) >= bytes;
+}
+
+}  // namespace
+
+unsigned int* DoneFlags::take()
+{
+    std::lock_guard<std::mutex> const hold(doneLock);
+    auto p = std::find_if(donePages.begin(), donePages.end(), [](DonePage const& d) { return d.used != ~0ull; });
+    if (p == donePages.end()) {
+        void* m = nullptr;
+        cuda_check(cudaHostAlloc(&m, 64 * kFlagBytes, cudaHostAllocMapped | cudaHostAllocPortable),
+                   "cudaHostAlloc(flags)");
+        donePages.push_back(DonePage{static_cast<char*>(m), 0ull});
+        p = donePages.end() - 1;
+    }
+    uint32_t const k = (uint32_t)__builtin_ctzll(~p->used);
+    p->used |= 1ull << k;
+    auto* const flag = reinterpret_cast<unsigned int*>(p->base + k * kFlagBytes);
+    *static_cast<unsigned int volatile*>(flag) = 0u;
+    return flag;
+}
+
+void DoneFlags::give(unsigned int* flag)
+{
+    std::lock_guard<std::mutex> const hold(doneLock);
+    char* const at = reinterpret_cast<char*>(flag);
+    auto const p = std::find_if(donePages.begin(), donePages.end(), [&](DonePage const& d) {
+        return at >= d.base && at < d.base + 64 * kFlagBytes;
+    });
+    if (p == donePages.end()) return;
+    p->used &= ~(1ull << ((at - p->base) / kFlagBytes));
+    if (p->used == 0ull) {
+        cudaFreeHost(p->base);
+        donePages.erase(p);
+    }
+}
+
+template <typename Ended>
+void Updater::awaitKernel(char const* what, Ended const& ended)
+{
+    // for a while the word that the kernel writes, then the stream, which also reports the error of a
+    // kernel that never got there
+    auto const until = std::chrono::steady_clock::now() + std::chrono::microseconds(kFlagWaitUs);
+    bool seen = false;
+    do {
+        for (int k = 0; k < 64 && !seen; ++k) {
+            seen = ended();
+            if (!seen) __builtin_ia32_pause();
+        }
+    } while (!seen && std::chrono::steady_clock::now() < until);
+    if (!seen) cuda_check(cudaStreamSynchronize(stream_), what);
+    std::atomic_thread_fence(std::memory_order_acquire);
+}
+
 void Updater::downloadPositions(int32_t* out)
 {
-    // the device puts the positions into the caller's order; one copy brings them over
+    // the device puts the positions into the caller's order: at once into a page-locked buffer, else, or
+    // for many, by way of a device buffer and a copy (kDirectReadBytes)
     cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
-    cuda_check(launch_gather_positions(dev_.h, dev_.slotOf, n_, dev_.xyzOut, stream_), "gather positions");
-    cuda_check(cudaMemcpyAsync(out, dev_.xyzOut, 12ull * n_, cudaMemcpyDeviceToHost, stream_), "download positions");
-    d2hBytes_ += 12ull * n_;
+    size_t const bytes = 12ull * n_;
+    d2hBytes_ += bytes;
+    if (bytes <= kDirectReadBytes && device_writable_host(out, bytes)) {
+        if (!done_) done_ = DoneFlags::take();
+        DoneSignal const d{done_, ++doneSeq_};
+        cuda_check(launch_gather_positions(dev_.h, dev_.slotOf, n_, out, d, stream_), "gather positions");
+        awaitKernel("download positions", [&] { return *static_cast<unsigned int const volatile*>(d.flag) == d.seq; });
+        checkReports();
+        return;
+    }
+    cuda_check(launch_gather_positions(dev_.h, dev_.slotOf, n_, dev_.xyzOut, DoneSignal{}, stream_), "gather positions");
+    cuda_check(cudaMemcpyAsync(out, dev_.xyzOut, bytes, cudaMemcpyDeviceToHost, stream_), "download positions");
     synchronize();
 }
 
@@ -1452,11 +1568,12 @@ void Updater::stats(uint64_t out[4])
     requireInit("stats");
     // the sums written into the mapped pinned staging by a kernel on the stream
     ensureStaging();
+    unsigned long long volatile* const sums = hStats_;
+    for (uint32_t c = 0; c < 3; ++c) sums[c] = ~0ull;   // no count of moves
+    std::atomic_thread_fence(std::memory_order_seq_cst);
     cuda_check(launch_publish_stats(dev_.h.stats, dStats_, stream_), "stats");
     d2hBytes_ += 3 * sizeof(unsigned long long);   // written into mapped host memory
-    cuda_check(cudaStreamSynchronize(stream_), "stats");
-    std::atomic_thread_fence(std::memory_order_acquire);
-    unsigned long long const volatile* const sums = hStats_;
+    awaitKernel("stats", [&] { return sums[0] != ~0ull && sums[1] != ~0ull && sums[2] != ~0ull; });
     for (uint32_t c = 0; c < 3; ++c) out[c] = sums[c];
     out[3] = mcsDone_;
 }
@@ -1658,6 +1775,13 @@ void Updater::freeDevice()
         pubEv_ = nullptr;
     }
     if (!graphs_.empty() && stream_) cudaStreamSynchronize(stream_);   // no graph of ours in flight
+    if (done_) {
+        if (*static_cast<unsigned int volatile*>(done_) != doneSeq_ && stream_)
+            cudaStreamSynchronize(stream_);   // (a failed read-back) no kernel of ours writes it any more
+        DoneFlags::give(done_);
+        done_ = nullptr;
+        doneSeq_ = 0;
+    }
     for (auto& g : graphs_) cudaGraphExecDestroy(g.exec);
     graphs_.clear();
     // stream-ordered frees: after this system's queued work (and whatever its stream waits on,

@@ -59,6 +59,12 @@ enum Mode : int {
     kModeCluster = 5,      // bond codes: one cluster of CTAs holds the system in shared memory
 };
 
+// Words of mapped host memory for DoneSignal, shared out over the process's updaters.
+struct DoneFlags {
+    static unsigned int* take();
+    static void give(unsigned int* flag);
+};
+
 class Updater {
 public:
     explicit Updater(int gpu);
@@ -197,6 +203,10 @@ private:
     void planCluster();   // the cluster size and chunks per warp of the cluster-resident kernel
     void enqueuePersistent(uint32_t nSteps);
     StepSource stepSource(uint32_t nSteps);   // the next nSteps entries, for one launch that runs them
+    // until ended() holds, which a kernel queued last makes true in host memory, or the stream is idle
+    template <typename Ended>
+    void awaitKernel(char const* what, Ended const& ended);
+    void checkReports();                // throws if a sweep that has ended reported a barrier timeout
     void fillSteps(uint32_t nSteps, StepEntry* hostBuf, bool residentParity);
     void freeDevice();
     void ensureStaging();
@@ -285,6 +295,8 @@ private:
     };
     std::vector<GraphExec> graphs_;
     cudaEvent_t stepsFree_ = nullptr;          // host staging may be rewritten after this event
+    unsigned int* done_ = nullptr;             // where kernels signal their end, and the last signal's number
+    unsigned int doneSeq_ = 0;
     uint64_t launches_ = 0;
     uint64_t h2dBytes_ = 0, d2hBytes_ = 0;
     int gridBlock_ = 0;

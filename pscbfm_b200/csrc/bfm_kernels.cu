@@ -319,26 +319,41 @@ __global__ void k_build_lattice(SysDev const* __restrict__ sysv, uint32_t n)
 // ------------------------------------------------------------------------ position read-back
 
 // Positions in the caller's monomer order, x y z interleaved: out[3 i + a] is coordinate a of the
-// monomer in sorted slot slotOf[i]. One copy of out then gives the caller's array. With bond codes
-// (rec != nullptr) x, y, z hold image offsets and the lattice address the rest (slot_coord).
-__global__ void k_gather_positions(int32_t const* __restrict__ x, int32_t const* __restrict__ y,
-                                   int32_t const* __restrict__ z, uint32_t const* __restrict__ rec, uint32_t recWords,
-                                   uint32_t m0, uint32_t m1, uint32_t m2, uint32_t const* __restrict__ slotOf,
-                                   uint32_t n, int32_t* __restrict__ out)
+// monomer in sorted slot slotOf[i]. With bond codes (rec != nullptr) x, y, z hold image offsets and the
+// lattice address the rest (slot_coord). out may be host memory: a warp turns its 32 triples around in
+// shared memory and stores 128 contiguous bytes per instruction (three stores with a stride of 12 bytes
+// reach the host as partial sectors).
+constexpr uint32_t kGatherBlock = 256;
+__global__ void __launch_bounds__(kGatherBlock)
+    k_gather_positions(int32_t const* __restrict__ x, int32_t const* __restrict__ y, int32_t const* __restrict__ z,
+                       uint32_t const* __restrict__ rec, uint32_t recWords, uint32_t m0, uint32_t m1, uint32_t m2,
+                       uint32_t const* __restrict__ slotOf, uint32_t n, int32_t* __restrict__ out,
+                       unsigned int* leaving, DoneSignal const done)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t const g = slotOf[i];
-        int32_t cx = x[g], cy = y[g], cz = z[g];
-        if (rec != nullptr) {
-            uint32_t const p = rec[(size_t)g * recWords];
-            cx += int32_t(axis_coord(p, m0));
-            cy += int32_t(axis_coord(p, m1));
-            cz += int32_t(axis_coord(p, m2));
+    __shared__ int32_t turn[3 * kGatherBlock];
+    uint32_t const lane = threadIdx.x & 31u;
+    int32_t* const mine = turn + 3u * (threadIdx.x - lane);   // this warp's triples
+    for (uint32_t first = (blockIdx.x * kGatherBlock + threadIdx.x) - lane; first < n; first += gridDim.x * kGatherBlock) {
+        uint32_t const i = first + lane;
+        if (i < n) {
+            uint32_t const g = slotOf[i];
+            int32_t cx = x[g], cy = y[g], cz = z[g];
+            if (rec != nullptr) {
+                uint32_t const p = rec[(size_t)g * recWords];
+                cx += int32_t(axis_coord(p, m0));
+                cy += int32_t(axis_coord(p, m1));
+                cz += int32_t(axis_coord(p, m2));
+            }
+            mine[3u * lane] = cx;
+            mine[3u * lane + 1u] = cy;
+            mine[3u * lane + 2u] = cz;
         }
-        out[3ull * i] = cx;
-        out[3ull * i + 1] = cy;
-        out[3ull * i + 2] = cz;
+        __syncwarp();
+        uint32_t const words = 3u * min(32u, n - first);
+        for (uint32_t k = lane; k < words; k += 32u) out[3ull * first + k] = mine[k];
+        __syncwarp();
     }
+    signal_done(done, leaving);
 }
 
 // Unfolded positions of every slot of a bond-code system in slot order (the MSD reference of the
@@ -354,8 +369,9 @@ __global__ void k_unfold_positions(SysDev const* __restrict__ sysv, int32_t* __r
     }
 }
 
-// One warp: each counter's slots summed with a warp reduction, written to host memory. The host
-// reads them only after an event behind this kernel has completed, so no fence is needed here.
+// One warp: each counter's slots summed with a warp reduction, written to host memory, each sum as one
+// 8-byte store. The host reads them after an event behind this kernel, or watches the words themselves
+// (14.4 -> 12.2 us from call to return), so no fence is needed here.
 __global__ void k_publish_stats(unsigned long long const* __restrict__ stats, unsigned long long* __restrict__ out)
 {
     uint32_t const lane = threadIdx.x;
@@ -429,14 +445,13 @@ cudaError_t launch_resident(SysDev const* dSys, uint32_t const* dList, uint32_t 
 }
 
 cudaError_t launch_gather_positions(SysDev const& h, uint32_t const* slotOf, uint32_t n, int32_t* out,
-                                    cudaStream_t s)
+                                    DoneSignal const& done, cudaStream_t s)
 {
-    uint32_t const block = 256;
-    uint32_t const grid = std::min((n + block - 1) / block, 148u * 8u);
+    uint32_t const grid = std::min((n + kGatherBlock - 1) / kGatherBlock, 148u * 8u);
     if (grid == 0) return cudaSuccess;
     bool const codes = h.codeMode != kCodeNone;
-    k_gather_positions<<<grid, block, 0, s>>>(h.x, h.y, h.z, codes ? h.rec : nullptr, rec_words(h.codeMode),
-                                              h.amask[0], h.amask[1], h.amask[2], slotOf, n, out);
+    k_gather_positions<<<grid, kGatherBlock, 0, s>>>(h.x, h.y, h.z, codes ? h.rec : nullptr, rec_words(h.codeMode),
+                                              h.amask[0], h.amask[1], h.amask[2], slotOf, n, out, &h.gs->leaving, done);
     return cudaGetLastError();
 }
 

@@ -165,7 +165,7 @@ cudaError_t launch_observables(SysDev const* dSys, ObsDev const& o, long long* d
 cudaError_t launch_build_lattice(SysDev const* dSys, uint32_t npad, cudaStream_t s);
 // Positions in the caller's order, x y z interleaved (out[3 i + a] from sorted slot slotOf[i]).
 cudaError_t launch_gather_positions(SysDev const& h, uint32_t const* slotOf, uint32_t n, int32_t* out,
-                                    cudaStream_t s);
+                                    DoneSignal const& done, cudaStream_t s);
 // Unfolded positions of every slot of bond-code system dSys[0] (image offsets plus the coordinates
 // of the lattice addresses) into ox, oy, oz, in slot order.
 cudaError_t launch_unfold_positions(SysDev const* dSys, uint32_t npad, int32_t* ox, int32_t* oy, int32_t* oz,
