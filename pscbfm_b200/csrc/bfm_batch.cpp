@@ -10,7 +10,8 @@
 // own sub-steps from its own stream exactly as it would alone, so its trajectory is unchanged by
 // batching.
 //
-// A run stages the step entries of all its sub-steps with one host-to-device copy; the resident
+// A run stages the members' streams, and the step entries that no kernel makes from them (grid-phase
+// members, callbacks), with one host-to-device copy; the resident
 // and the grid-phase launches then proceed on two streams without meeting until the run ends, and
 // the host returns as soon as the work is queued. The slab sweeps run on a stream of their own. Member streams are ordered before the run and
 // after it with events, never with host waits.
@@ -377,6 +378,24 @@ void Batch::ensureGraph()
     cuda_check(ie, "graph instantiate");
 }
 
+bool Batch::ownEntries(uint32_t m) const
+{
+    // a kernel that runs all of the member's sub-steps makes their entries (bond codes, counter stream)
+    return wholeRun_[m] && members_[m]->codeMode() != kCodeNone && members_[m]->countsDraws();
+}
+
+bool Batch::hostEntries() const
+{
+    for (uint32_t m = 0; m < (uint32_t)members_.size(); ++m)
+        if (!ownEntries(m)) return true;
+    return false;
+}
+
+size_t Batch::streamUnits() const
+{
+    return (sizeof(StepStream) * members_.size() + sizeof(StepEntry) - 1) / sizeof(StepEntry);
+}
+
 void Batch::prepare(int32_t const* mcs)
 {
     // one-time host work of a run (staging growth, graph capture), done ahead of a timed run
@@ -384,7 +403,7 @@ void Batch::prepare(int32_t const* mcs)
     uint64_t T = 0;
     for (uint32_t m = 0; m < M; ++m) T = std::max(T, (uint64_t)std::max(mcs[m], 0) * members_[m]->nColors());
     if (T == 0) return;
-    reserveSteps((size_t)T * M);
+    reserveSteps(streamUnits() + (hostEntries() ? (size_t)T * M : 0));
     if (!grid_.empty() && T >= stepCap_) ensureGraph();
 }
 
@@ -420,19 +439,27 @@ void Batch::run(int32_t const* mcs)
         T = std::max(T, need[m]);
     }
     if (T > 0) {
-        size_t const entries = (size_t)T * M;
+        // the members' streams, and the entries of those whose kernels don't make them
+        size_t const units = streamUnits(), entries = units + (hostEntries() ? (size_t)T * M : 0);
         reserveSteps(entries);
-        for (uint64_t t = 0; t < T; ++t)
-            for (uint32_t m = 0; m < M; ++m) {
-                StepEntry& e = hSteps_[(size_t)t * M + m];
-                if (t < need[m]) e = members_[m]->nextStep();
-                else e = StepEntry{kNoColor, 0u, 0u, kNoColor, 0u, 0u, 0u, 0u};
-            }
+        StepStream* const streams = reinterpret_cast<StepStream*>(hSteps_);
+        StepEntry* const host = hSteps_ + units;
+        std::vector<uint32_t> drawn;
+        for (uint32_t m = 0; m < M; ++m) {
+            streams[m] = StepStream{};
+            if (!ownEntries(m) || !members_[m]->streamSteps((uint32_t)need[m], streams[m])) drawn.push_back(m);
+        }
+        // sub-step by sub-step: members may share a callback's generator
+        for (uint64_t t = 0; t < T && !drawn.empty(); ++t)
+            for (uint32_t m : drawn)
+                host[(size_t)t * M + m] = t < need[m] ? members_[m]->nextStep()
+                                                      : StepEntry{kNoColor, 0u, 0u, kNoColor, 0u, 0u, 0u, 0u};
+        StepEntry const* const dEntries = dStepsAll_ + units;
         cuda_check(cudaMemcpyAsync(dStepsAll_, hSteps_, sizeof(StepEntry) * entries, cudaMemcpyHostToDevice, stream_),
                    "batch steps H2D");
         cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
         if (!resident_.empty() || !slab_.empty()) cuda_check(cudaEventRecord(fork_, stream_), "event");
-        StepSource const src{dStepsAll_, M, 0u, 0ull, 0ull};
+        StepSource const src{dEntries, reinterpret_cast<StepStream const*>(dStepsAll_), StepStream{}, M};
         if (!slab_.empty()) {
             cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
             for (auto const& w : slab_) {
@@ -451,7 +478,7 @@ void Batch::run(int32_t const* mcs)
             if (!slab_.empty() && residentsAfter_) cuda_check(cudaStreamWaitEvent(stream2_, sideJoin_, 0), "wait");
             for (auto const& g : resident_) {
                 cuda_check(g.codeMode == kCodeNone
-                               ? launch_resident(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, dStepsAll_,
+                               ? launch_resident(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, dEntries,
                                                  M, (uint32_t)T, g.smem, stream2_)
                                : launch_resident_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, src,
                                                     (uint32_t)T, g.smem, g.codeMode, stream2_),
@@ -464,14 +491,14 @@ void Batch::run(int32_t const* mcs)
                 uint32_t const chunk = (uint32_t)std::min<uint64_t>(stepCap_, T - t0);
                 if (chunk == stepCap_) {
                     // the captured graph reads its entries from the window
-                    cuda_check(cudaMemcpyAsync(dWindow_, dStepsAll_ + t0 * M, sizeof(StepEntry) * stepCap_ * M,
+                    cuda_check(cudaMemcpyAsync(dWindow_, dEntries + t0 * M, sizeof(StepEntry) * stepCap_ * M,
                                                cudaMemcpyDeviceToDevice, stream_),
                                "batch window");
                     ensureGraph();
                     cuda_check(cudaGraphLaunch(graph_, stream_), "batch graph launch");
                 } else {
                     for (uint32_t t = 0; t < chunk; ++t)
-                        cuda_check(launchGrid(dStepsAll_ + (t0 + t) * M), "batch grid launch");
+                        cuda_check(launchGrid(dEntries + (t0 + t) * M), "batch grid launch");
                 }
                 launches_ += 2ull * chunk * grid_.size();
             }

@@ -193,30 +193,36 @@ __device__ __forceinline__ void signal_done(DoneSignal const& d, unsigned int* l
     asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(d.flag), "r"(d.seq) : "memory");
 }
 
-// Where a kernel that runs many sub-steps takes their entries from: the host's array (entry of sub-step t
-// of system s at steps[t * stride + s]), or, on != 0 (one system), the counter stream itself: sub-step t
-// of the launch is sub-step t0 + t of the stream of `seed`. Such entries name no previous sub-step.
-// Made on the device, a run needs no copy of 32 bytes per sub-step ahead of the sweep and no host loop:
-// 10 MCS of the 1M-monomer melt with the positions read back 483 -> 465 us, one MCS of a
-// 64^3 chain system 60.5 -> 59.
+// The entries of n sub-steps of one system's counter stream: those of seed from sub-step t0 on, and idle
+// ones (kNoColor) after them. on == 0: the host's array holds the system's entries.
+struct StepStream {
+    unsigned long long seed, t0;
+    uint32_t n, on;
+};
+// Where a kernel that runs many sub-steps takes their entries from: entry of sub-step t of system s at
+// steps[t * stride + s], unless its stream (streams[s], or own where streams is nullptr) is on; then the
+// kernel makes them. Such entries name no previous sub-step.
+// Made on the device, a run needs no copy of 32 bytes per sub-step and system ahead of the sweep and no
+// host loop: 10 MCS of the 1M-monomer melt with the positions read back 483 -> 465 us, one MCS of a
+// 64^3 chain system 60.5 -> 59, 100 MCS of 128 systems of 1.6K monomers 803 -> 534.
 struct StepSource {
     StepEntry const* steps;
-    uint32_t stride, on;
-    unsigned long long seed, t0;
+    StepStream const* streams;
+    StepStream own;
+    uint32_t stride;
 };
-__device__ __forceinline__ StepEntry step_entry(StepSource const& src, uint32_t sys, uint32_t t, uint32_t const* grp,
-                                                uint32_t nColors)
+__device__ __forceinline__ StepEntry step_entry(StepSource const& src, StepStream const& own, uint32_t sys, uint32_t t,
+                                                uint32_t const* grp, uint32_t nColors)
 {
-    if (!src.on) return src.steps[(size_t)t * src.stride + sys];
-    uint64_t const at = src.t0 + t;
-    StepEntry e;
-    e.color = counter_draw(src.seed, 2 * at) % nColors;
-    e.seed = counter_draw(src.seed, 2 * at + 1);
+    if (!own.on) return src.steps[(size_t)t * src.stride + sys];
+    StepEntry e = {kNoColor, 0u, 0u, kNoColor, 0u, 0u, 0u, 0u};
+    if (t >= own.n) return e;
+    uint64_t const at = own.t0 + t;
+    e.color = counter_draw(own.seed, 2 * at) % nColors;
+    e.seed = counter_draw(own.seed, 2 * at + 1);
     e.parity = (uint32_t)(at & 1u);
-    e.prevColor = kNoColor;
     e.off = grp[2 * e.color];
     e.cnt = grp[2 * e.color + 1];
-    e.poff = e.pcnt = 0u;
     return e;
 }
 

@@ -1166,22 +1166,30 @@ void Updater::timeKernels(int32_t nMcs, double out[4])
     out[3] = (double)n;
 }
 
+bool Updater::streamSteps(uint32_t nSteps, StepStream& out)
+{
+    out = StepStream{};
+    if (drawKind_ != kDrawCounter) return false;
+    out = StepStream{drawSeed_, subStep_, nSteps, 1u};
+    subStep_ += nSteps;
+    return true;
+}
+
 StepSource Updater::stepSource(uint32_t nSteps)
 {
     // the entries of the next nSteps sub-steps for a kernel that runs them all: the counter stream's are
     // made on the device, a callback's go up in one copy
-    if (drawKind_ == kDrawCounter) {
-        StepSource const src{nullptr, 0u, 1u, drawSeed_, subStep_};
-        subStep_ += nSteps;
-        return src;
-    }
+    StepSource src{};
+    if (streamSteps(nSteps, src.own)) return src;
     cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
     fillSteps(nSteps, hSteps_, false);
     cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * nSteps, cudaMemcpyHostToDevice, stream_),
                "steps H2D");
     h2dBytes_ += sizeof(StepEntry) * nSteps;
     cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
-    return StepSource{dev_.dSteps, 1u, 0u, 0ull, 0ull};
+    src.steps = dev_.dSteps;
+    src.stride = 1;
+    return src;
 }
 
 void Updater::enqueueResident(uint32_t nSteps)

@@ -148,6 +148,9 @@ public:
     SysDev* deviceDesc() const { return dev_.dDesc; }
     uint32_t const* sortedSlot() const { return oldToNew_.data(); }
     StepEntry nextStep();                    // consumes the draws of one sub-step
+    // the next nSteps sub-steps for a kernel that makes their entries (the counter stream; else false)
+    bool streamSteps(uint32_t nSteps, StepStream& out);
+    bool countsDraws() const { return drawKind_ == kDrawCounter; }
     void scrubPending(cudaStream_t s);       // clears the temporary marks of the last sub-step
     // report: where a launch of the run may report a failed barrier (looked at by the next synchronise)
     void noteExternalRun(uint64_t subSteps, uint64_t mcs, bool pendingMarks, uint32_t lastColor,
@@ -430,6 +433,9 @@ private:
     void validateMembers(Updater* const* members, uint32_t n) const;
     cudaError_t launchGrid(StepEntry const* e);   // one sub-step of every grid group, entries [members]
     void reserveSteps(size_t entries);           // host staging and device entries for a run
+    bool ownEntries(uint32_t m) const;           // member m's kernel makes its entries
+    bool hostEntries() const;                    // some member's does not
+    size_t streamUnits() const;                  // the members' streams, in entries
     void ensureGraph();                          // capture the graph of stepCap_ sub-steps
     void prepare(int32_t const* mcs);            // both, for a run of mcs[i] MCS per member
     int gpu_;
@@ -457,7 +463,7 @@ private:
     size_t arenaBytes_ = 0, hStepsCap_ = 0, dStepsCap_ = 0;
     SysDev* dSys_ = nullptr;                   // descriptors of all members
     StepEntry* dWindow_ = nullptr;             // [stepCap_][members]: entries the captured graph reads
-    StepEntry* dStepsAll_ = nullptr;           // [sub-steps of the run][members]
+    StepEntry* dStepsAll_ = nullptr;           // the members' streams, then [sub-steps of the run][members]
     StepEntry* hSteps_ = nullptr;              // pinned staging of dStepsAll_
     size_t stepCap_ = 0;
     cudaEvent_t stepsFree_ = nullptr;

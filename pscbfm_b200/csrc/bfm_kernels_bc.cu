@@ -627,8 +627,8 @@ __host__ __device__ __forceinline__ bool slab_clear_all(uint32_t nwords, uint32_
 // CTAs with at most kSlabSmallSlots slots per colour have 256: fewer warps meet faster at the CTA's own
 // barriers (131K monomers 9.0 against 9.6 us per MCS, 210K 9.3 against 9.9, 60K 7.9 against 8.5).
 template <typename W, int B, bool kCache, bool kIdle>
-__device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& src, uint32_t sysId, uint32_t nSteps,
-                                           uint32_t C, uint32_t rank, uint32_t cap, uint32_t capG, bool clearAll,
+__device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& src, StepStream const& own,
+                                           uint32_t sysId, uint32_t nSteps, uint32_t C, uint32_t rank, uint32_t cap, uint32_t capG, bool clearAll,
                                            GridFault* report)
 {
     constexpr uint32_t kSlots = CodeWord<W>::kSlots;
@@ -759,7 +759,7 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& sr
     unsigned long long att = 0ull;
     auto fetch_steps = [&](uint32_t block) {   // the waiter's lanes
         uint32_t const t = block * kStepBlock + lane;
-        if (lane < kStepBlock && t < nSteps) stepSm[block & 1u][lane] = step_entry(src, sysId, t, S.grp, nColors);
+        if (lane < kStepBlock && t < nSteps) stepSm[block & 1u][lane] = step_entry(src, own, sysId, t, S.grp, nColors);
     };
     if (waiter) {
         fetch_steps(0);
@@ -1008,7 +1008,8 @@ __global__ void __launch_bounds__(B, 1)
     k_slab_bc(const __grid_constant__ SysDev S, const __grid_constant__ StepSource src, uint32_t nSteps, uint32_t cap,
               uint32_t capG, uint32_t clearAll, GridFault* report)
 {
-    slab_sweep<W, B, kCache, false>(S, src, 0u, nSteps, gridDim.x, blockIdx.x, cap, capG, clearAll != 0u, report);
+    slab_sweep<W, B, kCache, false>(S, src, src.own, 0u, nSteps, gridDim.x, blockIdx.x, cap, capG, clearAll != 0u,
+                                    report);
 }
 
 // Many systems in one cooperative launch: CTA b runs share refs[b].rank of system refs[b].sys with the
@@ -1019,14 +1020,16 @@ __global__ void __launch_bounds__(B, 1)
                     const __grid_constant__ StepSource src, uint32_t nSteps, GridFault* report)
 {
     __shared__ SysDev S;
+    __shared__ StepStream own;
     __shared__ uint32_t caps[3];
     SlabRef const r = refs[blockIdx.x];
+    if (threadIdx.x == 0) own = src.streams != nullptr ? src.streams[r.sys] : src.own;
     copy_desc(S, sysv + r.sys);
     __syncthreads();
     if (threadIdx.x == 0)
         slab_caps([&](uint32_t c) { return S.grp[2 * c + 1]; }, S.nColors, r.ctas, caps[0], caps[1], caps[2]);
     __syncthreads();
-    slab_sweep<W, B, true, true>(S, src, r.sys, nSteps, r.ctas, r.rank, caps[0], caps[1],
+    slab_sweep<W, B, true, true>(S, src, own, r.sys, nSteps, r.ctas, r.rank, caps[0], caps[1],
                                  slab_clear_all(S.nwords, caps[2]), report + r.sys);
 }
 
@@ -1126,9 +1129,11 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const*
     constexpr uint32_t kRefBits = slab_ref_bits(sizeof(W) == 8), kRefMask = (1u << kRefBits) - 1u;
     __shared__ SysDev S;
     __shared__ __align__(16) StepEntry stepSm[kStepBlock];
+    __shared__ StepStream own;
     __shared__ uint32_t nMov[2], nCand, maxGroup;   // nMov: per sub-step parity
     extern __shared__ unsigned long long smem[];
     uint32_t const sysId = sysList[blockIdx.x];
+    if (threadIdx.x == 0) own = src.streams != nullptr ? src.streams[sysId] : src.own;
     copy_desc(S, sysv + sysId);
     __syncthreads();
     uint32_t const nw = S.nwords, np = S.npad, maxc = S.maxc;
@@ -1205,7 +1210,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const*
     for (uint32_t t = 0; t < nSteps; ++t) {
         if (t % kStepBlock == 0) {   // (the last barrier of the sub-step before ended the reads of the old ones)
             uint32_t const n = min(kStepBlock, nSteps - t);
-            if (tid < n) stepSm[tid] = step_entry(src, sysId, t + tid, S.grp, S.nColors);
+            if (tid < n) stepSm[tid] = step_entry(src, own, sysId, t + tid, S.grp, S.nColors);
             __syncthreads();   // (the first also publishes the state loaded above)
             drawn = false;
         }
@@ -1400,9 +1405,11 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
     while ((1u << logC) < C) ++logC;   // a power of two (launch_cluster_bc)
     __shared__ SysDev S;
     __shared__ __align__(16) StepEntry stepSm[kStepBlock];
+    __shared__ StepStream own;
     __shared__ uint32_t nMov[2];   // per sub-step parity
     extern __shared__ unsigned long long smem[];
     uint32_t const sysId = sysList[blockIdx.x >> logC];
+    if (threadIdx.x == 0) own = src.streams != nullptr ? src.streams[sysId] : src.own;
     copy_desc(S, sysv + sysId);
     __syncthreads();
     uint32_t const np = S.npad, nwC = S.nwords >> logC, cap = cluster_slots_per_cta(np, logC), maxc = S.maxc;
@@ -1478,7 +1485,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
     for (uint32_t t = 0; t < nSteps; ++t) {
         if (t % kStepBlock == 0) {   // (the last barrier of the sub-step before ended the reads of the old ones)
             uint32_t const n = min(kStepBlock, nSteps - t);
-            if (tid < n) stepSm[tid] = step_entry(src, sysId, t + tid, S.grp, S.nColors);
+            if (tid < n) stepSm[tid] = step_entry(src, own, sysId, t + tid, S.grp, S.nColors);
             __syncthreads();
             drawn = false;
         }

@@ -100,6 +100,37 @@ def test_entries_made_on_the_device_vs_the_callbacks(mode):
             u.close()
 
 
+@pytest.mark.parametrize("cluster", [True, False])
+def test_batch_members_with_callbacks_beside_streams(cluster):
+    """Members on the counter stream, whose kernels make their entries, beside two that share one host
+    generator: its draws go to them sub-step by sub-step, in the members' order."""
+    systems = [S.serpentine_chains(32, 16, 0.3, seed=50), S.serpentine_chains(32, 16, 0.4, seed=51),
+               S.serpentine_chains(128, 32, 0.2, seed=52), S.serpentine_chains(64, 64, 0.3, seed=53)]
+    plan = [[5, 9, 3, 12], [4, 0, 6, 1]]
+    called = (1, 2)
+    draws = {m: [] for m in called}
+    at = 0
+    for mcs in plan:   # both have two colours: two draws per sub-step
+        for t in range(2 * max(mcs)):
+            for m in called:
+                if t < 2 * mcs[m]:
+                    draws[m] += [P.updater.counter_draw(77, at), P.updater.counter_draw(77, at + 1)]
+                    at += 2
+    k = iter(range(at))
+    members = [P.UpdaterGPUScBFM_AB_Type(0).load_system(s) for s in systems]
+    for m in called:
+        members[m].set_draw_callback(lambda: P.updater.counter_draw(77, next(k)))
+    b = P.Batch(members)
+    b.set_cluster(cluster)
+    for mcs in plan:
+        b.run_each(mcs)
+    for m, (s, u) in enumerate(zip(systems, members)):
+        mcs = sum(p[m] for p in plan)
+        want = O.run(s, mcs, draws=np.array(draws[m], dtype=np.uint32)) if m in called else O.run(s, mcs)
+        assert np.array_equal(u.get_coords(), want[0]), m
+    b.close()
+
+
 def test_idle_members_beside_longer_ones():
     """A batch whose members stop at different sub-steps: the shared-memory kernels skip the idle entries
     that follow a member's last sub-step, inside and across blocks of step entries."""
