@@ -2,7 +2,8 @@
 //
 // Systems whose lattices (and, in the bond-code representation, packed coordinates and bond
 // codes) fit one CTA's shared memory run in the resident kernel, one CTA per system, one launch
-// per run. Larger systems of the bond-code representation run in the slab sweep, each on CTAs of its
+// per run; where such systems leave SMs idle, the largest of them run on clusters of CTAs (planClusters).
+// Larger systems of the bond-code representation run in the slab sweep, each on CTAs of its
 // own, several systems in one cooperative launch per run (planSlabs). What fits neither shares
 // the grid-phase kernels: one check and one perform launch per
 // sub-step and representation cover the active colour group of every such system at once, and
@@ -26,6 +27,7 @@
 namespace bfm {
 
 namespace {
+constexpr double kClusterGain = 0.9;      // clusters are taken for at least a tenth of a batch's time
 constexpr uint32_t kBatchChunk = 64;      // sub-steps per captured graph of the grid phase
 size_t up256(size_t v) { return (v + 255) & ~size_t(255); }
 }  // namespace
@@ -75,6 +77,7 @@ uint32_t Batch::clusterCount() const
     uint32_t n = 0;
     for (auto const& w : slab_)
         for (SlabRef const& r : w.refs) n += r.rank == 0 ? 1u : 0u;
+    for (auto const& g : cluster_) n += (uint32_t)g.members.size();
     return n;
 }
 
@@ -122,7 +125,9 @@ void Batch::rebuild()
     };
     std::vector<char> slabbed;
     slab_ = planSlabs(slabbed, residentsAfter_);
-    if (!slab_.empty() && !side_) {
+    std::vector<char> clustered;
+    cluster_ = planClusters(clustered);
+    if (!(slab_.empty() && cluster_.empty()) && !side_) {
         cuda_check(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
         cuda_check(cudaEventCreateWithFlags(&sideJoin_, cudaEventDisableTiming), "cudaEventCreate");
     }
@@ -140,7 +145,9 @@ void Batch::rebuild()
     }
     for (uint32_t m = 0; m < M; ++m) {
         Updater* u = members_[m];
-        if (residentOn_ && u->residentEligible()) {
+        if (clustered[m]) {
+            wholeRun_[m] = 1;
+        } else if (residentOn_ && u->residentEligible()) {
             ResidentGroup& g = resGroup(u->codeMode());
             g.members.push_back(m);
             g.smem = std::max(g.smem, u->residentSmem());
@@ -162,6 +169,7 @@ void Batch::rebuild()
     for (auto const& g : grid_) total += up256(sizeof(TileRef) * g.tiles.size()) + up256(sizeof(TileRef) * g.ptiles.size());
     for (auto const& g : resident_) total += up256(sizeof(uint32_t) * g.members.size());
     for (auto const& w : slab_) total += up256(sizeof(SlabRef) * w.refs.size());
+    for (auto const& g : cluster_) total += up256(sizeof(uint32_t) * g.members.size());
     if (total > arenaBytes_) {   // grows only: membership changes reuse the arena
         if (arena_) cuda_check(cudaFreeAsync(arena_, stream_), "cudaFreeAsync(batch)");
         arena_ = nullptr;
@@ -203,6 +211,13 @@ void Batch::rebuild()
         cuda_check(cudaMemcpyAsync(w.dRefs, w.refs.data(), sizeof(SlabRef) * w.refs.size(), cudaMemcpyHostToDevice,
                                    stream_),
                    "upload slab CTAs");
+    }
+    for (auto& g : cluster_) {
+        g.dList = reinterpret_cast<uint32_t*>(p);
+        p += up256(sizeof(uint32_t) * g.members.size());
+        cuda_check(cudaMemcpyAsync(g.dList, g.members.data(), sizeof(uint32_t) * g.members.size(),
+                                   cudaMemcpyHostToDevice, stream_),
+                   "upload cluster list");
     }
     // the host vectors above die with this call: finish their copies now
     cuda_check(cudaStreamSynchronize(stream_), "batch uploads");
@@ -297,6 +312,64 @@ std::vector<Batch::SlabWave> Batch::planSlabs(std::vector<char>& taken, bool& re
         waves.push_back(std::move(wave));
     }
     return waves;
+}
+
+std::vector<Batch::ClusterGroup> Batch::planClusters(std::vector<char>& taken) const
+{
+    // A batch lasts as long as its largest member, and a member that fits one CTA takes longer there than
+    // on a cluster's CTAs (us per MCS with g slots per colour, fitted to 600 to 13K slots: 2.9 + 0.00185 g on
+    // one, 4.4 + 0.0046 g / C on C). Where every member fits one CTA and SMs are left over, the k largest go
+    // to clusters: C and k with the least time of the longest member. Sixteen systems of 0.4K to 10.5K
+    // monomers, on one CTA each, with slab sweeps on the SMs left over, and so: 14.2, 9.4 and 6.8 us per MCS;
+    // 7, 9, 16, 32 and 36 systems of 8K monomers 10.8 -> 5.8, 7.2, 9.5, 9.8 and 10.9.
+    uint32_t const M = (uint32_t)members_.size();
+    taken.assign(M, 0);
+    std::vector<ClusterGroup> groups;
+    if (!clusterOn_ || !residentOn_) return groups;
+    std::vector<uint32_t> order;
+    for (uint32_t m = 0; m < M; ++m) {
+        if (!members_[m]->residentEligible()) return groups;
+        if (members_[m]->codeMode() != kCodeNone) order.push_back(m);
+    }
+    std::stable_sort(order.begin(), order.end(),
+                     [&](uint32_t a, uint32_t b) { return members_[a]->maxGroup() > members_[b]->maxGroup(); });
+    auto slots = [&](size_t k) { return k < order.size() ? (double)members_[order[k]]->maxGroup() : 0.0; };
+    auto alone = [](double g) { return 2.9 + 0.00185 * g; };
+    auto spread = [](double g, double C) { return 4.4 + 0.0046 * g / C; };
+    double best = alone(slots(0)) * kClusterGain;
+    size_t bestCount = 0;
+    uint32_t bestLog = 0;
+    for (uint32_t logC = 4; logC >= 2; --logC) {
+        uint32_t const C = 1u << logC;
+        uint32_t atOnce = ~0u;   // clusters of the batch's share of the SMs
+        for (size_t k = 0; k < order.size(); ++k) {
+            ClusterPlan plan;
+            atOnce = std::min(atOnce, members_[order[k]]->clusterPlan(logC, plan) * slabSms_ / smCount_);
+            if (k + 1 > atOnce || (k + 1) * (C - 1u) + M > slabSms_) break;
+            double const time = std::max(spread(slots(0), C), alone(slots(k + 1)));
+            if (time < best) {
+                best = time;
+                bestCount = k + 1;
+                bestLog = logC;
+            }
+        }
+    }
+    for (size_t k = 0; k < bestCount; ++k) {
+        uint32_t const m = order[k];
+        Updater const& u = *members_[m];
+        ClusterPlan plan;
+        u.clusterPlan(bestLog, plan);
+        auto g = std::find_if(groups.begin(), groups.end(), [&](ClusterGroup const& c) { return c.codeMode == u.codeMode(); });
+        if (g == groups.end()) g = groups.insert(g, ClusterGroup{u.codeMode(), plan, {}, nullptr});
+        // one launch has one number of chunks per warp and one size of shared memory (descending groups: the
+        // first member's chunks do for all)
+        size_t const smem = u.clusterSmem(bestLog, g->plan.perWarp);
+        if (smem > kResidentMaxSmem) continue;
+        g->plan.smem = std::max(g->plan.smem, smem);
+        g->members.push_back(m);
+        taken[m] = 1;
+    }
+    return groups;
 }
 
 void Batch::setSlabSms(uint32_t sms)
@@ -458,10 +531,17 @@ void Batch::run(int32_t const* mcs)
         cuda_check(cudaMemcpyAsync(dStepsAll_, hSteps_, sizeof(StepEntry) * entries, cudaMemcpyHostToDevice, stream_),
                    "batch steps H2D");
         cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
-        if (!resident_.empty() || !slab_.empty()) cuda_check(cudaEventRecord(fork_, stream_), "event");
+        bool const sides = !slab_.empty() || !cluster_.empty();
+        if (!resident_.empty() || sides) cuda_check(cudaEventRecord(fork_, stream_), "event");
         StepSource const src{dEntries, reinterpret_cast<StepStream const*>(dStepsAll_), StepStream{}, M};
-        if (!slab_.empty()) {
+        if (sides) {
             cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
+            for (auto const& g : cluster_) {
+                cuda_check(launch_cluster_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.plan.logC, g.plan.perWarp,
+                                             src, (uint32_t)T, g.plan.smem, g.codeMode, side_),
+                           "batch cluster");
+                ++launches_;
+            }
             for (auto const& w : slab_) {
                 for (SlabRef const& r : w.refs)
                     if (r.rank == 0) members_[r.sys]->applyStall(side_);
@@ -507,7 +587,7 @@ void Batch::run(int32_t const* mcs)
             cuda_check(cudaEventRecord(join_, stream2_), "event");
             cuda_check(cudaStreamWaitEvent(stream_, join_, 0), "wait");
         }
-        if (!slab_.empty()) cuda_check(cudaStreamWaitEvent(stream_, sideJoin_, 0), "wait");
+        if (sides) cuda_check(cudaStreamWaitEvent(stream_, sideJoin_, 0), "wait");
     }
     cuda_check(cudaEventRecord(done_, stream_), "event");
     for (uint32_t m = 0; m < M; ++m) {
@@ -557,6 +637,7 @@ std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
         anyCluster[0] = anyCluster[0] || cl;
         anyCluster[1] = anyCluster[1] || (cl && !u->residentEligible());
     }
+    if (residentOn_ && clusterOn_) anyCluster[1] = anyCluster[1] || !cluster_.empty();
     // Three stages, each configuration timed over the same kind of MCS: first the paths (resident
     // kernel on / off x cluster kernel on / off, where either can matter) with the grid kernels'
     // defaults; then, for the best paths under which some member runs on the grid-phase kernels (with the

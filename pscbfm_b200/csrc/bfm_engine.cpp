@@ -1230,19 +1230,28 @@ void Updater::planCluster()
     // 8.2; in 128^3, 11K (network) 6.8 and 10.7, 26K 10.5 and 8.5, 45K 15.6 and 8.5).
     cluster_ = ClusterPlan{};
     clusterAuto_ = false;
-    if (codeMode_ == kCodeNone) return;
     uint32_t const chunks = (maxGroup_ + 31u) / 32u;
     for (uint32_t logC = 4; logC >= 1; --logC) {
-        uint32_t const C = 1u << logC, perCta = (chunks + C - 1u) / C, perWarp = (perCta + 31u) / 32u;
-        if (dev_.h.nwords < C || perCta > 256u) continue;
-        uint32_t per = 1;
-        while (per < perWarp) per *= 2;
-        size_t const smem = cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, per, maxc_, codeMode_);
-        if (smem > kResidentMaxSmem || !cluster_bc_runnable(logC, per, smem, codeMode_)) continue;
-        cluster_ = ClusterPlan{logC, per, smem};
+        if (clusterPlan(logC, cluster_) == 0) continue;
+        uint32_t const C = 1u << logC, perCta = (chunks + C - 1u) / C;
         clusterAuto_ = perCta * 128u + dev_.h.nwords / C <= 4352u;
         return;
     }
+    cluster_ = ClusterPlan{};
+}
+
+uint32_t Updater::clusterPlan(uint32_t logC, ClusterPlan& plan) const
+{
+    if (codeMode_ == kCodeNone) return 0;
+    uint32_t const C = 1u << logC, chunks = (maxGroup_ + 31u) / 32u;
+    uint32_t const perCta = (chunks + C - 1u) / C, perWarp = (perCta + 31u) / 32u;
+    if (dev_.h.nwords < C || perCta > 256u) return 0;
+    uint32_t per = 1;
+    while (per < perWarp) per *= 2;
+    size_t const smem = cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, per, maxc_, codeMode_);
+    if (smem > kResidentMaxSmem) return 0;
+    plan = ClusterPlan{logC, per, smem};
+    return cluster_bc_runnable(logC, per, smem, codeMode_);
 }
 
 void Updater::enqueueCluster(uint32_t nSteps)

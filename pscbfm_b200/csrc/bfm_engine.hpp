@@ -59,6 +59,12 @@ enum Mode : int {
     kModeCluster = 5,      // bond codes: one cluster of CTAs holds the system in shared memory
 };
 
+// log2 CTAs per cluster (0: none), chunks of 32 slots per warp and colour, dynamic shared memory per CTA.
+struct ClusterPlan {
+    uint32_t logC = 0, perWarp = 0;
+    size_t smem = 0;
+};
+
 // Words of mapped host memory for DoneSignal, shared out over the process's updaters.
 struct DoneFlags {
     static unsigned int* take();
@@ -136,6 +142,14 @@ public:
     bool residentEligible() const;
     bool clusterEligible() const { return cluster_.logC != 0; }
     // whether ctas CTAs hold the system in the slab sweep (bond codes), and how
+    // the cluster-resident kernel's plan on 2^logC CTAs: how many such clusters the device runs at a
+    // time (0: the system does not fit, or the device runs none); its shared memory per CTA with more
+    // chunks per warp than its own
+    uint32_t clusterPlan(uint32_t logC, ClusterPlan& plan) const;
+    size_t clusterSmem(uint32_t logC, uint32_t perWarp) const
+    {
+        return cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, perWarp, maxc_, codeMode_);
+    }
     bool slabPlan(uint32_t ctas, SlabPlan& plan) const
     {
         return slab_plan(grpSize_.data(), (uint32_t)grpSize_.size(), maxc_, dev_.h.nwords, codeMode_, ctas, plan);
@@ -282,12 +296,7 @@ private:
     bool gsPending_ = false;                   // a persistent launch may have reported to hGs_
     bool stallNext_ = false;                   // injectBarrierStall
     uint32_t smCount_ = 148;                   // SMs of the device (setGpu)
-    // the cluster-resident kernel's plan: log2 CTAs per cluster (0: does not fit), chunks of 32 slots
-    // per warp and colour, dynamic shared memory per CTA (planCluster)
-    struct ClusterPlan {
-        uint32_t logC = 0, perWarp = 0;
-        size_t smem = 0;
-    } cluster_;
+    ClusterPlan cluster_;                      // the cluster-resident kernel's plan (planCluster)
     bool clusterAuto_ = false;                 // AUTO takes the cluster-resident kernel
     SlabPlan slab_;                            // the persistent sweep's plan (ctas == 0: does not fit)
     uint32_t hStepCap_ = 0;
@@ -425,6 +434,14 @@ private:
         size_t smem = 0;
         SlabRef* dRefs = nullptr;
     };
+    // members in the cluster-resident kernel, one launch per run and group
+    struct ClusterGroup {
+        uint32_t codeMode;
+        ClusterPlan plan;
+        std::vector<uint32_t> members;
+        uint32_t* dList = nullptr;
+    };
+    std::vector<ClusterGroup> planClusters(std::vector<char>& taken) const;
     static constexpr uint32_t kSlabGrowSlots = 512;   // slots per CTA and colour, at least, where more CTAs join
     bool slabFits(Updater const& u) const;
     std::vector<SlabWave> planSlabs(std::vector<char>& taken, bool& residentsAfter) const;
@@ -440,15 +457,16 @@ private:
     void prepare(int32_t const* mcs);            // both, for a run of mcs[i] MCS per member
     int gpu_;
     std::vector<Updater*> members_;
-    std::vector<char> wholeRun_;               // member runs in a resident kernel or a slab sweep
+    std::vector<char> wholeRun_;               // member runs in one kernel for the whole run
     std::vector<GridGroup> grid_;
     std::vector<ResidentGroup> resident_;
     std::vector<SlabWave> slab_;
+    std::vector<ClusterGroup> cluster_;
     std::shared_ptr<GridFault> reports_;       // mapped host memory, one per member
     GridFault* dReports_ = nullptr;
     uint32_t reportCap_ = 0;
     bool residentsAfter_ = false;              // the resident kernels run after the slab sweeps
-    cudaStream_t side_ = nullptr;              // the slab sweeps' stream
+    cudaStream_t side_ = nullptr;              // the slab sweeps' or the clusters' stream
     cudaEvent_t sideJoin_ = nullptr;
     uint32_t smCount_ = 148, slabSms_ = 148;
     bool residentOn_ = true;

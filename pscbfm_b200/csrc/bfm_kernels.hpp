@@ -137,11 +137,11 @@ cudaError_t launch_slab_batch(SysDev const* dSys, SlabRef const* dRefs, uint32_t
 size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t maxc, uint32_t codeMode);
 // Cluster-resident sweep (bond codes): one cluster of 2^logC CTAs of kResidentBlock threads per
 // system of dList[0..nClusters) (logC 1..4), state in the cluster's shared memory for nSteps
-// sub-steps; perThread (1, 2, 4, 8) chunks of 32 slots per warp and colour. cluster_bc_runnable: whether
-// the device can run that configuration.
+// sub-steps; perThread (1, 2, 4, 8) chunks of 32 slots per warp and colour. cluster_bc_runnable: how many
+// such clusters the device runs at a time.
 size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t perThread, uint32_t maxc,
                              uint32_t codeMode);
-bool cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode);
+uint32_t cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode);
 cudaError_t launch_cluster_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
                               uint32_t perThread, StepSource const& src, uint32_t nSteps, size_t smem,
                               uint32_t codeMode, cudaStream_t s);

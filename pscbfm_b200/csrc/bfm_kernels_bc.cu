@@ -1918,16 +1918,16 @@ cudaLaunchConfig_t cluster_bc_config(uint32_t logC, size_t smem, cudaLaunchAttri
     return cfg;
 }
 
-// Whether the device runs clusters of 2^logC CTAs with all the shared memory a CTA may take: asked once
-// per device, thread, kernel and size (the question takes the driver most of a millisecond).
+// How many clusters of 2^logC CTAs the device runs at a time, with all the shared memory a CTA may take:
+// asked once per device, thread, kernel and size (the question takes the driver most of a millisecond).
 template <typename W, int K>
-bool cluster_bc_check(uint32_t logC)
+uint32_t cluster_bc_check(uint32_t logC)
 {
-    static thread_local signed char known[64][5] = {};
+    static thread_local short known[64][5] = {};
     static thread_local bool done[64] = {};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    signed char& k = known[dev & 63][logC];
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    short& k = known[dev & 63][logC];
     if (k == 0) {
         auto kernel = k_cluster_bc<W, K>;
         cudaLaunchAttribute attr[1];
@@ -1938,9 +1938,9 @@ bool cluster_bc_check(uint32_t logC)
             e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
         if (e != cudaSuccess) cudaGetLastError();   // a configuration the device refuses is an answer, not an error
-        k = e == cudaSuccess && clusters >= 1 ? 1 : -1;
+        k = e == cudaSuccess && clusters >= 1 ? (short)clusters : -1;
     }
-    return k > 0;
+    return k > 0 ? (uint32_t)k : 0u;
 }
 
 template <typename W, int K>
@@ -1948,7 +1948,7 @@ cudaError_t launch_cluster_bc_k(SysDev const* dSys, uint32_t const* dList, uint3
                                 StepSource const& src, uint32_t nSteps, size_t smem,
                                 cudaStream_t s)
 {
-    if (!cluster_bc_check<W, K>(logC)) return cudaErrorInvalidConfiguration;
+    if (cluster_bc_check<W, K>(logC) == 0) return cudaErrorInvalidConfiguration;
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t const cfg = cluster_bc_config(logC, smem, attr, nClusters, s);
     return cudaLaunchKernelEx(&cfg, k_cluster_bc<W, K>, dSys, dList, src, nSteps);
@@ -1969,25 +1969,25 @@ cudaError_t launch_cluster_bc_w(SysDev const* dSys, uint32_t const* dList, uint3
 }
 
 template <typename W>
-bool cluster_bc_runnable_w(uint32_t logC, uint32_t perThread)
+uint32_t cluster_bc_runnable_w(uint32_t logC, uint32_t perThread)
 {
     switch (perThread) {
     case 1: return cluster_bc_check<W, 1>(logC);
     case 2: return cluster_bc_check<W, 2>(logC);
     case 4: return cluster_bc_check<W, 4>(logC);
     case 8: return cluster_bc_check<W, 8>(logC);
-    default: return false;
+    default: return 0;
     }
 }
 
 }  // namespace
 
-bool cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode)
+uint32_t cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode)
 {
-    if (logC < 1 || logC > 4 || smem > kResidentMaxSmem) return false;
+    if (logC < 1 || logC > 4 || smem > kResidentMaxSmem) return 0;
     if (codeMode == kCode32) return cluster_bc_runnable_w<uint32_t>(logC, perThread);
     if (codeMode == kCode64) return cluster_bc_runnable_w<unsigned long long>(logC, perThread);
-    return false;
+    return 0;
 }
 
 cudaError_t launch_cluster_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,

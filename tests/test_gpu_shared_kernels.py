@@ -131,6 +131,34 @@ def test_batch_members_with_callbacks_beside_streams(cluster):
     b.close()
 
 
+@pytest.mark.parametrize("count", [1, 7, 8, 16, 40])
+def test_batch_members_on_clusters_vs_oracle(count):
+    """Members that fit one CTA on the SMs a batch leaves over: clusters of 16, 8 and 4 CTAs and none at
+    all, members of different sizes, 64-bit codes, a callback's member and idle ones in one launch."""
+    big = [S.serpentine_chains(64, 32, 0.25, seed=60), S.serpentine_chains(64, 31, 0.22, seed=61),
+           S.square_network(64), S.walled(S.serpentine_chains((64, 64, 50), 37, 0.2, seed=62), 4)]
+    systems = [big[k % 4] if k < 16 else S.serpentine_chains(32, 16, 0.3, seed=63) for k in range(count)]
+    members = [P.UpdaterGPUScBFM_AB_Type(0).load_system(s) for s in systems]
+    mcs = [9 - k % 5 for k in range(count)]
+    k = iter(range(10**6))
+    members[0].set_draw_callback(lambda: P.updater.counter_draw(systems[0].seed, next(k)))
+    b = P.Batch(members)
+    b.run_each(mcs)
+    b.set_cluster(False)
+    b.run_each(mcs)
+    b.set_cluster(True)
+    b.run_each(mcs)
+    want = {}
+    for s, m, t in zip(systems, members, mcs):
+        if (id(s), t) not in want:
+            want[id(s), t] = O.run(s, 3 * t)
+        assert np.array_equal(m.get_coords(), want[id(s), t][0])
+        st = m.stats()
+        assert (st["attempted"], st["tentative"], st["accepted"]) == want[id(s), t][1]
+        m.validate()
+    b.close()
+
+
 def test_idle_members_beside_longer_ones():
     """A batch whose members stop at different sub-steps: the shared-memory kernels skip the idle entries
     that follow a member's last sub-step, inside and across blocks of step entries."""
