@@ -1223,18 +1223,18 @@ void Updater::planCluster()
 {
     // Alone: the largest cluster the device can run (remote accesses, the barriers and each warp's chain
     // of dependent reads bound the kernel, so more CTAs with fewer slots are faster: 64^3 chains, N = 8192,
-    // us per MCS on 2, 4, 8, 16 CTAs: 11.4, 9.1, 6.6, 5.7; the 11K network on 8 and 16: 8.8, 6.8). AUTO
-    // takes it (clusterAuto_) while a CTA's chunks of 32 slots per colour and its share of the lattice
-    // stay small; beyond, the persistent sweep, which reads the lattice from the L2, is at least as fast
-    // (us per MCS, cluster against persistent: N = 8K in 64^3 5.7 and 8.3, 16K 7.0 and 8.2, 26K 8.5 and
-    // 8.2; in 128^3, 11K (network) 6.8 and 10.7, 26K 10.5 and 8.5, 45K 15.6 and 8.5).
+    // us per MCS on 2, 4, 8, 16 CTAs: 11.4, 9.1, 6.6, 5.7; the 11K network on 8 and 16: 8.8, 6.8).
+    // Its time per MCS grows with clusterCost_: a CTA's chunks of 32 slots per colour and its share of the
+    // lattice (each remote word and code costs), while the persistent sweep, which reads the lattice from
+    // the L2 and spreads the slots over all SMs, takes 7.7 us per MCS at every size here (11.4 with 64-bit
+    // codes). See autoMode.
     cluster_ = ClusterPlan{};
-    clusterAuto_ = false;
+    clusterCost_ = ~0u;
     uint32_t const chunks = (maxGroup_ + 31u) / 32u;
     for (uint32_t logC = 4; logC >= 1; --logC) {
         if (clusterPlan(logC, cluster_) == 0) continue;
         uint32_t const C = 1u << logC, perCta = (chunks + C - 1u) / C;
-        clusterAuto_ = perCta * 128u + dev_.h.nwords / C <= 4352u;
+        clusterCost_ = perCta * 128u + dev_.h.nwords / C * 3u / 8u;
         return;
     }
     cluster_ = ClusterPlan{};
@@ -1278,12 +1278,19 @@ int Updater::autoMode(int32_t nMcs) const
 {
     // One system on a B200, us per MCS: the resident kernel (one SM) while the largest colour group is
     // at most 1024 monomers (1.2K-monomer chains 3.5 against 4.6 on a cluster of 16 CTAs, 2K 4.3 against
-    // 4.6, 3.3K 5.3-5.6 against 4.8, 8K 10.6 against 5.7); then a cluster of CTAs holding the system in distributed shared
-    // memory (planCluster); then the persistent sweep (60K monomers 8.6 against 15.2 for the graph of
-    // launches, 131K 9.6 against 13.4, 1M 14.9 against 21.7), from three tiles per SM on only for runs of
-    // at least kSlabMcs MCS; else the graph.
+    // 4.6, 3.3K 5.3-5.6 against 4.8, 8K 10.6 against 5.7).
+    // Then a cluster of CTAs holding the system in distributed shared memory, up to the clusterCost_ where
+    // the persistent sweep draws level (cluster against persistent: 8K chains in 64^3, cost 1120, 5.8 and
+    // 7.7; 16K 2144 7.3-7.9 and 7.7; 20K 2656 8.1-8.6 and 7.7; 13K in 128^3 2432 7.3 and 7.8; 18K 3072 8.7
+    // and 7.8; 30K in 32 x 128 x 128 4032 11.9 and 7.7). A run of one MCS, mostly launch, keeps the cluster
+    // a little longer (26K 28.3 and 27.0 us in all, 30K 30.9 and 27.1); with 64-bit codes the persistent
+    // sweep is slower (11K network 7.0 and 11.4).
+    // Then the persistent sweep (60K monomers 7.9 against 15.2 for the graph of launches, 131K 9.0 against
+    // 13.4, 1M 14.5 against 21.7), from three tiles per SM on only for runs of at least kSlabMcs MCS; else
+    // the graph.
     if (residentEligible() && maxGroup_ <= kResidentBlock) return kModeResident;
-    if (clusterAuto_) return kModeCluster;
+    uint32_t const upTo = codeMode_ == kCode64 || slab_.ctas == 0 ? 4352u : nMcs == 1 ? 3450u : 2500u;
+    if (clusterCost_ <= upTo) return kModeCluster;
     if (slab_.ctas != 0) {
         uint32_t const tiles = (maxGroup_ + kBcTileSpan - 1) / kBcTileSpan;
         if (tiles <= 3u * smCount_ || nMcs >= kSlabMcs) return kModePersistent;

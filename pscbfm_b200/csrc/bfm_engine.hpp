@@ -297,7 +297,7 @@ private:
     bool stallNext_ = false;                   // injectBarrierStall
     uint32_t smCount_ = 148;                   // SMs of the device (setGpu)
     ClusterPlan cluster_;                      // the cluster-resident kernel's plan (planCluster)
-    bool clusterAuto_ = false;                 // AUTO takes the cluster-resident kernel
+    uint32_t clusterCost_ = ~0u;               // what decides between cluster_ and the persistent sweep (planCluster)
     SlabPlan slab_;                            // the persistent sweep's plan (ctas == 0: does not fit)
     uint32_t hStepCap_ = 0;
     struct GraphExec {

@@ -77,3 +77,21 @@ def test_auto_takes_one_launch_for_long_runs_of_the_melt():
     assert counts[1] <= 2 and counts[3] <= 2   # the sweep, and the scrub of the graph's last marks
     assert np.array_equal(u.get_coords(), O.run(s, 19)[0])
     u.close()
+
+
+@pytest.mark.parametrize("make", [lambda: S.serpentine_chains(64, 8, 0.5, seed=3), lambda: S.serpentine_chains(64, 64, 0.6, seed=3),
+                                  lambda: S.serpentine_chains((32, 128, 128), 8, 0.3, seed=3),
+                                  lambda: S.walled(S.serpentine_chains((64, 64, 50), 37, 0.7, seed=3), 4)])
+def test_auto_between_cluster_and_persistent(make):
+    """AUTO's choice between the cluster and the persistent sweep depends on the run's length: runs of one
+    MCS and longer ones in turn, on both sides of the line, give the oracle's positions and counters."""
+    s = make()
+    u = P.UpdaterGPUScBFM_AB_Type(0).load_system(s)
+    for n in (1, 3, 1, 2):
+        u.runSimulationOnGPU(n)
+    want, ost = O.run(s, 7)
+    st = u.stats()
+    assert np.array_equal(u.get_coords(), want)
+    assert (st["attempted"], st["tentative"], st["accepted"]) == ost
+    u.validate()
+    u.close()
