@@ -1277,7 +1277,7 @@ int Updater::path() const
 int Updater::autoMode(int32_t nMcs) const
 {
     // One system on a B200, us per MCS: the resident kernel (one SM) while the largest colour group is
-    // at most 1024 monomers (1.2K-monomer chains 3.5 against 4.6 on a cluster of 16 CTAs, 2K 4.3 against
+    // at most 1024 monomers (1.2K-monomer chains 3.3 against 4.6 on a cluster of 16 CTAs, 2K 4.3 against
     // 4.6, 3.3K 5.3-5.6 against 4.8, 8K 10.6 against 5.7).
     // Then a cluster of CTAs holding the system in distributed shared memory, up to the clusterCost_ where
     // the persistent sweep draws level (cluster against persistent: 8K chains in 64^3, cost 1120, 5.8 and

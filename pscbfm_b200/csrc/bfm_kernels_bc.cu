@@ -1110,16 +1110,21 @@ __host__ __device__ __forceinline__ size_t resident_layout(uint32_t nwords, uint
 // lattice per sub-step parity (the previous one cleared while the next check runs), lattice
 // addresses, bond codes, neighbour references (where they fit: 2 bytes each) and lists; one CTA per
 // system of sysList.
-// The bond test and the front plane are evaluated side by side, without branches, so that their
-// chains of dependent reads overlap; the directions of sub-step t + 1 are drawn during the perform
-// of t, whose movers take the threads from the last one down, where a small system has no slots.
+// The bond test and the front plane's masks are read side by side, so that their chains of dependent
+// reads overlap, the lattice only for slots that pass the test: two thirds of a melt's do not, and their
+// reads cost more in bank conflicts than the wait for the test. The directions of sub-step t + 1 are
+// drawn during the perform of t, whose movers take the threads from the last one down, where a small
+// system has no slots.
 // Two forms of the check:
 //   kDirect: each slot's bonds and plane by its own thread, two CTA barriers per sub-step (groups of at
 //   most 1024 slots, and those too large for 16-bit list entries);
 //   else the slots that pass the wall and bond tests (a third of a melt's) are listed first, so the
 //   planes run on full warps: three barriers, and less work from 2 slots per thread on.
 // Bound by shared-memory wavefronts (bank conflicts), the integer pipe and the chain of dependent reads
-// of each phase. us per MCS: 1.2K-monomer chains 3.9 -> 3.5, 2K 5.0 -> 4.3, 3.3K 6.3 -> 5.3, 8K 13.0 -> 10.6.
+// of each phase (1.2K monomers: about 1700 cycles of a sub-step in the check, 1300 in the perform). us per
+// MCS, with every slot's plane read and so: 1.2K-monomer chains 3.4 and 3.3, 1.6K 3.9 and 3.6, 2K 4.3 and
+// 4.1; 3.3K 5.3, 8K 10.6. Slower: each thread performing its own mover, all but the temporary lattice
+// read before the barrier and no list (3 %, issue); the movers spread over more warps (20 %).
 template <typename W, bool kDirect>
 __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const* __restrict__ sysv,
                                                                     uint32_t const* __restrict__ sysList,
@@ -1195,7 +1200,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const*
         return d;
     };
     // the check of slot l: the move's target, and whether the front plane is free and, if asked, the
-    // wall and bond tests pass, in one straight line of code
+    // wall and bond tests pass; only slots that pass them read the lattice
     auto check = [&](uint32_t l, uint32_t dir, bool tests, uint32_t& to) {
         uint32_t const p = pk[l];
         DirParams const D = dir_params(dtab, dir);
@@ -1203,7 +1208,8 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const*
         HalfPlane pl;
         half_plane(pl, masks, D, p, D.front, dir);
         to = addr_add(p, D.ma, D.step);
-        return ok & (half_hits(pl, lat) == 0u);
+        if (!ok) return false;
+        return half_hits(pl, lat) == 0u;
     };
     uint32_t par = 0, dirs = 0;
     bool drawn = false;   // dirs belong to the next active sub-step
