@@ -1389,28 +1389,28 @@ __host__ __device__ __forceinline__ size_t cluster_layout(uint32_t nwords, uint3
 // neighbours' codes held by another CTA are reached through distributed shared memory, the
 // neighbours' at addresses mapped once. Two cluster barriers per sub-step (after the check, after the
 // perform); the temporary lattice has one copy per sub-step parity. Between the two halves of the
-// first barrier a CTA clears its words of the previous copy and draws the directions of the next
-// sub-step, which nobody waits for. Every CTA of a cluster runs the same system and so reaches the
+// first barrier a CTA clears its words of the previous copy, draws the directions of the next sub-step and
+// makes the step entries a block ahead (made at the start of their block, with a barrier and the first
+// directions after them, they took 4 % of the run), which nobody waits for. Every CTA of a cluster runs the same system and so reaches the
 // same barriers. A CTA leaves only after the last barrier, when no other CTA accesses its shared
 // memory any more. Grid: one cluster per system of sysList. K: chunks of 32 slots per warp and colour, at most.
 // Bound by remote accesses (0.33 remote atomics per clock and SM), two barriers of 0.3 us and the
 // chain of dependent reads of each phase; a lattice word is read only where the bond test passed and the
-// plane touches it. us per MCS, 16 CTAs: 8K chains 5.7 (8.6 on the four CTAs of one chunk per warp),
-// the 11K network 6.8 (8.3 on eight), 16K chains 7.0 (8.4).
+// plane touches it. us per MCS, 16 CTAs: 8K chains 5.5, the 11K network 6.8, 16K chains 7.2.
 template <typename W, int K>
 __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* __restrict__ sysv,
                                                                    uint32_t const* __restrict__ sysList,
                                                                    StepSource const src, uint32_t nSteps)
 {
     namespace cg = cooperative_groups;
-    constexpr uint32_t kSlots = CodeWord<W>::kSlots, B = kResidentBlock;
+    constexpr uint32_t kSlots = CodeWord<W>::kSlots, B = kResidentBlock, kFetchWarp = 15;
     static_assert(K <= 10, "a thread's directions share one word, three bits each");
     cg::cluster_group cluster = cg::this_cluster();
     uint32_t const C = cluster.num_blocks(), rank = cluster.block_rank();
     uint32_t logC = 0;
     while ((1u << logC) < C) ++logC;   // a power of two (launch_cluster_bc)
     __shared__ SysDev S;
-    __shared__ __align__(16) StepEntry stepSm[kStepBlock];
+    __shared__ __align__(16) StepEntry stepSm[2][kStepBlock];   // the block of entries in use, and the next
     __shared__ StepStream own;
     __shared__ uint32_t nMov[2];   // per sub-step parity
     extern __shared__ unsigned long long smem[];
@@ -1488,16 +1488,26 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
     uint32_t nTent = 0, nAcc = 0, par = 0, dirs = 0;
     bool drawn = false;   // dirs belong to the next active sub-step
     unsigned long long nAtt = 0;
+    auto fetch_steps = [&](uint32_t block) {   // one warp
+        uint32_t const k = tid - kFetchWarp * 32u, t = block * kStepBlock + k;
+        if (k < kStepBlock && t < nSteps) stepSm[block & 1u][k] = step_entry(src, own, sysId, t, S.grp, S.nColors);
+    };
+    fetch_steps(0);
+    fetch_steps(1);
+    __syncthreads();
     for (uint32_t t = 0; t < nSteps; ++t) {
-        if (t % kStepBlock == 0) {   // (the last barrier of the sub-step before ended the reads of the old ones)
-            uint32_t const n = min(kStepBlock, nSteps - t);
-            if (tid < n) stepSm[tid] = step_entry(src, own, sysId, t + tid, S.grp, S.nColors);
-            __syncthreads();
-            drawn = false;
+        StepEntry const st = stepSm[t / kStepBlock & 1u][t % kStepBlock];
+        StepEntry const& next = stepSm[(t + 1u) / kStepBlock & 1u][(t + 1u) % kStepBlock];
+        // the block before the one in use has been read by all: the next one takes its place
+        bool const refill = t != 0 && t % kStepBlock == 0;
+        if (st.color == kNoColor) {
+            if (refill) {   // (the same on every thread)
+                __syncthreads();
+                fetch_steps(t / kStepBlock + 1u);
+                __syncthreads();
+            }
+            continue;
         }
-        uint32_t const ts = t % kStepBlock;
-        StepEntry const st = stepSm[ts];
-        if (st.color == kNoColor) continue;
         if (!drawn) dirs = directions(st);
         if (rank == 0) nAtt += st.cnt;
         uint32_t const marks = tmpAddr + par * 8u * nwC;
@@ -1527,8 +1537,9 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
         for (uint32_t w = B - 1u - tid; w < nwC; w += B)
             reinterpret_cast<unsigned long long*>(tmp + (par ^ 1u) * 2u * nwC)[w] = 0ull;
         if (tid == 0) nMov[par ^ 1u] = 0u;
-        drawn = t + 1 < nSteps && ts + 1u < kStepBlock && stepSm[ts + 1u].color != kNoColor;
-        if (drawn) dirs = directions(stepSm[ts + 1u]);
+        drawn = t + 1 < nSteps && next.color != kNoColor;
+        if (drawn) dirs = directions(next);
+        if (refill) fetch_steps(t / kStepBlock + 1u);
         cluster_wait();   // every CTA's marks are in place
         // perform over this CTA's movers, from the last thread down
         uint32_t const n = nMov[par];

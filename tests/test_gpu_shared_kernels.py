@@ -159,6 +159,22 @@ def test_batch_members_on_clusters_vs_oracle(count):
     b.close()
 
 
+def test_idle_cluster_members_across_blocks_of_entries():
+    """Members on clusters that idle for several blocks of step entries while another runs, one that is
+    idle from the start, and runs that end on the first and the last entry of a block."""
+    systems = [S.serpentine_chains(64, 32, 0.25, seed=64), S.serpentine_chains(64, 31, 0.22, seed=65),
+               S.square_network(64)]
+    members = [P.UpdaterGPUScBFM_AB_Type(0).load_system(s) for s in systems]
+    b = P.Batch(members)
+    plan = [[40, 1, 13], [4, 25, 0], [8, 8, 8], [0, 12, 31]]
+    for mcs in plan:
+        b.run_each(mcs)
+    for s, m, t in zip(systems, members, np.sum(plan, axis=0)):
+        assert np.array_equal(m.get_coords(), O.run(s, int(t))[0]), s.name
+        m.validate()
+    b.close()
+
+
 def test_idle_members_beside_longer_ones():
     """A batch whose members stop at different sub-steps: the shared-memory kernels skip the idle entries
     that follow a member's last sub-step, inside and across blocks of step entries."""
