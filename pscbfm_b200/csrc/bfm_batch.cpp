@@ -363,7 +363,7 @@ std::vector<Batch::ClusterGroup> Batch::planClusters(std::vector<char>& taken) c
         if (g == groups.end()) g = groups.insert(g, ClusterGroup{u.codeMode(), plan, {}, nullptr});
         // one launch has one number of chunks per warp and one size of shared memory (descending groups: the
         // first member's chunks do for all)
-        size_t const smem = u.clusterSmem(bestLog, g->plan.perWarp);
+        size_t const smem = u.clusterSmem(bestLog, g->plan.chunks);
         if (smem > kResidentMaxSmem) continue;
         g->plan.smem = std::max(g->plan.smem, smem);
         g->members.push_back(m);
@@ -537,7 +537,7 @@ void Batch::run(int32_t const* mcs)
         if (sides) {
             cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
             for (auto const& g : cluster_) {
-                cuda_check(launch_cluster_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.plan.logC, g.plan.perWarp,
+                cuda_check(launch_cluster_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.plan.logC, g.plan.chunks,
                                              src, (uint32_t)T, g.plan.smem, g.codeMode, side_),
                            "batch cluster");
                 ++launches_;

@@ -1223,7 +1223,7 @@ void Updater::planCluster()
 {
     // Alone: the largest cluster the device can run (remote accesses, the barriers and each warp's chain
     // of dependent reads bound the kernel, so more CTAs with fewer slots are faster: 64^3 chains, N = 8192,
-    // us per MCS on 2, 4, 8, 16 CTAs: 11.4, 9.1, 6.6, 5.7; the 11K network on 8 and 16: 8.8, 6.8).
+    // us per MCS on 2, 4, 8, 16 CTAs of 1024 threads: 11.4, 9.1, 6.6, 5.7; the 11K network on 8 and 16: 8.8, 6.8).
     // Its time per MCS grows with clusterCost_: a CTA's chunks of 32 slots per colour and its share of the
     // lattice (each remote word and code costs), while the persistent sweep, which reads the lattice from
     // the L2 and spreads the slots over all SMs, takes 7.7 us per MCS at every size here (11.4 with 64-bit
@@ -1243,15 +1243,14 @@ void Updater::planCluster()
 uint32_t Updater::clusterPlan(uint32_t logC, ClusterPlan& plan) const
 {
     if (codeMode_ == kCodeNone) return 0;
-    uint32_t const C = 1u << logC, chunks = (maxGroup_ + 31u) / 32u;
-    uint32_t const perCta = (chunks + C - 1u) / C, perWarp = (perCta + 31u) / 32u;
+    uint32_t const C = 1u << logC, perCta = ((maxGroup_ + 31u) / 32u + C - 1u) / C;
     if (dev_.h.nwords < C || perCta > 256u) return 0;
-    uint32_t per = 1;
-    while (per < perWarp) per *= 2;
-    size_t const smem = cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, per, maxc_, codeMode_);
+    uint32_t chunks = 16;   // the kernel's forms: 16, 32, 64, 128 and 256 chunks per CTA and colour
+    while (chunks < perCta) chunks *= 2;
+    size_t const smem = cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, chunks, maxc_, codeMode_);
     if (smem > kResidentMaxSmem) return 0;
-    plan = ClusterPlan{logC, per, smem};
-    return cluster_bc_runnable(logC, per, smem, codeMode_);
+    plan = ClusterPlan{logC, chunks, smem};
+    return cluster_bc_runnable(logC, chunks, smem, codeMode_);
 }
 
 void Updater::enqueueCluster(uint32_t nSteps)
@@ -1259,7 +1258,7 @@ void Updater::enqueueCluster(uint32_t nSteps)
     scrubPending(stream_);
     for (uint32_t done = 0; done < nSteps;) {
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
-        cuda_check(launch_cluster_bc(dev_.dDesc, dev_.dList, 1, cluster_.logC, cluster_.perWarp, stepSource(chunk), chunk,
+        cuda_check(launch_cluster_bc(dev_.dDesc, dev_.dList, 1, cluster_.logC, cluster_.chunks, stepSource(chunk), chunk,
                                      cluster_.smem, codeMode_, stream_),
                    "cluster");
         ++launches_;
@@ -1277,14 +1276,14 @@ int Updater::path() const
 int Updater::autoMode(int32_t nMcs) const
 {
     // One system on a B200, us per MCS: the resident kernel (one SM) while the largest colour group is
-    // at most 1024 monomers (1.2K-monomer chains 3.3 against 4.6 on a cluster of 16 CTAs, 2K 4.3 against
-    // 4.6, 3.3K 5.3-5.6 against 4.8, 8K 10.6 against 5.7).
+    // at most 1024 monomers (1.2K-monomer chains 3.3 against 3.9 on a cluster of 16 CTAs, 2K 4.1 against
+    // 4.0-4.1, 3.3K 5.6 against 4.2, 8K 10.6 against 5.0).
     // Then a cluster of CTAs holding the system in distributed shared memory, up to the clusterCost_ where
-    // the persistent sweep draws level (cluster against persistent: 8K chains in 64^3, cost 1120, 5.8 and
-    // 7.7; 16K 2144 7.3-7.9 and 7.7; 20K 2656 8.1-8.6 and 7.7; 13K in 128^3 2432 7.3 and 7.8; 18K 3072 8.7
-    // and 7.8; 30K in 32 x 128 x 128 4032 11.9 and 7.7). A run of one MCS, mostly launch, keeps the cluster
+    // the persistent sweep draws level (cluster against persistent: 8K chains in 64^3, cost 1120, 5.0 and
+    // 7.7; 16K 2144 6.7 and 7.6; 20K 2656 8.5 and 7.6; 13K in 128^3 2432 6.4 and 7.7; 18K 3072 8.3 and 7.7;
+    // 30K in 32 x 128 x 128 4032 11.9 and 7.7). A run of one MCS, mostly launch, keeps the cluster
     // a little longer (26K 28.3 and 27.0 us in all, 30K 30.9 and 27.1); with 64-bit codes the persistent
-    // sweep is slower (11K network 7.0 and 11.4).
+    // sweep is slower (11K network 6.2 and 11.4).
     // Then the persistent sweep (60K monomers 7.9 against 15.2 for the graph of launches, 131K 9.0 against
     // 13.4, 1M 14.5 against 21.7), from three tiles per SM on only for runs of at least kSlabMcs MCS; else
     // the graph.

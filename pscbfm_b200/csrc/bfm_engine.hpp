@@ -59,9 +59,9 @@ enum Mode : int {
     kModeCluster = 5,      // bond codes: one cluster of CTAs holds the system in shared memory
 };
 
-// log2 CTAs per cluster (0: none), chunks of 32 slots per warp and colour, dynamic shared memory per CTA.
+// log2 CTAs per cluster (0: none), chunks of 32 slots per CTA and colour at most, dynamic shared memory per CTA.
 struct ClusterPlan {
-    uint32_t logC = 0, perWarp = 0;
+    uint32_t logC = 0, chunks = 0;
     size_t smem = 0;
 };
 
@@ -144,11 +144,11 @@ public:
     // whether ctas CTAs hold the system in the slab sweep (bond codes), and how
     // the cluster-resident kernel's plan on 2^logC CTAs: how many such clusters the device runs at a
     // time (0: the system does not fit, or the device runs none); its shared memory per CTA with more
-    // chunks per warp than its own
+    // chunks than its own
     uint32_t clusterPlan(uint32_t logC, ClusterPlan& plan) const;
-    size_t clusterSmem(uint32_t logC, uint32_t perWarp) const
+    size_t clusterSmem(uint32_t logC, uint32_t chunks) const
     {
-        return cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, perWarp, maxc_, codeMode_);
+        return cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, chunks, maxc_, codeMode_);
     }
     bool slabPlan(uint32_t ctas, SlabPlan& plan) const
     {

@@ -13,6 +13,7 @@ namespace bfm {
 
 constexpr uint32_t kGridBlock = 256;          // threads per CTA of the grid-phase kernels
 constexpr uint32_t kResidentBlock = 1024;     // threads per CTA of the resident kernel
+constexpr uint32_t kClusterSmallBlock = 512;  // threads per CTA of the cluster kernel with few slots per CTA
 // dynamic shared memory of the resident kernel: the 227 KB opt-in limit minus room for its
 // static shared memory (the copied system descriptor)
 constexpr size_t kResidentMaxSmem = 226 * 1024;
@@ -135,15 +136,15 @@ cudaError_t launch_slab_batch(SysDev const* dSys, SlabRef const* dRefs, uint32_t
                               cudaStream_t s);
 // Dynamic shared memory of the bond-code resident kernel, with the neighbour references where they fit too.
 size_t resident_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t maxGroup, uint32_t maxc, uint32_t codeMode);
-// Cluster-resident sweep (bond codes): one cluster of 2^logC CTAs of kResidentBlock threads per
+// Cluster-resident sweep (bond codes): one cluster of 2^logC CTAs per
 // system of dList[0..nClusters) (logC 1..4), state in the cluster's shared memory for nSteps
-// sub-steps; perThread (1, 2, 4, 8) chunks of 32 slots per warp and colour. cluster_bc_runnable: how many
-// such clusters the device runs at a time.
-size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t perThread, uint32_t maxc,
+// sub-steps; at most `chunks` (16, 32: CTAs of kClusterSmallBlock threads; 64, 128, 256: of kResidentBlock)
+// chunks of 32 slots per CTA and colour. cluster_bc_runnable: how many such clusters the device runs at a time.
+size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t chunks, uint32_t maxc,
                              uint32_t codeMode);
-uint32_t cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode);
+uint32_t cluster_bc_runnable(uint32_t logC, uint32_t chunks, size_t smem, uint32_t codeMode);
 cudaError_t launch_cluster_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
-                              uint32_t perThread, StepSource const& src, uint32_t nSteps, size_t smem,
+                              uint32_t chunks, StepSource const& src, uint32_t nSteps, size_t smem,
                               uint32_t codeMode, cudaStream_t s);
 cudaError_t launch_resident_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nCta, uint32_t perThread,
                                StepSource const& src, uint32_t nSteps, size_t smem, uint32_t codeMode, cudaStream_t s);

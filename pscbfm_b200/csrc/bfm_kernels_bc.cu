@@ -1382,7 +1382,7 @@ __host__ __device__ __forceinline__ size_t cluster_layout(uint32_t nwords, uint3
            (size_t)groupSlots * 4 + cap * nb * 4;
 }
 
-// One thread-block cluster of 2^logC CTAs (1024 threads each) owns a system whose lattice,
+// One thread-block cluster of 2^logC CTAs (kBlock threads each) owns a system whose lattice,
 // temporary lattices, addresses and codes fit their shared memory together, for a whole run of
 // sub-steps (half bricks dealt out as cluster_word_rank says, slots as cluster_slot_rank). Each CTA
 // checks the slots it holds, lists its own tentative movers and performs them; words and
@@ -1394,16 +1394,19 @@ __host__ __device__ __forceinline__ size_t cluster_layout(uint32_t nwords, uint3
 // directions after them, they took 4 % of the run), which nobody waits for. Every CTA of a cluster runs the same system and so reaches the
 // same barriers. A CTA leaves only after the last barrier, when no other CTA accesses its shared
 // memory any more. Grid: one cluster per system of sysList. K: chunks of 32 slots per warp and colour, at most.
+// CTAs of at most 32 chunks per colour have 512 threads: half of the warps of 1024 had nothing to do but
+// arrive at the barriers (8K chains, 8 chunks per CTA, 5.5 -> 5.0 us per MCS on 512 threads, 5.1 on 256; 16K,
+// 16 chunks, 7.2 -> 6.7, 7.2 on 256; 26K, 26 chunks, 9.8 -> 9.2 with two chunks per warp).
 // Bound by remote accesses (0.33 remote atomics per clock and SM), two barriers of 0.3 us and the
 // chain of dependent reads of each phase; a lattice word is read only where the bond test passed and the
-// plane touches it. us per MCS, 16 CTAs: 8K chains 5.5, the 11K network 6.8, 16K chains 7.2.
-template <typename W, int K>
-__global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* __restrict__ sysv,
-                                                                   uint32_t const* __restrict__ sysList,
-                                                                   StepSource const src, uint32_t nSteps)
+// plane touches it. us per MCS, 16 CTAs: 4K chains 4.3, 8K 5.0, 16K 6.7, the 11K network 6.2.
+template <typename W, int K, int kBlock>
+__global__ void __launch_bounds__(kBlock, 1) k_cluster_bc(SysDev const* __restrict__ sysv,
+                                                          uint32_t const* __restrict__ sysList,
+                                                          StepSource const src, uint32_t nSteps)
 {
     namespace cg = cooperative_groups;
-    constexpr uint32_t kSlots = CodeWord<W>::kSlots, B = kResidentBlock, kFetchWarp = 15;
+    constexpr uint32_t kSlots = CodeWord<W>::kSlots, B = kBlock, kFetchWarp = B / 64 - 1;
     static_assert(K <= 10, "a thread's directions share one word, three bits each");
     cg::cluster_group cluster = cg::this_cluster();
     uint32_t const C = cluster.num_blocks(), rank = cluster.block_rank();
@@ -1427,7 +1430,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
     W* const code = reinterpret_cast<W*>(tmp + 4u * nwC);                    // cap slots
     uint32_t* const pk = reinterpret_cast<uint32_t*>(code + cap);            // cap slots
     uint8_t* const mok = reinterpret_cast<uint8_t*>(pk + cap);               // 512 move-table bytes
-    uint32_t* const list = reinterpret_cast<uint32_t*>(mok + 512);           // K x 1024 movers: local slot | dir << 28
+    uint32_t* const list = reinterpret_cast<uint32_t*>(mok + 512);           // K x B movers: local slot | dir << 28
     uint32_t* const refs = list + K * B;                                     // maxc x cap references, where they fit
     uint32_t dynBytes;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynBytes));
@@ -1468,7 +1471,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
         return (v0 & r.m.x) | (v1 & r.m.y) | (v2 & r.m.z) | (v3 & r.m.w);
     };
     // this warp's chunks of a colour group (which starts at a chunk): the k-th starts at slot
-    // chunk(e) * 32 + k * 1024 C
+    // chunk(e) * 32 + k * B C
     auto chunk = [&](StepEntry const& e) {
         uint32_t const c0 = e.off >> 5;
         return c0 + ((rank - c0) & (C - 1u)) + warp * C;
@@ -1515,7 +1518,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_cluster_bc(SysDev const* 
         uint32_t const end = st.off + st.cnt, c0 = chunk(st);
 #pragma unroll
         for (uint32_t k = 0; k < (uint32_t)K; ++k) {
-            uint32_t const g = (c0 + k * 32u * C) * 32u + lane;
+            uint32_t const g = (c0 + k * (B / 32u) * C) * 32u + lane;
             if (g - lane >= end) break;   // the same for the whole warp
             uint32_t const l = cluster_slot_local(g, logC), dir = (dirs >> (3u * k)) & 7u, p = pk[l];
             DirParams const D = dir_params(dtab, dir);
@@ -1907,19 +1910,19 @@ cudaError_t launch_resident_bc(SysDev const* dSys, uint32_t const* dList, uint32
     return cudaErrorInvalidValue;
 }
 
-size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t perThread, uint32_t maxc,
+size_t cluster_bc_smem_bytes(uint32_t nwords, uint32_t npad, uint32_t logC, uint32_t chunks, uint32_t maxc,
                              uint32_t codeMode)
 {
     uint32_t const w = codeMode == kCode64 ? 8 : 4;
-    size_t const all = cluster_layout(nwords, npad, logC, perThread * kResidentBlock, w, maxc);
-    return all <= kResidentMaxSmem ? all : cluster_layout(nwords, npad, logC, perThread * kResidentBlock, w, 0);
+    size_t const all = cluster_layout(nwords, npad, logC, chunks * 32u, w, maxc);
+    return all <= kResidentMaxSmem ? all : cluster_layout(nwords, npad, logC, chunks * 32u, w, 0);
 }
 
 namespace {
 
-// The launch of nClusters clusters of 2^logC CTAs.
-cudaLaunchConfig_t cluster_bc_config(uint32_t logC, size_t smem, cudaLaunchAttribute* attr, uint32_t nClusters,
-                                     cudaStream_t s)
+// The launch of nClusters clusters of 2^logC CTAs of `block` threads.
+cudaLaunchConfig_t cluster_bc_config(uint32_t logC, uint32_t block, size_t smem, cudaLaunchAttribute* attr,
+                                     uint32_t nClusters, cudaStream_t s)
 {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1u << logC;
@@ -1927,7 +1930,7 @@ cudaLaunchConfig_t cluster_bc_config(uint32_t logC, size_t smem, cudaLaunchAttri
     attr[0].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nClusters << logC);
-    cfg.blockDim = dim3(kResidentBlock);
+    cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attr;
@@ -1937,7 +1940,7 @@ cudaLaunchConfig_t cluster_bc_config(uint32_t logC, size_t smem, cudaLaunchAttri
 
 // How many clusters of 2^logC CTAs the device runs at a time, with all the shared memory a CTA may take:
 // asked once per device, thread, kernel and size (the question takes the driver most of a millisecond).
-template <typename W, int K>
+template <typename W, int K, int B>
 uint32_t cluster_bc_check(uint32_t logC)
 {
     static thread_local short known[64][5] = {};
@@ -1946,9 +1949,9 @@ uint32_t cluster_bc_check(uint32_t logC)
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     short& k = known[dev & 63][logC];
     if (k == 0) {
-        auto kernel = k_cluster_bc<W, K>;
+        auto kernel = k_cluster_bc<W, K, B>;
         cudaLaunchAttribute attr[1];
-        cudaLaunchConfig_t const cfg = cluster_bc_config(logC, kResidentMaxSmem, attr, 1, nullptr);
+        cudaLaunchConfig_t const cfg = cluster_bc_config(logC, B, kResidentMaxSmem, attr, 1, nullptr);
         int clusters = 0;
         cudaError_t e = allow_smem(kernel, done);
         if (e == cudaSuccess && logC > 3)
@@ -1960,63 +1963,65 @@ uint32_t cluster_bc_check(uint32_t logC)
     return k > 0 ? (uint32_t)k : 0u;
 }
 
-template <typename W, int K>
+template <typename W, int K, int B>
 cudaError_t launch_cluster_bc_k(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
                                 StepSource const& src, uint32_t nSteps, size_t smem,
                                 cudaStream_t s)
 {
-    if (cluster_bc_check<W, K>(logC) == 0) return cudaErrorInvalidConfiguration;
+    if (cluster_bc_check<W, K, B>(logC) == 0) return cudaErrorInvalidConfiguration;
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t const cfg = cluster_bc_config(logC, smem, attr, nClusters, s);
-    return cudaLaunchKernelEx(&cfg, k_cluster_bc<W, K>, dSys, dList, src, nSteps);
+    cudaLaunchConfig_t const cfg = cluster_bc_config(logC, B, smem, attr, nClusters, s);
+    return cudaLaunchKernelEx(&cfg, k_cluster_bc<W, K, B>, dSys, dList, src, nSteps);
 }
 
 template <typename W>
 cudaError_t launch_cluster_bc_w(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
-                                uint32_t perThread, StepSource const& src, uint32_t nSteps,
+                                uint32_t chunks, StepSource const& src, uint32_t nSteps,
                                 size_t smem, cudaStream_t s)
 {
-    switch (perThread) {
-    case 1: return launch_cluster_bc_k<W, 1>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
-    case 2: return launch_cluster_bc_k<W, 2>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
-    case 4: return launch_cluster_bc_k<W, 4>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
-    case 8: return launch_cluster_bc_k<W, 8>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
+    switch (chunks) {
+    case 16: return launch_cluster_bc_k<W, 1, kClusterSmallBlock>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
+    case 32: return launch_cluster_bc_k<W, 2, kClusterSmallBlock>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
+    case 64: return launch_cluster_bc_k<W, 2, kResidentBlock>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
+    case 128: return launch_cluster_bc_k<W, 4, kResidentBlock>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
+    case 256: return launch_cluster_bc_k<W, 8, kResidentBlock>(dSys, dList, nClusters, logC, src, nSteps, smem, s);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename W>
-uint32_t cluster_bc_runnable_w(uint32_t logC, uint32_t perThread)
+uint32_t cluster_bc_runnable_w(uint32_t logC, uint32_t chunks)
 {
-    switch (perThread) {
-    case 1: return cluster_bc_check<W, 1>(logC);
-    case 2: return cluster_bc_check<W, 2>(logC);
-    case 4: return cluster_bc_check<W, 4>(logC);
-    case 8: return cluster_bc_check<W, 8>(logC);
+    switch (chunks) {
+    case 16: return cluster_bc_check<W, 1, kClusterSmallBlock>(logC);
+    case 32: return cluster_bc_check<W, 2, kClusterSmallBlock>(logC);
+    case 64: return cluster_bc_check<W, 2, kResidentBlock>(logC);
+    case 128: return cluster_bc_check<W, 4, kResidentBlock>(logC);
+    case 256: return cluster_bc_check<W, 8, kResidentBlock>(logC);
     default: return 0;
     }
 }
 
 }  // namespace
 
-uint32_t cluster_bc_runnable(uint32_t logC, uint32_t perThread, size_t smem, uint32_t codeMode)
+uint32_t cluster_bc_runnable(uint32_t logC, uint32_t chunks, size_t smem, uint32_t codeMode)
 {
     if (logC < 1 || logC > 4 || smem > kResidentMaxSmem) return 0;
-    if (codeMode == kCode32) return cluster_bc_runnable_w<uint32_t>(logC, perThread);
-    if (codeMode == kCode64) return cluster_bc_runnable_w<unsigned long long>(logC, perThread);
+    if (codeMode == kCode32) return cluster_bc_runnable_w<uint32_t>(logC, chunks);
+    if (codeMode == kCode64) return cluster_bc_runnable_w<unsigned long long>(logC, chunks);
     return 0;
 }
 
 cudaError_t launch_cluster_bc(SysDev const* dSys, uint32_t const* dList, uint32_t nClusters, uint32_t logC,
-                              uint32_t perThread, StepSource const& src, uint32_t nSteps,
+                              uint32_t chunks, StepSource const& src, uint32_t nSteps,
                               size_t smem, uint32_t codeMode, cudaStream_t s)
 {
     if (nClusters == 0 || nSteps == 0) return cudaSuccess;
     if (logC < 1 || logC > 4 || smem > kResidentMaxSmem) return cudaErrorInvalidValue;
     if (codeMode == kCode32)
-        return launch_cluster_bc_w<uint32_t>(dSys, dList, nClusters, logC, perThread, src, nSteps, smem, s);
+        return launch_cluster_bc_w<uint32_t>(dSys, dList, nClusters, logC, chunks, src, nSteps, smem, s);
     if (codeMode == kCode64)
-        return launch_cluster_bc_w<unsigned long long>(dSys, dList, nClusters, logC, perThread, src, nSteps,
+        return launch_cluster_bc_w<unsigned long long>(dSys, dList, nClusters, logC, chunks, src, nSteps,
                                                        smem, s);
     return cudaErrorInvalidValue;
 }

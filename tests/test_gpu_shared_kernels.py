@@ -58,6 +58,23 @@ def test_shared_memory_kernels_vs_oracle(name, mode):
     u.close()
 
 
+@pytest.mark.parametrize("n, side", [(8192, 64), (8193, 64), (16384, 64), (16385, 64), (32768, 128), (32769, 128)])
+def test_cluster_forms_vs_oracle(n, side):
+    """16, 17, 32, 33, 64 and 65 chunks of 32 slots per CTA of a cluster of 16: both sides of the edges
+    between the cluster kernel's forms."""
+    s = _free(n, side)
+    u = P.UpdaterGPUScBFM_AB_Type(0).load_system(s, mode=P.MODE_CLUSTER)
+    assert u.path() == P.MODE_CLUSTER
+    for mcs in (1, 9):
+        u.runSimulationOnGPU(mcs)
+    want, ost = O.run(s, 10)
+    st = u.stats()
+    assert np.array_equal(u.get_coords(), want)
+    assert (st["attempted"], st["tentative"], st["accepted"]) == ost
+    u.validate()
+    u.close()
+
+
 @pytest.mark.parametrize("mode", ["resident", "cluster", "persistent"])
 def test_entries_made_on_the_device_vs_the_callbacks(mode):
     """Kernels that run many sub-steps make the counter stream's entries themselves; a callback's come
