@@ -469,12 +469,23 @@ size_t Batch::streamUnits() const
     return (sizeof(StepStream) * members_.size() + sizeof(StepEntry) - 1) / sizeof(StepEntry);
 }
 
+uint32_t Batch::longest(int32_t const* mcs) const
+{
+    uint64_t T = 0;
+    for (size_t m = 0; m < members_.size(); ++m) {
+        if (mcs[m] < 0) throw std::invalid_argument("[Batch::run] negative MCS count");
+        T = std::max(T, (uint64_t)mcs[m] * members_[m]->nColors());
+    }
+    // the kernels count the sub-steps of a run in 32 bits, as Updater::run does
+    if (T > 0xFFFFFFFFull) throw std::invalid_argument("[Batch::run] too many sub-steps in one call");
+    return (uint32_t)T;
+}
+
 void Batch::prepare(int32_t const* mcs)
 {
     // one-time host work of a run (staging growth, graph capture), done ahead of a timed run
     uint32_t const M = (uint32_t)members_.size();
-    uint64_t T = 0;
-    for (uint32_t m = 0; m < M; ++m) T = std::max(T, (uint64_t)std::max(mcs[m], 0) * members_[m]->nColors());
+    uint32_t const T = longest(mcs);
     if (T == 0) return;
     reserveSteps(streamUnits() + (hostEntries() ? (size_t)T * M : 0));
     if (!grid_.empty() && T >= stepCap_) ensureGraph();
@@ -490,8 +501,7 @@ void Batch::run(int32_t nMcs)
 void Batch::run(int32_t const* mcs)
 {
     uint32_t const M = (uint32_t)members_.size();
-    for (uint32_t m = 0; m < M; ++m)
-        if (mcs[m] < 0) throw std::invalid_argument("[Batch::run] negative MCS count");
+    uint32_t const T = longest(mcs);
     cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
     if (!built_) rebuild();
     // pending grid-path marks of members that run in a resident or cluster kernel are cleared on
@@ -505,12 +515,8 @@ void Batch::run(int32_t const* mcs)
         cuda_check(cudaStreamWaitEvent(stream_, ready_, 0), "wait");
     }
 
-    std::vector<uint64_t> need(M);
-    uint64_t T = 0;
-    for (uint32_t m = 0; m < M; ++m) {
-        need[m] = (uint64_t)mcs[m] * members_[m]->nColors();
-        T = std::max(T, need[m]);
-    }
+    std::vector<uint32_t> need(M);
+    for (uint32_t m = 0; m < M; ++m) need[m] = (uint32_t)mcs[m] * members_[m]->nColors();   // at most T
     if (T > 0) {
         // the members' streams, and the entries of those whose kernels don't make them
         size_t const units = streamUnits(), entries = units + (hostEntries() ? (size_t)T * M : 0);
@@ -520,10 +526,10 @@ void Batch::run(int32_t const* mcs)
         std::vector<uint32_t> drawn;
         for (uint32_t m = 0; m < M; ++m) {
             streams[m] = StepStream{};
-            if (!ownEntries(m) || !members_[m]->streamSteps((uint32_t)need[m], streams[m])) drawn.push_back(m);
+            if (!ownEntries(m) || !members_[m]->streamSteps(need[m], streams[m])) drawn.push_back(m);
         }
         // sub-step by sub-step: members may share a callback's generator
-        for (uint64_t t = 0; t < T && !drawn.empty(); ++t)
+        for (uint32_t t = 0; t < T && !drawn.empty(); ++t)
             for (uint32_t m : drawn)
                 host[(size_t)t * M + m] = t < need[m] ? members_[m]->nextStep()
                                                       : StepEntry{kNoColor, 0u, 0u, kNoColor, 0u, 0u, 0u, 0u};
@@ -538,14 +544,14 @@ void Batch::run(int32_t const* mcs)
             cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
             for (auto const& g : cluster_) {
                 cuda_check(launch_cluster_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.plan.logC, g.plan.chunks,
-                                             src, (uint32_t)T, g.plan.smem, g.codeMode, side_),
+                                             src, T, g.plan.smem, g.codeMode, side_),
                            "batch cluster");
                 ++launches_;
             }
             for (auto const& w : slab_) {
                 for (SlabRef const& r : w.refs)
                     if (r.rank == 0) members_[r.sys]->applyStall(side_);
-                cuda_check(launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, src, (uint32_t)T,
+                cuda_check(launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, src, T,
                                              dReports_, w.codeMode, side_),
                            "batch slab");
                 ++launches_;
@@ -559,9 +565,9 @@ void Batch::run(int32_t const* mcs)
             for (auto const& g : resident_) {
                 cuda_check(g.codeMode == kCodeNone
                                ? launch_resident(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, dEntries,
-                                                 M, (uint32_t)T, g.smem, stream2_)
+                                                 M, T, g.smem, stream2_)
                                : launch_resident_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, src,
-                                                    (uint32_t)T, g.smem, g.codeMode, stream2_),
+                                                    T, g.smem, g.codeMode, stream2_),
                            "batch resident");
                 ++launches_;
             }

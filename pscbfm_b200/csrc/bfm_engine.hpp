@@ -454,6 +454,7 @@ private:
     bool hostEntries() const;                    // some member's does not
     size_t streamUnits() const;                  // the members' streams, in entries
     void ensureGraph();                          // capture the graph of stepCap_ sub-steps
+    uint32_t longest(int32_t const* mcs) const;  // the most sub-steps of a member; throws beyond 32 bits
     void prepare(int32_t const* mcs);            // both, for a run of mcs[i] MCS per member
     int gpu_;
     std::vector<Updater*> members_;
