@@ -1,11 +1,11 @@
 // Batch: many independent systems advanced together on one GPU.
 //
 // Systems whose lattices (and, in the bond-code representation, packed coordinates and bond
-// codes) fit one CTA's shared memory run in the resident kernel, one CTA per system, one launch
-// per run; where such systems leave SMs idle, the largest of them run on clusters of CTAs (planClusters).
+// codes) fit one CTA's shared memory run in the resident kernel, one CTA per system; where such systems
+// leave SMs idle, the largest of them run on clusters of CTAs (planClusters).
 // Larger systems of the bond-code representation run in the slab sweep, each on CTAs of its
-// own, several systems in one cooperative launch per run (planSlabs). What fits neither shares
-// the grid-phase kernels: one check and one perform launch per
+// own, several systems in one cooperative launch (planSlabs). A launch of these kernels runs up to
+// kLaunchSteps sub-steps. What fits neither shares the grid-phase kernels: one check and one perform launch per
 // sub-step and representation cover the active colour group of every such system at once, and
 // chunks of those launches are captured into a CUDA graph once and replayed. Each system draws its
 // own sub-steps from its own stream exactly as it would alone, so its trajectory is unchanged by
@@ -539,38 +539,46 @@ void Batch::run(int32_t const* mcs)
         cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
         bool const sides = !slab_.empty() || !cluster_.empty();
         if (!resident_.empty() || sides) cuda_check(cudaEventRecord(fork_, stream_), "event");
-        StepSource const src{dEntries, reinterpret_cast<StepStream const*>(dStepsAll_), StepStream{}, M};
-        if (sides) {
-            cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
-            for (auto const& g : cluster_) {
-                cuda_check(launch_cluster_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.plan.logC, g.plan.chunks,
-                                             src, T, g.plan.smem, g.codeMode, side_),
-                           "batch cluster");
+        // a whole-run kernel's launches on one stream: launch(source, sub-steps), kLaunchSteps at a time
+        auto wholeRun = [&](char const* what, auto const& launch) {
+            for (uint32_t t0 = 0, n = 0; t0 < T; t0 += n) {
+                n = std::min(T - t0, kLaunchSteps);
+                cuda_check(launch(StepSource{dEntries + (size_t)t0 * M, reinterpret_cast<StepStream const*>(dStepsAll_),
+                                             StepStream{}, M, t0},
+                                  n),
+                           what);
                 ++launches_;
             }
+        };
+        if (sides) {
+            cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
+            for (auto const& g : cluster_)
+                wholeRun("batch cluster", [&](StepSource const& src, uint32_t n) {
+                    return launch_cluster_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.plan.logC, g.plan.chunks,
+                                             src, n, g.plan.smem, g.codeMode, side_);
+                });
             for (auto const& w : slab_) {
                 for (SlabRef const& r : w.refs)
                     if (r.rank == 0) members_[r.sys]->applyStall(side_);
-                cuda_check(launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, src, T,
-                                             dReports_, w.codeMode, side_),
-                           "batch slab");
-                ++launches_;
+                wholeRun("batch slab", [&](StepSource const& src, uint32_t n) {
+                    return launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, src, n, dReports_,
+                                             w.codeMode, side_);
+                });
             }
             cuda_check(cudaEventRecord(sideJoin_, side_), "event");
         }
         if (!resident_.empty()) {
-            // one launch per group for the whole run, on the second stream
+            // on the second stream
             cuda_check(cudaStreamWaitEvent(stream2_, fork_, 0), "wait");
             if (!slab_.empty() && residentsAfter_) cuda_check(cudaStreamWaitEvent(stream2_, sideJoin_, 0), "wait");
-            for (auto const& g : resident_) {
-                cuda_check(g.codeMode == kCodeNone
-                               ? launch_resident(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, dEntries,
-                                                 M, T, g.smem, stream2_)
-                               : launch_resident_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, src,
-                                                    T, g.smem, g.codeMode, stream2_),
-                           "batch resident");
-                ++launches_;
-            }
+            for (auto const& g : resident_)
+                wholeRun("batch resident", [&](StepSource const& src, uint32_t n) {
+                    return g.codeMode == kCodeNone
+                               ? launch_resident(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, src.steps, M,
+                                                 n, g.smem, stream2_)
+                               : launch_resident_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.perThread, src, n,
+                                                    g.smem, g.codeMode, stream2_);
+                });
         }
         if (!grid_.empty()) {
             for (uint64_t t0 = 0; t0 < T; t0 += stepCap_) {

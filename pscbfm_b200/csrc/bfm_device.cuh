@@ -205,12 +205,22 @@ struct StepStream {
 // Made on the device, a run needs no copy of 32 bytes per sub-step and system ahead of the sweep and no
 // host loop: 10 MCS of the 1M-monomer melt with the positions read back 483 -> 465 us, one MCS of a
 // 64^3 chain system 60.5 -> 59, 100 MCS of 128 systems of 1.6K monomers 803 -> 534.
+// first: sub-steps of streams[] that earlier launches of the run have done (steps starts behind them).
 struct StepSource {
     StepEntry const* steps;
     StepStream const* streams;
     StepStream own;
-    uint32_t stride;
+    uint32_t stride, first;
 };
+// The stream of system sys, from the launch's first sub-step on.
+__device__ __forceinline__ StepStream step_stream(StepSource const& src, uint32_t sys)
+{
+    if (src.streams == nullptr) return src.own;
+    StepStream s = src.streams[sys];
+    s.t0 += src.first;
+    s.n -= min(s.n, src.first);
+    return s;
+}
 __device__ __forceinline__ StepEntry step_entry(StepSource const& src, StepStream const& own, uint32_t sys, uint32_t t,
                                                 uint32_t const* grp, uint32_t nColors)
 {

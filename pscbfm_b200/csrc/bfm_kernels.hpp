@@ -30,6 +30,11 @@ cudaError_t allow_smem(F* kernel, bool (&done)[64])
     done[dev & 63] = e == cudaSuccess;
     return e;
 }
+// Sub-steps of one launch of the kernels that run many (resident, cluster, slab), at most; a longer run is
+// several launches. A CTA holds at most kCtaSlots slots of a colour and counts its moves in 32 bits, and no
+// CTA keeps its SM from other work for more than a second or so (65536 sub-steps of 8K slots in one CTA 0.35 s).
+constexpr uint32_t kLaunchSteps = 1u << 16, kCtaSlots = 16 * kResidentBlock;
+static_assert((unsigned long long)kLaunchSteps * kCtaSlots < (1ull << 32), "a launch's move counts fit 32 bits");
 constexpr int32_t kPadCoord = INT32_MIN;      // x of an unused (padding) slot
 
 // One CTA of a grid-phase launch: system index and first in-colour index it covers.

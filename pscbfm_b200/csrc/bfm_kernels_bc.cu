@@ -1023,7 +1023,7 @@ __global__ void __launch_bounds__(B, 1)
     __shared__ StepStream own;
     __shared__ uint32_t caps[3];
     SlabRef const r = refs[blockIdx.x];
-    if (threadIdx.x == 0) own = src.streams != nullptr ? src.streams[r.sys] : src.own;
+    if (threadIdx.x == 0) own = step_stream(src, r.sys);
     copy_desc(S, sysv + r.sys);
     __syncthreads();
     if (threadIdx.x == 0)
@@ -1138,7 +1138,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const*
     __shared__ uint32_t nMov[2], nCand, maxGroup;   // nMov: per sub-step parity
     extern __shared__ unsigned long long smem[];
     uint32_t const sysId = sysList[blockIdx.x];
-    if (threadIdx.x == 0) own = src.streams != nullptr ? src.streams[sysId] : src.own;
+    if (threadIdx.x == 0) own = step_stream(src, sysId);
     copy_desc(S, sysv + sysId);
     __syncthreads();
     uint32_t const nw = S.nwords, np = S.npad, maxc = S.maxc;
@@ -1418,7 +1418,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_cluster_bc(SysDev const* __restri
     __shared__ uint32_t nMov[2];   // per sub-step parity
     extern __shared__ unsigned long long smem[];
     uint32_t const sysId = sysList[blockIdx.x >> logC];
-    if (threadIdx.x == 0) own = src.streams != nullptr ? src.streams[sysId] : src.own;
+    if (threadIdx.x == 0) own = step_stream(src, sysId);
     copy_desc(S, sysv + sysId);
     __syncthreads();
     uint32_t const np = S.npad, nwC = S.nwords >> logC, cap = cluster_slots_per_cta(np, logC), maxc = S.maxc;
@@ -1847,7 +1847,7 @@ cudaError_t launch_slab_bc(SysDev const& hostDesc, StepSource const& src, uint32
                            GridFault* report, uint32_t codeMode, cudaStream_t s)
 {
     if (nSteps == 0) return cudaSuccess;
-    if (plan.ctas == 0 || codeMode == kCodeNone) return cudaErrorInvalidValue;
+    if (plan.ctas == 0 || codeMode == kCodeNone || nSteps > kLaunchSteps) return cudaErrorInvalidValue;
     return slab_dispatch(codeMode, plan, SlabLaunch{hostDesc, src, nSteps, plan, report, s});
 }
 
@@ -1856,6 +1856,7 @@ cudaError_t launch_slab_batch(SysDev const* dSys, SlabRef const* dRefs, uint32_t
                               cudaStream_t s)
 {
     if (ctas == 0 || nSteps == 0) return cudaSuccess;
+    if (nSteps > kLaunchSteps) return cudaErrorInvalidValue;
     if (codeMode == kCode32)
         return launch_slab_batch_w<uint32_t, (int)kSlabBlock32>(dSys, dRefs, ctas, smem, src, nSteps, report, s);
     if (codeMode == kCode64)
@@ -1902,7 +1903,7 @@ cudaError_t launch_resident_bc(SysDev const* dSys, uint32_t const* dList, uint32
                                cudaStream_t s)
 {
     if (nCta == 0 || nSteps == 0) return cudaSuccess;
-    if (smem > kResidentMaxSmem) return cudaErrorInvalidValue;
+    if (smem > kResidentMaxSmem || nSteps > kLaunchSteps) return cudaErrorInvalidValue;
     if (codeMode == kCode32)
         return launch_resident_bc_w<uint32_t>(dSys, dList, nCta, perThread, src, nSteps, smem, s);
     if (codeMode == kCode64)
@@ -2017,7 +2018,7 @@ cudaError_t launch_cluster_bc(SysDev const* dSys, uint32_t const* dList, uint32_
                               size_t smem, uint32_t codeMode, cudaStream_t s)
 {
     if (nClusters == 0 || nSteps == 0) return cudaSuccess;
-    if (logC < 1 || logC > 4 || smem > kResidentMaxSmem) return cudaErrorInvalidValue;
+    if (logC < 1 || logC > 4 || smem > kResidentMaxSmem || nSteps > kLaunchSteps) return cudaErrorInvalidValue;
     if (codeMode == kCode32)
         return launch_cluster_bc_w<uint32_t>(dSys, dList, nClusters, logC, chunks, src, nSteps, smem, s);
     if (codeMode == kCode64)

@@ -37,3 +37,29 @@ def test_batch_refuses_runs_past_32_bits_of_sub_steps():
     for s, m in zip(systems, members):
         assert np.array_equal(m.get_coords(), O.run(s, 5)[0])
     b.close()
+
+
+@pytest.mark.parametrize("name", ["resident", "gather", "cluster", "slab"])
+def test_long_batch_runs_are_several_launches(name):
+    """The kernels that hold a system for many sub-steps count a CTA's moves in 32 bits: a launch has at most
+    65536 sub-steps (times 16384 slots of a colour: 2^30 moves), and a longer run is several launches of the
+    same trajectory and counters, for members that end within the first or the second of them."""
+    mcs = 32768 + 700   # of two colours: 65536 sub-steps and 1400
+    s = {"cluster": S.small_chains(), "slab": S.serpentine_chains(64, 64, 0.8, seed=13)}.get(
+        name, S.serpentine_chains(32, 16, 0.05, seed=40))
+    repr_ = P.REPR_GATHER if name == "gather" else P.REPR_AUTO
+    members = [load(s, seed=q, representation=repr_) for q in (5, 6, 7)]
+    b = P.Batch(members, cluster=name in ("cluster", "slab"))
+    b.run(1)
+    n0 = b.launch_count()
+    b.run_each([mcs, 900, mcs - 600])
+    assert b.launch_count() - n0 == 2
+    for q, m, k in zip((5, 6, 7), members, (mcs, 900, mcs - 600)):
+        u = load(s, seed=q, representation=repr_)
+        u.runSimulationOnGPU(1)
+        u.runSimulationOnGPU(k)
+        assert m.stats() == u.stats() and m.substep() == u.substep()
+        assert np.array_equal(m.get_coords(), u.get_coords())
+        m.validate()
+        u.close()
+    b.close()
