@@ -951,7 +951,9 @@ void Updater::noteExternalRun(uint64_t subSteps, uint64_t mcs, bool pendingMarks
                               std::shared_ptr<GridFault> report)
 {
     (void)subSteps;
-    if (report) batchReport_ = std::move(report);
+    // (a report that has not been looked at stays: an earlier run's failure is not lost to a later run)
+    if (report && std::find(batchReports_.begin(), batchReports_.end(), report) == batchReports_.end())
+        batchReports_.push_back(std::move(report));
     lastRunSnap_ = false;
     lastRunLead_ = false;   // the batch flushed this system's waiting tickets before it ran
     mcsDone_ += mcs;
@@ -1381,11 +1383,11 @@ void Updater::checkReports()
         std::atomic_thread_fence(std::memory_order_acquire);
         failed(hGs_);
     }
-    if (batchReport_) {
-        std::shared_ptr<GridFault> const r = std::move(batchReport_);
-        batchReport_ = nullptr;
+    if (!batchReports_.empty()) {
+        std::vector<std::shared_ptr<GridFault>> reports;
+        reports.swap(batchReports_);
         std::atomic_thread_fence(std::memory_order_acquire);
-        failed(r.get());
+        for (auto const& r : reports) failed(r.get());
     }
 }
 
@@ -1854,7 +1856,7 @@ void Updater::freeDevice()
         for (uint32_t k = 0; k < kStatRing; ++k) statTicket_[k] = 0;
     }
     pendingTickets_.clear();
-
+    batchReports_.clear();   // of a state that is gone
 }
 
 void Updater::cleanup()

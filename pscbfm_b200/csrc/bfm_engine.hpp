@@ -268,7 +268,7 @@ private:
     uint32_t genOn_ = 0;                       // the device producer's `on`, as last written
     GridFault* hGs_ = nullptr;                 // mapped report of the persistent kernel's barrier
     GridFault* dGs_ = nullptr;                 // the same, as the device addresses it
-    std::shared_ptr<GridFault> batchReport_;   // the report of a Batch run not yet synchronised
+    std::vector<std::shared_ptr<GridFault>> batchReports_;   // those of Batch runs not yet synchronised
     unsigned long long* hStats_ = nullptr;     // pinned copy of the move counters (stats)
     unsigned long long* hStatRing_ = nullptr;  // kStatRing mapped pinned slots (statsEnqueue)
     unsigned long long* dStatRing_ = nullptr;  // the same, as the device addresses them

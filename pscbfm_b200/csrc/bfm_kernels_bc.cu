@@ -642,12 +642,11 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& sr
     constexpr uint32_t kFarBit = 1u << 31;
     __shared__ SlabPart P;
     __shared__ __align__(16) StepEntry stepSm[2][kStepBlock];   // the block of entries in use, and the next
-    __shared__ uint32_t nCand, nMov, tallyA;
+    __shared__ uint32_t nCand, nMov, tallyA, failed;
     extern __shared__ unsigned long long smem[];
     uint32_t const tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     bool const waiter = warp == nWork;
     GridSync* const gs = S.gs;
-    if (ld_acquire_gpu(&gs->fault) != 0u) return;   // an earlier launch failed: the state is not usable
     uint32_t const nColors = S.nColors, np = S.npad;
     if (tid == 0) {
         uint32_t b = 0;
@@ -660,6 +659,7 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& sr
             b += 32u * (hi - lo);
         }
         nCand = nMov = tallyA = 0u;
+        failed = ld_acquire_gpu(&gs->fault);
     }
     unsigned long long* const ptab = smem;                                   // 768 plane masks
     uint32_t* const dtab = reinterpret_cast<uint32_t*>(smem + 768);          // kDirTab words
@@ -675,6 +675,10 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& sr
     if (tid < kDirTab) dtab[tid] = S.dirTab[tid];
     for (uint32_t w = tid; w < 512; w += B) mok[w] = S.moveOk[w];
     __syncthreads();
+    if (failed != 0u) {   // an earlier launch failed: the state is not usable, and this run's caller learns of it too
+        if (tid == 0) report->fault = 1u;   // (where: the barrier it failed at, where the report is the same)
+        return;
+    }
     using RV = typename SlotRec<W>::V;
     for (uint32_t c = 0; c < nColors; ++c)
         for (uint32_t d = tid; d < P.count[c]; d += B) {

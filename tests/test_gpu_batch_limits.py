@@ -63,3 +63,36 @@ def test_long_batch_runs_are_several_launches(name):
         m.validate()
         u.close()
     b.close()
+
+
+def test_failed_sweep_is_reported_by_every_later_sweep():
+    """A system whose sweep timed out (injected on the host) is not advanced again, and no later sweep of it
+    returns as if it were: in the batch after its plan was made anew, in another batch, alone; a run that was
+    never waited for is reported too. The other members go on, and a system set up again is a new one."""
+    s = S.serpentine_chains(128, 32, 0.1, seed=3)
+    a, c = load(s, seed=1), load(s, seed=2)
+    b = P.Batch([a, c])
+    a.inject_barrier_stall()
+    with pytest.raises(P.BfmCudaError, match="timed out"):
+        b.run(2)
+    for on in (False, True):   # (the plan is made again, with reports of its own)
+        b.set_cluster(on)
+    with pytest.raises(P.BfmCudaError, match="timed out"):
+        b.run(1)
+    other = P.Batch([a])
+    with pytest.raises(P.BfmCudaError, match="timed out"):
+        other.run(1)
+    other.run_async(1)         # two runs of two batches, neither waited for
+    b.run_async(1)
+    with pytest.raises(P.BfmCudaError, match="timed out"):
+        a.synchronize()
+    other.close()
+    a.set_mode(P.MODE_PERSISTENT)
+    with pytest.raises(P.BfmCudaError, match="timed out"):
+        a.runSimulationOnGPU(1)
+    b.close()
+    assert np.array_equal(c.get_coords(), O.run(s, 4, seed=2)[0])
+    a.cleanup()
+    load_again = a.load_system(s, seed=1, mode=P.MODE_PERSISTENT)
+    load_again.runSimulationOnGPU(3)
+    assert np.array_equal(a.get_coords(), O.run(s, 3, seed=1)[0])
