@@ -131,7 +131,7 @@ int bfm_set_perform(bfm_handle h, int warps, int group);
 int bfm_get_path(bfm_handle h, int* mode);
 /* Fault injection for tests (no counterpart in the reference): the next BFM_MODE_PERSISTENT launch
  * of this handle (or the next run of a batch that holds it on CTAs of its own) starts its grid-barrier arrival count where no barrier can complete, so every
- * CTA's wait runs out at its time limit (20 s) and the run reports the timeout
+ * CTA's wait runs out at its time limit (2 s) and the run reports the timeout
  * (BFM_ERR_CUDA).
  * Nothing faults on the GPU and the device stays usable; this system's state is not. */
 int bfm_inject_barrier_stall(bfm_handle h);

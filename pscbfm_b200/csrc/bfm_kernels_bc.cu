@@ -476,9 +476,12 @@ __global__ void __launch_bounds__(32 * PW) k_perform_bc(const __grid_constant__ 
 
 // ---------------------------------------------------------------------------------- persistent
 
-// A wait longer than this is a fault: a launch's first wait ends only once every CTA has found a free SM,
-// and another stream's kernel may hold some for a while.
-constexpr unsigned long long kBarrierTimeoutNs = 20000000000ull;
+// A wait longer than this is a fault. The CTAs of a cooperative launch start together, once all of them have
+// an SM (B200: behind a kernel that holds 100 SMs for 50 ms all 148 start within 10 us of its end, behind
+// another cooperative launch they never start between its CTAs), so other streams' kernels delay a launch
+// but none of its waits. kBarrierPolls bounds a wait without the timer (as many polls take longer).
+constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;
+constexpr unsigned int kBarrierPolls = 1u << 24;
 
 __device__ __forceinline__ unsigned int ld_acquire_gpu(unsigned int const* p)
 {
@@ -516,7 +519,7 @@ __device__ __forceinline__ bool grid_meet(GridSync* gs, unsigned int& target, un
             // a time limit, and a poll count as a second bound that does not trust the timer
             if ((++polls & 255u) == 0u) {
                 if (ld_acquire_gpu(&gs->fault) != 0u) return false;
-                if (global_ns() - t0 > kBarrierTimeoutNs || polls > (1u << 27)) {
+                if (global_ns() - t0 > kBarrierTimeoutNs || polls > kBarrierPolls) {
                     gs->fault = 1u;
                     return false;
                 }

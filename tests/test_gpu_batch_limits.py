@@ -96,3 +96,22 @@ def test_failed_sweep_is_reported_by_every_later_sweep():
     load_again = a.load_system(s, seed=1, mode=P.MODE_PERSISTENT)
     load_again.runSimulationOnGPU(3)
     assert np.array_equal(a.get_coords(), O.run(s, 3, seed=1)[0])
+
+
+def test_stalled_sweep_ends_at_its_limit_of_two_seconds():
+    """A wait that cannot end (injected on the host) ends after 2 s, alone and in a batch: the GPU is not held
+    longer. (The CTAs of a cooperative launch start together, so no wait depends on other streams' work.)"""
+    import time
+    s = S.serpentine_chains(128, 32, 0.1, seed=3)
+    u = load(s, mode=P.MODE_PERSISTENT)
+    u.runSimulationOnGPU(1)
+    m = load(s)
+    b = P.Batch([m])
+    b.run(1)
+    for stalled, run in ((u, lambda: u.runSimulationOnGPU(2)), (m, lambda: b.run(2))):
+        stalled.inject_barrier_stall()
+        t = time.perf_counter()
+        with pytest.raises(P.BfmCudaError, match="timed out"):
+            run()
+        assert 1.0 < time.perf_counter() - t < 8.0
+    b.close()
