@@ -123,8 +123,10 @@ void Batch::rebuild()
         resident_.push_back(ResidentGroup{mode, {}, nullptr, 1, 0});
         return resident_.back();
     };
-    std::vector<char> slabbed;
-    slab_ = planSlabs(slabbed, residentsAfter_);
+    SlabWaves plan = planSlabs();
+    slab_.swap(plan.waves);
+    residentsAfter_ = plan.residentsAfter;
+    std::vector<char> const slabbed = std::move(plan.taken);
     std::vector<char> clustered;
     cluster_ = planClusters(clustered);
     if (!(slab_.empty() && cluster_.empty()) && !side_) {
@@ -228,63 +230,67 @@ void Batch::rebuild()
     built_ = true;
 }
 
+namespace {
+// The fewest of at most `most` CTAs that hold the member in the slab sweep, and how; false: it does not fit.
+template <typename Plan>
+bool slab_least(Plan const& plan, uint32_t most, SlabPlan& out)
+{
+    for (uint32_t C = 1; C <= most; ++C)
+        if (plan(C, out) && out.cache) return true;
+    return false;
+}
+}  // namespace
+
 bool Batch::slabFits(Updater const& u) const
 {
     SlabPlan plan;
-    return u.slabPlan(smCount_ / 2u, plan) && plan.cache;
+    return slab_least([&](uint32_t C, SlabPlan& p) { return u.slabPlan(C, p); }, std::min(smCount_ / 2u, slabSms_), plan);
 }
 
-std::vector<Batch::SlabWave> Batch::planSlabs(std::vector<char>& taken, bool& residentsAfter) const
+SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, uint32_t share)
 {
     // The members in the slab sweep (taken) and their CTAs, in cooperative launches of at most `budget` CTAs
     // that run one after the other. Each CTA takes an SM, so the fewest CTAs that hold a member do the most
     // work per SM (moves per us and SM at 0.9K, 1.9K, 3.7K and 7.5K slots per CTA and colour: 208, 331, 419
     // and 458); members are packed that way, longest first. The SMs a wave leaves idle then go, one by one,
     // to its member with the most slots per CTA, which runs longest. A member the grid-phase kernels
-    // have to take anyway (it does not fit, or gathers) keeps half of the SMs.
-    uint32_t const M = (uint32_t)members_.size();
-    taken.assign(M, 0);
-    residentsAfter = false;
-    std::vector<SlabWave> waves;
-    if (!clusterOn_) return waves;
+    // have to take anyway (it does not fit the budget, or gathers) keeps half of the SMs.
+    SlabWaves out;
+    out.taken.assign(members.size(), 0);
     uint32_t residents = 0;
-    bool gridAnyway = false;
+    for (SlabMember const& m : members) residents += m.resident ? 1u : 0u;
+    // A cooperative launch waits until all its CTAs have found an SM, so it must never queue behind the
+    // batch's own resident kernels, which keep theirs for the whole run: a few residents get SMs of
+    // their own, many run after the slab sweeps.
+    bool const residentsAfter = residents > share / 4u;
     struct Item {
         uint32_t m;
         SlabPlan plan;
     };
     std::vector<Item> items;
-    for (uint32_t m = 0; m < M; ++m) {
-        Updater const& u = *members_[m];
-        if (residentOn_ && u.residentEligible()) {
-            ++residents;
-            continue;
+    bool gridAnyway = false;
+    uint32_t budget = 0;
+    for (;;) {   // a member that does not fit leaves the others half of the SMs, which one more may not fit
+        budget = std::max(1u, gridAnyway ? share / 2u : share - (residentsAfter ? 0u : residents));
+        bool const before = gridAnyway;
+        items.clear();
+        for (uint32_t m = 0; m < (uint32_t)members.size(); ++m) {
+            if (members[m].resident) continue;
+            Item it{m, {}};
+            if (slab_least(members[m].plan, std::min(budget, sms / 2u), it.plan)) items.push_back(it);
+            else gridAnyway = true;
         }
-        if (!slabFits(u)) {
-            gridAnyway = true;
-            continue;
-        }
-        Item it{m, {}};
-        for (uint32_t C = 1; !(u.slabPlan(C, it.plan) && it.plan.cache); ++C) {}   // ends: slabFits
-        items.push_back(it);
+        if (gridAnyway == before) break;
     }
-    // A cooperative launch waits until all its CTAs have found an SM, so it must never queue behind the
-    // batch's own resident kernels, which keep theirs for the whole run: a few residents get SMs of
-    // their own, many run after the slab sweeps.
-    residentsAfter = residents > slabSms_ / 4u;
-    uint32_t const budget =
-        std::max(1u, gridAnyway ? slabSms_ / 2u : slabSms_ - (residentsAfter ? 0u : residents));
-    std::stable_sort(items.begin(), items.end(), [&](Item const& a, Item const& b) {
-        return members_[a.m]->nMonomers() > members_[b.m]->nMonomers();
-    });
+    out.residentsAfter = residentsAfter;
+    std::stable_sort(items.begin(), items.end(),
+                     [&](Item const& a, Item const& b) { return members[a.m].monomers > members[b.m].monomers; });
     std::vector<std::vector<Item>> packed;
     std::vector<uint32_t> used;
     for (Item const& it : items) {
-        uint32_t const mode = members_[it.m]->codeMode();
+        uint32_t const mode = members[it.m].codeMode;
         size_t w = 0;
-        while (w < packed.size() &&
-               (used[w] + it.plan.ctas > budget || members_[packed[w][0].m]->codeMode() != mode))
-            ++w;
+        while (w < packed.size() && (used[w] + it.plan.ctas > budget || members[packed[w][0].m].codeMode != mode)) ++w;
         if (w == packed.size()) {
             packed.emplace_back();
             used.push_back(0);
@@ -298,20 +304,31 @@ std::vector<Batch::SlabWave> Batch::planSlabs(std::vector<char>& taken, bool& re
             for (Item& it : packed[w])
                 if (it.plan.perCta > kSlabGrowSlots && (!pick || it.plan.perCta > pick->plan.perCta)) pick = &it;
             SlabPlan next;
-            if (!pick || used[w] >= budget || !members_[pick->m]->slabPlan(pick->plan.ctas + 1u, next) || !next.cache)
-                break;
+            if (!pick || used[w] >= budget || !members[pick->m].plan(pick->plan.ctas + 1u, next) || !next.cache) break;
             pick->plan = next;
             ++used[w];
         }
-        SlabWave wave{members_[packed[w][0].m]->codeMode(), {}, 0, nullptr};
+        SlabWave wave{members[packed[w][0].m].codeMode, {}, 0, nullptr};
         for (Item const& it : packed[w]) {
             for (uint32_t r = 0; r < it.plan.ctas; ++r) wave.refs.push_back(SlabRef{it.m, r, it.plan.ctas, 0u});
             wave.smem = std::max(wave.smem, it.plan.smem);
-            taken[it.m] = 1;
+            out.taken[it.m] = 1;
         }
-        waves.push_back(std::move(wave));
+        out.waves.push_back(std::move(wave));
     }
-    return waves;
+    return out;
+}
+
+SlabWaves Batch::planSlabs() const
+{
+    std::vector<SlabMember> members;
+    if (clusterOn_)
+        for (Updater const* u : members_)
+            members.push_back(SlabMember{u->nMonomers(), u->codeMode(), residentOn_ && u->residentEligible(),
+                                         [u](uint32_t C, SlabPlan& p) { return u->slabPlan(C, p); }});
+    SlabWaves plan = plan_slab_waves(members, smCount_, slabSms_);
+    plan.taken.resize(members_.size(), 0);
+    return plan;
 }
 
 std::vector<Batch::ClusterGroup> Batch::planClusters(std::vector<char>& taken) const

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -349,6 +350,28 @@ public:
     size_t residentSmem() const;
 };
 
+// The slab sweeps of a Batch (plan_slab_waves): members of one representation in one cooperative launch of
+// at most the batch's share of the SMs; the launches run one after the other.
+constexpr uint32_t kSlabGrowSlots = 512;   // slots per CTA and colour, at least, where more CTAs join
+struct SlabMember {
+    uint32_t monomers, codeMode;
+    bool resident;                                      // runs in the resident kernel instead
+    std::function<bool(uint32_t, SlabPlan&)> plan;      // how so many CTAs hold it, if they do
+};
+struct SlabWave {
+    uint32_t codeMode;
+    std::vector<SlabRef> refs;      // the launch's CTAs
+    size_t smem = 0;
+    SlabRef* dRefs = nullptr;
+};
+struct SlabWaves {
+    std::vector<SlabWave> waves;
+    std::vector<char> taken;        // per member: it runs in one of them
+    bool residentsAfter = false;    // the resident kernels run after them
+};
+// sms: of the device; share: those the sweeps may fill.
+SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, uint32_t share);
+
 // A set of initialised updaters on one GPU advanced together: systems that fit one CTA run in the
 // resident kernel and larger bond-code systems in the slab sweep on several CTAs each (one
 // launch per run and group), the others share one grid-phase launch per phase and sub-step,
@@ -426,14 +449,6 @@ private:
         uint32_t perThread = 1;
         size_t smem = 0;
     };
-    // members of one representation in the slab sweep, one cooperative launch per run and wave, in order on
-    // one stream (side_[side])
-    struct SlabWave {
-        uint32_t codeMode;
-        std::vector<SlabRef> refs;      // the launch's CTAs
-        size_t smem = 0;
-        SlabRef* dRefs = nullptr;
-    };
     // members in the cluster-resident kernel, one launch per run and group
     struct ClusterGroup {
         uint32_t codeMode;
@@ -442,9 +457,8 @@ private:
         uint32_t* dList = nullptr;
     };
     std::vector<ClusterGroup> planClusters(std::vector<char>& taken) const;
-    static constexpr uint32_t kSlabGrowSlots = 512;   // slots per CTA and colour, at least, where more CTAs join
     bool slabFits(Updater const& u) const;
-    std::vector<SlabWave> planSlabs(std::vector<char>& taken, bool& residentsAfter) const;
+    SlabWaves planSlabs() const;
     void checkReports();                       // throws if a slab sweep of the last run failed
     void rebuild();
     void validateMembers(Updater* const* members, uint32_t n) const;
