@@ -14,7 +14,8 @@
 // A run stages the members' streams, and the step entries that no kernel makes from them (grid-phase
 // members, callbacks), with one host-to-device copy; the resident
 // and the grid-phase launches then proceed on two streams without meeting until the run ends, and
-// the host returns as soon as the work is queued. The slab sweeps run on a stream of their own. Member streams are ordered before the run and
+// the host returns as soon as the work is queued. The slab sweeps run on a stream of
+// their own, each group of clusters on another. Member streams are ordered before the run and
 // after it with events, never with host waits.
 
 #include <algorithm>
@@ -51,7 +52,7 @@ Batch::~Batch()
     cudaSetDevice(gpu_);
     if (stream_) cudaStreamSynchronize(stream_);
     if (stream2_) cudaStreamSynchronize(stream2_);
-    if (side_) cudaStreamSynchronize(side_);
+    for (Side const& q : side_) cudaStreamSynchronize(q.stream);
     if (graph_) cudaGraphExecDestroy(graph_);
     if (arena_) cudaFreeAsync(arena_, stream_);
     if (dStepsAll_) cudaFreeAsync(dStepsAll_, stream_);
@@ -59,8 +60,10 @@ Batch::~Batch()
     cudaFreeHost(hSteps_);
     for (cudaEvent_t e : {join_, fork_, stepsFree_, done_, ready_})
         if (e) cudaEventDestroy(e);
-    if (sideJoin_) cudaEventDestroy(sideJoin_);
-    if (side_) cudaStreamDestroy(side_);
+    for (Side const& q : side_) {
+        if (q.join) cudaEventDestroy(q.join);
+        cudaStreamDestroy(q.stream);
+    }
     if (stream_) cudaStreamDestroy(stream_);
     if (stream2_) cudaStreamDestroy(stream2_);
 }
@@ -106,7 +109,7 @@ void Batch::rebuild()
     // the previous launches may still read the arena
     cuda_check(cudaStreamSynchronize(stream_), "batch");
     cuda_check(cudaStreamSynchronize(stream2_), "batch");
-    if (side_) cuda_check(cudaStreamSynchronize(side_), "batch");
+    for (Side const& q : side_) cuda_check(cudaStreamSynchronize(q.stream), "batch");
     uint32_t const M = (uint32_t)members_.size();
     grid_.clear();
     resident_.clear();
@@ -129,9 +132,12 @@ void Batch::rebuild()
     std::vector<char> const slabbed = std::move(plan.taken);
     std::vector<char> clustered;
     cluster_ = planClusters(clustered);
-    if (!(slab_.empty() && cluster_.empty()) && !side_) {
-        cuda_check(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
-        cuda_check(cudaEventCreateWithFlags(&sideJoin_, cudaEventDisableTiming), "cudaEventCreate");
+    sides_ = std::max<size_t>(cluster_.size(), slab_.empty() ? 0 : 1);
+    while (side_.size() < sides_) {   // kept from one plan to the next
+        cudaStream_t q = nullptr;
+        cuda_check(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreate");
+        side_.push_back(Side{q, nullptr});
+        cuda_check(cudaEventCreateWithFlags(&side_.back().join, cudaEventDisableTiming), "cudaEventCreate");
     }
     bool faulted = false;   // a report belongs to the member it was made for: kept by it, not reused
     for (uint32_t m = 0; m < reportCap_; ++m) faulted = faulted || reports_.get()[m].fault != 0u;
@@ -554,8 +560,7 @@ void Batch::run(int32_t const* mcs)
         cuda_check(cudaMemcpyAsync(dStepsAll_, hSteps_, sizeof(StepEntry) * entries, cudaMemcpyHostToDevice, stream_),
                    "batch steps H2D");
         cuda_check(cudaEventRecord(stepsFree_, stream_), "event");
-        bool const sides = !slab_.empty() || !cluster_.empty();
-        if (!resident_.empty() || sides) cuda_check(cudaEventRecord(fork_, stream_), "event");
+        if (!resident_.empty() || sides_ != 0) cuda_check(cudaEventRecord(fork_, stream_), "event");
         // a whole-run kernel's launches on one stream: launch(source, sub-steps), kLaunchSteps at a time
         auto wholeRun = [&](char const* what, auto const& launch) {
             for (uint32_t t0 = 0, n = 0; t0 < T; t0 += n) {
@@ -567,27 +572,32 @@ void Batch::run(int32_t const* mcs)
                 ++launches_;
             }
         };
-        if (sides) {
-            cuda_check(cudaStreamWaitEvent(side_, fork_, 0), "wait");
-            for (auto const& g : cluster_)
+        for (size_t i = 0; i < sides_; ++i) {
+            // a cluster group each, side by side; or all slab sweeps, one after the other
+            cudaStream_t const q = side_[i].stream;
+            cuda_check(cudaStreamWaitEvent(q, fork_, 0), "wait");
+            if (i < cluster_.size()) {
+                ClusterGroup const& g = cluster_[i];
                 wholeRun("batch cluster", [&](StepSource const& src, uint32_t n) {
                     return launch_cluster_bc(dSys_, g.dList, (uint32_t)g.members.size(), g.plan.logC, g.plan.chunks,
-                                             src, n, g.plan.smem, g.codeMode, side_);
-                });
-            for (auto const& w : slab_) {
-                for (SlabRef const& r : w.refs)
-                    if (r.rank == 0) members_[r.sys]->applyStall(side_);
-                wholeRun("batch slab", [&](StepSource const& src, uint32_t n) {
-                    return launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, src, n, dReports_,
-                                             w.codeMode, side_);
+                                             src, n, g.plan.smem, g.codeMode, q);
                 });
             }
-            cuda_check(cudaEventRecord(sideJoin_, side_), "event");
+            for (size_t k = 0; i == 0 && k < slab_.size(); ++k) {
+                SlabWave const& w = slab_[k];
+                for (SlabRef const& r : w.refs)
+                    if (r.rank == 0) members_[r.sys]->applyStall(q);
+                wholeRun("batch slab", [&](StepSource const& src, uint32_t n) {
+                    return launch_slab_batch(dSys_, w.dRefs, (uint32_t)w.refs.size(), w.smem, src, n, dReports_,
+                                             w.codeMode, q);
+                });
+            }
+            cuda_check(cudaEventRecord(side_[i].join, q), "event");
         }
         if (!resident_.empty()) {
             // on the second stream
             cuda_check(cudaStreamWaitEvent(stream2_, fork_, 0), "wait");
-            if (!slab_.empty() && residentsAfter_) cuda_check(cudaStreamWaitEvent(stream2_, sideJoin_, 0), "wait");
+            if (!slab_.empty() && residentsAfter_) cuda_check(cudaStreamWaitEvent(stream2_, side_[0].join, 0), "wait");
             for (auto const& g : resident_)
                 wholeRun("batch resident", [&](StepSource const& src, uint32_t n) {
                     return g.codeMode == kCodeNone
@@ -618,7 +628,7 @@ void Batch::run(int32_t const* mcs)
             cuda_check(cudaEventRecord(join_, stream2_), "event");
             cuda_check(cudaStreamWaitEvent(stream_, join_, 0), "wait");
         }
-        if (sides) cuda_check(cudaStreamWaitEvent(stream_, sideJoin_, 0), "wait");
+        for (size_t i = 0; i < sides_; ++i) cuda_check(cudaStreamWaitEvent(stream_, side_[i].join, 0), "wait");
     }
     cuda_check(cudaEventRecord(done_, stream_), "event");
     for (uint32_t m = 0; m < M; ++m) {

@@ -481,8 +481,12 @@ private:
     GridFault* dReports_ = nullptr;
     uint32_t reportCap_ = 0;
     bool residentsAfter_ = false;              // the resident kernels run after the slab sweeps
-    cudaStream_t side_ = nullptr;              // the slab sweeps' or the clusters' stream
-    cudaEvent_t sideJoin_ = nullptr;
+    struct Side {
+        cudaStream_t stream;
+        cudaEvent_t join;
+    };
+    std::vector<Side> side_;                   // streams of the cluster groups; the first is the slab sweeps'
+    size_t sides_ = 0;                         // those of this plan
     uint32_t smCount_ = 148, slabSms_ = 148;
     bool residentOn_ = true;
     bool clusterOn_ = true;

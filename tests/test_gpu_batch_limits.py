@@ -115,3 +115,33 @@ def test_stalled_sweep_ends_at_its_limit_of_two_seconds():
             run()
         assert 1.0 < time.perf_counter() - t < 8.0
     b.close()
+
+
+def test_clusters_of_both_code_widths_run_side_by_side():
+    """Chains (32-bit codes) and chains linked across (64-bit) on clusters are two launches; neither waits
+    for the other: together they take less than one after the other."""
+    chains = S.serpentine_chains((64, 64, 32), 32, 0.6, seed=64)
+    rows, cols = chains.bonds()
+    at = {tuple(r): i for i, r in enumerate(chains.xyz)}
+    across = [(i, at[q]) for r, i in at.items() for q in ((r[0], r[1] + 2, r[2]), (r[0], r[1], r[2] + 2))
+              if q in at and abs(at[q] - i) > 1][::3]
+    bonds = {(int(min(p)), int(max(p))) for p in [*zip(rows, cols), *across]}
+    linked = S.from_bonds(chains.box, chains.xyz, sorted(bonds), seed=65)
+    assert linked.nbr_count.max() > 3
+    kinds = [chains, linked]
+
+    def timed(systems):
+        members = [load(s) for s in systems]
+        b = P.Batch(members)
+        n0 = b.launch_count()
+        b.run(20)
+        assert b.launch_count() - n0 == len(systems)   # a cluster launch each, and no resident one
+        ms = min(b.run_timed(300) for _ in range(3))
+        for s, m in zip(systems, members):
+            assert np.array_equal(m.get_coords(), O.run(s, 20 + 3 * 300)[0])
+            m.validate()
+        b.close()
+        return ms
+
+    one, other, both = timed(kinds[:1]), timed(kinds[1:]), timed(kinds)
+    assert both < 0.85 * (one + other), (one, other, both)
