@@ -258,7 +258,7 @@ SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, 
     // The members in the slab sweep (taken) and their CTAs, in cooperative launches of at most `budget` CTAs
     // that run one after the other. Each CTA takes an SM, so the fewest CTAs that hold a member do the most
     // work per SM (moves per us and SM at 0.9K, 1.9K, 3.7K and 7.5K slots per CTA and colour: 208, 331, 419
-    // and 458); members are packed that way, longest first. The SMs a wave leaves idle then go, one by one,
+    // and 458); members are packed by those, longest first. The SMs a wave leaves idle then go, one by one,
     // to its member with the most slots per CTA, which runs longest. A member the grid-phase kernels
     // have to take anyway (it does not fit the budget, or gathers) keeps half of the SMs.
     SlabWaves out;
@@ -291,31 +291,67 @@ SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, 
     out.residentsAfter = residentsAfter;
     std::stable_sort(items.begin(), items.end(),
                      [&](Item const& a, Item const& b) { return members[a.m].monomers > members[b.m].monomers; });
-    std::vector<std::vector<Item>> packed;
-    std::vector<uint32_t> used;
+    struct Wave {
+        uint32_t codeMode, used = 0;
+        uint64_t monomers = 0;
+        std::vector<Item> items;
+    };
+    auto put = [&](Wave& w, Item const& it) {
+        w.items.push_back(it);
+        w.used += it.plan.ctas;
+        w.monomers += members[it.m].monomers;
+    };
+    auto takes = [&](Wave const& w, Item const& it) {
+        return w.codeMode == members[it.m].codeMode && w.used + it.plan.ctas <= budget;
+    };
+    // The idle SMs of each wave handed out; returns the waves' time in all, us per MCS: a CTA's time grows with
+    // its slots per colour, and jumps where the movers of a sub-step, about an eighth, pass one per thread
+    // (one wave each, 128^3 boxes, at 640, 1664, 3350, 4928 and 6048 slots: 8, 11, 17, 21 and 41).
+    auto grow = [&](std::vector<Wave>& waves) {
+        double time = 0.0;
+        for (Wave& w : waves) {
+            uint32_t most = 0;
+            for (;;) {
+                Item* pick = nullptr;
+                for (Item& it : w.items)
+                    if (!pick || it.plan.perCta > pick->plan.perCta) pick = &it;
+                most = pick->plan.perCta;
+                SlabPlan next;
+                if (most <= kSlabGrowSlots || w.used >= budget || !members[pick->m].plan(pick->plan.ctas + 1u, next) ||
+                    !next.cache)
+                    break;
+                pick->plan = next;
+                ++w.used;
+            }
+            time += 5.5 + 0.0033 * most + (most > kSlabPassSlots ? 14.0 : 0.0);
+        }
+        return time;
+    };
+    // Members by first fit, the fewest waves; or as evenly over as many waves, each member, longest first, into
+    // the one of its kind with the fewest monomers: whichever takes less time. First fit fills its waves to
+    // the brim and leaves little to the last (32 systems of 60K, 29 and 3, 50 us per MCS and, 16 and 16, 38;
+    // 64 systems of 30K, 49 of 3 CTAs each and 15, 31 and, 32 and 32, 35).
+    std::vector<Wave> first;
     for (Item const& it : items) {
-        uint32_t const mode = members[it.m].codeMode;
-        size_t w = 0;
-        while (w < packed.size() && (used[w] + it.plan.ctas > budget || members[packed[w][0].m].codeMode != mode)) ++w;
-        if (w == packed.size()) {
-            packed.emplace_back();
-            used.push_back(0);
-        }
-        packed[w].push_back(it);
-        used[w] += it.plan.ctas;
+        auto w = std::find_if(first.begin(), first.end(), [&](Wave const& q) { return takes(q, it); });
+        if (w == first.end()) w = first.insert(w, Wave{members[it.m].codeMode});
+        put(*w, it);
     }
-    for (size_t w = 0; w < packed.size(); ++w) {
-        for (;;) {
-            Item* pick = nullptr;
-            for (Item& it : packed[w])
-                if (it.plan.perCta > kSlabGrowSlots && (!pick || it.plan.perCta > pick->plan.perCta)) pick = &it;
-            SlabPlan next;
-            if (!pick || used[w] >= budget || !members[pick->m].plan(pick->plan.ctas + 1u, next) || !next.cache) break;
-            pick->plan = next;
-            ++used[w];
-        }
-        SlabWave wave{members[packed[w][0].m].codeMode, {}, 0, nullptr};
-        for (Item const& it : packed[w]) {
+    std::vector<Wave> even;
+    for (Wave const& w : first) even.push_back(Wave{w.codeMode});
+    bool room = first.size() > 1;
+    for (size_t i = 0; room && i < items.size(); ++i) {
+        Wave* best = nullptr;
+        for (Wave& w : even)
+            if (takes(w, items[i]) && (!best || w.monomers < best->monomers)) best = &w;
+        room = best != nullptr;
+        if (room) put(*best, items[i]);
+    }
+    double const time = grow(first);
+    if (room && grow(even) < time) first.swap(even);
+    for (Wave const& w : first) {
+        SlabWave wave{w.codeMode, {}, 0, nullptr};
+        for (Item const& it : w.items) {
             for (uint32_t r = 0; r < it.plan.ctas; ++r) wave.refs.push_back(SlabRef{it.m, r, it.plan.ctas, 0u});
             wave.smem = std::max(wave.smem, it.plan.smem);
             out.taken[it.m] = 1;

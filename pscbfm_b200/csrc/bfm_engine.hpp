@@ -353,6 +353,7 @@ public:
 // The slab sweeps of a Batch (plan_slab_waves): members of one representation in one cooperative launch of
 // at most the batch's share of the SMs; the launches run one after the other.
 constexpr uint32_t kSlabGrowSlots = 512;   // slots per CTA and colour, at least, where more CTAs join
+constexpr uint32_t kSlabPassSlots = 5120;  // slots per CTA and colour whose movers are one per thread, about
 struct SlabMember {
     uint32_t monomers, codeMode;
     bool resident;                                      // runs in the resident kernel instead

@@ -17,11 +17,11 @@ using namespace bfm;
         }                                                                                           \
     } while (0)
 
-static SlabMember member(uint32_t n, uint32_t mode, bool resident)
+static SlabMember member(uint32_t n, uint32_t mode, bool resident, uint32_t nwords = 1u << 18)
 {
     return SlabMember{n, mode, resident, [=](uint32_t C, SlabPlan& p) {
                           uint32_t const grp[2] = {n / 2, n - n / 2};
-                          return slab_plan(grp, 2, mode == kCode64 ? 4 : 2, 1u << 18, mode, C, p);
+                          return slab_plan(grp, 2, mode == kCode64 ? 4 : 2, nwords, mode, C, p);
                       }};
 }
 
@@ -77,8 +77,18 @@ int main()
     // beside a gathering member the lane's sweeps have 18 SMs: 300K need 19
     if (check(1, {member(300000, kCode32, false), member(9000, kCodeNone, false), member(30000, kCode32, false)}, 148, 37))
         return 1;
+    // two waves where one is not enough, as evenly as their sizes allow: none to the brim beside one nearly empty
+    {
+        number = 2;
+        std::vector<SlabMember> const members(32, member(60288, kCode32, false, 1u << 15));
+        SlabWaves const w = plan_slab_waves(members, 148, 148);
+        REQUIRE(w.waves.size() == 2 && w.waves[0].refs.size() == 148 && w.waves[1].refs.size() == 148);
+        size_t first = 0;
+        for (SlabRef const& r : w.waves[0].refs) first += r.rank == 0;
+        REQUIRE(first == 16);
+    }
     std::mt19937 rng(12345);
-    for (number = 2; number < 3000; ++number) {
+    for (number = 3; number < 3000; ++number) {
         std::uniform_real_distribution<double> u(0.0, 1.0);
         std::vector<SlabMember> members;
         size_t const count = 1 + size_t(40 * u(rng) * u(rng));
