@@ -240,8 +240,9 @@ int bfm_batch_synchronize(bfm_batch_handle b);
 int bfm_batch_set_resident(bfm_batch_handle b, int on);
 /* 1 (default): bond-code systems too large for one CTA run on CTAs of their own for the whole run, as
  * many as hold them in shared memory and share the SMs evenly (to about 500 K monomers; beside a larger
- * or a gather system, which needs the grid-phase kernels, they take at most half of the SMs); 0: they
- * share the grid-phase kernels. Results do not change. */
+ * or a gather system, which needs the grid-phase kernels, they take at most half of the SMs; runs of one to
+ * five MCS of many or large ones take the grid-phase kernels); 0: they share the grid-phase kernels.
+ * Results do not change. */
 int bfm_batch_set_cluster(bfm_batch_handle b, int on);
 /* Member i advances mcs[i] MCS (0 = it idles); one launch sequence for all, like bfm_batch_run. */
 int bfm_batch_run_each(bfm_batch_handle b, const int32_t* mcs);

@@ -4,7 +4,8 @@
 // codes) fit one CTA's shared memory run in the resident kernel, one CTA per system; where such systems
 // leave SMs idle, the largest of them run on clusters of CTAs (planClusters).
 // Larger systems of the bond-code representation run in the slab sweep, each on CTAs of its
-// own, several systems in one cooperative launch (planSlabs). A launch of these kernels runs up to
+// own, several systems in one cooperative launch (plan_slab_waves; runs of few MCS take the grid phase where
+// the launches' loading of the slots would take longer). A launch of these kernels runs up to
 // kLaunchSteps sub-steps. What fits neither shares the grid-phase kernels: one check and one perform launch per
 // sub-step and representation cover the active colour group of every such system at once, and
 // chunks of those launches are captured into a CUDA graph once and replayed. Each system draws its
@@ -129,6 +130,8 @@ void Batch::rebuild()
     SlabWaves plan = planSlabs();
     slab_.swap(plan.waves);
     residentsAfter_ = plan.residentsAfter;
+    leastMcs_ = plan.leastMcs;
+    shortMembers_ = false;
     std::vector<char> const slabbed = std::move(plan.taken);
     std::vector<char> clustered;
     cluster_ = planClusters(clustered);
@@ -349,6 +352,20 @@ SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, 
     }
     double const time = grow(first);
     if (room && grow(even) < time) first.swap(even);
+    // A launch loads its CTAs' slots and writes them back, about 10 us per 1000 slots of a CTA and colour. us
+    // of 1, 2, 4 and 6 MCS in the grid phase and in the sweeps, `load` their launches' slots: 16 x 60K (load 3350)
+    // 59, 102, 180, 264 and 61, 77, 114, 153; 12 x 118K (4928) 67, 112, 200, 291 and 77, 100, 143, 188; 32 x 60K
+    // (6700) 92, 154, 277, 403 and 118, 156, 225, 301; 48 x 60K (10048) 124, 211, 385, 562 and 174, 227, 322,
+    // 424; 100 x 30K (10368) 138, 204, 347, 481 and 198, 248, 347, 448. Residents that run after the sweeps run
+    // beside the grid phase: 64 mixed systems 145, 212, 333, 469 and 195, 248, 356, 467; 256 624, 822, 1251, 1669 and
+    // 808, 961, 1266, 1565.
+    uint32_t load = 0;
+    for (Wave const& w : first) {
+        uint32_t most = 0;
+        for (Item const& it : w.items) most = std::max(most, it.plan.perCta);
+        load += most;
+    }
+    out.leastMcs = load <= 4000u ? 1u : (load <= 9500u ? 2u : 4u) + (residentsAfter ? 2u : 0u);
     for (Wave const& w : first) {
         SlabWave wave{w.codeMode, {}, 0, nullptr};
         for (Item const& it : w.items) {
@@ -540,12 +557,36 @@ uint32_t Batch::longest(int32_t const* mcs) const
     return (uint32_t)T;
 }
 
+Batch* Batch::shortFor(int32_t const* mcs)
+{
+    if (!shortRuns_ || slab_.empty()) return nullptr;
+    for (size_t m = 0; m < members_.size(); ++m)
+        if ((uint32_t)mcs[m] >= leastMcs_) return nullptr;
+    if (!short_) {
+        short_.reset(new Batch(gpu_, members_.data(), (uint32_t)members_.size()));
+        short_->setClusterEnabled(false);
+    } else if (!shortMembers_) {
+        short_->setMembers(members_.data(), (uint32_t)members_.size());
+    }
+    shortMembers_ = true;
+    short_->setResidentEnabled(residentOn_);
+    short_->setShape(shape_);
+    short_->setBlock(block_);
+    short_->setPerformShape(perfWarps_, perfGroup_);
+    return short_.get();
+}
+
 void Batch::prepare(int32_t const* mcs)
 {
     // one-time host work of a run (staging growth, graph capture), done ahead of a timed run
     uint32_t const M = (uint32_t)members_.size();
     uint32_t const T = longest(mcs);
     if (T == 0) return;
+    if (Batch* const b = shortFor(mcs)) {
+        if (!b->built_) b->rebuild();
+        b->prepare(mcs);
+        return;
+    }
     reserveSteps(streamUnits() + (hostEntries() ? (size_t)T * M : 0));
     if (!grid_.empty() && T >= stepCap_) ensureGraph();
 }
@@ -563,6 +604,11 @@ void Batch::run(int32_t const* mcs)
     uint32_t const T = longest(mcs);
     cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
     if (!built_) rebuild();
+    if (Batch* const b = shortFor(mcs)) {
+        b->run(mcs);   // (the members' streams order it after this batch's runs and before the next)
+        cuda_check(cudaStreamWaitEvent(stream_, b->done_, 0), "wait");
+        return;
+    }
     // pending grid-path marks of members that run in a resident or cluster kernel are cleared on
     // their own streams; then the batch waits for every member stream (uploads, scrubs,
     // observables) on the device
@@ -722,6 +768,11 @@ std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
     // check's register budget (kGridShapes) x its CTA size (128, 256, 512 threads), as the
     // reference sweeps its block size (CRITICAL.cu:445-487); last, for the best of those, the
     // perform's warps per CTA x warps per tile.
+    struct Whole {   // the trials are of the paths they name, however short
+        bool& on;
+        explicit Whole(bool& o) : on(o) { on = false; }
+        ~Whole() { on = true; }
+    } const whole(shortRuns_);
     std::vector<Trial> trials;
     auto time_it = [&](bool resident, bool cl, int shape, int block, int pw, int pg) {
         setResidentEnabled(resident);

@@ -369,6 +369,7 @@ struct SlabWaves {
     std::vector<SlabWave> waves;
     std::vector<char> taken;        // per member: it runs in one of them
     bool residentsAfter = false;    // the resident kernels run after them
+    uint32_t leastMcs = 1;          // shorter runs are faster on the grid-phase kernels
 };
 // sms: of the device; share: those the sweeps may fill.
 SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, uint32_t share);
@@ -431,7 +432,7 @@ public:
     cudaStream_t stream() const { return stream_; }
     uint32_t residentCount() const;
     uint32_t clusterCount() const;
-    uint64_t launches() const { return launches_; }
+    uint64_t launches() const { return launches_ + (short_ ? short_->launches_ : 0); }
 
 private:
     // members of one representation (codeMode) on one path
@@ -470,6 +471,7 @@ private:
     size_t streamUnits() const;                  // the members' streams, in entries
     void ensureGraph();                          // capture the graph of stepCap_ sub-steps
     uint32_t longest(int32_t const* mcs) const;  // the most sub-steps of a member; throws beyond 32 bits
+    Batch* shortFor(int32_t const* mcs);         // short_, if the run is one for it, else nullptr
     void prepare(int32_t const* mcs);            // both, for a run of mcs[i] MCS per member
     int gpu_;
     std::vector<Updater*> members_;
@@ -489,6 +491,10 @@ private:
     std::vector<Side> side_;                   // streams of the cluster groups; the first is the slab sweeps'
     size_t sides_ = 0;                         // those of this plan
     uint32_t smCount_ = 148, slabSms_ = 148;
+    uint32_t leastMcs_ = 1;                    // shorter runs go to short_ (SlabWaves)
+    bool shortRuns_ = true;
+    std::unique_ptr<Batch> short_;             // the same members without slab sweeps, from the first short run on
+    bool shortMembers_ = false;                // short_ has this batch's members
     bool residentOn_ = true;
     bool clusterOn_ = true;
     bool built_ = false;

@@ -145,3 +145,38 @@ def test_clusters_of_both_code_widths_run_side_by_side():
 
     one, other, both = timed(kinds[:1]), timed(kinds[1:]), timed(kinds)
     assert both < 0.85 * (one + other), (one, other, both)
+
+
+def test_short_runs_of_many_large_members_take_the_grid_phase():
+    """64 systems of 29K monomers are two launches of slab sweeps, which load and write back every slot: a run of
+    one MCS takes the grid-phase kernels instead (two launches per sub-step). The trajectories go on across both,
+    and across changes of the members and of the kernels' settings."""
+    s = S.serpentine_chains(64, 64, 0.9, seed=5)
+    members = [load(s, seed=200 + i) for i in range(64)]
+    b = P.Batch(members)
+
+    def launches(run, *a):
+        n0 = b.launch_count()
+        run(*a)
+        return b.launch_count() - n0
+
+    assert launches(b.run, 1) == 4
+    assert launches(b.run, 3) == 2
+    assert launches(b.run, 1) == 4
+    b.set_block(128)
+    assert launches(b.run, 1) == 4
+    assert launches(b.run_each, [2] * 3 + [1] * 61) == 2
+    b.set_cluster(False)
+    assert launches(b.run, 2) == 8
+    b.set_cluster(True)
+    b.run_timed(1)
+    b.run_async(1)
+    b.run_async(2)
+    for i in (0, 2, 3, 40, 63):
+        k = 1 + 3 + 1 + 1 + (2 if i < 3 else 1) + 2 + 1 + 1 + 2
+        want, ost = O.run(s, k, seed=200 + i)
+        st = members[i].stats()
+        assert np.array_equal(members[i].get_coords(), want), i
+        assert (st["attempted"], st["tentative"], st["accepted"]) == ost and st["mcs"] == k
+        members[i].validate()
+    b.close()
