@@ -256,7 +256,7 @@ bool Batch::slabFits(Updater const& u) const
     return slab_least([&](uint32_t C, SlabPlan& p) { return u.slabPlan(C, p); }, std::min(smCount_ / 2u, slabSms_), plan);
 }
 
-SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, uint32_t share)
+SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, uint32_t share, uint32_t most)
 {
     // The members in the slab sweep (taken) and their CTAs, in cooperative launches of at most `budget` CTAs
     // that run one after the other. Each CTA takes an SM, so the fewest CTAs that hold a member do the most
@@ -313,20 +313,20 @@ SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, 
     auto grow = [&](std::vector<Wave>& waves) {
         double time = 0.0;
         for (Wave& w : waves) {
-            uint32_t most = 0;
+            uint32_t slots = 0;
             for (;;) {
                 Item* pick = nullptr;
                 for (Item& it : w.items)
                     if (!pick || it.plan.perCta > pick->plan.perCta) pick = &it;
-                most = pick->plan.perCta;
+                slots = pick->plan.perCta;
                 SlabPlan next;
-                if (most <= kSlabGrowSlots || w.used >= budget || !members[pick->m].plan(pick->plan.ctas + 1u, next) ||
+                if (slots <= kSlabGrowSlots || w.used >= budget || !members[pick->m].plan(pick->plan.ctas + 1u, next) ||
                     !next.cache)
                     break;
                 pick->plan = next;
                 ++w.used;
             }
-            time += 5.5 + 0.0033 * most + (most > kSlabPassSlots ? 14.0 : 0.0);
+            time += 5.5 + 0.0033 * slots + (slots > kSlabPassSlots ? 14.0 : 0.0);
         }
         return time;
     };
@@ -339,6 +339,10 @@ SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, 
         auto w = std::find_if(first.begin(), first.end(), [&](Wave const& q) { return takes(q, it); });
         if (w == first.end()) w = first.insert(w, Wave{members[it.m].codeMode});
         put(*w, it);
+    }
+    if (first.size() > most) {
+        out.residentsAfter = false;
+        return out;
     }
     std::vector<Wave> even;
     for (Wave const& w : first) even.push_back(Wave{w.codeMode});
@@ -361,9 +365,9 @@ SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, 
     // 808, 961, 1266, 1565.
     uint32_t load = 0;
     for (Wave const& w : first) {
-        uint32_t most = 0;
-        for (Item const& it : w.items) most = std::max(most, it.plan.perCta);
-        load += most;
+        uint32_t slots = 0;
+        for (Item const& it : w.items) slots = std::max(slots, it.plan.perCta);
+        load += slots;
     }
     out.leastMcs = load <= 4000u ? 1u : (load <= 9500u ? 2u : 4u) + (residentsAfter ? 2u : 0u);
     for (Wave const& w : first) {
@@ -385,7 +389,7 @@ SlabWaves Batch::planSlabs() const
         for (Updater const* u : members_)
             members.push_back(SlabMember{u->nMonomers(), u->codeMode(), residentOn_ && u->residentEligible(),
                                          [u](uint32_t C, SlabPlan& p) { return u->slabPlan(C, p); }});
-    SlabWaves plan = plan_slab_waves(members, smCount_, slabSms_);
+    SlabWaves plan = plan_slab_waves(members, smCount_, slabSms_, slabLaunches_);
     plan.taken.resize(members_.size(), 0);
     return plan;
 }
@@ -446,6 +450,12 @@ std::vector<Batch::ClusterGroup> Batch::planClusters(std::vector<char>& taken) c
         taken[m] = 1;
     }
     return groups;
+}
+
+void Batch::setSlabLaunches(uint32_t most)
+{
+    if (most != slabLaunches_) built_ = false;
+    slabLaunches_ = most;
 }
 
 void Batch::setSlabSms(uint32_t sms)

@@ -371,8 +371,8 @@ struct SlabWaves {
     bool residentsAfter = false;    // the resident kernels run after them
     uint32_t leastMcs = 1;          // shorter runs are faster on the grid-phase kernels
 };
-// sms: of the device; share: those the sweeps may fill.
-SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, uint32_t share);
+// sms: of the device; share: those the sweeps may fill; most: launches at most, or none at all.
+SlabWaves plan_slab_waves(std::vector<SlabMember> const& members, uint32_t sms, uint32_t share, uint32_t most = ~0u);
 
 // A set of initialised updaters on one GPU advanced together: systems that fit one CTA run in the
 // resident kernel and larger bond-code systems in the slab sweep on several CTAs each (one
@@ -428,6 +428,8 @@ public:
     }
     // SMs the slab sweeps may fill (default: all; a server's lanes share them)
     void setSlabSms(uint32_t sms);
+    // slab sweeps only where at most so many launches hold their members, else the grid phase (default: any)
+    void setSlabLaunches(uint32_t most);
     uint32_t smCount() const { return smCount_; }
     cudaStream_t stream() const { return stream_; }
     uint32_t residentCount() const;
@@ -490,7 +492,7 @@ private:
     };
     std::vector<Side> side_;                   // streams of the cluster groups; the first is the slab sweeps'
     size_t sides_ = 0;                         // those of this plan
-    uint32_t smCount_ = 148, slabSms_ = 148;
+    uint32_t smCount_ = 148, slabSms_ = 148, slabLaunches_ = ~0u;
     uint32_t leastMcs_ = 1;                    // shorter runs go to short_ (SlabWaves)
     bool shortRuns_ = true;
     std::unique_ptr<Batch> short_;             // the same members without slab sweeps, from the first short run on

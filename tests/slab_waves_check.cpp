@@ -86,6 +86,9 @@ int main()
         size_t first = 0;
         for (SlabRef const& r : w.waves[0].refs) first += r.rank == 0;
         REQUIRE(first == 16);
+        // at most one launch: none for these, one for a lane's few
+        SlabWaves const none = plan_slab_waves(members, 148, 148, 1), few = plan_slab_waves({members[0], members[1]}, 148, 37, 1);
+        REQUIRE(none.waves.empty() && none.taken == std::vector<char>(32, 0) && few.waves.size() == 1 && few.taken[1]);
     }
     std::mt19937 rng(12345);
     for (number = 3; number < 3000; ++number) {
