@@ -262,7 +262,8 @@ int bfm_batch_get_perform(bfm_batch_handle b, int* warps, int* group);
  * (shape) x CTA size (128, 256, 512 threads; the reference sweeps its block size,
  * CRITICAL.cu:445-487); for the best of those the perform's warps per CTA x per tile ((8,4),
  * (4,2), (8,8), (2,2) beside the default (4,4)). The last two stages run only when some member is
- * on the grid-phase kernels. trials (may be NULL) receives up to capacity sextuples (shape, paths,
+ * on the grid-phase kernels. ms per MCS is that of a long run: what a run costs however long it is (by the
+ * trials' runs of 1 and of mcs_per_trial MCS, where that is more than 1) is left out. trials (may be NULL) receives up to capacity sextuples (shape, paths,
  * block, perform warps, perform warps per tile, ms per MCS; 0 for a default). */
 int bfm_batch_autotune(bfm_batch_handle b, int32_t mcs_per_trial, int* shape, int* paths, float* ms_per_mcs,
                        float* trials, uint32_t capacity, uint32_t* n_trials);

@@ -610,7 +610,6 @@ void Batch::run(int32_t nMcs)
 
 void Batch::run(int32_t const* mcs)
 {
-    uint32_t const M = (uint32_t)members_.size();
     uint32_t const T = longest(mcs);
     cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
     if (!built_) rebuild();
@@ -619,6 +618,12 @@ void Batch::run(int32_t const* mcs)
         cuda_check(cudaStreamWaitEvent(stream_, b->done_, 0), "wait");
         return;
     }
+    enqueue(mcs, T);
+}
+
+void Batch::enqueue(int32_t const* mcs, uint32_t T)
+{
+    uint32_t const M = (uint32_t)members_.size();
     // pending grid-path marks of members that run in a resident or cluster kernel are cleared on
     // their own streams; then the batch waits for every member stream (uploads, scrubs,
     // observables) on the device
@@ -758,7 +763,11 @@ void Batch::setPerformShape(int warps, int group)
 std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
 {
     // Every configuration gives the same trajectories, so the trials are ordinary MCS of the run:
-    // each configuration runs 1 MCS (graph capture, warm-up) and then mcsPerTrial timed MCS.
+    // each configuration runs 1 MCS and then mcsPerTrial MCS, both timed. What a run costs however long it is
+    // (slots loaded and written back, streams joined) would have few MCS per trial choose for runs as short as
+    // the trials (40 systems of 60K, 2 MCS 95 us per MCS in slab sweeps and 88 in the grid phase, 100 MCS 46
+    // and 65): the paths are compared by the time that the further MCS take, their kernels' shapes by the
+    // longer run less the path's fixed time.
     if (mcsPerTrial <= 0) throw std::invalid_argument("[Batch::autotune] trials need at least one MCS");
     cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
     if (!built_) rebuild();
@@ -784,16 +793,27 @@ std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
         ~Whole() { on = true; }
     } const whole(shortRuns_);
     std::vector<Trial> trials;
-    auto time_it = [&](bool resident, bool cl, int shape, int block, int pw, int pg) {
+    float fixed[2][2] = {};   // ms of a run on each path before its first MCS
+    auto time_it = [&](bool resident, bool cl, int shape, int block, int pw, int pg, bool path = false) {
         setResidentEnabled(resident);
         setClusterEnabled(cl);
         setShape(shape);
         setBlock(block);
         setPerformShape(pw, pg);
         rebuild();
-        runTimed(1);
-        trials.push_back(
-            Trial{shape_, resident, cl, block_, pw, pg, runTimed(mcsPerTrial) / (float)mcsPerTrial});
+        std::vector<int32_t> const none(members_.size(), 0);
+        float idle = 0.f;   // every kernel, all members idle (the first time it is loaded as well)
+        for (int rep = 0; rep < 4; ++rep) {
+            for (Updater* u : members_) u->synchronize();
+            float const t = timed([&] { enqueue(none.data(), 1); });
+            idle = rep < 2 ? t : std::min(idle, t);
+        }
+        float const one = runTimed(1), ms = runTimed(mcsPerTrial), k = (float)mcsPerTrial;
+        float& f = fixed[resident][cl];
+        // (a run of 1 MCS that was held up must not make a path look fast: the MCS take at least the time
+        // of the run less that of an idle one)
+        if (path && mcsPerTrial > 1) f = std::max(0.f, ms - std::max(k * (ms - one) / (k - 1.f), ms - idle));
+        trials.push_back(Trial{shape_, resident, cl, block_, pw, pg, std::max(ms - f, 0.1f * ms) / k});
         return trials.back();
     };
     Trial best{};
@@ -802,7 +822,7 @@ std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
         if (!resident && !anyResident) break;   // the same configuration as resident on
         for (int cl = 1; cl >= 0; --cl) {
             if (!cl && !anyCluster[resident]) break;   // the same configuration as cluster on
-            Trial const t = time_it(resident != 0, cl != 0, -1, 0, 0, 0);
+            Trial const t = time_it(resident != 0, cl != 0, -1, 0, 0, 0, true);
             if (first || t.msPerMcs < best.msPerMcs) best = t;
             first = false;
         }
@@ -837,6 +857,24 @@ std::vector<Batch::Trial> Batch::autotune(int32_t mcsPerTrial)
     return trials;
 }
 
+template <typename Queue>
+float Batch::timed(Queue const& queue)
+{
+    cudaEvent_t a, b;
+    cuda_check(cudaEventCreate(&a), "cudaEventCreate");
+    cuda_check(cudaEventCreate(&b), "cudaEventCreate");
+    cuda_check(cudaEventRecord(a, stream_), "event");
+    queue();   // the other streams join stream_ before it returns
+    cuda_check(cudaEventRecord(b, stream_), "event");
+    cuda_check(cudaEventSynchronize(b), "timed batch");
+    float ms = 0.f;
+    cuda_check(cudaEventElapsedTime(&ms, a, b), "elapsed");
+    cudaEventDestroy(a);
+    cudaEventDestroy(b);
+    checkReports();
+    return ms;
+}
+
 float Batch::runTimed(int32_t nMcs)
 {
     cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
@@ -846,19 +884,7 @@ float Batch::runTimed(int32_t nMcs)
         std::vector<int32_t> each(members_.size(), nMcs);
         prepare(each.data());
     }
-    cudaEvent_t a, b;
-    cuda_check(cudaEventCreate(&a), "cudaEventCreate");
-    cuda_check(cudaEventCreate(&b), "cudaEventCreate");
-    cuda_check(cudaEventRecord(a, stream_), "event");
-    run(nMcs);   // the resident stream joins stream_ before run() returns
-    cuda_check(cudaEventRecord(b, stream_), "event");
-    cuda_check(cudaEventSynchronize(b), "timed batch");
-    float ms = 0.f;
-    cuda_check(cudaEventElapsedTime(&ms, a, b), "elapsed");
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    checkReports();
-    return ms;
+    return timed([&] { run(nMcs); });
 }
 
 void Batch::synchronize()

@@ -400,7 +400,8 @@ public:
     bool residentEnabled() const { return residentOn_; }
     bool clusterEnabled() const { return clusterOn_; }
     // Runs the members under each configuration (kernel shape x resident path on / off x cluster
-    // path on / off) for 1 + mcsPerTrial MCS, keeps the fastest per MCS and returns every trial.
+    // path on / off) for 1 + mcsPerTrial MCS, keeps the fastest per MCS (less what a run costs however long it
+    // is) and returns every trial.
     // The MCS count as ordinary steps of the run: the results do not depend on the configuration.
     struct Trial {
         int shape;
@@ -473,6 +474,9 @@ private:
     size_t streamUnits() const;                  // the members' streams, in entries
     void ensureGraph();                          // capture the graph of stepCap_ sub-steps
     uint32_t longest(int32_t const* mcs) const;  // the most sub-steps of a member; throws beyond 32 bits
+    void enqueue(int32_t const* mcs, uint32_t T);   // the run by this batch's own plan, of T sub-steps at most
+    template <typename Queue>
+    float timed(Queue const& queue);             // ms of the work that queue() puts on the batch's streams
     Batch* shortFor(int32_t const* mcs);         // short_, if the run is one for it, else nullptr
     void prepare(int32_t const* mcs);            // both, for a run of mcs[i] MCS per member
     int gpu_;

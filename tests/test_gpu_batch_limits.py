@@ -180,3 +180,24 @@ def test_short_runs_of_many_large_members_take_the_grid_phase():
         assert (st["attempted"], st["tentative"], st["accepted"]) == ost and st["mcs"] == k
         members[i].validate()
     b.close()
+
+
+def test_autotuner_with_short_trials_picks_the_path_of_long_runs():
+    """Trials of two MCS are no measure of what a launch costs however long it runs: 40 systems of 60K monomers,
+    whose slab sweeps take longer than the grid phase for two MCS and less for a hundred, are tuned for the sweeps."""
+    s = S.serpentine_chains(128, 64, 0.23, seed=5)
+    members = [load(s, seed=300 + i) for i in range(40)]
+    b = P.Batch(members)
+    b.run(3)
+    rep = b.autotune(2)
+    spent = 3 + rep["mcs_spent"]
+    assert rep["cluster"], rep["trials"]
+    tuned = min(b.run_timed(60) for _ in range(2))
+    b.set_cluster(False)
+    other = min(b.run_timed(60) for _ in range(2))
+    assert tuned < other
+    want, ost = O.run(s, spent + 240, seed=339)
+    st = members[39].stats()
+    assert np.array_equal(members[39].get_coords(), want)
+    assert (st["attempted"], st["tentative"], st["accepted"]) == ost
+    b.close()
