@@ -212,14 +212,16 @@ struct StepSource {
     StepStream own;
     uint32_t stride, first;
 };
-// The stream of system sys, from the launch's first sub-step on.
+// The stream of system sys: loaded by one thread, then, after a CTA barrier, brought to the launch's first
+// sub-step by another. (Both by the loading thread, the resident kernel built from it was 0.4 % slower.)
 __device__ __forceinline__ StepStream step_stream(StepSource const& src, uint32_t sys)
 {
-    if (src.streams == nullptr) return src.own;
-    StepStream s = src.streams[sys];
-    s.t0 += src.first;
-    s.n -= min(s.n, src.first);
-    return s;
+    return src.streams != nullptr ? src.streams[sys] : src.own;
+}
+__device__ __forceinline__ void step_stream_from(StepStream& s, uint32_t first)
+{
+    s.t0 += first;
+    s.n -= min(s.n, first);
 }
 __device__ __forceinline__ StepEntry step_entry(StepSource const& src, StepStream const& own, uint32_t sys, uint32_t t,
                                                 uint32_t const* grp, uint32_t nColors)

@@ -602,7 +602,9 @@ __host__ __device__ __forceinline__ void slab_caps(F size, uint32_t nColors, uin
     }
 }
 // Dense systems clear the temporary lattice whole: nwords x 8 B written in order, against one scattered
-// write per mark.
+// write per mark. The two draw level at about two words per slot (us per MCS, whole and per mark: 128^3 at 6.3
+// words per slot 7.72 and 7.42, 3.1 7.75 and 7.67, 2.0 7.68 and 7.68, 1.6 7.61 and 7.63; 256^3 at 6.3 8.22 and 7.92,
+// 2.0 8.32 and 8.26, 1.25 8.75 and 8.71, 0.6 10.25 and 10.31, 0.3 14.23 and 14.37).
 __host__ __device__ __forceinline__ bool slab_clear_all(uint32_t nwords, uint32_t nSlots) { return nwords <= 2u * nSlots; }
 
 // The sweep of one system by C CTAs (this one's rank among them), a whole run of sub-steps in one launch.
@@ -645,7 +647,7 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& sr
     constexpr uint32_t kFarBit = 1u << 31;
     __shared__ SlabPart P;
     __shared__ __align__(16) StepEntry stepSm[2][kStepBlock];   // the block of entries in use, and the next
-    __shared__ uint32_t nCand, nMov, tallyA, failed;
+    __shared__ uint32_t nCand, nMov, tallyA;
     extern __shared__ unsigned long long smem[];
     uint32_t const tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     bool const waiter = warp == nWork;
@@ -662,7 +664,6 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& sr
             b += 32u * (hi - lo);
         }
         nCand = nMov = tallyA = 0u;
-        failed = ld_acquire_gpu(&gs->fault);
     }
     unsigned long long* const ptab = smem;                                   // 768 plane masks
     uint32_t* const dtab = reinterpret_cast<uint32_t*>(smem + 768);          // kDirTab words
@@ -677,8 +678,8 @@ __device__ __forceinline__ void slab_sweep(SysDev const& S, StepSource const& sr
     for (uint32_t w = tid; w < 768; w += B) ptab[(w & 2u ? 384u : 0u) + (w >> 2) * 2u + (w & 1u)] = S.planeTab[w];
     if (tid < kDirTab) dtab[tid] = S.dirTab[tid];
     for (uint32_t w = tid; w < 512; w += B) mok[w] = S.moveOk[w];
-    __syncthreads();
-    if (failed != 0u) {   // an earlier launch failed: the state is not usable, and this run's caller learns of it too
+    // an earlier launch failed: the state is not usable, and this run's caller learns of it too
+    if (__syncthreads_or(tid == 0 && ld_acquire_gpu(&gs->fault) != 0u) != 0) {
         if (tid == 0) report->fault = 1u;   // (where: the barrier it failed at, where the report is the same)
         return;
     }
@@ -1035,6 +1036,7 @@ __global__ void __launch_bounds__(B, 1)
     __syncthreads();
     if (threadIdx.x == 0)
         slab_caps([&](uint32_t c) { return S.grp[2 * c + 1]; }, S.nColors, r.ctas, caps[0], caps[1], caps[2]);
+    if (threadIdx.x == 32) step_stream_from(own, src.first);
     __syncthreads();
     slab_sweep<W, B, true, true>(S, src, own, r.sys, nSteps, r.ctas, r.rank, caps[0], caps[1],
                                  slab_clear_all(S.nwords, caps[2]), report + r.sys);
@@ -1148,6 +1150,7 @@ __global__ void __launch_bounds__(kResidentBlock, 1) k_resident_bc(SysDev const*
     if (threadIdx.x == 0) own = step_stream(src, sysId);
     copy_desc(S, sysv + sysId);
     __syncthreads();
+    if (threadIdx.x == 32) step_stream_from(own, src.first);   // (read after the next barrier)
     uint32_t const nw = S.nwords, np = S.npad, maxc = S.maxc;
     uint32_t const tid = threadIdx.x, lane = tid & 31u;
     if (tid == 0) {
@@ -1428,6 +1431,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_cluster_bc(SysDev const* __restri
     if (threadIdx.x == 0) own = step_stream(src, sysId);
     copy_desc(S, sysv + sysId);
     __syncthreads();
+    if (threadIdx.x == 32) step_stream_from(own, src.first);   // (read after the next barrier)
     uint32_t const np = S.npad, nwC = S.nwords >> logC, cap = cluster_slots_per_cta(np, logC), maxc = S.maxc;
     uint32_t const tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     uint4* const masks = reinterpret_cast<uint4*>(smem);                     // kHalfPlanes entries
