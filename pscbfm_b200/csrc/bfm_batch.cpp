@@ -397,8 +397,10 @@ SlabWaves Batch::planSlabs() const
 std::vector<Batch::ClusterGroup> Batch::planClusters(std::vector<char>& taken) const
 {
     // A batch lasts as long as its largest member, and a member that fits one CTA takes longer there than
-    // on a cluster's CTAs (us per MCS with g slots per colour, fitted to 600 to 13K slots: 2.9 + 0.00185 g on
-    // one, 4.4 + 0.0046 g / C on C). Where every member fits one CTA and SMs are left over, the k largest go
+    // on a cluster's CTAs. The weights, us per MCS with g slots per colour, 2.9 + 0.00185 g on one CTA and
+    // 4.4 + 0.0046 g / C on C, are those of lone systems on earlier forms of the kernels. A lone cluster takes
+    // less now (3.7 + 0.006 g / C), but many at once take longer than one, and with that fit the plans
+    // were worse (16 systems of 8K monomers 8.8 -> 11.2), so the older weights stay. Where every member fits one CTA and SMs are left over, the k largest go
     // to clusters: C and k with the least time of the longest member. Sixteen systems of 0.4K to 10.5K
     // monomers, on one CTA each, with slab sweeps on the SMs left over, and so: 14.2, 9.4 and 6.8 us per MCS;
     // 7, 9, 16, 32 and 36 systems of 8K monomers 10.8 -> 5.8, 7.2, 9.5, 9.8 and 10.9.
@@ -729,7 +731,7 @@ void Batch::enqueue(int32_t const* mcs, uint32_t T)
     }
     cuda_check(cudaEventRecord(done_, stream_), "event");
     for (uint32_t m = 0; m < M; ++m) {
-        members_[m]->noteExternalRun(need[m], (uint64_t)mcs[m], !wholeRun_[m], members_[m]->lastColor(),
+        members_[m]->noteExternalRun((uint64_t)mcs[m], !wholeRun_[m], members_[m]->lastColor(),
                                      slab_.empty() ? nullptr : std::shared_ptr<GridFault>(reports_, reports_.get() + m));
         members_[m]->streamWait(done_);
     }

@@ -893,7 +893,7 @@ StepEntry Updater::nextStep()
     return e;
 }
 
-void Updater::fillSteps(uint32_t nSteps, StepEntry* buf, bool)
+void Updater::fillSteps(uint32_t nSteps, StepEntry* buf)
 {
     for (uint32_t t = 0; t < nSteps; ++t) buf[t] = nextStep();
     chainValid_ = false;   // the host's entries go to the device's entry slots
@@ -947,10 +947,9 @@ void Updater::scrubPending(cudaStream_t s)
     lastColor_ = kNoColor;
 }
 
-void Updater::noteExternalRun(uint64_t subSteps, uint64_t mcs, bool pendingMarks, uint32_t lastColor,
+void Updater::noteExternalRun(uint64_t mcs, bool pendingMarks, uint32_t lastColor,
                               std::shared_ptr<GridFault> report)
 {
-    (void)subSteps;
     // (a report that has not been looked at stays: an earlier run's failure is not lost to a later run)
     if (report && std::find(batchReports_.begin(), batchReports_.end(), report) == batchReports_.end())
         batchReports_.push_back(std::move(report));
@@ -966,7 +965,7 @@ void Updater::enqueueLaunch(uint32_t nSteps)
     for (uint32_t done = 0; done < nSteps;) {
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
         cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
-        fillSteps(chunk, hSteps_, false);
+        fillSteps(chunk, hSteps_);
         cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * chunk, cudaMemcpyHostToDevice, stream_),
                    "steps H2D");
         h2dBytes_ += sizeof(StepEntry) * chunk;
@@ -1077,7 +1076,7 @@ void Updater::enqueueGraph(uint32_t nSteps)
         } else {
             producerOff(stream_);
             cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
-            fillSteps(chunk, hSteps_, false);
+            fillSteps(chunk, hSteps_);
             cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * chunk, cudaMemcpyHostToDevice,
                                        stream_),
                        "steps H2D");
@@ -1137,7 +1136,7 @@ void Updater::timeKernels(int32_t nMcs, double out[4])
     for (uint32_t done = 0; done < nSteps;) {
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
         cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
-        fillSteps(chunk, hSteps_, false);
+        fillSteps(chunk, hSteps_);
         cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * chunk, cudaMemcpyHostToDevice, stream_),
                    "steps H2D");
         h2dBytes_ += sizeof(StepEntry) * chunk;
@@ -1184,7 +1183,7 @@ StepSource Updater::stepSource(uint32_t nSteps)
     StepSource src{};
     if (streamSteps(nSteps, src.own)) return src;
     cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
-    fillSteps(nSteps, hSteps_, false);
+    fillSteps(nSteps, hSteps_);
     cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * nSteps, cudaMemcpyHostToDevice, stream_),
                "steps H2D");
     h2dBytes_ += sizeof(StepEntry) * nSteps;
@@ -1204,7 +1203,7 @@ void Updater::enqueueResident(uint32_t nSteps)
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
         if (codeMode_ == kCodeNone) {
             cuda_check(cudaEventSynchronize(stepsFree_), "steps staging");
-            fillSteps(chunk, hSteps_, true);
+            fillSteps(chunk, hSteps_);
             cuda_check(cudaMemcpyAsync(dev_.dSteps, hSteps_, sizeof(StepEntry) * chunk, cudaMemcpyHostToDevice, stream_),
                        "steps H2D");
             h2dBytes_ += sizeof(StepEntry) * chunk;
@@ -1279,7 +1278,7 @@ int Updater::autoMode(int32_t nMcs) const
 {
     // One system on a B200, us per MCS: the resident kernel (one SM) while the largest colour group is
     // at most 1024 monomers (1.2K-monomer chains 3.3 against 3.9 on a cluster of 16 CTAs, 2K 4.1 against
-    // 4.0-4.1, 3.3K 5.6 against 4.2, 8K 10.6 against 5.0).
+    // 4.0-4.1, 3.3K 5.3 against 4.2, 8K 10.6 against 5.0).
     // Then a cluster of CTAs holding the system in distributed shared memory, up to the clusterCost_ where
     // the persistent sweep draws level (cluster against persistent: 8K chains in 64^3, cost 1120, 5.0 and
     // 7.7; 16K 2144 6.7 and 7.6; 20K 2656 8.5 and 7.6; 13K in 128^3 2432 6.4 and 7.7; 18K 3072 8.3 and 7.7;

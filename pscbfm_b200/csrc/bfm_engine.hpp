@@ -142,7 +142,6 @@ public:
     uint32_t maxGroup() const { return maxGroup_; }
     bool residentEligible() const;
     bool clusterEligible() const { return cluster_.logC != 0; }
-    // whether ctas CTAs hold the system in the slab sweep (bond codes), and how
     // the cluster-resident kernel's plan on 2^logC CTAs: how many such clusters the device runs at a
     // time (0: the system does not fit, or the device runs none); its shared memory per CTA with more
     // chunks than its own
@@ -151,6 +150,7 @@ public:
     {
         return cluster_bc_smem_bytes(dev_.h.nwords, npad_, logC, chunks, maxc_, codeMode_);
     }
+    // whether ctas CTAs hold the system in the slab sweep (bond codes), and how
     bool slabPlan(uint32_t ctas, SlabPlan& plan) const
     {
         return slab_plan(grpSize_.data(), (uint32_t)grpSize_.size(), maxc_, dev_.h.nwords, codeMode_, ctas, plan);
@@ -168,7 +168,7 @@ public:
     bool countsDraws() const { return drawKind_ == kDrawCounter; }
     void scrubPending(cudaStream_t s);       // clears the temporary marks of the last sub-step
     // report: where a launch of the run may report a failed barrier (looked at by the next synchronise)
-    void noteExternalRun(uint64_t subSteps, uint64_t mcs, bool pendingMarks, uint32_t lastColor,
+    void noteExternalRun(uint64_t mcs, bool pendingMarks, uint32_t lastColor,
                          std::shared_ptr<GridFault> report = nullptr);
     uint32_t lastColor() const { return lastColor_; }
     void streamWait(cudaEvent_t e);          // orders this system's later work after e
@@ -225,7 +225,7 @@ private:
     template <typename Ended>
     void awaitKernel(char const* what, Ended const& ended);
     void checkReports();                // throws if a sweep that has ended reported a barrier timeout
-    void fillSteps(uint32_t nSteps, StepEntry* hostBuf, bool residentParity);
+    void fillSteps(uint32_t nSteps, StepEntry* hostBuf);
     void freeDevice();
     void ensureStaging();
 
