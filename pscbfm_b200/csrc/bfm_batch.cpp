@@ -571,7 +571,7 @@ uint32_t Batch::longest(int32_t const* mcs) const
 
 Batch* Batch::shortFor(int32_t const* mcs)
 {
-    if (!shortRuns_ || slab_.empty()) return nullptr;
+    if (!shortRuns_ || leastMcs_ <= 1 || slab_.empty()) return nullptr;
     for (size_t m = 0; m < members_.size(); ++m)
         if ((uint32_t)mcs[m] >= leastMcs_) return nullptr;
     if (!short_) {

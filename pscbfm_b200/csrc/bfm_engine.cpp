@@ -1254,13 +1254,44 @@ uint32_t Updater::clusterPlan(uint32_t logC, ClusterPlan& plan) const
     return cluster_bc_runnable(logC, chunks, smem, codeMode_);
 }
 
+namespace {
+// Per device, the updaters whose cluster or slab sweep has been queued and not waited for.
+std::atomic<uint32_t> sweepsQueued[64];
+}  // namespace
+
+uint32_t Updater::beginSweep()
+{
+    if (sweepOn_ < 0) {
+        sweepOn_ = gpu_ & 63;
+        ++sweepsQueued[sweepOn_];
+    }
+    return sweepsQueued[sweepOn_].load(std::memory_order_relaxed);
+}
+
+void Updater::endSweep()
+{
+    if (sweepOn_ >= 0) --sweepsQueued[sweepOn_];
+    sweepOn_ = -1;
+}
+
 void Updater::enqueueCluster(uint32_t nSteps)
 {
     scrubPending(stream_);
+    // Beside sweeps of other updaters (threads, streams) the largest cluster of which the device runs as many
+    // at a time (us per MCS of all, 8 threads with 8K chains each, one run of 1000 MCS, on 16 CTAs and so: 10.1
+    // and 6.5; 16 threads 15.2 and 13.5).
+    ClusterPlan plan = cluster_;
+    uint32_t const n = beginSweep();
+    for (uint32_t logC = cluster_.logC; n > 1 && logC >= 1; --logC) {
+        ClusterPlan p;
+        if (clusterPlan(logC, p) < n) continue;
+        plan = p;
+        break;
+    }
     for (uint32_t done = 0; done < nSteps;) {
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
-        cuda_check(launch_cluster_bc(dev_.dDesc, dev_.dList, 1, cluster_.logC, cluster_.chunks, stepSource(chunk), chunk,
-                                     cluster_.smem, codeMode_, stream_),
+        cuda_check(launch_cluster_bc(dev_.dDesc, dev_.dList, 1, plan.logC, plan.chunks, stepSource(chunk), chunk,
+                                     plan.smem, codeMode_, stream_),
                    "cluster");
         ++launches_;
         done += chunk;
@@ -1340,10 +1371,20 @@ void Updater::applyStall(cudaStream_t s)
 void Updater::enqueuePersistent(uint32_t nSteps)
 {
     scrubPending(stream_);   // marks of a previous grid-phase run, left for the next check
+    // Cooperative launches that do not fit side by side run one after the other. Where this one would not fit
+    // beside the sweeps of other updaters (threads, streams) it takes its share of the SMs instead, if that
+    // holds the system with at most kSlabPassSlots slots per CTA and colour (us per MCS of all, threads that run
+    // 100 MCS at a time, with the largest plan and so: 4 and 8 x 60K monomers 17.1, 33.9 and 10.2, 11.4; 4 and 8
+    // x 131K 18.5, 36.8 and 11.7, 16.9).
+    SlabPlan plan = slab_, part;
+    uint32_t const n = beginSweep();
+    if (n > 1 && n * slab_.ctas > slab_ctas_per_sm(slab_, codeMode_) * smCount_ && slabPlan(smCount_ / n, part) &&
+        part.cache && part.perCta <= kSlabPassSlots)
+        plan = part;
     for (uint32_t done = 0; done < nSteps;) {
         uint32_t const chunk = std::min(nSteps - done, hStepCap_);
         applyStall(stream_);
-        cuda_check(launch_slab_bc(dev_.h, stepSource(chunk), chunk, slab_, dGs_, codeMode_, stream_), "persistent sweep");
+        cuda_check(launch_slab_bc(dev_.h, stepSource(chunk), chunk, plan, dGs_, codeMode_, stream_), "persistent sweep");
         ++launches_;
         done += chunk;
     }
@@ -1365,6 +1406,7 @@ void Updater::streamWait(cudaEvent_t e)
 void Updater::synchronize()
 {
     if (stream_) cuda_check(cudaStreamSynchronize(stream_), "sweep");
+    endSweep();
     checkReports();
 }
 
@@ -1480,6 +1522,7 @@ void Updater::awaitKernel(char const* what, Ended const& ended)
         }
     } while (!seen && std::chrono::steady_clock::now() < until);
     if (!seen) cuda_check(cudaStreamSynchronize(stream_), what);
+    endSweep();
     std::atomic_thread_fence(std::memory_order_acquire);
 }
 
@@ -1788,6 +1831,7 @@ void Updater::validate()
 
 void Updater::freeDevice()
 {
+    endSweep();
     // the publishing stream reads the arena's snapshots and writes the host ring: done first
     if (pubStream_) {
         cudaStreamSynchronize(pubStream_);

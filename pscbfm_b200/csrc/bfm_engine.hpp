@@ -220,6 +220,8 @@ private:
     void enqueueCluster(uint32_t nSteps);
     void planCluster();   // the cluster size and chunks per warp of the cluster-resident kernel
     void enqueuePersistent(uint32_t nSteps);
+    uint32_t beginSweep();   // counts this updater's queued sweep; how many updaters of the device have one
+    void endSweep();         // it has ended
     StepSource stepSource(uint32_t nSteps);   // the next nSteps entries, for one launch that runs them
     // until ended() holds, which a kernel queued last makes true in host memory, or the stream is idle
     template <typename Ended>
@@ -296,6 +298,7 @@ private:
     cudaEvent_t pubEv_ = nullptr;
     bool gsPending_ = false;                   // a persistent launch may have reported to hGs_
     bool stallNext_ = false;                   // injectBarrierStall
+    int sweepOn_ = -1;                         // the device that beginSweep counted on
     uint32_t smCount_ = 148;                   // SMs of the device (setGpu)
     ClusterPlan cluster_;                      // the cluster-resident kernel's plan (planCluster)
     uint32_t clusterCost_ = ~0u;               // what decides between cluster_ and the persistent sweep (planCluster)

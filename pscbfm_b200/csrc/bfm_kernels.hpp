@@ -133,6 +133,8 @@ bool slab_plan(uint32_t const* grpSize, uint32_t nColors, uint32_t maxc, uint32_
                uint32_t ctas, SlabPlan& plan);
 // CTAs of a cooperative launch for a system whose largest colour group is maxGroup
 uint32_t slab_ctas(uint32_t maxGroup, uint32_t sms);
+// CTAs of such a launch that an SM holds at a time (0: the question failed).
+uint32_t slab_ctas_per_sm(SlabPlan const& plan, uint32_t codeMode);
 cudaError_t launch_slab_bc(SysDev const& hostDesc, StepSource const& src, uint32_t nSteps, SlabPlan const& plan,
                            GridFault* report, uint32_t codeMode, cudaStream_t s);
 // Plans with the cache only; dRefs: the launch's CTAs; the reports are report[system].

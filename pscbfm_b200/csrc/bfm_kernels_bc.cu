@@ -1841,6 +1841,22 @@ struct SlabLaunch {
     cudaError_t operator()() const { return launch_slab_bc_w<W, B, kCache>(S, src, nSteps, plan, report, s); }
 };
 
+struct SlabPerSm {
+    SlabPlan const& plan;
+    template <typename W, int B, bool kCache>
+    uint32_t operator()() const
+    {
+        static thread_local bool done[64] = {};
+        int n = 0;
+        if (allow_smem(k_slab_bc<W, B, kCache>, done) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_slab_bc<W, B, kCache>, B, plan.smem) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return (uint32_t)n;
+    }
+};
+
 template <typename W, int B>
 cudaError_t launch_slab_batch_w(SysDev const* dSys, SlabRef const* dRefs, uint32_t ctas, size_t smem, StepSource src,
                                 uint32_t nSteps, GridFault* report, cudaStream_t s)
@@ -1854,6 +1870,11 @@ cudaError_t launch_slab_batch_w(SysDev const* dSys, SlabRef const* dRefs, uint32
 }
 
 }  // namespace
+
+uint32_t slab_ctas_per_sm(SlabPlan const& plan, uint32_t codeMode)
+{
+    return plan.ctas == 0 || codeMode == kCodeNone ? 0u : slab_dispatch(codeMode, plan, SlabPerSm{plan});
+}
 
 cudaError_t launch_slab_bc(SysDev const& hostDesc, StepSource const& src, uint32_t nSteps, SlabPlan const& plan,
                            GridFault* report, uint32_t codeMode, cudaStream_t s)

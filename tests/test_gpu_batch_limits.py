@@ -201,3 +201,42 @@ def test_autotuner_with_short_trials_picks_the_path_of_long_runs():
     assert np.array_equal(members[39].get_coords(), want)
     assert (st["attempted"], st["tentative"], st["accepted"]) == ost
     b.close()
+
+
+@pytest.mark.parametrize("name,most", [("60K", 2.5), ("131K", 2.8), ("8K", 2.5)])
+def test_threads_share_the_sms(name, most):
+    """Eight threads that each run a system of their own again and again: sweeps that take most of the SMs alone run
+    side by side on fewer, with the trajectories of each alone, in much less time than one after the other."""
+    import threading
+    import time
+    s = {"60K": lambda: S.serpentine_chains(128, 64, 0.23, seed=5), "131K": lambda: S.serpentine_chains(128, 256, 0.5),
+         "8K": S.small_chains}[name]()
+    us = [load(s, seed=400 + i) for i in range(8)]
+
+    def timed(some):
+        def again(u):
+            for _ in range(8):
+                u.runSimulationOnGPU(100)
+
+        best = 1e9
+        for _ in range(3):
+            threads = [threading.Thread(target=again, args=(u,)) for u in some]
+            t = time.perf_counter()
+            for x in threads:
+                x.start()
+            for x in threads:
+                x.join()
+            best = min(best, time.perf_counter() - t)
+        return best
+
+    one, all8 = timed([load(s, seed=1)]), timed(us)
+    for k in (7, 1):
+        for u in us:
+            u.run_async(k)
+    for i in (0, 3, 7):
+        v = load(s, seed=400 + i, mode=P.MODE_GRAPH)
+        v.runSimulationOnGPU(3 * 800 + 8)
+        assert us[i].stats() == v.stats() and np.array_equal(us[i].get_coords(), v.get_coords())
+        us[i].validate()
+        v.close()
+    assert all8 < most * one, (one, all8)
