@@ -39,7 +39,8 @@ extern "C" {
 /* engine paths (bfm_set_mode) */
 #define BFM_MODE_AUTO 0     /* resident for small systems (largest colour group <= 1024 and fits one CTA),
                                cluster where a cluster of up to 16 CTAs holds the system with few slots
-                               per CTA (to about 26 K monomers in a 64^3 box), persistent up to about
+                               per CTA (to about 18 K monomers in a 64^3 box, 26 K for a run of one
+                               MCS, 64-bit bond codes further), persistent up to about
                                three 512-monomer tiles per SM (bond codes), else graph, with
                                persistent runs of 6 MCS or more where the slots fit the SMs */
 #define BFM_MODE_LAUNCH 1   /* check + perform launch per sub-step (the reference's structure) */
@@ -130,10 +131,10 @@ int bfm_set_perform(bfm_handle h, int warps, int group);
  * BFM_MODE_GRAPH. */
 int bfm_get_path(bfm_handle h, int* mode);
 /* Fault injection for tests (no counterpart in the reference): the next BFM_MODE_PERSISTENT launch
- * of this handle (or the next run of a batch that holds it on CTAs of its own) starts its grid-barrier arrival count where no barrier can complete, so every
- * CTA's wait runs out at its time limit (2 s) and the run reports the timeout
- * (BFM_ERR_CUDA).
- * Nothing faults on the GPU and the device stays usable; this system's state is not. */
+ * of this handle (or the next run of a batch that holds it on CTAs of its own) starts its grid-barrier
+ * arrival count where no barrier can complete, so every CTA's wait runs out at its time limit (2 s) and the
+ * run reports the timeout (BFM_ERR_CUDA). Nothing faults on the GPU and the device stays usable; this
+ * system's state is not, and every later sweep of it, alone or in a batch, reports the failure again. */
 int bfm_inject_barrier_stall(bfm_handle h);
 /* Device representation of the bonds, chosen before bfm_initialize: BFM_REPR_AUTO (bond codes —
  * each monomer keeps the table indices of its bonds, updated exactly when it or a neighbour moves
