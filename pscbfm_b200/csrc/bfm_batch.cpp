@@ -31,6 +31,7 @@ namespace bfm {
 namespace {
 constexpr double kClusterGain = 0.9;      // clusters are taken for at least a tenth of a batch's time
 constexpr uint32_t kBatchChunk = 64;      // sub-steps per captured graph of the grid phase
+constexpr uint32_t kCalmRuns = 8;         // runs beside fewer others before a batch's share of the SMs grows
 size_t up256(size_t v) { return (v + 255) & ~size_t(255); }
 }  // namespace
 
@@ -45,11 +46,12 @@ Batch::Batch(int gpu, Updater* const* members, uint32_t n) : gpu_(gpu)
         cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, gpu_) == cudaSuccess && sms > 0)
-        smCount_ = slabSms_ = (uint32_t)sms;
+        smCount_ = slabSms_ = share_ = (uint32_t)sms;
 }
 
 Batch::~Batch()
 {
+    SweepUsers::end(gpu_, this);
     cudaSetDevice(gpu_);
     if (stream_) cudaStreamSynchronize(stream_);
     if (stream2_) cudaStreamSynchronize(stream2_);
@@ -389,7 +391,7 @@ SlabWaves Batch::planSlabs() const
         for (Updater const* u : members_)
             members.push_back(SlabMember{u->nMonomers(), u->codeMode(), residentOn_ && u->residentEligible(),
                                          [u](uint32_t C, SlabPlan& p) { return u->slabPlan(C, p); }});
-    SlabWaves plan = plan_slab_waves(members, smCount_, slabSms_, slabLaunches_);
+    SlabWaves plan = plan_slab_waves(members, smCount_, share_, slabLaunches_);
     plan.taken.resize(members_.size(), 0);
     return plan;
 }
@@ -426,8 +428,8 @@ std::vector<Batch::ClusterGroup> Batch::planClusters(std::vector<char>& taken) c
         uint32_t atOnce = ~0u;   // clusters of the batch's share of the SMs
         for (size_t k = 0; k < order.size(); ++k) {
             ClusterPlan plan;
-            atOnce = std::min(atOnce, members_[order[k]]->clusterPlan(logC, plan) * slabSms_ / smCount_);
-            if (k + 1 > atOnce || (k + 1) * (C - 1u) + M > slabSms_) break;
+            atOnce = std::min(atOnce, members_[order[k]]->clusterPlan(logC, plan) * share_ / smCount_);
+            if (k + 1 > atOnce || (k + 1) * (C - 1u) + M > share_) break;
             double const time = std::max(spread(slots(0), C), alone(slots(k + 1)));
             if (time < best) {
                 best = time;
@@ -463,7 +465,28 @@ void Batch::setSlabLaunches(uint32_t most)
 void Batch::setSlabSms(uint32_t sms)
 {
     if (sms != slabSms_) built_ = false;
-    slabSms_ = sms;
+    slabSms_ = share_ = sms;
+    calm_ = 0;
+}
+
+void Batch::takeShare()
+{
+    // Beside other users of the device (SweepUsers) the plan takes their number's share of the SMs: sweeps of
+    // batches in several threads then run at once instead of one after the other (us per MCS of all, 8 threads with
+    // a batch each: 2 systems of 60K monomers 76 and 20, 8 of 30K 76 and 35, 4 of 8K 24 and 9; 16 of 60K 155 and
+    // 171, each batch then several launches).
+    // The share shrinks at once and by halves, and grows after kCalmRuns runs in which it could have: a new
+    // plan costs the host what several short runs take.
+    if (!clusterOn_ || slabSms_ < smCount_) return;   // (a server's lanes have their shares)
+    if (built_ && slab_.empty() && cluster_.empty() && share_ == slabSms_) return;
+    uint32_t parts = 1;
+    for (uint32_t const n = SweepUsers::others(gpu_, this) + 1u; parts < n;) parts *= 2u;
+    uint32_t const want = std::max(1u, std::min(slabSms_, smCount_ / parts));
+    calm_ = want > share_ ? calm_ + 1u : 0u;
+    if (want >= share_ && calm_ < kCalmRuns) return;
+    share_ = want;
+    calm_ = 0;
+    built_ = false;
 }
 
 cudaError_t Batch::launchGrid(StepEntry const* e)
@@ -614,6 +637,7 @@ void Batch::run(int32_t const* mcs)
 {
     uint32_t const T = longest(mcs);
     cuda_check(cudaSetDevice(gpu_), "cudaSetDevice");
+    takeShare();
     if (!built_) rebuild();
     if (Batch* const b = shortFor(mcs)) {
         b->run(mcs);   // (the members' streams order it after this batch's runs and before the next)
@@ -632,6 +656,7 @@ void Batch::enqueue(int32_t const* mcs, uint32_t T)
     for (uint32_t m = 0; m < M; ++m)
         if (wholeRun_[m]) members_[m]->scrubPending(members_[m]->stream());
     for (Updater* u : members_) {
+        u->endSweep();       // (this run comes after the member's own)
         u->flushTickets();   // a member's ticket still waiting for a snapshot reads its counters now
         cuda_check(cudaEventRecord(ready_, u->stream()), "event");
         cuda_check(cudaStreamWaitEvent(stream_, ready_, 0), "wait");
@@ -730,6 +755,7 @@ void Batch::enqueue(int32_t const* mcs, uint32_t T)
         for (size_t i = 0; i < sides_; ++i) cuda_check(cudaStreamWaitEvent(stream_, side_[i].join, 0), "wait");
     }
     cuda_check(cudaEventRecord(done_, stream_), "event");
+    if (sides_ != 0) SweepUsers::add(gpu_, this, done_);
     for (uint32_t m = 0; m < M; ++m) {
         members_[m]->noteExternalRun((uint64_t)mcs[m], !wholeRun_[m], members_[m]->lastColor(),
                                      slab_.empty() ? nullptr : std::shared_ptr<GridFault>(reports_, reports_.get() + m));

@@ -1255,22 +1255,54 @@ uint32_t Updater::clusterPlan(uint32_t logC, ClusterPlan& plan) const
 }
 
 namespace {
-// Per device, the updaters whose cluster or slab sweep has been queued and not waited for.
-std::atomic<uint32_t> sweepsQueued[64];
+struct SweepUser {
+    int gpu;
+    void const* who;
+    cudaEvent_t done;
+};
+std::mutex usersLock;
+std::vector<SweepUser> users;
 }  // namespace
 
-uint32_t Updater::beginSweep()
+void SweepUsers::add(int gpu, void const* who, cudaEvent_t done)
 {
-    if (sweepOn_ < 0) {
-        sweepOn_ = gpu_ & 63;
-        ++sweepsQueued[sweepOn_];
-    }
-    return sweepsQueued[sweepOn_].load(std::memory_order_relaxed);
+    std::lock_guard<std::mutex> const hold(usersLock);
+    for (SweepUser const& u : users)
+        if (u.who == who) return;
+    users.push_back(SweepUser{gpu, who, done});
+}
+
+void SweepUsers::end(int gpu, void const* who)
+{
+    std::lock_guard<std::mutex> const hold(usersLock);
+    users.erase(std::remove_if(users.begin(), users.end(),
+                               [&](SweepUser const& u) { return u.gpu == gpu && u.who == who; }),
+                users.end());
+}
+
+uint32_t SweepUsers::others(int gpu, void const* who)
+{
+    std::lock_guard<std::mutex> const hold(usersLock);
+    users.erase(std::remove_if(users.begin(), users.end(),
+                               [&](SweepUser const& u) {
+                                   return u.who != who && u.done && cudaEventQuery(u.done) == cudaSuccess;
+                               }),
+                users.end());
+    return (uint32_t)std::count_if(users.begin(), users.end(),
+                                   [&](SweepUser const& u) { return u.gpu == gpu && u.who != who; });
+}
+
+void Updater::beginSweep()
+{
+    if (sweepOn_ >= 0) return;
+    sweepOn_ = gpu_;
+    SweepUsers::add(sweepOn_, this, nullptr);
 }
 
 void Updater::endSweep()
 {
-    if (sweepOn_ >= 0) --sweepsQueued[sweepOn_];
+    if (sweepOn_ < 0) return;
+    SweepUsers::end(sweepOn_, this);
     sweepOn_ = -1;
 }
 
@@ -1281,7 +1313,8 @@ void Updater::enqueueCluster(uint32_t nSteps)
     // at a time (us per MCS of all, 8 threads with 8K chains each, one run of 1000 MCS, on 16 CTAs and so: 10.1
     // and 6.5; 16 threads 15.2 and 13.5).
     ClusterPlan plan = cluster_;
-    uint32_t const n = beginSweep();
+    beginSweep();
+    uint32_t const n = SweepUsers::others(gpu_, this) + 1u;
     for (uint32_t logC = cluster_.logC; n > 1 && logC >= 1; --logC) {
         ClusterPlan p;
         if (clusterPlan(logC, p) < n) continue;
@@ -1377,7 +1410,8 @@ void Updater::enqueuePersistent(uint32_t nSteps)
     // 100 MCS at a time, with the largest plan and so: 4 and 8 x 60K monomers 17.1, 33.9 and 10.2, 11.4; 4 and 8
     // x 131K 18.5, 36.8 and 11.7, 16.9).
     SlabPlan plan = slab_, part;
-    uint32_t const n = beginSweep();
+    beginSweep();
+    uint32_t const n = SweepUsers::others(gpu_, this) + 1u;
     if (n > 1 && n * slab_.ctas > slab_ctas_per_sm(slab_, codeMode_) * smCount_ && slabPlan(smCount_ / n, part) &&
         part.cache && part.perCta <= kSlabPassSlots)
         plan = part;
@@ -1744,6 +1778,7 @@ void Updater::statsWait(uint64_t ticket, uint64_t out[4])
                         "replays ahead of the read)");
     for (uint32_t c = 0; c < 3; ++c) out[c] = slot[c];
     out[3] = statMcs_[k];
+    if (statMcs_[k] == mcsDone_) endSweep();   // nothing has run since
 }
 
 void Updater::validate()

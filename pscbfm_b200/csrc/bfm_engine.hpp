@@ -72,6 +72,15 @@ struct DoneFlags {
     static void give(unsigned int* flag);
 };
 
+// The updaters and batches of each device whose cluster or slab sweeps have been queued and have not ended: they
+// share its SMs.
+struct SweepUsers {
+    // who is one, until done has passed, or where there is no event until end()
+    static void add(int gpu, void const* who, cudaEvent_t done);
+    static void end(int gpu, void const* who);
+    static uint32_t others(int gpu, void const* who);   // how many there are beside who
+};
+
 class Updater {
 public:
     explicit Updater(int gpu);
@@ -171,6 +180,8 @@ public:
     void noteExternalRun(uint64_t mcs, bool pendingMarks, uint32_t lastColor,
                          std::shared_ptr<GridFault> report = nullptr);
     uint32_t lastColor() const { return lastColor_; }
+    void beginSweep();                       // a cluster or slab sweep is queued (SweepUsers)
+    void endSweep();                         // it has ended, or is followed by a batch's
     void streamWait(cudaEvent_t e);          // orders this system's later work after e
     void flushTickets();                     // tickets waiting for a snapshot: from the counters, now
 
@@ -220,8 +231,6 @@ private:
     void enqueueCluster(uint32_t nSteps);
     void planCluster();   // the cluster size and chunks per warp of the cluster-resident kernel
     void enqueuePersistent(uint32_t nSteps);
-    uint32_t beginSweep();   // counts this updater's queued sweep; how many updaters of the device have one
-    void endSweep();         // it has ended
     StepSource stepSource(uint32_t nSteps);   // the next nSteps entries, for one launch that runs them
     // until ended() holds, which a kernel queued last makes true in host memory, or the stream is idle
     template <typename Ended>
@@ -298,7 +307,7 @@ private:
     cudaEvent_t pubEv_ = nullptr;
     bool gsPending_ = false;                   // a persistent launch may have reported to hGs_
     bool stallNext_ = false;                   // injectBarrierStall
-    int sweepOn_ = -1;                         // the device that beginSweep counted on
+    int sweepOn_ = -1;                         // the device of a queued cluster or slab sweep (SweepUsers)
     uint32_t smCount_ = 148;                   // SMs of the device (setGpu)
     ClusterPlan cluster_;                      // the cluster-resident kernel's plan (planCluster)
     uint32_t clusterCost_ = ~0u;               // what decides between cluster_ and the persistent sweep (planCluster)
@@ -500,6 +509,8 @@ private:
     std::vector<Side> side_;                   // streams of the cluster groups; the first is the slab sweeps'
     size_t sides_ = 0;                         // those of this plan
     uint32_t smCount_ = 148, slabSms_ = 148, slabLaunches_ = ~0u;
+    void takeShare();                          // share_ for the next run, beside the device's other users
+    uint32_t share_ = 148, calm_ = 0;          // SMs of the plan; runs in a row that could have had more
     uint32_t leastMcs_ = 1;                    // shorter runs go to short_ (SlabWaves)
     bool shortRuns_ = true;
     std::unique_ptr<Batch> short_;             // the same members without slab sweeps, from the first short run on

@@ -183,53 +183,57 @@ def test_short_runs_of_many_large_members_take_the_grid_phase():
 
 
 def test_autotuner_with_short_trials_picks_the_path_of_long_runs():
-    """Trials of two MCS are no measure of what a launch costs however long it runs: 40 systems of 60K monomers,
+    """Trials of two MCS are no measure of what a launch costs however long it runs: 96 systems of 60K monomers,
     whose slab sweeps take longer than the grid phase for two MCS and less for a hundred, are tuned for the sweeps."""
     s = S.serpentine_chains(128, 64, 0.23, seed=5)
-    members = [load(s, seed=300 + i) for i in range(40)]
+    members = [load(s, seed=300 + i) for i in range(96)]
     b = P.Batch(members)
     b.run(3)
     rep = b.autotune(2)
     spent = 3 + rep["mcs_spent"]
     assert rep["cluster"], rep["trials"]
-    tuned = min(b.run_timed(60) for _ in range(2))
+    tuned = min(b.run_timed(40) for _ in range(2))
     b.set_cluster(False)
-    other = min(b.run_timed(60) for _ in range(2))
+    other = min(b.run_timed(40) for _ in range(2))
     assert tuned < other
-    want, ost = O.run(s, spent + 240, seed=339)
-    st = members[39].stats()
-    assert np.array_equal(members[39].get_coords(), want)
+    want, ost = O.run(s, spent + 160, seed=395)
+    st = members[95].stats()
+    assert np.array_equal(members[95].get_coords(), want)
     assert (st["attempted"], st["tentative"], st["accepted"]) == ost
     b.close()
+
+
+def timed_in_threads(runs, times=3):
+    """The least wall time of `times` rounds in which every function of runs is called 8 times on a thread of its own."""
+    import threading
+    import time
+
+    def again(run):
+        for _ in range(8):
+            run()
+
+    best = 1e9
+    for _ in range(times):
+        threads = [threading.Thread(target=again, args=(r,)) for r in runs]
+        t = time.perf_counter()
+        for x in threads:
+            x.start()
+        for x in threads:
+            x.join()
+        best = min(best, time.perf_counter() - t)
+    return best
 
 
 @pytest.mark.parametrize("name,most", [("60K", 2.5), ("131K", 2.8), ("8K", 2.5)])
 def test_threads_share_the_sms(name, most):
     """Eight threads that each run a system of their own again and again: sweeps that take most of the SMs alone run
     side by side on fewer, with the trajectories of each alone, in much less time than one after the other."""
-    import threading
-    import time
     s = {"60K": lambda: S.serpentine_chains(128, 64, 0.23, seed=5), "131K": lambda: S.serpentine_chains(128, 256, 0.5),
          "8K": S.small_chains}[name]()
     us = [load(s, seed=400 + i) for i in range(8)]
-
-    def timed(some):
-        def again(u):
-            for _ in range(8):
-                u.runSimulationOnGPU(100)
-
-        best = 1e9
-        for _ in range(3):
-            threads = [threading.Thread(target=again, args=(u,)) for u in some]
-            t = time.perf_counter()
-            for x in threads:
-                x.start()
-            for x in threads:
-                x.join()
-            best = min(best, time.perf_counter() - t)
-        return best
-
-    one, all8 = timed([load(s, seed=1)]), timed(us)
+    alone = load(s, seed=1)
+    one = timed_in_threads([lambda: alone.runSimulationOnGPU(100)])
+    all8 = timed_in_threads([lambda u=u: u.runSimulationOnGPU(100) for u in us])
     for k in (7, 1):
         for u in us:
             u.run_async(k)
@@ -240,3 +244,27 @@ def test_threads_share_the_sms(name, most):
         us[i].validate()
         v.close()
     assert all8 < most * one, (one, all8)
+
+
+@pytest.mark.parametrize("name,most", [("2x60K", 4.0), ("4x8K", 3.0)])
+def test_batches_in_threads_share_the_sms(name, most):
+    """The same for batches in eight threads, whose plans change with the number of others beside them, and change
+    back when a batch runs alone again."""
+    s, each = (S.serpentine_chains(128, 64, 0.23, seed=5), 2) if name == "2x60K" else (S.small_chains(), 4)
+    members = [[load(s, seed=500 + each * i + k) for k in range(each)] for i in range(8)]
+    batches = [P.Batch(m) for m in members]
+    one = timed_in_threads([lambda: batches[0].run(100)])
+    all8 = timed_in_threads([lambda b=b: b.run(100) for b in batches])
+    again = timed_in_threads([lambda: batches[0].run(100)], times=4)
+    for b in batches:
+        b.run_async(3)
+    for i, total in ((0, 10 * 800 + 3), (3, 3 * 800 + 3), (7, 3 * 800 + 3)):
+        m = members[i][-1]
+        v = load(s, seed=500 + each * i + each - 1, mode=P.MODE_GRAPH)
+        v.runSimulationOnGPU(total)
+        assert m.stats() == v.stats() and np.array_equal(m.get_coords(), v.get_coords())
+        m.validate()
+        v.close()
+    assert all8 < most * one and again < 1.5 * one, (one, all8, again)
+    for b in batches:
+        b.close()
